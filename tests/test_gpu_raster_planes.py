@@ -1,0 +1,109 @@
+"""k_raster's crossing planes against the oracle, byte for byte: crossings
+that share a sample column (one to three of a direction stay in the planes,
+four go to the counters), fills with more edges in a band than the planes are
+tried for, both rules, every anti-aliasing mode, widths around the 32-pixel
+blocks and the 256-pixel tiles, pixel src_over fills (the plain variant),
+other operators and gradients, one surface and several."""
+import numpy as np
+import pytest
+
+from backends import GpuBackend
+from z2d_gb300 import abi, painter
+from z2d_gb300.path import Path
+from z2d_gb300.surface import Surface
+from z2d_gb300.types import Color, FillOptions, Gradient, Pattern, Pixel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    return GpuBackend()
+
+
+def _copies(n, w, h, turn=False):
+    """n equal triangles, the last third of them wound the other way with
+    `turn`: n crossings of a column on every sample row of both sides."""
+    p = Path()
+    a, b, c = (0.3 * w + 0.37, 1.2), (0.81 * w, h - 1.7), (3.6, 0.55 * h)
+    for k in range(n):
+        pts = (a, c, b) if turn and k >= n - n // 3 else (a, b, c)
+        p.move_to(*pts[0])
+        p.line_to(*pts[1])
+        p.line_to(*pts[2])
+        p.close()
+    return p.to_array()
+
+
+def _off_surface():
+    """Nodes that send the call to the full pipeline and draw nothing."""
+    p = Path()
+    p.move_to(-5000, -5000)
+    for k in range(4200):
+        p.line_to(-4000 - (k % 7), -5000 + k * 0.01)
+    p.close()
+    return p.to_array()
+
+
+def _surface(fmt, w, h, seed):
+    s = Surface.init(fmt, w, h)
+    d = np.random.default_rng(seed).integers(0, 256, s.data.size, dtype=np.uint8)
+    if fmt == "rgba":
+        d = d.reshape(-1, 4)
+        d[:, :3] = np.minimum(d[:, :3], d[:, 3:])
+    s.data[:] = d.reshape(-1)
+    return s
+
+
+PIX = Pattern.from_pixel(Pixel.rgba(120, 40, 20, 180))
+
+
+def _both(gpu, oracle, w, h, fmt, pat, nodes, opts, what):
+    ref = _surface(fmt, w, h, 5)
+    assert oracle.fill(ref, pat, nodes, opts) == abi.OK
+    one, many = _surface(fmt, w, h, 5), _surface(fmt, w, h, 5)
+    assert gpu.fill(one, pat, nodes, opts) == abi.OK
+    assert np.array_equal(one.numpy(), ref.numpy()), f"{what}: single call"
+    painter.fill_batch(many, [(pat, nodes, opts), (pat, _off_surface(), opts)], ctx=gpu.ctx)
+    assert np.array_equal(many.numpy(), ref.numpy()), f"{what}: pipeline"
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 9, 84, 85, 86, 127, 128, 129, 200])
+@pytest.mark.parametrize("rule", ["non_zero", "even_odd"])
+@pytest.mark.parametrize("aa", ["default", "supersample_4x", "none"])
+def test_shared_columns(gpu, oracle, n, rule, aa):
+    for turn in (False, True):
+        _both(gpu, oracle, 61, 23, "rgba", PIX, _copies(n, 61, 23, turn), FillOptions(anti_aliasing=aa, fill_rule=rule),
+              f"{n}/{rule}/{aa}/{turn}")
+
+
+@pytest.mark.parametrize("w", [1, 7, 8, 31, 32, 33, 255, 256, 257, 289, 511, 513])
+@pytest.mark.parametrize("fmt", ["rgba", "rgb", "alpha8", "alpha4", "alpha1"])
+def test_widths(gpu, oracle, w, fmt):
+    for n in (2, 4, 90):
+        _both(gpu, oracle, w, 9, fmt, PIX, _copies(n, w, 9, True), FillOptions(), f"{w}/{fmt}/{n}")
+
+
+@pytest.mark.parametrize("op", ["xor", "src_in", "dst_atop", "multiply"])
+def test_general_variant(gpu, oracle, op):
+    g = Gradient.linear(0, 0, 200, 10).add_stop(0.0, Color.rgb(1, 0, 0, 1)).add_stop(1.0, Color.rgb(0, 0, 1, 0.3))
+    for pat in (PIX, Pattern.from_gradient(g)):
+        for n in (1, 3, 4, 100):
+            _both(gpu, oracle, 290, 13, "rgba", pat, _copies(n, 290, 13, True), FillOptions(operator=op), f"{op}/{n}")
+
+
+def test_several_surfaces(gpu, oracle):
+    sizes = [(5, 3), (33, 9), (300, 17), (257, 6), (64, 64), (1, 1), (40, 8), (90, 33), (512, 5)]
+    jobs, refs = [], []
+    for k, (w, h) in enumerate(sizes):
+        fills = [(PIX, _copies(n, w, h, n % 2 == 1), FillOptions(fill_rule=("non_zero", "even_odd")[n % 3 == 0]))
+                 for n in (1, 3, 4, 7, 95)[:1 + k % 5]]
+        ref = _surface("rgba", w, h, k)
+        jobs.append((_surface("rgba", w, h, k).to_device(), fills))
+        for pat, nodes, opts in fills:
+            assert oracle.fill(ref, pat, nodes, opts) == abi.OK
+        refs.append(ref)
+    painter.fill_jobs(jobs, ctx=gpu.ctx)
+    gpu.ctx.synchronize()
+    for (s, _), ref, size in zip(jobs, refs, sizes):
+        assert np.array_equal(s.numpy(), ref.numpy()), size

@@ -58,29 +58,24 @@ __device__ __forceinline__ void add_edge(const FillCmd &F, DEdge *out, double x0
         e.top = ay;
         e.x_start = ax;
         e.x_inc = f64_div_dev(bx - ax, by - ay);
-        e.dir = -1;
         e.rb = round_i32(by);
     } else if (f64_lt(by, ay)) {
         e.top = by;
         e.x_start = bx;
         e.x_inc = f64_div_dev(ax - bx, ay - by);
-        e.dir = 1;
         e.rb = round_i32(ay);
     } else {
         e.top = 0;
         e.x_start = 0;
         e.x_inc = 0;
-        e.fxs = e.fxi = e.ftp = 0.0f;
-        e.dir = 0;
+        e.xi = 0;
+        e.fx = e.fxi = e.fdt = 0.0f;
         e.rt = 1;
         e.rb = 0;  // horizontal: never active
         *out = e;
         return;
     }
-    e.rt = round_i32(e.top);
-    e.fxs = to_f32(e.x_start);
-    e.fxi = to_f32(e.x_inc);
-    e.ftp = to_f32(e.top);
+    if (!edge_fields(e, down)) e.rt = f64_round_i32_hw(e.top);
     const double bot = down ? by : ay;
     const bool lr = f64_lt(ax, bx);
     const double l = lr ? ax : bx, r = lr ? bx : ax;

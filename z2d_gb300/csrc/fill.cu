@@ -43,6 +43,7 @@
 #include "host_pool.h"
 #include "edges.cuh"
 #include "spline.cuh"
+#include "raster.cuh"
 #include "raster_px.cuh"
 #include "stroke_gpu.cuh"
 
@@ -800,7 +801,6 @@ __global__ void k_fill_setup(const FillCmd *__restrict__ fills, FillState *__res
 // Band range of an edge's active sample rows within the fill's draw rows.
 __device__ __forceinline__ bool edge_bands(const DEdge &e, const FillCmd &F, const FillState &S, int32_t &b0,
                                            int32_t &b1) {
-    if (e.dir == 0) return false;
     const int32_t S_ = (int32_t)F.scale;
     const int32_t lo = max(e.rt, S.start_y * S_), hi = min(e.rb, (S.end_y + 1) * S_);
     if (lo >= hi) return false;
@@ -865,11 +865,19 @@ __global__ void k_bin_count(const FillCmd *__restrict__ fills, const FillState *
     });
 }
 
+// The rasteriser reads an edge once per tile column and row of a band: the
+// bin holds what it reads, one coalesced 32-byte record per entry, instead of
+// an index to gather it by.
 __global__ void k_bin_fill(const FillCmd *__restrict__ fills, const FillState *__restrict__ st,
                            const DEdge *__restrict__ edges, const int32_t *__restrict__ edge_fill, int32_t n_edges,
-                           int32_t *__restrict__ fb_cursor, int32_t *__restrict__ bins) {
-    for_edge_bands(fills, st, edges, edge_fill, n_edges,
-                   [&](int32_t edge, int32_t fb) { bins[atomicAdd(&fb_cursor[fb], 1)] = edge; });
+                           int32_t *__restrict__ fb_cursor, BinEdge *__restrict__ bins) {
+    for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t edge, int32_t fb) {
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(edges + edge));
+        const int2 r = __ldg(reinterpret_cast<const int2 *>(&edges[edge].rt));
+        int4 *out = reinterpret_cast<int4 *>(bins + atomicAdd(&fb_cursor[fb], 1));
+        out[0] = a;
+        out[1] = make_int4(r.x, r.y, edge, 0);
+    });
 }
 
 // Edge -> fill map (edges of one fill are contiguous).
@@ -896,16 +904,22 @@ __device__ __forceinline__ int32_t job_of(const DevJob *__restrict__ jobs, int32
 
 // One CTA per global band: the job's fills touching the band, in call order
 // (ordered compaction), with the tile-column range each one can affect and
-// the fill's (fill, band) slot of the band.
+// the fill's (fill, band) slot of the band, and (several surfaces) the
+// records of the band's tiles.
 __global__ void __launch_bounds__(256) k_band_lists(const FillState *__restrict__ st, const DevJob *__restrict__ jobs,
                                                     int32_t n_jobs, int32_t *__restrict__ band_count,
-                                                    int4 *__restrict__ band_fills) {
+                                                    int4 *__restrict__ band_fills, TileRec *__restrict__ tiles) {
     const int32_t gb = blockIdx.x;
     const int32_t j = job_of(jobs, n_jobs, gb, [](const DevJob &J) { return (long long)J.gband_base; });
     const DevJob J = jobs[j];
     const int32_t lb = gb - J.gband_base;
     const int32_t b = J.band_lo + lb;
     const int32_t nf = J.fill1 - J.fill0;
+    if (tiles) {
+        const int32_t nc = J.tcol_hi - J.tcol_lo + 1;
+        for (int32_t t = threadIdx.x; t < nc; t += blockDim.x)
+            tiles[J.tile_base + (long long)lb * nc + t] = TileRec{j, lb, t, 0};
+    }
     __shared__ int32_t warp_tot[8];
     __shared__ int32_t base;
     if (threadIdx.x == 0) base = 0;
@@ -990,7 +1004,7 @@ __global__ void k_exact(const FillCmd *__restrict__ fills, const FillState *__re
     int32_t *bp = xv + S.n_edges;
     int32_t n = 0;
     for (int32_t i = 0; i < S.n_edges; i++)
-        if (E[i].dir != 0) perm[n++] = i;
+        if (E[i].rt < E[i].rb) perm[n++] = i;
     int32_t nbp = 0;
     for (int32_t i = 0; i < n; i++) {
         bp[nbp++] = E[perm[i]].rt;
@@ -1039,10 +1053,10 @@ __global__ void k_exact(const FillCmd *__restrict__ fills, const FillState *__re
                 for (int32_t from = 0; from < n_active; from++) {
                     xv[to] = xv[from];
                     if (wn == 0) {
-                        wn += E[perm[from]].dir;
+                        wn += edge_dir(E[perm[from]]);
                         to++;
                     } else {
-                        wn += E[perm[from]].dir;
+                        wn += edge_dir(E[perm[from]]);
                         if (wn == 0) to++;
                     }
                 }
@@ -1077,396 +1091,6 @@ __global__ void k_exact(const FillCmd *__restrict__ fills, const FillState *__re
     }
 }
 
-// --------------------------------------------------------- compositing
-// The supersample mask value of a pixel whose 4x4 sample block has n covered
-// samples, as 8-bit alpha: the mask is alpha8, or the surface's own format
-// for alpha4/2/1 surfaces (supersample.zig:69-83), each covered sample is
-// opaque, and downsampleBuffer averages the 16 (surface.zig:447-469).
-__device__ __forceinline__ uint32_t ss_mask8(int n, int fmt) {
-    if (fmt >= Z2D_FORMAT_ALPHA4) return scale_alpha(((uint32_t)n * fmt_max(fmt)) / 16u, fmt_bits(fmt), 8);
-    return ((uint32_t)n * 255u) / 16u;
-}
-
-// One pixel of the supersample batch [dst_in(dst = pattern, src = mask), op]
-// (supersample.zig:171-184) as StrideCompositor.runPrecision evaluates it
-// (compositor.zig:540-621): the mask reads as alpha-only lanes.
-static __device__ __noinline__ I16 apply_ssaa(const FillCmd &F, int32_t x, int32_t y, uint32_t m8, I16 d) {
-    if (F.precision == Z2D_PRECISION_INTEGER) {
-        const I16 r = int_op(Z2D_OP_DST_IN, src_i16_fast(F.src, x, y, 0), I16{0, 0, 0, m8});
-        return int_op_any(F.op, d, r);
-    }
-    const F4 r = float_op(Z2D_OP_DST_IN, src_f4_fast(F.src, x, y, 0), decode_raw(I16{0, 0, 0, m8}));
-    return encode_raw(float_op_any(F.op, decode_raw(d), r));
-}
-
-// multisample.run's clears for unbounded operators (multisample.zig:96-110),
-// including its quirks: the rows below the draw box are cleared up to the
-// surface WIDTH, and the right-hand clear starts at x = 0.
-__device__ __forceinline__ bool msaa_unbounded_clear(const FillState &S, int32_t x, int32_t y, int32_t sw) {
-    if (y < S.start_y) return true;
-    if (y > S.end_y) return y < sw;
-    return (S.start_x > 0 && x < S.start_x) || (S.end_x < sw && x < sw - S.end_x);
-}
-
-struct RasterArgs {
-    DevJob job0;                // the job of a one-surface batch, by value
-    const DevJob *jobs;
-    const FillCmd *fills;
-    const FillState *st;
-    const DEdge *edges;
-    const int32_t *bins;
-    const int32_t *bin_off;
-    const int32_t *band_count;  // per global band
-    const int4 *band_fills;     // {fill, cull_x0, cull_x1, (fill, band) slot} per band, in call order
-    const RasterFill *rfills;
-    const uint8_t *masks;
-    int32_t n_jobs;
-    unsigned long long *queue;  // work-queue counter, zero at launch
-    unsigned long long n_items; // tiles (CTA items) or tiles x rows (warp items)
-    const int32_t *order;       // tile order of the queue, or null (tile index order)
-    int32_t one_per_tile;       // not persistent: CTA i draws the i-th tile of the queue
-};
-
-// Winding deltas of one warp: up to 4 sample rows x 1024 sample columns,
-// two biased 16-bit counters per word (bias 0x8000; a fill with at most
-// kMaxBandEdges edges in a band can never carry a counter across halves).
-constexpr int kWordsPerSubRow = 512;
-constexpr int kTouchOff = 4 * kWordsPerSubRow;  // then 4 x 32 words: pairs touched per (sample row, lane)
-constexpr int kTotOff = kTouchOff + 4 * 32;     // then 4 x 32 words: winding change per (sample row, lane)
-constexpr int kWarpWords = kTotOff + 4 * 32;
-constexpr uint32_t kBias2 = 0x80008000u;
-
-// Sample column c of a sub-scanline belongs to lane c / per (per = sample
-// columns per lane: 32 with 4x sampling, 8 without); the pair holding it is
-// stored at ((c % per) / 2) * 32 + lane, so a warp reading pair k of every
-// lane touches 32 consecutive words.
-
-// One work item is one pixel row of a tile of 4 rows x 256 pixels: lane l
-// owns the row's pixels [8l, 8l+8).  The warp walks the band's fills in call
-// order, accumulates the winding deltas of its row's 4 (or 1) sample rows
-// from the fill's band edges, prefix-scans them across the warp, turns the
-// inside bits into coverage and composites its 8 pixels, which stay in
-// registers from the first fill to the last.  `words` is the warp's own
-// shared-memory scratch.  MULTI = false draws a one-surface batch from
-// A.job0, whose fields are kernel parameters (warp-uniform values that need
-// no registers); MULTI = true finds the tile's job in the job table.
-template <bool MULTI>
-__device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t tile, const int warp, const int lane,
-                                           uint32_t *words) {
-    // tile -> (job, band, tile column): jobs hold consecutive tile ranges
-    int32_t jb = 0;
-    if constexpr (MULTI) jb = job_of(A.jobs, A.n_jobs, tile, [](const DevJob &J) { return (long long)J.tile_base; });
-    const DevJob &JB = MULTI ? A.jobs[jb] : A.job0;
-    const int32_t local = tile - JB.tile_base, ncols = JB.tcol_hi - JB.tcol_lo + 1;
-    const int32_t lb = local / ncols;
-    const int32_t b = JB.band_lo + lb;
-    const int32_t cnt = A.band_count[JB.gband_base + lb];
-    if (cnt == 0) return;
-    const int32_t x0 = (JB.tcol_lo + local % ncols) * kTileCols, y = b * kTileRows + warp;
-    const int32_t W = JB.sfc.w, H = JB.sfc.h, fmt = JB.sfc.fmt;
-    if (y >= H) return;
-    const int4 *list = A.band_fills + JB.list_base + (long long)lb * (JB.fill1 - JB.fill0);
-    const int32_t px0 = x0 + lane * 8;  // this lane's first pixel
-
-    for (int i = lane; i < kWarpWords; i += 32) words[i] = i < kTouchOff ? kBias2 : 0u;
-    uint32_t raw[8];
-    uint32_t touched = 0;
-    {
-        const DevSurface dst = JB.sfc;
-#pragma unroll
-        for (int q = 0; q < 8; q++) raw[q] = (px0 + q < W) ? load_raw(dst, (size_t)W * y + px0 + q) : 0u;
-    }
-    __syncwarp();
-
-    // The band's fill list is read 32 entries at a time, one per lane; the
-    // fills that overlap this tile are then walked in order from a ballot.
-    for (int32_t k0 = 0; k0 < cnt; k0 += 32) {
-        int4 ent = make_int4(0, 0, 0, 0);
-        const bool valid = k0 + lane < cnt;
-        if (valid) ent = list[k0 + lane];
-        uint32_t hits = __ballot_sync(0xffffffffu, valid && ent.z > x0 && ent.y < x0 + kTileCols);
-        while (hits) {
-            const int src = __ffs(hits) - 1;
-            const int32_t f = __shfl_sync(0xffffffffu, ent.x, src);
-            const int32_t fb = __shfl_sync(0xffffffffu, ent.w, src);
-            hits &= hits - 1;
-            const int4 ra = __ldg(reinterpret_cast<const int4 *>(A.rfills + f));
-            const int4 rb = __ldg(reinterpret_cast<const int4 *>(A.rfills + f) + 1);
-            // the band's edge range, loaded alongside the record rather than
-            // after the tests on it (fb is a valid slot either way)
-            const int32_t e0 = __ldg(A.bin_off + fb), e1 = __ldg(A.bin_off + fb + 1);
-            const int32_t start_x = ra.x, end_x = ra.y, start_y = ra.z, end_y = ra.w;
-            const uint32_t meta = (uint32_t)rb.x;
-            const int32_t aa = (int32_t)((meta >> RF_AA_SHIFT) & 3u);
-            const bool bounded = (meta & RF_BOUNDED) != 0;
-            const bool ssaa = aa == Z2D_AA_SUPERSAMPLE_4X;
-            const bool boxed = bounded || ssaa;  // touches only [start_x, end_x) x [start_y, end_y]
-            if (boxed && (end_x <= x0 || start_x >= x0 + kTileCols)) continue;
-            const bool direct = aa == Z2D_AA_NONE;
-            const bool exact = (meta & RF_EXACT) != 0;
-            const bool in_rows = y >= start_y && y <= end_y;
-            if (!in_rows && boxed) continue;
-            const int32_t sc = direct ? 1 : 4, per = 8 * sc, lg_per = direct ? 3 : 5;
-            // coverage of pixel q (0..16) is byte q / 2 of cov_ev (q even)
-            // or cov_od (q odd)
-            uint32_t cov_ev = 0, cov_od = 0;
-            if (!exact && in_rows && !(meta & RF_SS_ZERO)) {
-                const int32_t sub0 = y * sc, col0 = x0 * sc, ncol = kTileCols * sc;
-                // sample rows stay below 2^22, where sr + 0.5 is exact in f32
-                const bool f32_ok = sub0 < (1 << 22);
-                const float fsub = (float)sub0 + 0.5f;
-                // one edge per lane; crossings at or left of the tile's
-                // first sample column all land on column 0, so they are
-                // summed across the warp and added once (instead of one
-                // atomic per edge on the same word)
-                for (int32_t base = e0; base < e1; base += 32) {
-                    const int32_t ei = base + lane;
-                    int32_t id = 0, dir = 0, lo = 0, hi = 0;
-                    float4 ef = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (ei < e1) {
-                        id = A.bins[ei];
-                        ef = __ldg(reinterpret_cast<const float4 *>(A.edges + id));
-                        const int2 er = __ldg(reinterpret_cast<const int2 *>(&A.edges[id].rt));
-                        dir = __float_as_int(ef.w);
-                        lo = max(er.x, sub0);
-                        hi = min(er.y, sub0 + sc);
-                    }
-                    for (int r = 0; r < sc; r++) {  // uniform across the warp
-                        const int32_t sr = sub0 + r;
-                        int32_t left = 0;
-                        if (sr >= lo && sr < hi) {
-                            int32_t X;
-                            if (!(f32_ok && crossing_f32(ef.x, ef.y, ef.z, fsub + (float)r, X))) {
-                                const DEdge &e = A.edges[id];
-                                X = (int32_t)round(e.x_start + (e.x_inc * (((double)sr + 0.5) - e.top)));
-                            }
-                            const int32_t c = X - col0;
-                            if (c <= 0) {
-                                left = dir;
-                            } else if (c < ncol) {
-                                // per is 8 or 32 and c > 0: shifts and masks
-                                const int lane_c = c >> lg_per, pair = (c & (per - 1)) >> 1;
-                                const uint32_t inc = (c & 1) ? ((uint32_t)dir << 16) : (uint32_t)dir;
-                                atomicAdd(&words[r * kWordsPerSubRow + ((pair << 5) | lane_c)], inc);
-                                atomicOr(&words[kTouchOff + r * 32 + lane_c], 1u << pair);
-                                atomicAdd(&words[kTotOff + r * 32 + lane_c], (uint32_t)dir);
-                            }
-                        }
-                        // column 0 is the low half of lane 0's pair 0; a net
-                        // zero changes no winding and needs no visit
-                        const int32_t sum = __reduce_add_sync(0xffffffffu, left);
-                        if (lane == 0 && sum != 0) {
-                            atomicAdd(&words[r * kWordsPerSubRow], (uint32_t)sum);
-                            atomicOr(&words[kTouchOff + r * 32], 1u);
-                            atomicAdd(&words[kTotOff + r * 32], (uint32_t)sum);
-                        }
-                    }
-                }
-                __syncwarp();
-                // no crossing in or left of the tile on any sample row: the
-                // winding is 0 across the tile, nothing is covered
-                uint32_t any_touch = 0;
-#pragma unroll
-                for (int s = 0; s < 4; s++)
-                    if (s < sc) any_touch |= words[kTouchOff + s * 32 + lane];
-                if (!__any_sync(0xffffffffu, any_touch != 0)) {
-                    if (bounded) continue;  // zero coverage draws nothing
-                    goto composite;         // unbounded operators still clear
-                }
-                {
-                const bool eo = (meta & RF_EVEN_ODD) != 0;
-                // each lane's winding change per sample row, then the
-                // winding at the lane's first column: the exclusive scans of
-                // rows (0, 1) and (2, 3) run packed as lo + 65536 hi (every
-                // partial sum is bounded by the band's edge count, at most
-                // kMaxBandEdges < 2^15 in magnitude, so the halves stay apart)
-                // (the crossings also summed each lane's winding change)
-                int32_t tot[4] = {0, 0, 0, 0};
-#pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    if (s >= sc) break;
-                    tot[s] = (int32_t)words[kTotOff + s * 32 + lane];
-                    words[kTotOff + s * 32 + lane] = 0u;
-                }
-                const int32_t t01 = tot[0] + tot[1] * 65536, t23 = tot[2] + tot[3] * 65536;
-                int32_t i01 = t01, i23 = t23;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int32_t u01 = __shfl_up_sync(0xffffffffu, i01, o);
-                    const int32_t u23 = __shfl_up_sync(0xffffffffu, i23, o);
-                    if (lane >= o) {
-                        i01 += u01;
-                        i23 += u23;
-                    }
-                }
-                const int32_t x01 = i01 - t01, x23 = i23 - t23;
-                int32_t wrow[4];
-                wrow[0] = (int32_t)(int16_t)(x01 & 0xFFFF);
-                wrow[1] = (x01 - wrow[0]) >> 16;
-                wrow[2] = (int32_t)(int16_t)(x23 & 0xFFFF);
-                wrow[3] = (x23 - wrow[2]) >> 16;
-#pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    if (s >= sc) break;
-                    uint32_t *row = words + s * kWordsPerSubRow;
-                    uint32_t *touch = words + kTouchOff + s * 32 + lane;
-                    const uint32_t touched = *touch;  // pairs of this lane that received crossings
-                    int32_t wnd = wrow[s];
-                    // Between touched pairs the winding is constant, so inside
-                    // bits are filled a range at a time.
-                    bool in = eo ? ((wnd & 1) != 0) : (wnd != 0);
-                    uint32_t bits = 0;
-                    int pos = 0;
-                    for (uint32_t m = touched; m; m &= m - 1) {
-                        const int kk = __ffs(m) - 1, s0 = 2 * kk;
-                        const int idx = (kk << 5) | lane;
-                        const uint32_t v = row[idx];
-                        row[idx] = kBias2;
-                        if (in) bits |= ((1u << s0) - 1u) & ~((1u << pos) - 1u);
-                        wnd += (int32_t)(v & 0xFFFFu) - 0x8000;
-                        in = eo ? ((wnd & 1) != 0) : (wnd != 0);
-                        bits |= (uint32_t)in << s0;
-                        wnd += (int32_t)(v >> 16) - 0x8000;
-                        in = eo ? ((wnd & 1) != 0) : (wnd != 0);
-                        bits |= (uint32_t)in << (s0 + 1);
-                        pos = s0 + 2;
-                    }
-                    if (in && pos < 32) bits |= ~((1u << pos) - 1u);
-                    *touch = 0u;
-                    if (direct) {  // one sample row: bit q is pixel q's sample
-#pragma unroll
-                        for (int q = 0; q < 8; q += 2) {
-                            cov_ev |= ((bits >> q) & 1u) << (4 * q);
-                            cov_od |= ((bits >> (q + 1)) & 1u) << (4 * q);
-                        }
-                    } else {  // nibble q holds pixel q's 4 samples of this row
-                        uint32_t n = bits - ((bits >> 1) & 0x55555555u);
-                        n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
-                        cov_ev += n & 0x0F0F0F0Fu;
-                        cov_od += (n >> 4) & 0x0F0F0F0Fu;
-                    }
-                }
-                __syncwarp();
-                }
-            }
-        composite:
-            if (((meta >> RF_FAST_SHIFT) & 3u) == FAST_PIXEL_SRC_OVER && !exact && bounded) {
-                // Pixel source, integer src_over: the compositeOpaque /
-                // compositeOpacity paths reduce to src_over(d, pixel) at full
-                // coverage and src_over(d, dst_in(pixel, opacity)) otherwise.
-                // The supersample batch [dst_in(pixel, mask), src_over] is the
-                // same with the downsampled mask value as opacity; at zero
-                // coverage both leave the pixel as it is.
-                // (A bounded fill outside its rows was skipped above.)
-                const uint32_t pw = (uint32_t)rb.y;
-                const I16 px{pw & 0xFFu, (pw >> 8) & 0xFFu, (pw >> 16) & 0xFFu, pw >> 24};
-                const int full = direct ? 1 : 16;
-                const int32_t xlo = start_x, xhi = direct ? W : min(end_x, W);
-                if (fmt <= Z2D_FORMAT_RGBA) {
-                    // Lane k holds the source word for coverage k: the pixel
-                    // at k = full, dst_in(pixel, opacity(k)) below it.
-                    I16 s = px;
-                    if (lane < full) {
-                        const uint32_t op8 = ssaa ? ss_mask8(lane, fmt) : (uint32_t)max(lane * 16 - 1, 0);
-                        s = I16{(px.r * op8) / 255u, (px.g * op8) / 255u, (px.b * op8) / 255u, (px.a * op8) / 255u};
-                    }
-                    const uint32_t lut_w = i16_to_word(s, word_order(fmt));
-                    const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const int c = (int)((((q & 1) ? cov_od : cov_ev) >> (8 * (q >> 1))) & 0xFFu);
-                        const uint32_t L = __shfl_sync(0xffffffffu, lut_w, c);
-                        const int32_t x = px0 + q;
-                        // without a branch: the lanes of a warp mostly agree
-                        // on composing, and a select costs less than a split
-                        const bool on = c != 0 && x >= xlo && x < xhi;
-                        const uint32_t nv = word_src_over(raw[q], L, has_alpha);
-                        raw[q] = on ? nv : raw[q];
-                        touched |= (uint32_t)on << q;
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int32_t x = px0 + q;
-                    const int c = (int)((((q & 1) ? cov_od : cov_ev) >> (8 * (q >> 1))) & 0xFFu);
-                    if (c == 0 || x < xlo || x >= xhi) continue;
-                    I16 s = px;
-                    if (c < full) {
-                        const uint32_t op8 = ssaa ? ss_mask8(c, fmt) : (uint32_t)(c * 16 - 1);
-                        s = I16{(px.r * op8) / 255u, (px.g * op8) / 255u, (px.b * op8) / 255u, (px.a * op8) / 255u};
-                    }
-                    raw[q] = i16_to_raw(int_op(Z2D_OP_SRC_OVER, raw_to_i16(raw[q], fmt), s), fmt);
-                    touched |= 1u << q;
-                }
-                continue;
-            }
-            const FillState &S = A.st[f];
-            const FillCmd &F = A.fills[f];
-            if (ssaa) {
-                // every pixel of the composite region runs the batch
-                // [dst_in(pattern, mask), op] (supersample.zig:171-184)
-#pragma unroll 1
-                for (int q = 0; q < 8; q++) {
-                    const int32_t x = px0 + q;
-                    if (x >= W || x < S.start_x || x >= S.end_x) continue;
-                    int c = (int)((((q & 1) ? cov_od : cov_ev) >> (8 * (q >> 1))) & 0xFFu);
-                    if (exact && x >= S.mask_x0 && x < S.mask_x0 + S.mask_w)
-                        c = A.masks[S.mask_base + (long long)(y - S.start_y) * S.mask_w + (x - S.mask_x0)] & 0x1F;
-                    uint32_t rq = raw[0];
-#pragma unroll
-                    for (int j = 1; j < 8; j++)
-                        if (q == j) rq = raw[j];
-                    rq = i16_to_raw(apply_ssaa(F, x, y, ss_mask8(c, fmt), raw_to_i16(rq, fmt)), fmt);
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (q == j) raw[j] = rq;
-                    touched |= 1u << q;
-                }
-                continue;
-            }
-#pragma unroll 1
-            for (int q = 0; q < 8; q++) {
-                const int32_t x = px0 + q;
-                if (x >= W) continue;
-                // raw[] is read and written with constant indices only, so it
-                // stays in registers
-                int c = (int)((((q & 1) ? cov_od : cov_ev) >> (8 * (q >> 1))) & 0xFFu);
-                uint32_t rq = raw[0];
-#pragma unroll
-                for (int j = 1; j < 8; j++)
-                    if (q == j) rq = raw[j];
-                bool clear = false;
-                if (exact && in_rows && x >= S.mask_x0 && x < S.mask_x0 + S.mask_w) {
-                    const uint8_t m = A.masks[S.mask_base + (long long)(y - S.start_y) * S.mask_w + (x - S.mask_x0)];
-                    c = m & 0x1F;
-                    if (direct) clear = (m & kMaskClear) != 0;
-                }
-                if (!direct && !bounded) clear = msaa_unbounded_clear(S, x, y, W);
-                const bool in_box = in_rows && (direct ? true : (x >= S.start_x && x < S.end_x));
-                if (!clear && !(in_box && c > 0)) continue;
-                I16 d = clear ? normalize(I16{0, 0, 0, 0}, fmt) : raw_to_i16(rq, fmt);
-                if (in_box && c > 0) d = apply_fill(F, fmt, x, y, c, direct ? 1 : 16, d);
-                rq = i16_to_raw(d, fmt);
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (q == j) raw[j] = rq;
-                touched |= 1u << q;
-            }
-        }
-    }
-    // the surface pointer is read again here rather than kept in registers
-    // through the fill loop
-    DevSurface dst;
-    dst.data = MULTI ? *reinterpret_cast<uint8_t *const volatile *>(&A.jobs[jb].sfc.data) : A.job0.sfc.data;
-    dst.fmt = fmt;
-    dst.w = W;
-    dst.h = 0;  // unused by the stores
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-        if ((touched >> q) & 1u) store_raw(dst, (size_t)W * y + px0 + q, raw[q]);
-}
-
 // Work estimate of each raster tile for the cost-ordered queue: the number
 // of fills in its band's list (every one is visited by the tile's rows).
 __global__ void k_tile_cost(const DevJob *__restrict__ jobs, int32_t n_jobs, const int32_t *__restrict__ band_count,
@@ -1478,51 +1102,6 @@ __global__ void k_tile_cost(const DevJob *__restrict__ jobs, int32_t n_jobs, con
     const int32_t ncols = J.tcol_hi - J.tcol_lo + 1;
     cost[t] = band_count[J.gband_base + (t - J.tile_base) / ncols];
     idx[t] = t;
-}
-
-// Persistent rasteriser: a grid of resident CTAs that take items from a
-// device work queue (one 64-bit counter) until it is empty; tiles are
-// queued job after job, or in the order of A.order when given.
-//  * CTA_ITEMS: an item is a whole tile; the CTA's four warps draw its four
-//    rows and meet at a barrier before the next tile, so the rows share the
-//    band's fill list and edges in the SM's L1.
-//  * otherwise an item is one (tile, row) pair, numbered tile * 4 + row,
-//    taken by a single warp: a warp that finishes a cheap row takes the
-//    next item at once instead of holding its CTA until the slowest warp of
-//    the tile is done.
-template <bool MULTI, bool CTA_ITEMS>
-__global__ void __launch_bounds__(kRasterThreads, 6) k_raster(const RasterArgs A) {
-    extern __shared__ uint32_t smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *words = smem + warp * kWarpWords;
-    if constexpr (CTA_ITEMS) {
-        if (A.one_per_tile) {  // a grid of one CTA per tile, dispatched in queue order
-            const int32_t tile = A.order ? A.order[blockIdx.x] : (int32_t)blockIdx.x;
-            raster_row<MULTI>(A, tile, warp, lane, words);
-            return;
-        }
-        __shared__ unsigned long long next_tile;
-        for (;;) {
-            if (threadIdx.x == 0) next_tile = atomicAdd(A.queue, 1ull);
-            __syncthreads();
-            const unsigned long long t = next_tile;
-            __syncthreads();  // every thread has read it before it is replaced
-            if (t >= A.n_items) break;
-            const int32_t tile = A.order ? A.order[t] : (int32_t)t;
-            raster_row<MULTI>(A, tile, warp, lane, words);
-        }
-    } else {
-        for (;;) {
-            unsigned long long item = 0;
-            if (lane == 0) item = atomicAdd(A.queue, 1ull);
-            item = __shfl_sync(0xffffffffu, item, 0);
-            if (item >= A.n_items) break;
-            const long long t = (long long)(item / kTileRows);
-            const int32_t tile = A.order ? A.order[t] : (int32_t)t;
-            __syncwarp();  // the previous item's reads of `words` are done before it is reset
-            raster_row<MULTI>(A, tile, (int)(item % kTileRows), lane, words);
-        }
-    }
 }
 
 // The fill owning each node: warp f writes f over fill f's node range (the
@@ -1537,20 +1116,6 @@ __global__ void k_node_owner(const FillCmd *__restrict__ fills, int32_t n_fills,
 
 // ----------------------------------------------------------- host side
 static inline unsigned grid_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
-
-// k_raster's shared-memory attributes: per device, set once on each.
-static int raster_attributes(Ctx &c) {
-    static std::atomic<uint64_t> attr_set{0};
-    const uint64_t dev_bit = 1ull << (c.device & 63);
-    if (attr_set.load(std::memory_order_relaxed) & dev_bit) return Z2D_OK;
-    const size_t smem = sizeof(uint32_t) * kWarpWords * kTileRows;
-    for (auto k : {k_raster<false, false>, k_raster<true, false>, k_raster<false, true>, k_raster<true, true>}) {
-        Z2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        Z2D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    }
-    attr_set.fetch_or(dev_bit, std::memory_order_relaxed);
-    return Z2D_OK;
-}
 
 int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n_nodes, std::vector<FillCmd> &fills,
              const std::vector<DevGradient> &grads,
@@ -1876,22 +1441,25 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         set_error("a fill has more than 32000 edges inside one 4-row band");
         return rb[1];
     }
-    if (c.bins.ensure(sizeof(int32_t) * (size_t)std::max(n_bin_entries, 1))) return Z2D_ERR_OUT_OF_MEMORY;
+    if (c.bins.ensure(sizeof(BinEdge) * (size_t)std::max(n_bin_entries, 1))) return Z2D_ERR_OUT_OF_MEMORY;
     // scatter with the counts array reused as cursors
     Z2D_CUDA(cudaMemcpyAsync(d_fb_cnt, d_fb_off, sizeof(int32_t) * (size_t)(n_fb + 1), cudaMemcpyDeviceToDevice, c.stream));
     tb = c.timer_begin(c.t_bins);
     if (n_edges > 0 && n_bin_entries > 0) {
         k_bin_fill<<<grid_for(n_edges, 256), 256, 0, c.stream>>>(d_fills, d_st, d_edges, d_edge_fill, n_edges, d_fb_cnt,
-                                                                  c.bins.as<int32_t>());
+                                                                  c.bins.as<BinEdge>());
         c.launches++;
     }
 
     // ---- ordered fill lists per global band
     const size_t count_bytes = ((sizeof(int32_t) * (size_t)n_gbands) + 15) & ~(size_t)15;
-    if (c.band_fills.ensure(count_bytes + sizeof(int4) * (size_t)std::max(n_slots, 1ll))) return Z2D_ERR_OUT_OF_MEMORY;
+    const size_t tile_bytes = n_jobs > 1 ? sizeof(TileRec) * (size_t)n_tiles : 0;
+    if (c.band_fills.ensure(count_bytes + tile_bytes + sizeof(int4) * (size_t)std::max(n_slots, 1ll)))
+        return Z2D_ERR_OUT_OF_MEMORY;
     int32_t *d_band_count = c.band_fills.as<int32_t>();
-    int4 *d_band_fills = reinterpret_cast<int4 *>(c.band_fills.as<uint8_t>() + count_bytes);
-    k_band_lists<<<(unsigned)n_gbands, 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, d_band_count, d_band_fills);
+    TileRec *d_tiles = n_jobs > 1 ? reinterpret_cast<TileRec *>(c.band_fills.as<uint8_t>() + count_bytes) : nullptr;
+    int4 *d_band_fills = reinterpret_cast<int4 *>(c.band_fills.as<uint8_t>() + count_bytes + tile_bytes);
+    k_band_lists<<<(unsigned)n_gbands, 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, d_band_count, d_band_fills, d_tiles);
     c.launches++;
 
     // ---- exact path
@@ -1911,32 +1479,27 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     A.fills = d_fills;
     A.st = d_st;
     A.edges = d_edges;
-    A.bins = c.bins.as<int32_t>();
+    A.bins = c.bins.as<BinEdge>();
     A.bin_off = d_fb_off;
     A.band_count = d_band_count;
     A.band_fills = d_band_fills;
     A.rfills = d_rf;
+    A.tiles = d_tiles;
     A.masks = c.masks.as<uint8_t>();
     A.n_jobs = n_jobs;
     A.job0 = jobs[0];
-    const size_t smem = sizeof(uint32_t) * kWarpWords * kTileRows;
-    {
-        const int rc = raster_attributes(c);
-        if (rc) return rc;
-    }
     {
         const int rc = c.await_surface();  // a host surface's upload
         if (rc) return rc;
     }
     // persistent grid: every SM filled to the kernel's residency (or the
     // tuned CTAs per SM), never more CTAs than tiles
-    static std::atomic<int> occ_cache[2];
-    int occ = occ_cache[n_jobs == 1 ? 0 : 1].load(std::memory_order_relaxed);
-    if (occ <= 0) {
-        if (n_jobs == 1) Z2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<false, false>, kRasterThreads, smem));
-        else Z2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<true, false>, kRasterThreads, smem));
-        occ = std::max(occ, 1);
-        occ_cache[n_jobs == 1 ? 0 : 1].store(occ, std::memory_order_relaxed);
+    RasterVariant variant{n_jobs > 1, false, n_exact == 0, false};
+    for (const FillCmd &F : fills) variant.plain &= F.fast_kind == FAST_PIXEL_SRC_OVER;
+    int occ = 1;
+    {
+        const int rc = raster_occupancy(c, variant, occ);
+        if (rc) return rc;
     }
     // the schedule: forced on the context, or the tuner's for this kind of pass
     const TuneKey key = tune_key(n_jobs, n_tiles, n_slots, n_gbands);
@@ -1986,20 +1549,16 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         A.order = order;
     }
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
-    if (plan.cta_items) {
-        if (n_jobs == 1) k_raster<false, true><<<grid, kRasterThreads, smem, c.stream>>>(A);
-        else k_raster<true, true><<<grid, kRasterThreads, smem, c.stream>>>(A);
-    } else {
-        if (n_jobs == 1) k_raster<false, false><<<grid, kRasterThreads, smem, c.stream>>>(A);
-        else k_raster<true, false><<<grid, kRasterThreads, smem, c.stream>>>(A);
+    variant.cta_items = plan.cta_items != 0;
+    {
+        const int rc = raster_launch(c, variant, A, grid);
+        if (rc) return rc;
     }
     c.timer_end(c.t_raster, t0);
     if (plan.candidate >= 0) {
         Z2D_CUDA(cudaEventRecord(tune_t1, c.stream));
         c.tune_pending.push_back(TunePending{key, plan.candidate, tune_t0, tune_t1});
     }
-    c.launches++;
-    Z2D_CUDA(cudaGetLastError());
     return pads.finish(c);
 }
 
@@ -2051,13 +1610,11 @@ struct HostFlatten {
             e.top = ay;
             e.x_start = ax;
             e.x_inc = (bx - ax) / (by - ay);
-            e.dir = -1;
             e.rb = (int32_t)std::round(by);
         } else if (ay > by) {
             e.top = by;
             e.x_start = bx;
             e.x_inc = (ax - bx) / (ay - by);
-            e.dir = 1;
             e.rb = (int32_t)std::round(ay);
         } else {
             e.rt = 1;
@@ -2066,9 +1623,7 @@ struct HostFlatten {
             return;
         }
         e.rt = (int32_t)std::round(e.top);
-        e.fxs = (float)e.x_start;
-        e.fxi = (float)e.x_inc;
-        e.ftp = (float)e.top;
+        e.fdt = ay < by ? -0.0f : 0.0f;  // (k_raster's gathering variants fill the f32 fields in)
         const double bot = ay < by ? by : ay;
         const double l = ax < bx ? ax : bx, r = ax < bx ? bx : ax;
         if (!any) {
@@ -2350,6 +1905,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     }
     // ---- bins: each edge in the bands of its active sample rows (edge_bands)
     static thread_local std::vector<int32_t> cnt, off, bins, bcount;
+    static thread_local std::vector<TileRec> tiles;
     static thread_local std::vector<int4> blist;
     cnt.assign((size_t)n_fb + 1, 0);
     auto for_bands = [&](auto &&visit) {
@@ -2359,7 +1915,6 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
             const int32_t S_ = (int32_t)fills[f].scale;
             for (int32_t k = 0; k < S.n_edges; k++) {
                 const DEdge &e = edges[(size_t)(S.edge_base + k)];
-                if (e.dir == 0) continue;
                 const int32_t lo = std::max(e.rt, S.start_y * S_), hi = std::min(e.rb, (S.end_y + 1) * S_);
                 if (lo >= hi) continue;
                 const int32_t b0 = lo / (kTileRows * S_), b1 = (hi - 1) / (kTileRows * S_);
@@ -2389,11 +1944,15 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     // ---- band lists (k_band_lists): the job's fills touching each band, in order
     bcount.assign(std::max<long long>(n_gbands, 1), 0);
     blist.assign(std::max<long long>(n_slots, 1), make_int4(0, 0, 0, 0));
+    tiles.clear();
     for (const DevJob &jb : J) {
         if (jb.band_hi < jb.band_lo) continue;
         const int32_t nf = jb.fill1 - jb.fill0;
         for (int32_t b = jb.band_lo; b <= jb.band_hi; b++) {
             const int32_t lb = b - jb.band_lo;
+            if (n_jobs > 1)  // (tiles are numbered in this order)
+                for (int32_t t = 0; t <= jb.tcol_hi - jb.tcol_lo; t++)
+                    tiles.push_back(TileRec{(int32_t)(&jb - J.data()), lb, t, 0});
             int4 *out = blist.data() + jb.list_base + (long long)lb * nf;
             int32_t k = 0;
             for (int32_t f = jb.fill0; f < jb.fill1; f++) {
@@ -2414,7 +1973,8 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     const size_t o_cnt = o_off + al(sizeof(int32_t) * ((size_t)n_fb + 1));
     const size_t o_list = o_cnt + al(sizeof(int32_t) * bcount.size());
     const size_t o_grad = o_list + al(sizeof(int4) * blist.size());
-    const size_t total = o_grad + al(sizeof(DevGradient) * std::max<size_t>(grads.size(), 1));
+    const size_t o_tile = o_grad + al(sizeof(DevGradient) * std::max<size_t>(grads.size(), 1));
+    const size_t total = o_tile + al(sizeof(TileRec) * tiles.size());
     const int slot = c.small_slot;
     c.small_slot ^= 1;
     HostBuf &hb = c.small_stage[slot];
@@ -2432,6 +1992,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     memcpy(h + o_rf, rf.data(), sizeof(RasterFill) * n_fills);
     if (!edges.empty()) memcpy(h + o_edges, edges.data(), sizeof(DEdge) * edges.size());
     memcpy(h + o_bins, bins.data(), sizeof(int32_t) * bins.size());
+    if (!tiles.empty()) memcpy(h + o_tile, tiles.data(), sizeof(TileRec) * tiles.size());
     memcpy(h + o_off, off.data(), sizeof(int32_t) * ((size_t)n_fb + 1));
     memcpy(h + o_cnt, bcount.data(), sizeof(int32_t) * bcount.size());
     memcpy(h + o_list, blist.data(), sizeof(int4) * blist.size());
@@ -2446,30 +2007,28 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     A.fills = reinterpret_cast<const FillCmd *>(dv + o_fill);
     A.st = reinterpret_cast<const FillState *>(dv + o_st);
     A.edges = reinterpret_cast<const DEdge *>(dv + o_edges);
-    A.bins = reinterpret_cast<const int32_t *>(dv + o_bins);
+    A.bins = dv + o_bins;
     A.bin_off = reinterpret_cast<const int32_t *>(dv + o_off);
     A.band_count = reinterpret_cast<const int32_t *>(dv + o_cnt);
     A.band_fills = reinterpret_cast<const int4 *>(dv + o_list);
     A.rfills = reinterpret_cast<const RasterFill *>(dv + o_rf);
+    A.tiles = reinterpret_cast<const TileRec *>(dv + o_tile);
     A.masks = nullptr;
     A.n_jobs = (int32_t)n_jobs;
     A.queue = nullptr;
     A.n_items = (unsigned long long)n_tiles;
     A.order = nullptr;
     A.one_per_tile = 1;
-    const int rc = raster_attributes(c);
-    if (rc) return rc;
     {
         const int rs = c.await_surface();
         if (rs) return rs;
     }
-    const size_t smem = sizeof(uint32_t) * kWarpWords * kTileRows;
+    RasterVariant variant{n_jobs > 1, true, true, true};
+    for (const FillCmd &F : fills) variant.plain &= F.fast_kind == FAST_PIXEL_SRC_OVER;
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
-    if (n_jobs == 1) k_raster<false, true><<<(unsigned)n_tiles, kRasterThreads, smem, c.stream>>>(A);
-    else k_raster<true, true><<<(unsigned)n_tiles, kRasterThreads, smem, c.stream>>>(A);
+    const int rc = raster_launch(c, variant, A, (unsigned)n_tiles);
+    if (rc) return rc;
     c.timer_end(c.t_raster, t0);
-    c.launches++;
-    Z2D_CUDA(cudaGetLastError());
     return Z2D_OK;
 }
 

@@ -1,6 +1,8 @@
 // fill.cuh -- device structures of the fill pipeline (fill.cu).
 #pragma once
+#include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "z2d_internal.h"
 
@@ -47,42 +49,113 @@ struct NodeInfo {
 };
 
 // Polygon.Edge plus its rounded active range: the edge is active on sample
-// row y exactly when rt <= y < rb (top < y+0.5 <= bottom, Polygon.zig:284-285).
-// fxs/fxi/ftp are x_start/x_inc/top rounded to f32 for crossing_f32; the
-// first 16 bytes load as one vector.
+// row y exactly when rt <= y < rb (top < y+0.5 <= bottom, Polygon.zig:284-285;
+// a horizontal edge has rt = 1, rb = 0 and is never active).  The first 16
+// bytes hold what crossing_f32 needs, as one vector: x_start split
+// into a whole part xi and a rest fx, the slope, and fdt = rt + 0.5 - top,
+// whose sign bit is the direction (set: -1 down, clear: +1 up).
 struct DEdge {
-    float fxs, fxi, ftp;
-    int32_t dir;  // -1 down, +1 up, 0 horizontal (dropped)
+    int32_t xi;
+    float fx, fxi, fdt;
     int32_t rt, rb;
     double x_start, x_inc, top;
 };
 
 static_assert(sizeof(DEdge) == 48, "DEdge layout: 16-byte f32 block, ranges, f64 fields");
 
+Z2D_HD float f32_of_bits(uint32_t b) {
+    float f;
+    memcpy(&f, &b, 4);
+    return f;
+}
+
+// |v| as 32.32 fixed point (truncated), from the bits of v: no f64
+// instruction.  False for |v| >= 2^26 and for what is not finite.
+Z2D_HD bool fixed_coord(double v, uint32_t &whole, uint32_t &frac, bool &neg) {
+    uint64_t b;
+    memcpy(&b, &v, 8);
+    const int32_t sh = 31 + 1023 - (int32_t)((b >> 52) & 0x7FFu);  // 31 - exponent
+    neg = (b >> 63) != 0;
+    const uint64_t q = ((b << 11) | (1ull << 63)) >> (sh < 0 ? 0 : sh > 63 ? 63 : sh);
+    whole = (uint32_t)(q >> 32);
+    frac = (uint32_t)q;
+    return sh >= 6;
+}
+// A 32-bit fraction as an f32 in [0, 1), truncated to 23 bits.
+Z2D_HD float frac_f32(uint32_t f) { return f32_of_bits(0x3F800000u | (f >> 9)) - 1.0f; }
+
+// The f32 fields and rt of an edge whose x_start, x_inc and top are set.
+// rt is round(top), half away from zero.  Every field is truncated, not
+// rounded: fx is within 2^-23 of x_start - xi, fdt within 2^-23 of
+// rt + 0.5 - top (in [0, 1]), fxi within 2^-23 of x_inc relatively.  What
+// does not fit (coordinates of 2^26 and more, slopes outside f32's normal
+// range) leaves a NaN in fx: every crossing of the edge is then evaluated
+// in f64.  False when top does not fit: rt is then the caller's to set.
+Z2D_HD bool edge_fields(DEdge &e, bool down) {
+    uint32_t w, f;
+    bool neg;
+    bool ok = fixed_coord(e.x_start, w, f, neg);
+    const float fx = frac_f32(f);
+    e.xi = neg ? -(int32_t)w : (int32_t)w;
+    e.fx = neg ? -fx : fx;
+    uint64_t b;
+    memcpy(&b, &e.x_inc, 8);
+    const int32_t se = (int32_t)((b >> 52) & 0x7FFu) - 1023 + 127;
+    const bool zero = (b << 1) == 0;
+    ok &= zero || (se > 0 && se < 255);
+    e.fxi = zero ? 0.0f
+                 : f32_of_bits(((uint32_t)(b >> 32) & 0x80000000u) | ((uint32_t)se << 23) |
+                               ((uint32_t)(b >> 29) & 0x7FFFFFu));
+    const bool top_ok = fixed_coord(e.top, w, f, neg);
+    // away from zero by one where the fraction is 1/2 or more
+    const uint32_t up = f >> 31;
+    const float r = frac_f32(f), m = (float)up;
+    const float d = neg ? (0.5f - m) + r : (0.5f + m) - r;
+    e.rt = neg ? -(int32_t)(w + up) : (int32_t)(w + up);
+    e.fdt = down ? -d : d;
+    if (!(ok && top_ok)) e.fx = f32_of_bits(0x7FC00000u);
+    return top_ok;
+}
+
+// The direction of a (not horizontal) edge.
+Z2D_HD int32_t edge_dir(const DEdge &e) {
+    uint32_t b;
+    memcpy(&b, &e.fdt, 4);
+    return (b >> 31) ? -1 : 1;
+}
+
 // The crossing of an edge with sample row sr is
 //   X = round(x_start + x_inc * ((sr + 0.5) - top))      (Polygon.zig:272-276)
-// in f64, rounded half away from zero.  crossing_f32 evaluates the same
-// expression in f32 from the f32-rounded inputs (s = sr + 0.5, exact) and
-// bounds its distance from the f64 value.  With u = 2^-24 and every f32
-// operation correctly rounded, to first order
-//   |fv - v| <= u * (|fv| + |fxs| + |fp| + |fxi| * (|ftp| + 2|ft|))
-// (input roundings of x_start, x_inc and top, then one rounding per
-// operation); the f64 evaluation's own error is ~2^-29 of that.  The bound
-// used is 1.25x the first-order one.  When fv is farther than the bound
-// from the nearest half-integer, the f64 value lies on the same side of it
-// and rounds to the same integer; otherwise the caller evaluates in f64.
-// Returns false when the f32 result does not decide X.
-Z2D_HD bool crossing_f32(float fxs, float fxi, float ftp, float s, int32_t &X) {
-    const float ft = s - ftp;
-    const float fp = fxi * ft;
-    const float fv = fxs + fp;
-    const float bound =
-        (fabsf(fv) + fabsf(fxs) + fabsf(fp) + fabsf(fxi) * (fabsf(ftp) + 2.0f * fabsf(ft))) * 7.450580596923828e-8f;
-    const float fl = floorf(fv);
-    const float h = fl + 0.5f;
-    if (!(fabsf(fv - h) > bound) || !(fabsf(fv) < 4194304.0f)) return false;  // NaN/inf fail here too
-    X = (int32_t)fl + (fv > h ? 1 : 0);
-    return true;
+// in f64, rounded half away from zero.  With the edge's split fields,
+// X = xi + round(fx + fxi * t), t = (sr - rt) + fdt >= 0: the f32 value
+// carries the distance along the edge only, not the coordinates.  With
+// u = 2^-24, T the largest t asked of the edge and p = |fxi| T, to first
+// order its error is at most
+//   u (2 p (slope) + 3 p (t: two sums and the conversion)
+//      + 3 |fxi| (fdt) + 2 (fx) + (1 + p) (the fused multiply-add's rounding))
+// and the f64 evaluation's own error is below u / 4 for |x_start| < 2^26 (a
+// larger one has fx = NaN), p < 2^21.  The bound used is 1.25 times
+// u (7 p + 3 |fxi| + 5).  A value farther than the bound from every
+// half-integer rounds as the f64 value does; the others, and those
+// whose bound is 1/2 or more (so p stays below 2^21 where rounding by adding
+// 1.5 * 2^23 is exact), have to be evaluated in f64.
+constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr int32_t kRoundMagicBits = 0x4B400000;
+// The largest distance from the rounded value that decides it.
+Z2D_HD float crossing_limit(float fxi, float t_max) {
+    const float s = fabsf(fxi), p = s * t_max;
+    return 0.5f - 7.450580596923828e-8f * (7.0f * p + 3.0f * s + 5.0f);
+}
+// round(fx + fxi * t) + kRoundMagicBits; false when f32 does not decide it.
+Z2D_HD bool crossing_f32(float fx, float fxi, float t, float limit, int32_t &n) {
+#ifdef __CUDA_ARCH__
+    const float v = __fmaf_rn(fxi, t, fx);
+#else
+    const float v = fmaf(fxi, t, fx);
+#endif
+    const float m = v + kRoundMagic;
+    memcpy(&n, &m, 4);
+    return fabsf(v - (m - kRoundMagic)) <= limit;  // NaN fails
 }
 
 enum : int32_t {
@@ -126,6 +199,7 @@ enum : uint32_t {
     RF_EXACT = 1u << 10,      // FILL_EXACT
     RF_SS_ZERO = 1u << 11,    // FILL_SS_ZERO
     RF_BOUNDED = 1u << 12,    // the operator is bounded
+    RF_IN_ROWS = 1u << 31,    // set by k_raster: the row is one of the draw box
 };
 
 // counters (int32 slots; the mask byte count is a 64-bit pair)

@@ -1,0 +1,699 @@
+// raster.cu -- the tile rasteriser: coverage of the binned edges of a batch's
+// fills, composited in call order (WorkingEdgeSet, multisample.run,
+// raster/shared.zig, Surface.paintStride/compositeStride).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "raster.cuh"
+#include "raster_px.cuh"
+#include "z2d_internal.h"
+
+namespace z2dg {
+
+// --------------------------------------------------------- compositing
+// The supersample mask value of a pixel whose 4x4 sample block has n covered
+// samples, as 8-bit alpha: the mask is alpha8, or the surface's own format
+// for alpha4/2/1 surfaces (supersample.zig:69-83), each covered sample is
+// opaque, and downsampleBuffer averages the 16 (surface.zig:447-469).
+__device__ __forceinline__ uint32_t ss_mask8(int n, int fmt) {
+    if (fmt >= Z2D_FORMAT_ALPHA4) return scale_alpha(((uint32_t)n * fmt_max(fmt)) / 16u, fmt_bits(fmt), 8);
+    return ((uint32_t)n * 255u) / 16u;
+}
+
+// One pixel of the supersample batch [dst_in(dst = pattern, src = mask), op]
+// (supersample.zig:171-184) as StrideCompositor.runPrecision evaluates it
+// (compositor.zig:540-621): the mask reads as alpha-only lanes.
+static __device__ __noinline__ I16 apply_ssaa(const FillCmd &F, int32_t x, int32_t y, uint32_t m8, I16 d) {
+    if (F.precision == Z2D_PRECISION_INTEGER) {
+        const I16 r = int_op(Z2D_OP_DST_IN, src_i16_fast(F.src, x, y, 0), I16{0, 0, 0, m8});
+        return int_op_any(F.op, d, r);
+    }
+    const F4 r = float_op(Z2D_OP_DST_IN, src_f4_fast(F.src, x, y, 0), decode_raw(I16{0, 0, 0, m8}));
+    return encode_raw(float_op_any(F.op, decode_raw(d), r));
+}
+
+// multisample.run's clears for unbounded operators (multisample.zig:96-110),
+// including its quirks: the rows below the draw box are cleared up to the
+// surface WIDTH, and the right-hand clear starts at x = 0.
+__device__ __forceinline__ bool msaa_unbounded_clear(const FillState &S, int32_t x, int32_t y, int32_t sw) {
+    if (y < S.start_y) return true;
+    if (y > S.end_y) return y < sw;
+    return (S.start_x > 0 && x < S.start_x) || (S.end_x < sw && x < sw - S.end_x);
+}
+
+// Crossings of one warp's pixel row: up to 4 sample rows of 1024 sample
+// columns, one 32-bit word of columns per lane.  Sample column c belongs to
+// lane c / per (per = sample columns per lane: 32 with 4x sampling, 8
+// without) and is bit c % per of the lane's word.
+//   even-odd: one plane per sample row; a crossing toggles its bit.
+//   non-zero: planes U0 D0 U1 D1 U2 D2 per sample row; the first upward
+//     crossing of a column sets its bit of U0, the second one that of U1, the
+//     third one that of U2 (D for downward).  A fourth crossing of one
+//     column, row and direction sends the (fill, row) to winding_bits.
+// Against 16-bit counters per column this is one atomic per crossing instead
+// of three, and the even-odd rule needs no walk over the crossings at all:
+// the inside bits are the prefix XOR of the toggles.  Issue bound: a fill
+// costs a row and tile of the 2,000-path 4096x4096 batch (2.9 M of them, 28
+// edges each on average) about 600 warp instructions instead of 1,250, and
+// the kernel takes 2.45 ms instead of 4.30.
+constexpr int kPlanes = 6;
+constexpr int kSubWords = kPlanes * 32;         // one sample row
+constexpr int kDenseWords = 2 * 16 * 32 + 2 * 32;  // or winding_bits' counters
+constexpr int kCovOff = kDenseWords > 4 * kSubWords ? kDenseWords : 4 * kSubWords;  // then 256 coverage bytes
+constexpr int kWarpWords = kCovOff + kTileCols / 4;
+
+// An edge as a pixel row's sample rows see it (crossing_f32).
+struct RowEdge {
+    float fx, fxi, t0, rt_rest, lim;  // t = (t0 + r) + rt_rest
+    int32_t c0;        // xi - (tile's first sample column) - the bits of 1.5 * 2^23
+    int32_t id;
+    uint32_t rows;     // sample rows on which the edge is active
+    bool down;
+};
+template <bool GATHER>
+__device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const DEdge *__restrict__ edges,
+                                            int32_t bin, bool valid, int32_t sub0, int32_t sc, int32_t col0) {
+    RowEdge R{};
+    if (!valid) return R;
+    int4 f, er;
+    if constexpr (GATHER) {
+        R.id = __ldg(reinterpret_cast<const int32_t *>(bins) + bin);
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(edges + R.id));
+        const int4 b = __ldg(reinterpret_cast<const int4 *>(edges + R.id) + 1);
+        const int4 c = __ldg(reinterpret_cast<const int4 *>(edges + R.id) + 2);
+        DEdge e;
+        e.x_start = __hiloint2double(b.w, b.z);
+        e.x_inc = __hiloint2double(c.y, c.x);
+        e.top = __hiloint2double(c.w, c.z);
+        edge_fields(e, a.w < 0);
+        f = make_int4(e.xi, __float_as_int(e.fx), __float_as_int(e.fxi), __float_as_int(e.fdt));
+        er = make_int4(b.x, b.y, R.id, 0);
+    } else {
+        f = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin);
+        er = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin + 1);
+        R.id = er.z;
+    }
+    const int32_t lo = max(er.x - sub0, 0), hi = min(er.y - sub0, sc);
+    if (lo < hi) R.rows = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+    R.fx = __int_as_float(f.y);
+    R.fxi = __int_as_float(f.z);
+    R.rt_rest = fabsf(__int_as_float(f.w));
+    R.down = f.w < 0;
+    const int32_t rel = sub0 - er.x;
+    R.t0 = (float)rel;
+    R.lim = crossing_limit(R.fxi, (float)(rel + hi));
+    R.c0 = f.x - col0 - kRoundMagicBits;
+    return R;
+}
+
+// Sample column, relative to the tile's first, where edge R crosses sample
+// row sub0 + r (r one of R.rows).
+__device__ __forceinline__ int32_t edge_crossing(const DEdge *__restrict__ edges, const RowEdge &R, int32_t r,
+                                                 int32_t sub0, int32_t col0) {
+    const float t = (R.t0 + (float)r) + R.rt_rest;
+    int32_t n;
+    if (crossing_f32(R.fx, R.fxi, t, R.lim, n)) return n + R.c0;
+    const DEdge &e = edges[R.id];
+    return (int32_t)round(e.x_start + (e.x_inc * (((double)(sub0 + r) + 0.5) - e.top))) - col0;
+}
+
+// Inside bits of the lane's columns on the row's sample rows by the non-zero
+// rule, for any number of crossings per column: two sample rows at a time,
+// with biased 16-bit counters per column (two a word; at most
+// kMaxBandEdges < 2^15 crossings, so no half carries) in `words`, which is
+// clear before and after.  For rows where four crossings of one direction
+// share a sample column, and without trying the planes first for
+// kDenseEdges edges and more: of 320 surfaces with fills and strokes, 12 % of
+// the non-zero rows with 128-256 edges in their band run over the planes,
+// 56 % of those with 256-512 and 90 % of those with more (strokes drawn over
+// themselves, paths much smaller than their detail).  Out of line, for the
+// registers of the common path.
+constexpr int32_t kDenseEdges = 256;
+template <bool GATHER>
+static __device__ __noinline__ uint4 winding_bits(const void *bins, const DEdge *edges, int32_t e0, int32_t ne,
+                                                  int32_t sub0, int32_t sc, int32_t col0, uint32_t *words, int lane) {
+    constexpr uint32_t kBias2 = 0x80008000u;
+    constexpr int kRow = 16 * 32;              // a sample row's counters
+    uint32_t *touch = words + 2 * kRow;        // column pairs touched, per sample row and lane
+    const int32_t lg_per = sc == 1 ? 3 : 5, per = 1 << lg_per;
+    uint32_t out[4] = {0u, 0u, 0u, 0u};
+    __syncwarp();
+    for (int i = lane; i < 2 * kRow; i += 32) words[i] = kBias2;
+    __syncwarp();
+#pragma unroll
+    for (int s0 = 0; s0 < 4; s0 += 2) {
+        if (s0 >= sc) break;
+        int32_t left = 0;  // rows s0 and s0 + 1 as lo + 65536 hi
+        for (int32_t base = 0; base < ne; base += 32) {
+            const RowEdge R = row_edge<GATHER>(bins, edges, e0 + base + lane, base + lane < ne, sub0, sc, col0);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (!((R.rows >> (s0 + h)) & 1u)) continue;
+                const int32_t c = edge_crossing(edges, R, s0 + h, sub0, col0);
+                if (c <= 0) {
+                    left += R.down ? (h ? -65536 : -1) : (h ? 65536 : 1);
+                } else if (c < 32 * per) {
+                    // a lane's pairs of columns lie 32 words apart: every
+                    // lane reads its own bank
+                    const int32_t pair = (c & (per - 1)) >> 1, own = c >> lg_per;
+                    const uint32_t d = R.down ? 0xFFFFFFFFu : 1u;
+                    atomicAdd(&words[h * kRow + ((pair << 5) | own)], (c & 1) ? d << 16 : d);
+                    atomicOr(&touch[h * 32 + own], 1u << pair);
+                }
+            }
+        }
+        left = __reduce_add_sync(0xffffffffu, left);
+        __syncwarp();
+        int32_t tot[2];
+        uint32_t pairs[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            pairs[h] = touch[h * 32 + lane];
+            touch[h * 32 + lane] = 0u;
+            tot[h] = 0;
+            for (uint32_t m = pairs[h]; m; m &= m - 1) {
+                const uint32_t v = words[h * kRow + (__ffs(m) - 1) * 32 + lane];
+                tot[h] += (int32_t)(v & 0xFFFFu) + (int32_t)(v >> 16) - 0x10000;
+            }
+        }
+        const int32_t t = tot[0] + tot[1] * 65536;
+        int32_t incl = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        incl += left - t;
+        const int32_t lo = (int32_t)(int16_t)(incl & 0xFFFF);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            int32_t wnd = h ? (incl - lo) >> 16 : lo;
+            uint32_t bits = wnd != 0 ? 0xFFFFFFFFu : 0u;
+            for (uint32_t m = pairs[h]; m; m &= m - 1) {
+                const int k = __ffs(m) - 1;
+                uint32_t *w = words + h * kRow + k * 32 + lane;
+                const uint32_t v = *w;
+                *w = kBias2;
+                bool was = wnd != 0;
+                wnd += (int32_t)(v & 0xFFFFu) - 0x8000;
+                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << (2 * k);
+                was = wnd != 0;
+                wnd += (int32_t)(v >> 16) - 0x8000;
+                if ((wnd != 0) != was) bits ^= 0xFFFFFFFEu << (2 * k);
+            }
+            out[s0 + h] = bits;
+        }
+        __syncwarp();
+    }
+    for (int i = lane; i < 2 * kRow; i += 32) words[i] = 0u;
+    __syncwarp();
+    return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+// One work item is one pixel row of a tile of 4 rows x 256 pixels.  The warp
+// walks the band's fills in call order: the fill's crossings with the row's
+// 4 (or 1) sample rows go to the planes, where lane l owns the 32 (or 8)
+// sample columns of pixels [8l, 8l+8); it turns them into inside bits and
+// coverage, which pass through shared memory to the lanes that composite:
+// lane l holds pixels l, l + 32, ..., l + 224 of the row in registers from
+// the first fill to the last.  A block of 32 consecutive pixels that the fill
+// leaves uncovered is skipped by the whole warp, and loads and stores are
+// coalesced.  `words` is the warp's own shared-memory scratch.
+// MULTI = false draws a one-surface batch from A.job0, whose fields are
+// kernel parameters (warp-uniform values that need no registers);
+// MULTI = true finds the tile's job in the job table.
+template <bool MULTI, bool PLAIN, bool GATHER>
+__device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t tile, const int warp, const int lane,
+                                           uint32_t *words) {
+    // tile -> (job, band, tile column)
+    int32_t jb = 0, lb, col;
+    if constexpr (MULTI) {
+        const int4 t = __ldg(reinterpret_cast<const int4 *>(A.tiles + tile));
+        jb = t.x;
+        lb = t.y;
+        col = t.z;
+    } else {
+        const int32_t ncols = A.job0.tcol_hi - A.job0.tcol_lo + 1;
+        lb = tile / ncols;
+        col = tile - lb * ncols;
+    }
+    const DevJob &JB = MULTI ? A.jobs[jb] : A.job0;
+    const int32_t b = JB.band_lo + lb;
+    const int32_t cnt = A.band_count[JB.gband_base + lb];
+    if (cnt == 0) return;
+    const int32_t x0 = (JB.tcol_lo + col) * kTileCols, y = b * kTileRows + warp;
+    const int32_t W = JB.sfc.w, H = JB.sfc.h, fmt = JB.sfc.fmt;
+    if (y >= H) return;
+    const int4 *list = A.band_fills + JB.list_base + (long long)lb * (JB.fill1 - JB.fill0);
+    const int32_t px0 = x0 + lane;  // this lane's first pixel; the others follow 32 apart
+    constexpr uint32_t kAll = 0xffffffffu;
+    const uint32_t below = (1u << lane) - 1u;  // the lanes before this one
+
+    for (int i = lane; i < kCovOff; i += 32) words[i] = 0u;
+    uint32_t raw[8];
+    uint32_t touched = 0;  // blocks of 32 pixels to store (the same in every lane)
+    {
+        const DevSurface dst = JB.sfc;
+#pragma unroll
+        for (int q = 0; q < 8; q++) raw[q] = (px0 + 32 * q < W) ? load_raw(dst, (size_t)W * y + px0 + 32 * q) : 0u;
+    }
+    __syncwarp();
+
+    // The band's fill list is read 32 entries at a time, one per lane.  Each
+    // lane also loads its fill's record and edge range and tests them, so
+    // that the fills that matter to this row are known, with their
+    // records in registers, before the first of them is drawn.
+    for (int32_t k0 = 0; k0 < cnt; k0 += 32) {
+        int32_t my_f = 0, my_e0 = 0, my_ne = 0;
+        uint32_t my_meta = 0, my_px = 0, my_box = 0;
+        bool hit = false;
+        if (k0 + lane < cnt) {
+            const int4 ent = list[k0 + lane];
+            if (ent.z > x0 && ent.y < x0 + kTileCols) {
+                const int4 ra = __ldg(reinterpret_cast<const int4 *>(A.rfills + ent.x));
+                const int2 rb = __ldg(reinterpret_cast<const int2 *>(A.rfills + ent.x) + 2);
+                my_e0 = __ldg(A.bin_off + ent.w);
+                my_ne = __ldg(A.bin_off + ent.w + 1) - my_e0;
+                my_f = ent.x;
+                my_meta = (uint32_t)rb.x;
+                my_px = (uint32_t)rb.y;
+                const int32_t aa = (int32_t)((my_meta >> RF_AA_SHIFT) & 3u);
+                const bool bounded = (my_meta & RF_BOUNDED) != 0;
+                const bool boxed = bounded || aa == Z2D_AA_SUPERSAMPLE_4X;  // touches only its box
+                const bool in_rows = y >= ra.z && y <= ra.w;
+                hit = !boxed || (in_rows && ra.y > x0 && ra.x < x0 + kTileCols);
+                // no edge in the band: nothing is covered, and a bounded
+                // operator draws nothing (see the same test below)
+                if (PLAIN ? my_ne == 0 || (my_meta & RF_SS_ZERO)
+                          : bounded && my_ne == 0 && !(my_meta & (RF_EXACT | RF_SS_ZERO)))
+                    hit = false;
+                if (in_rows) my_meta |= RF_IN_ROWS;
+                // the box's columns within the tile
+                const int32_t xhi = aa == Z2D_AA_NONE ? W : min(ra.y, W);
+                my_box = (uint32_t)max(0, min(ra.x - x0, kTileCols)) |
+                         ((uint32_t)max(0, min(xhi - x0, kTileCols)) << 16);
+            }
+        }
+        for (uint32_t hits = __ballot_sync(kAll, hit); hits; hits &= hits - 1) {
+            const int src = __ffs(hits) - 1;
+            const uint32_t meta = __shfl_sync(kAll, my_meta, src);
+            const int32_t e0 = __shfl_sync(kAll, my_e0, src), ne = __shfl_sync(kAll, my_ne, src);
+            const int32_t aa = (int32_t)((meta >> RF_AA_SHIFT) & 3u);
+            const bool bounded = PLAIN || (meta & RF_BOUNDED) != 0;
+            const bool ssaa = aa == Z2D_AA_SUPERSAMPLE_4X;
+            const bool direct = aa == Z2D_AA_NONE;
+            const bool exact = !PLAIN && (meta & RF_EXACT) != 0;
+            const bool in_rows = PLAIN || (meta & RF_IN_ROWS) != 0;
+            const int32_t sc = direct ? 1 : 4, per = 8 * sc, lg_per = direct ? 3 : 5;
+            uint32_t cov_any = 0;  // lanes with a covered pixel among [8l, 8l+8)
+            if (PLAIN || (!exact && in_rows && !(meta & RF_SS_ZERO))) {
+                const int32_t sub0 = y * sc, col0 = x0 * sc, ncol = kTileCols * sc;
+                const bool eo = (meta & RF_EVEN_ODD) != 0;
+                // One edge per lane.  Crossings at or left of the tile's
+                // first sample column all count from column 0: they are
+                // summed per sample row (rows 0, 1 and 2, 3 packed as
+                // lo + 65536 hi: every sum is at most kMaxBandEdges < 2^15
+                // in magnitude, so the halves stay apart).
+                int32_t l01 = 0, l23 = 0;
+                uint32_t flags = 0;  // 1: a crossing in the tile, 2: a second of its column, 4: a fourth
+                const bool dense = !eo && ne >= kDenseEdges;
+                if (dense) flags = 4u;
+                for (int32_t base = dense ? ne : 0; base < ne; base += 32) {
+                    const RowEdge R = row_edge<GATHER>(A.bins, A.edges, e0 + base + lane, base + lane < ne, sub0, sc, col0);
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        if (r >= sc) break;
+                        if (!((R.rows >> r) & 1u)) continue;
+                        const int32_t c = edge_crossing(A.edges, R, r, sub0, col0);
+                        if (c <= 0) {
+                            const int32_t d = R.down ? -1 : 1;
+                            if (r < 2) l01 += r == 0 ? d : d * 65536;
+                            else l23 += r == 2 ? d : d * 65536;
+                        } else if (c < ncol) {
+                            uint32_t *w = words + r * kSubWords + (c >> lg_per);
+                            const uint32_t bit = 1u << (c & (per - 1));
+                            flags |= 1u;
+                            if (eo) {
+                                atomicXor(w, bit);
+                            } else {
+                                if (R.down) w += 32;
+                                if (atomicOr(w, bit) & bit) {
+                                    flags |= 2u;
+                                    if ((atomicOr(w + 64, bit) & bit) && (atomicOr(w + 128, bit) & bit)) flags |= 4u;
+                                }
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+                flags = __reduce_or_sync(kAll, flags);
+                l01 = __reduce_add_sync(kAll, l01);
+                l23 = __reduce_add_sync(kAll, l23);
+                // no crossing in the tile and none left of it in balance: the
+                // winding is 0 across the tile, nothing is covered
+                if (flags == 0 && l01 == 0 && l23 == 0) {
+                    if (bounded) continue;  // zero coverage draws nothing
+                    goto composite;         // unbounded operators still clear
+                }
+                {
+                // coverage of pixel q (0..16) of the lane's [8l, 8l+8) is byte
+                // q / 2 of cov_ev (q even) or cov_od (q odd)
+                uint32_t cov_ev = 0, cov_od = 0;
+                int32_t wl[4];  // winding left of the lane's columns (even-odd: its parity)
+                wl[0] = (int32_t)(int16_t)(l01 & 0xFFFF);
+                wl[1] = (l01 - wl[0]) >> 16;
+                wl[2] = (int32_t)(int16_t)(l23 & 0xFFFF);
+                wl[3] = (l23 - wl[2]) >> 16;
+                auto cover = [&](uint32_t bits) {
+                    if (direct) {  // one sample row: bit q is pixel q's sample
+#pragma unroll
+                        for (int q = 0; q < 8; q += 2) {
+                            cov_ev |= ((bits >> q) & 1u) << (4 * q);
+                            cov_od |= ((bits >> (q + 1)) & 1u) << (4 * q);
+                        }
+                    } else {  // nibble q holds pixel q's 4 samples of this row
+                        uint32_t n = bits - ((bits >> 1) & 0x55555555u);
+                        n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+                        cov_ev += n & 0x0F0F0F0Fu;
+                        cov_od += (n >> 4) & 0x0F0F0F0Fu;
+                    }
+                };
+                if (eo) {
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        uint32_t *w = words + s * kSubWords + lane;
+                        uint32_t t = *w;
+                        *w = 0u;
+                        // the crossings of the lanes before this one, and of
+                        // the columns left of the tile
+                        const uint32_t odd = __ballot_sync(kAll, __popc(t) & 1);
+                        const uint32_t in = (uint32_t)(__popc(odd & below) + wl[s]) & 1u;
+                        t ^= t << 1;
+                        t ^= t << 2;
+                        t ^= t << 4;
+                        t ^= t << 8;
+                        t ^= t << 16;
+                        cover(t ^ (0u - in));
+                    }
+                } else if (flags & 4u) {
+                    if (!dense) {  // clear the planes
+                        for (int i = lane; i < 4 * kSubWords; i += 32) words[i] = 0u;
+                    }
+                    const uint4 in = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, sc, col0, words, lane);
+                    cover(in.x);
+                    if (sc > 1) {
+                        cover(in.y);
+                        cover(in.z);
+                        cover(in.w);
+                    }
+                } else {
+                    uint32_t up[4], dn[4];
+                    int32_t tot[4] = {0, 0, 0, 0};  // the lane's winding change
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        uint32_t *w = words + s * kSubWords + lane;
+                        up[s] = w[0];
+                        dn[s] = w[32];
+                        w[0] = 0u;
+                        w[32] = 0u;
+                        tot[s] = __popc(up[s]) - __popc(dn[s]);
+                        if (flags & 2u) tot[s] += __popc(w[64]) + __popc(w[128]) - __popc(w[96]) - __popc(w[160]);
+                    }
+                    const int32_t t01 = tot[0] + tot[1] * 65536, t23 = tot[2] + tot[3] * 65536;
+                    int32_t i01 = t01, i23 = t23;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int32_t u01 = __shfl_up_sync(kAll, i01, o);
+                        const int32_t u23 = __shfl_up_sync(kAll, i23, o);
+                        if (lane >= o) {
+                            i01 += u01;
+                            i23 += u23;
+                        }
+                    }
+                    i01 += l01 - t01;
+                    i23 += l23 - t23;
+                    wl[0] = (int32_t)(int16_t)(i01 & 0xFFFF);
+                    wl[1] = (i01 - wl[0]) >> 16;
+                    wl[2] = (int32_t)(int16_t)(i23 & 0xFFFF);
+                    wl[3] = (i23 - wl[2]) >> 16;
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        // the inside state changes where the winding leaves
+                        // or reaches zero
+                        int32_t wnd = wl[s];
+                        uint32_t bits = wnd != 0 ? 0xFFFFFFFFu : 0u;
+                        if (flags & 2u) {
+                            uint32_t *w = words + s * kSubWords + lane;
+                            const uint32_t u1 = w[64], d1 = w[96], u2 = w[128], d2 = w[160];
+                            w[64] = w[96] = w[128] = w[160] = 0u;
+                            for (uint32_t m = up[s] | dn[s]; m; m &= m - 1) {
+                                const int k = __ffs(m) - 1;
+                                const bool was = wnd != 0;
+                                wnd += (int32_t)(((up[s] >> k) & 1u) + ((u1 >> k) & 1u) + ((u2 >> k) & 1u)) -
+                                       (int32_t)(((dn[s] >> k) & 1u) + ((d1 >> k) & 1u) + ((d2 >> k) & 1u));
+                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                            }
+                        } else {
+                            for (uint32_t m = up[s] | dn[s]; m; m &= m - 1) {
+                                const int k = __ffs(m) - 1;
+                                const bool was = wnd != 0;
+                                wnd += (int32_t)((up[s] >> k) & 1u) - (int32_t)((dn[s] >> k) & 1u);
+                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                            }
+                        }
+                        cover(bits);
+                    }
+                }
+                // only the box's columns are drawn
+                const uint32_t box = __shfl_sync(kAll, my_box, src);
+                if (box != ((uint32_t)kTileCols << 16)) {
+                    const int lo = (int)(box & 0xFFFFu) - 8 * lane, hi = (int)(box >> 16) - 8 * lane;
+                    uint32_t m = hi >= 8 ? 0xFFu : hi <= 0 ? 0u : (1u << hi) - 1u;
+                    if (lo > 0) m &= lo >= 8 ? 0u : 0xFFu << lo;
+                    if (m != 0xFFu) {
+                        // bit q of m -> byte q / 2 of the even or odd bytes
+                        const uint32_t ev = m & 0x55u, od = (m >> 1) & 0x55u;
+                        cov_ev &= (((ev & 1u) | ((ev & 4u) << 6) | ((ev & 16u) << 12) | ((ev & 64u) << 18))) * 0xFFu;
+                        cov_od &= (((od & 1u) | ((od & 4u) << 6) | ((od & 16u) << 12) | ((od & 64u) << 18))) * 0xFFu;
+                    }
+                }
+                cov_any = __ballot_sync(kAll, (cov_ev | cov_od) != 0u);
+                reinterpret_cast<uint2 *>(words + kCovOff)[lane] =
+                    make_uint2(__byte_perm(cov_ev, cov_od, 0x5140), __byte_perm(cov_ev, cov_od, 0x7362));
+                // the planes are clear again and the coverage is written
+                __syncwarp();
+                }
+            }
+        composite:
+            // coverage of this lane's pixel of block q; blocks whose bit of
+            // `blocks` is clear are uncovered (the coverage bytes are written
+            // only where some lane has coverage)
+            uint32_t blocks = 0;
+            if (cov_any) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) blocks |= ((cov_any >> (4 * q)) & 0xFu ? 1u : 0u) << q;
+            }
+            const uint8_t *cov = reinterpret_cast<const uint8_t *>(words + kCovOff) + lane;
+            if (PLAIN || (((meta >> RF_FAST_SHIFT) & 3u) == FAST_PIXEL_SRC_OVER && !exact && bounded)) {
+                // Pixel source, integer src_over: the compositeOpaque /
+                // compositeOpacity paths reduce to src_over(d, pixel) at full
+                // coverage and src_over(d, dst_in(pixel, opacity)) otherwise.
+                // The supersample batch [dst_in(pixel, mask), src_over] is the
+                // same with the downsampled mask value as opacity; at zero
+                // coverage both leave the pixel as it is.
+                // (A bounded fill outside its rows was skipped above.)
+                if (!blocks) continue;
+                const uint32_t pw = __shfl_sync(kAll, my_px, src);
+                const int full = direct ? 1 : 16;
+                // Lane k holds the source word for coverage k: the pixel at
+                // k = full, dst_in(pixel, opacity(k)) below it.
+                I16 s{pw & 0xFFu, (pw >> 8) & 0xFFu, (pw >> 16) & 0xFFu, pw >> 24};
+                if (lane < full) {
+                    const uint32_t op8 = ssaa ? ss_mask8(lane, fmt) : (uint32_t)max(lane * 16 - 1, 0);
+                    s = I16{(s.r * op8) / 255u, (s.g * op8) / 255u, (s.b * op8) / 255u, (s.a * op8) / 255u};
+                }
+                touched |= blocks;
+                if (fmt <= Z2D_FORMAT_RGBA) {
+                    const uint32_t lut_w = i16_to_word(s, word_order(fmt));
+                    const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        if (!((blocks >> q) & 1u)) continue;
+                        const int c = cov[32 * q];
+                        const uint32_t L = __shfl_sync(kAll, lut_w, c);
+                        const uint32_t nv = word_src_over_x4(raw[q], L, has_alpha);
+                        raw[q] = c != 0 ? nv : raw[q];
+                    }
+                } else {  // alpha formats: the alpha lane of src_over alone
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        if (!((blocks >> q) & 1u)) continue;
+                        const int c = cov[32 * q];
+                        const uint32_t sa = __shfl_sync(kAll, s.a, c), da = raw_to_i16(raw[q], fmt).a;
+                        const uint32_t nv = i16_to_raw(I16{0, 0, 0, sa + da - (sa * da) / 255u}, fmt);
+                        raw[q] = c != 0 ? nv : raw[q];
+                    }
+                }
+                continue;
+            }
+            if constexpr (!PLAIN) {
+            const int32_t f = __shfl_sync(kAll, my_f, src);
+            const FillState &S = A.st[f];
+            const FillCmd &F = A.fills[f];
+            // with a bounded operator only covered pixels are drawn
+            const bool sparse = bounded && !ssaa && !exact;
+#pragma unroll 1
+            for (int q = 0; q < 8; q++) {
+                const bool some = (blocks >> q) & 1u;
+                if (sparse && !some) continue;
+                const int32_t x = px0 + 32 * q;
+                // raw[] is read and written with constant indices only, so it
+                // stays in registers
+                uint32_t rq = raw[0];
+#pragma unroll
+                for (int j = 1; j < 8; j++)
+                    if (q == j) rq = raw[j];
+                int c = some ? cov[32 * q] : 0;
+                bool on;
+                if (ssaa) {
+                    // every pixel of the composite region runs the batch
+                    // [dst_in(pattern, mask), op] (supersample.zig:171-184)
+                    on = x < W && x >= S.start_x && x < S.end_x;
+                    if (on) {
+                        if (exact && x >= S.mask_x0 && x < S.mask_x0 + S.mask_w)
+                            c = A.masks[S.mask_base + (long long)(y - S.start_y) * S.mask_w + (x - S.mask_x0)] & 0x1F;
+                        rq = i16_to_raw(apply_ssaa(F, x, y, ss_mask8(c, fmt), raw_to_i16(rq, fmt)), fmt);
+                    }
+                } else {
+                    bool clear = false;
+                    if (exact && in_rows && x >= S.mask_x0 && x < S.mask_x0 + S.mask_w) {
+                        const uint8_t m = A.masks[S.mask_base + (long long)(y - S.start_y) * S.mask_w + (x - S.mask_x0)];
+                        c = m & 0x1F;
+                        if (direct) clear = (m & kMaskClear) != 0;
+                    }
+                    if (!direct && !bounded) clear = msaa_unbounded_clear(S, x, y, W);
+                    const bool in_box = in_rows && (direct ? true : (x >= S.start_x && x < S.end_x));
+                    on = x < W && (clear || (in_box && c > 0));
+                    if (on) {
+                        I16 d = clear ? normalize(I16{0, 0, 0, 0}, fmt) : raw_to_i16(rq, fmt);
+                        if (in_box && c > 0) d = apply_fill(F, fmt, x, y, c, direct ? 1 : 16, d);
+                        rq = i16_to_raw(d, fmt);
+                    }
+                }
+                if (!__any_sync(kAll, on)) continue;
+                touched |= 1u << q;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (q == j) raw[j] = rq;
+            }
+            }
+        }
+    }
+    // the surface pointer is read again here rather than kept in registers
+    // through the fill loop
+    DevSurface dst;
+    dst.data = MULTI ? *reinterpret_cast<uint8_t *const volatile *>(&A.jobs[jb].sfc.data) : A.job0.sfc.data;
+    dst.fmt = fmt;
+    dst.w = W;
+    dst.h = 0;  // unused by the stores
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        if (((touched >> q) & 1u) && px0 + 32 * q < W) store_raw(dst, (size_t)W * y + px0 + 32 * q, raw[q]);
+}
+
+// Persistent rasteriser: a grid of resident CTAs that take items from a
+// device work queue (one 64-bit counter) until it is empty; tiles are
+// queued job after job, or in the order of A.order when given.
+//  * CTA_ITEMS: an item is a whole tile; the CTA's four warps draw its four
+//    rows and meet at a barrier before the next tile, so the rows share the
+//    band's fill list and edges in the SM's L1.
+//  * otherwise an item is one (tile, row) pair, numbered tile * 4 + row,
+//    taken by a single warp: a warp that finishes a cheap row takes the
+//    next item at once instead of holding its CTA until the slowest warp of
+//    the tile is done.
+template <bool MULTI, bool CTA_ITEMS, bool PLAIN, bool GATHER = false>
+__global__ void __launch_bounds__(kRasterThreads, PLAIN ? 8 : 6) k_raster(const RasterArgs A) {
+    extern __shared__ uint32_t smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t *words = smem + warp * kWarpWords;
+    if constexpr (CTA_ITEMS) {
+        __shared__ unsigned long long next_tile;
+        for (;;) {
+            unsigned long long t = blockIdx.x;  // one_per_tile: a grid of one CTA per tile, dispatched in queue order
+            if (!A.one_per_tile) {
+                if (threadIdx.x == 0) next_tile = atomicAdd(A.queue, 1ull);
+                __syncthreads();
+                t = next_tile;
+                __syncthreads();  // every thread has read it before it is replaced
+                if (t >= A.n_items) break;
+            }
+            const int32_t tile = A.order ? A.order[t] : (int32_t)t;
+            raster_row<MULTI, PLAIN, GATHER>(A, tile, warp, lane, words);
+            if (A.one_per_tile) break;
+        }
+    } else {
+        for (;;) {
+            unsigned long long item = 0;
+            if (lane == 0) item = atomicAdd(A.queue, 1ull);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            if (item >= A.n_items) break;
+            const long long t = (long long)(item / kTileRows);
+            const int32_t tile = A.order ? A.order[t] : (int32_t)t;
+            __syncwarp();  // the previous item's reads of `words` are done before it is reset
+            raster_row<MULTI, PLAIN, GATHER>(A, tile, (int)(item % kTileRows), lane, words);
+        }
+    }
+}
+
+static size_t raster_smem() { return sizeof(uint32_t) * kWarpWords * kTileRows; }
+
+template <class F>
+static int with_variant(RasterVariant v, F &&f) {
+    const int k = (v.gather ? 8 : 0) | (v.multi ? 4 : 0) | (v.cta_items ? 2 : 0) | (v.plain ? 1 : 0);
+    switch (k) {
+        case 0: return f(k_raster<false, false, false>, k);
+        case 1: return f(k_raster<false, false, true>, k);
+        case 2: return f(k_raster<false, true, false>, k);
+        case 3: return f(k_raster<false, true, true>, k);
+        case 4: return f(k_raster<true, false, false>, k);
+        case 5: return f(k_raster<true, false, true>, k);
+        case 6: return f(k_raster<true, true, false>, k);
+        case 7: return f(k_raster<true, true, true>, k);
+        case 10: return f(k_raster<false, true, false, true>, k);
+        case 11: return f(k_raster<false, true, true, true>, k);
+        case 14: return f(k_raster<true, true, false, true>, k);
+        case 15: return f(k_raster<true, true, true, true>, k);
+        default: return Z2D_ERR_INVALID_ARGUMENT;  // (gathered edges come a tile per CTA)
+    }
+}
+
+// A variant's resident CTAs per SM, asked once per variant.
+int raster_occupancy(Ctx &, RasterVariant v, int &ctas_per_sm) {
+    static std::atomic<int> cache[16];
+    return with_variant(v, [&](auto kernel, int k) -> int {
+        int occ = cache[k].load(std::memory_order_relaxed);
+        if (occ <= 0) {
+            Z2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRasterThreads, raster_smem()));
+            occ = std::max(occ, 1);
+            cache[k].store(occ, std::memory_order_relaxed);
+        }
+        ctas_per_sm = occ;
+        return Z2D_OK;
+    });
+}
+
+int raster_launch(Ctx &c, RasterVariant v, const RasterArgs &A, unsigned grid) {
+    return with_variant(v, [&](auto kernel, int) -> int {
+        kernel<<<grid, kRasterThreads, raster_smem(), c.stream>>>(A);
+        c.launches++;
+        Z2D_CUDA(cudaGetLastError());
+        return Z2D_OK;
+    });
+}
+
+}  // namespace z2dg

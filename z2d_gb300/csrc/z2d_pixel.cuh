@@ -146,6 +146,18 @@ Z2D_HD uint32_t word_src_over(uint32_t w, uint32_t L, bool has_alpha) {
     }
     return out;
 }
+// The same for the rasteriser, whose ALU work counts: d_a - floor(s_a * d_a /
+// 255) is ceil(d_a * (255 - s_a) / 255), the colours' division with 254 added
+// first (65,279 at most, where div255x2's shift is still exact), so alpha
+// rides in the upper half of the second pair.  (In the memory-bound mask
+// batch the form above is 2 % faster: its alpha runs beside the pairs.)
+Z2D_HD uint32_t word_src_over_x4(uint32_t w, uint32_t L, bool has_alpha) {
+    const uint32_t inv = 255u - (L >> 24);
+    const uint32_t e = div255x2((w & 0x00FF00FFu) * inv) + (L & 0x00FF00FFu);
+    const uint32_t o = div255x2(((w >> 8) & 0x00FF00FFu) * inv + 0x00FE0000u) + ((L >> 8) & 0x00FF00FFu);
+    const uint32_t out = (e & 0x00FF00FFu) | ((o & 0x00FF00FFu) << 8);
+    return has_alpha ? out : out & 0x00FFFFFFu;
+}
 
 // Surface access by flat pixel index (w*y+x).  Packed formats are LSB
 // first (src/pixel.zig:664-677).
