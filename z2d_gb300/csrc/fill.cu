@@ -197,232 +197,82 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_fill_scan(const z2d_node *_
 }
 
 
-// ------------------------------------------- warp-cooperative flattening
-// One warp per curve.  The subdivision tree of Spline.decomposeInto is first
-// expanded breadth-first into an ordered frontier of up to kFrontier
-// subcurves (z2d's depth-first order is the frontier order), then lane l
-// walks frontier items l and l+32 depth-first.  Warp scans give each lane
-// the number of points emitted before it and the point emitted just before
-// its first one, so edges land where the sequential walk would put them.
-constexpr int kFrontier = 64;
+// ------------------------------------------------------- curve flattening
 constexpr int kFlattenWarps = 4;
+constexpr int kScratch = 64;  // leaf points a lane keeps
 
-struct WarpFrontier {
-    Knots k[kFrontier];
-    uint8_t leaf[kFrontier];  // 1: error below tolerance already established
-};
-
-// Expands the frontier of the curve from (ax, ay) through p[0..5].
-__device__ int frontier_expand(double ax, double ay, const double *p, const Tol &tol, WarpFrontier &fr, int lane) {
-    if (lane == 0) {
-        fr.k[0] = Knots{ax, ay, p[0], p[1], p[2], p[3], p[4], p[5]};
-        fr.leaf[0] = 0;
-    }
-    __syncwarp();
-    int n = 1;
-    for (int round = 0; round < 8 && n < 32; round++) {
-        Knots k{};
-        bool leaf = true;
-        int grow = 0;
-        if (lane < n) {
-            k = fr.k[lane];
-            leaf = fr.leaf[lane] || below_tol(k, tol);
-            grow = leaf ? 1 : 2;
-        }
-        int incl = grow;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        const bool all_leaf = __all_sync(0xffffffffu, leaf);
-        __syncwarp();
-        if (all_leaf || total > kFrontier) {
-            if (lane < n) fr.leaf[lane] = leaf ? 1 : 0;
-            __syncwarp();
-            break;
-        }
-        const int pos = incl - grow;
-        if (lane < n) {
-            if (leaf) {
-                fr.k[pos] = k;
-                fr.leaf[pos] = 1;
-            } else {
-                const Knots second = de_casteljau(k);
-                fr.k[pos] = k;
-                fr.leaf[pos] = 0;
-                fr.k[pos + 1] = second;
-                fr.leaf[pos + 1] = 0;
-            }
-        }
-        __syncwarp();
-        n = total;
-    }
-    return n;
-}
-
-// Depth-first walk of one frontier item (Spline.zig:56-71): leaf(k) for
-// every subcurve that decomposeInto stops at, in order.
-template <class L>
-__device__ __forceinline__ bool walk_leaves(const Knots &k0, bool is_leaf, const Tol &tol, L &&leaf) {
-    if (is_leaf) {
-        leaf(k0);
-        return true;
-    }
-    Knots stack[kSplineStack];
-    int sp = 0;
-    stack[sp++] = k0;
-    int32_t budget = kSplineMaxSplits;
-    while (sp > 0) {
-        Knots k = stack[--sp];
-        while (true) {
-            if (--budget < 0) return false;
-            if (below_tol(k, tol)) {
-                leaf(k);
-                break;
-            }
-            const Knots second = de_casteljau(k);
-            if (sp >= kSplineStack) return false;
-            stack[sp++] = second;
-        }
-    }
-    return true;
-}
-
-// emit(x, y) for each leaf start that differs from the curve start: the
-// lineTo calls of decomposeInto.  The final lineTo(d) is not part of an item.
-template <class F>
-__device__ __forceinline__ bool walk_item(const Knots &k0, bool is_leaf, double ax, double ay, const Tol &tol, F &&emit) {
-    return walk_leaves(k0, is_leaf, tol, [&](const Knots &k) {
-        if (!pt_eq(k.ax, k.ay, ax, ay)) emit(k.ax, k.ay);
-    });
-}
-
-// "Last valid value before this lane" across the warp, seeded with carry.
-__device__ __forceinline__ void prev_point_scan(bool has, double lx, double ly, double cx, double cy, int lane,
+// "Last valid value before this lane" within groups of G lanes, seeded with
+// the group's carry.
+__device__ __forceinline__ void prev_point_scan(bool has, double lx, double ly, double cx, double cy, int j, int G,
                                                 double &px, double &py) {
     // inclusive "most recent valid" scan, then shift by one lane
     int v = has ? 1 : 0;
     double x = lx, y = ly;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int tv = __shfl_up_sync(0xffffffffu, v, o);
-        const double tx = __shfl_up_sync(0xffffffffu, x, o);
-        const double ty = __shfl_up_sync(0xffffffffu, y, o);
-        if (lane >= o && !v) {
+    for (int o = 1; o < G; o <<= 1) {
+        const int tv = __shfl_up_sync(0xffffffffu, v, o, G);
+        const double tx = __shfl_up_sync(0xffffffffu, x, o, G);
+        const double ty = __shfl_up_sync(0xffffffffu, y, o, G);
+        if (j >= o && !v) {
             v = tv;
             x = tx;
             y = ty;
         }
     }
-    const int pv = __shfl_up_sync(0xffffffffu, v, 1);
-    const double qx = __shfl_up_sync(0xffffffffu, x, 1);
-    const double qy = __shfl_up_sync(0xffffffffu, y, 1);
-    if (lane > 0 && pv) {
+    px = cx;
+    py = cy;
+    if (G == 1) return;
+    const int pv = __shfl_up_sync(0xffffffffu, v, 1, G);
+    const double qx = __shfl_up_sync(0xffffffffu, x, 1, G);
+    const double qy = __shfl_up_sync(0xffffffffu, y, 1, G);
+    if (j > 0 && pv) {
         px = qx;
         py = qy;
-    } else {
-        px = cx;
-        py = cy;
     }
 }
 
-__device__ __forceinline__ int warp_excl_sum(int v, int lane, int &total) {
+// Exclusive sum over the lanes of a group of G, and the group's total.
+__device__ __forceinline__ int group_excl_sum(int v, int j, int G, int &total) {
     int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+    for (int o = 1; o < G; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o, G);
+        if (j >= o) incl += t;
     }
-    total = __shfl_sync(0xffffffffu, incl, 31);
+    total = __shfl_sync(0xffffffffu, incl, G - 1, G);
     return incl - v;
 }
 
-// Counts the lineTo calls (n_emit) and the points they add (n_added) of the
-// curve from (sx, sy) through p, cooperatively.  Result valid in all lanes.
-// Counts the lineTo calls (n_emit) and the points PointBuffer keeps
-// (n_added) of one curve, and the leaves of each frontier item
-// (item_leaves[0..kFrontier)).  chords is set when the curve's edges are
-// exactly its leaves' chords: every leaf start but the first differs from the
-// curve start (consecutive leaves share their end points, so the lineTo
-// sequence start, a1, a2, ..., d is the chord sequence), and every item has
-// fewer than 65536 leaves.
-// Each lane also keeps the start points of the leaves it walks, up to
-// kScratch of them, interleaved across the warp in `scr` (scr_n counts
-// them, beyond kScratch too); n_items and leaves return the frontier size
-// and the curve's leaf count.
-constexpr int kScratch = 64;
-__device__ bool curve_count_warp(double sx, double sy, const double *p, double tol, WarpFrontier &fr, int lane,
-                                 int32_t &n_emit, int32_t &n_added, uint16_t *item_leaves, int32_t &chords,
-                                 double2 *scr, int32_t &scr_n, int &n_items, int32_t &leaves_out) {
-    chords = 0;
-    scr_n = 0;
-    n_items = 0;
-    leaves_out = 0;
-    if (pt_eq(sx, sy, p[0], p[1]) && pt_eq(p[2], p[3], p[4], p[5])) {  // Spline.zig:39-42
-        n_emit = 1;
-        n_added = pt_eq(sx, sy, p[4], p[5]) ? 0 : 1;
-        return true;
-    }
-    const Tol tol2 = make_tol(tol);
-    const int n = frontier_expand(sx, sy, p, tol2, fr, lane);
-    n_items = n;
-    bool ok = true, small = true;
-    int32_t emit_tot = 0, add_tot = 0, leaf_tot = 0;
-    double carry_x = sx, carry_y = sy;
-    for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        int32_t cnt = 0, internal = 0, leaves = 0;
-        double fx = 0, fy = 0, lx = 0, ly = 0;
-        if (i < n) {
-            ok &= walk_leaves(fr.k[i], fr.leaf[i] != 0, tol2, [&](const Knots &k) {
-                leaves++;
-                if (scr_n < kScratch) scr[scr_n * 32 + lane] = make_double2(k.ax, k.ay);
-                scr_n++;
-                if (pt_eq(k.ax, k.ay, sx, sy)) return;  // decomposeInto plots no point equal to the start
-                const double x = k.ax, y = k.ay;
-                if (cnt == 0) {
-                    fx = x;
-                    fy = y;
-                } else if (!pt_eq(x, y, lx, ly)) {
-                    internal++;
-                }
-                lx = x;
-                ly = y;
-                cnt++;
-            });
-            small &= leaves < 65536;
-            item_leaves[i] = (uint16_t)leaves;
+// What a lane's share of a curve gives the curve: the lineTo calls its
+// leaves issue (those whose start is not the curve's start: decomposeInto
+// plots no such point), the points among them that differ from the one
+// before, the first and the last point.
+struct LaneCurve {
+    int32_t cnt = 0, internal = 0, leaves = 0;
+    double fx = 0, fy = 0, lx = 0, ly = 0;
+    bool ok = true;
+};
+template <class P>
+__device__ __forceinline__ LaneCurve walk_lane(double sx, double sy, const double *p, const Tol &tol, int g, int j,
+                                               P &&leaf_start) {
+    LaneCurve r;
+    Knots k{sx, sy, p[0], p[1], p[2], p[3], p[4], p[5]};
+    bool is_leaf;
+    int open;
+    if (!lane_subtree(k, g, j, tol, is_leaf, open)) return r;
+    r.ok = walk_leaves(k, is_leaf, open, tol, [&](const Knots &q) {
+        leaf_start(r.leaves, q);
+        r.leaves++;
+        if (pt_eq(q.ax, q.ay, sx, sy)) return;
+        if (r.cnt == 0) {
+            r.fx = q.ax;
+            r.fy = q.ay;
+        } else if (!pt_eq(q.ax, q.ay, r.lx, r.ly)) {
+            r.internal++;
         }
-        int lt = 0;
-        warp_excl_sum(leaves, lane, lt);
-        leaf_tot += lt;
-        double px, py;
-        prev_point_scan(cnt > 0, lx, ly, carry_x, carry_y, lane, px, py);
-        const int32_t first_add = (cnt > 0 && !pt_eq(fx, fy, px, py)) ? 1 : 0;
-        int rt = 0;
-        warp_excl_sum(cnt, lane, rt);
-        emit_tot += rt;
-        int at = 0;
-        warp_excl_sum(internal + first_add, lane, at);
-        add_tot += at;
-        // carry: the last point emitted so far
-        const unsigned m = __ballot_sync(0xffffffffu, cnt > 0);
-        if (m) {
-            const int src = 31 - __clz(m);
-            carry_x = __shfl_sync(0xffffffffu, lx, src);
-            carry_y = __shfl_sync(0xffffffffu, ly, src);
-        }
-    }
-    // final lineTo(d)
-    chords = (__all_sync(0xffffffffu, small) && leaf_tot == emit_tot + 1) ? 1 : 0;
-    leaves_out = leaf_tot;
-    emit_tot += 1;
-    add_tot += pt_eq(p[4], p[5], carry_x, carry_y) ? 0 : 1;
-    n_emit = emit_tot;
-    n_added = add_tot;
-    return __all_sync(0xffffffffu, ok);
+        r.lx = q.ax;
+        r.ly = q.ay;
+        r.cnt++;
+    });
+    return r;
 }
 
 // Appends idx to a device list (one atomic per warp); all lanes call it.
@@ -438,7 +288,7 @@ __device__ __forceinline__ void queue_push(bool push, int32_t idx, int32_t *list
 
 // The node kernels take 32 consecutive nodes per warp: every lane handles
 // its own line, move and close_path node and queues its curve, if it has
-// one; the curve kernels then subdivide one queued curve per warp.
+// one, with the curves of its class (curve_class).
 __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_count_w(const z2d_node *__restrict__ nodes,
                                                                      const int32_t *__restrict__ node_fill,
                                                                      const FillCmd *__restrict__ fills,
@@ -450,7 +300,7 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_count_w(const z2d_n
          base += gridDim.x * kFlattenWarps * 32) {
         const int32_t i = base + lane;
         NodeInfo inf{};
-        bool curve = false;
+        int curve = -1;  // its length class
         if (i < n_nodes) {
             const int32_t f = node_fill[i];
             if (f >= 0) {  // else no fill owns the node
@@ -462,146 +312,170 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_count_w(const z2d_n
                                                                  pv.tag == Z2D_CURVE_TO);
                     if (!static_start) {
                         inf.n_emit = -1;  // resolved by k_fill_scan
-                    } else if (nd.tag == Z2D_LINE_TO) {
+                    } else {
                         const double sx = pv.tag == Z2D_CURVE_TO ? pv.p[4] : pv.p[0];
                         const double sy = pv.tag == Z2D_CURVE_TO ? pv.p[5] : pv.p[1];
-                        inf.n_emit = 1;
-                        inf.n_added = pt_eq(sx, sy, nd.p[0], nd.p[1]) ? 0 : 1;
-                    } else {
-                        curve = true;  // k_curve_count_w fills in its info
+                        if (nd.tag == Z2D_LINE_TO) {
+                            inf.n_emit = 1;
+                            inf.n_added = pt_eq(sx, sy, nd.p[0], nd.p[1]) ? 0 : 1;
+                        } else if (pt_eq(sx, sy, nd.p[0], nd.p[1]) && pt_eq(nd.p[2], nd.p[3], nd.p[4], nd.p[5])) {
+                            inf.n_emit = 1;  // a straight one: lineTo(d) (Spline.zig:39-42)
+                            inf.n_added = pt_eq(sx, sy, nd.p[4], nd.p[5]) ? 0 : 1;
+                        } else {  // k_curve_count_w fills in its info
+                            curve = curve_class(sx, sy, nd.p, fills[f].tol);
+                        }
                     }
                 }
             }
         }
         inf.pool = -1;
-        if (i < n_nodes && !curve) info[i] = inf;
-        queue_push(curve, i, curves, counters + CNT_CURVES, lane);
+        if (i < n_nodes && curve < 0) info[i] = inf;
+        for (int k = 0; k < kCurveClasses; k++)
+            queue_push(curve == k, i, curves + k * (size_t)n_nodes, counters + CNT_CURVES + k, lane);
     }
 }
 
-// Besides the counts, a chord curve whose leaves all fit the lanes' scratch
-// leaves its polyline (leaf starts, then d) in the curve pool, so that the
-// emit pass copies points instead of subdividing the curve again.
+// Counts every queued curve's lineTo calls (n_emit) and the points
+// PointBuffer keeps of them (n_added).  2^g neighbouring lanes walk a curve:
+// about 8 leaves each (g = 0 for class 0, g = k - 3 for a curve of about 2^k
+// leaves), fewer while the grid has lanes to spare.  The lanes of a warp then
+// have walks of like length, and the splits that every lane of a curve
+// repeats stay few against the leaves.  (A warp per curve left most lanes
+// idle on short curves: 1,024 glyphs of 110 curves 655 us, now 157; 320
+// surfaces with 16 k fills 2.1 ms, now 0.76; 2,000 paths of long curves 396
+// us, now 285.  Three classes of 1, 8 and 32 lanes: 222, 925 and 309 us.)
+// A curve's edges are its leaves' chords when every leaf start but the first
+// differs from the curve's start (consecutive leaves share their end points,
+// so the lineTo sequence start, a1, a2, ..., d is the chord sequence): such a
+// curve, if its leaves fit the lanes' scratch, leaves its polyline (leaf
+// starts, then d) in the curve pool, and the emit pass reads points instead
+// of subdividing again.  Bound by the issue of the subdivision (below_tol,
+// de_casteljau).
 __global__ void __launch_bounds__(32 * kFlattenWarps) k_curve_count_w(const z2d_node *__restrict__ nodes,
                                                                       const int32_t *__restrict__ node_fill,
                                                                       const FillCmd *__restrict__ fills,
-                                                                      NodeInfo *__restrict__ info,
+                                                                      NodeInfo *__restrict__ info, int32_t n_nodes,
                                                                       const int32_t *__restrict__ curves,
                                                                       int32_t *__restrict__ counters,
-                                                                      uint16_t *__restrict__ item_leaves,
                                                                       int32_t *__restrict__ status,
                                                                       double2 *__restrict__ scratch,
                                                                       double2 *__restrict__ pool, int32_t pool_cap) {
-    __shared__ WarpFrontier frs[kFlattenWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned all = 0xffffffffu;
-    WarpFrontier &fr = frs[w];
     double2 *scr = scratch + (size_t)(blockIdx.x * kFlattenWarps + w) * (32 * kScratch);
-    const int32_t n = counters[CNT_CURVES];
-    for (int32_t q = blockIdx.x * kFlattenWarps + w; q < n; q += gridDim.x * kFlattenWarps) {
-        const int32_t i = curves[q];
-        const z2d_node nd = nodes[i];
-        const z2d_node pv = nodes[i - 1];
-        const double sx = pv.tag == Z2D_CURVE_TO ? pv.p[4] : pv.p[0];
-        const double sy = pv.tag == Z2D_CURVE_TO ? pv.p[5] : pv.p[1];
-        NodeInfo inf{};
-        int32_t scr_n = 0, leaves = 0;
-        int n_items = 0;
-        uint16_t *il = item_leaves + (size_t)i * kFrontier;
-        const bool ok = curve_count_warp(sx, sy, nd.p, fills[node_fill[i]].tol, fr, lane, inf.n_emit, inf.n_added, il,
-                                         inf.chords, scr, scr_n, n_items, leaves);
-        if (!ok && lane == 0) atomicExch(status, Z2D_ERR_INVALID_STATE);
-        inf.pool = -1;
-        if (ok && inf.chords && __all_sync(all, scr_n <= kScratch)) {
-            int32_t base = -1;
+    const int32_t warps = gridDim.x * kFlattenWarps;
+    int32_t n[kCurveClasses];
+    long long lanes = 0;
+    for (int k = 0; k < kCurveClasses; k++) {
+        n[k] = counters[CNT_CURVES + k];
+        lanes += (long long)n[k] << k;
+    }
+    int spare = 0;
+    while (spare < kCurveClasses - 1 && (lanes << (spare + 1)) <= 32ll * warps) spare++;
+    // chunks of 32 >> g curves, the longest class first
+    int32_t chunks = 0;
+    for (int k = 0; k < kCurveClasses; k++)
+        chunks += (int32_t)((((long long)n[k] << min(k + spare, 5)) + 31) >> 5);
+    for (int32_t c0 = blockIdx.x * kFlattenWarps + w; c0 < chunks; c0 += warps) {
+        int32_t c = c0;
+        int k = kCurveClasses - 1;
+        for (; k > 0; k--) {
+            const int32_t m = (int32_t)((((long long)n[k] << min(k + spare, 5)) + 31) >> 5);
+            if (c < m) break;
+            c -= m;
+        }
+        const int g = min(k + spare, 5), G = 1 << g;
+        const int j = lane & (G - 1);
+        const int32_t q = c * (32 >> g) + (lane >> g);
+        int32_t nk = n[0];
+#pragma unroll
+        for (int i = 1; i < kCurveClasses; i++)
+            if (k == i) nk = n[i];
+        const bool live = q < nk;
+        int32_t i = 0;
+        double sx = 0, sy = 0, dx = 0, dy = 0;
+        LaneCurve r;
+        if (live) {
+            i = curves[k * (size_t)n_nodes + q];
+            const z2d_node nd = nodes[i];
+            const z2d_node pv = nodes[i - 1];
+            sx = pv.tag == Z2D_CURVE_TO ? pv.p[4] : pv.p[0];
+            sy = pv.tag == Z2D_CURVE_TO ? pv.p[5] : pv.p[1];
+            dx = nd.p[4];
+            dy = nd.p[5];
+            r = walk_lane(sx, sy, nd.p, make_tol(fills[node_fill[i]].tol), g, j, [&](int32_t m, const Knots &q) {
+                if (m < kScratch) scr[m * 32 + lane] = make_double2(q.ax, q.ay);
+            });
+            if (!r.ok) atomicExch(status, Z2D_ERR_INVALID_STATE);
+        }
+        __syncwarp();
+        double px, py;
+        prev_point_scan(r.cnt > 0, r.lx, r.ly, sx, sy, j, G, px, py);
+        const int32_t first_add = (r.cnt > 0 && !pt_eq(r.fx, r.fy, px, py)) ? 1 : 0;
+        int32_t emit = 0, added = 0, leaves = 0, unfit = 0;
+        group_excl_sum(r.cnt, j, G, emit);
+        group_excl_sum(r.internal + first_add, j, G, added);
+        const int32_t at = group_excl_sum(r.leaves, j, G, leaves);
+        group_excl_sum(r.leaves > kScratch || !r.ok ? 1 : 0, j, G, unfit);
+        const bool chords = leaves == emit + 1;
+        // the group's last lane sees the last point before d
+        const bool last = live && j == G - 1;
+        const double ex = r.cnt > 0 ? r.lx : px, ey = r.cnt > 0 ? r.ly : py;
+        // room for the polylines of the warp's curves: one reservation
+        const bool keep = live && chords && unfit == 0;
+        int32_t room = 0;
+        const int32_t mine = group_excl_sum(last && keep ? leaves + 1 : 0, lane, 32, room);
+        int32_t base = -1;
+        if (room > 0) {
             if (lane == 0) {
                 const unsigned long long b = atomicAdd(reinterpret_cast<unsigned long long *>(&counters[CNT_POOL]),
-                                                       (unsigned long long)(leaves + 1));
-                base = (b + (unsigned long long)(leaves + 1) <= (unsigned long long)pool_cap) ? (int32_t)b : -1;
+                                                       (unsigned long long)room);
+                base = (b + (unsigned long long)room <= (unsigned long long)pool_cap) ? (int32_t)b : -1;
             }
-            base = __shfl_sync(all, base, 0);
-            if (base >= 0) {
-                __syncwarp();  // item_leaves of the other lanes are visible
-                int32_t off = 0, src = 0;
-                for (int b0 = 0; b0 < n_items; b0 += 32) {
-                    const int i2 = b0 + lane;
-                    const int32_t cnt = i2 < n_items ? (int32_t)il[i2] : 0;
-                    int tot = 0;
-                    const int32_t at = off + warp_excl_sum(cnt, lane, tot);
-                    for (int32_t j = 0; j < cnt; j++) pool[base + at + j] = scr[(src + j) * 32 + lane];
-                    src += cnt;
-                    off += tot;
-                }
-                if (lane == 0) pool[base + leaves] = make_double2(nd.p[4], nd.p[5]);
-                inf.pool = base;
-            }
+            base = __shfl_sync(0xffffffffu, base, 0);
         }
-        if (lane == 0) info[i] = inf;
+        // (the last lane's own sum is that of the curves before)
+        const int32_t first = __shfl_sync(0xffffffffu, mine, G - 1, G) + base;
+        const bool pooled = keep && base >= 0;
+        if (pooled) {
+            double2 *out = pool + first + at;
+            for (int32_t m = 0; m < r.leaves; m++) out[m] = scr[m * 32 + lane];
+            if (last) pool[first + leaves] = make_double2(dx, dy);
+        }
+        if (last) {
+            NodeInfo inf{};
+            inf.n_emit = emit + 1;  // with the final lineTo(d)
+            inf.n_added = added + (pt_eq(dx, dy, ex, ey) ? 0 : 1);
+            inf.pool = pooled ? first : -1;
+            info[i] = inf;
+        }
         __syncwarp();
     }
 }
 
-// Emits the edges of one curve with the whole warp.
+// Emits the edges of one curve with the whole warp: its leaves counted by
+// one walk, emitted by another.
 __device__ __forceinline__ void curve_emit_warp(const FillCmd &F, DEdge *out, const NodeInfo &inf, const double *p,
-                                                const uint16_t *il, WarpFrontier &fr, int lane, double &et, double &eb,
-                                                double &el, double &er, bool &any) {
-    const Tol tol2 = make_tol(F.tol);
-    const int n = frontier_expand(inf.sx, inf.sy, p, tol2, fr, lane);
-    if (inf.chords) {
-        // One walk: the edges are the leaves' chords (a -> d), and the
-        // count pass left each frontier item's leaf count.
-        int32_t base_off = 0;
-        for (int base = 0; base < n; base += 32) {
-            const int i2 = base + lane;
-            const int32_t cnt = i2 < n ? (int32_t)il[i2] : 0;
-            int tot = 0;
-            const int off = base_off + warp_excl_sum(cnt, lane, tot);
-            if (i2 < n && cnt > 0) {
-                int32_t k = off;
-                walk_leaves(fr.k[i2], fr.leaf[i2] != 0, tol2, [&](const Knots &kn) {
-                    if (k < inf.n_emit) add_edge(F, out + k, kn.ax, kn.ay, kn.dx, kn.dy, et, eb, el, er, any);
-                    k++;
-                });
-            }
-            base_off += tot;
-        }
-        return;
+                                                int lane, double &et, double &eb, double &el, double &er, bool &any) {
+    const Tol tol = make_tol(F.tol);
+    const LaneCurve r = walk_lane(inf.sx, inf.sy, p, tol, 5, lane, [](int32_t, const Knots &) {});
+    __syncwarp();
+    double px, py;
+    prev_point_scan(r.cnt > 0, r.lx, r.ly, inf.sx, inf.sy, lane, 32, px, py);
+    int tot = 0;
+    const int off = group_excl_sum(r.cnt, lane, 32, tot);
+    const double ex = r.cnt > 0 ? r.lx : px, ey = r.cnt > 0 ? r.ly : py;
+    if (r.cnt > 0) {
+        int32_t k = off;
+        walk_lane(inf.sx, inf.sy, p, tol, 5, lane, [&](int32_t, const Knots &q) {
+            if (pt_eq(q.ax, q.ay, inf.sx, inf.sy)) return;
+            if (k < inf.n_emit) add_edge(F, out + k, px, py, q.ax, q.ay, et, eb, el, er, any);
+            k++;
+            px = q.ax;
+            py = q.ay;
+        });
     }
-    int32_t base_off = 0;
-    double carry_x = inf.sx, carry_y = inf.sy;
-    for (int base = 0; base < n; base += 32) {
-        const int i2 = base + lane;
-        int32_t cnt = 0;
-        double lx = 0, ly = 0;
-        if (i2 < n)
-            walk_item(fr.k[i2], fr.leaf[i2] != 0, inf.sx, inf.sy, tol2, [&](double x, double y) {
-                cnt++;
-                lx = x;
-                ly = y;
-            });
-        double px, py;
-        prev_point_scan(cnt > 0, lx, ly, carry_x, carry_y, lane, px, py);
-        int tot = 0;
-        const int off = base_off + warp_excl_sum(cnt, lane, tot);
-        if (i2 < n && cnt > 0) {
-            int32_t k = off;
-            walk_item(fr.k[i2], fr.leaf[i2] != 0, inf.sx, inf.sy, tol2, [&](double x, double y) {
-                if (k < inf.n_emit) add_edge(F, out + k, px, py, x, y, et, eb, el, er, any);
-                k++;
-                px = x;
-                py = y;
-            });
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, cnt > 0);
-        if (m) {
-            const int src = 31 - __clz(m);
-            carry_x = __shfl_sync(0xffffffffu, lx, src);
-            carry_y = __shfl_sync(0xffffffffu, ly, src);
-        }
-        base_off += tot;
-    }
-    if (lane == 0 && base_off < inf.n_emit)  // final lineTo(d)
-        add_edge(F, out + base_off, carry_x, carry_y, p[4], p[5], et, eb, el, er, any);
+    if (lane == 31 && tot < inf.n_emit)  // final lineTo(d)
+        add_edge(F, out + tot, ex, ey, p[4], p[5], et, eb, el, er, any);
 }
 
 __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_emit_w(const z2d_node *__restrict__ nodes,
@@ -639,6 +513,11 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_emit_w(const z2d_no
     }
 }
 
+// Emits the queued curves' edges.  A warp takes up to 32 curves (as many as
+// give every warp of the grid some) and goes through the edges of those with
+// a polyline 32 at a time, whichever curve they belong to: a curve of a few
+// edges does not idle the other lanes.  Edge k of a curve joins points k and
+// k + 1.
 __global__ void __launch_bounds__(32 * kFlattenWarps) k_curve_emit_w(const z2d_node *__restrict__ nodes,
                                                                      const int32_t *__restrict__ node_fill,
                                                                      const FillCmd *__restrict__ fills,
@@ -647,32 +526,59 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_curve_emit_w(const z2d_n
                                                                      DEdge *__restrict__ edges,
                                                                      const int32_t *__restrict__ curves,
                                                                      const int32_t *__restrict__ counters,
-                                                                     const uint16_t *__restrict__ item_leaves,
                                                                      const double2 *__restrict__ pool) {
-    __shared__ WarpFrontier frs[kFlattenWarps];
+    constexpr uint32_t all = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WarpFrontier &fr = frs[w];
-    const int32_t n = counters[CNT_CURVES_EMIT];
-    for (int32_t q = blockIdx.x * kFlattenWarps + w; q < n; q += gridDim.x * kFlattenWarps) {
-        const int32_t i = curves[q];
-        const NodeInfo inf = info[i];
-        const int32_t f = node_fill[i];
-        const FillCmd &F = fills[f];
-        DEdge *out = edges + st[f].edge_base + inf.edge_off;
-        double et = 0, eb = 0, el = 0, er = 0;
-        bool any = false;
-        if (inf.pool >= 0) {  // the count pass kept the polyline: edge k joins points k and k + 1
-            const double2 *P = pool + inf.pool;
-            for (int32_t k = lane; k < inf.n_emit; k += 32) {
-                const double2 a = P[k], b = P[k + 1];
-                add_edge(F, out + k, a.x, a.y, b.x, b.y, et, eb, el, er, any);
+    const int32_t n = counters[CNT_CURVES_EMIT], warps = gridDim.x * kFlattenWarps;
+    const int32_t per = max(1, min(32, (n + warps - 1) / warps));
+    for (int32_t q0 = (blockIdx.x * kFlattenWarps + w) * per; q0 < n; q0 += warps * per) {
+        int32_t i = -1, f = -1, cnt = 0, src = 0;
+        long long dst = 0;
+        if (lane < per && q0 + lane < n) {
+            i = curves[q0 + lane];
+            f = node_fill[i];
+            const NodeInfo &inf = info[i];
+            if (inf.pool >= 0) {
+                cnt = inf.n_emit;
+                src = inf.pool;
+                dst = (long long)st[f].edge_base + inf.edge_off;
+                i = -1;
             }
-        } else {
-            const z2d_node nd = nodes[i];
-            curve_emit_warp(F, out, inf, nd.p, item_leaves + (size_t)i * kFrontier, fr, lane, et, eb, el, er, any);
         }
-        merge_extents(st, f, any, et, eb, el, er);
-        __syncwarp();
+        int32_t total;
+        const int32_t excl = group_excl_sum(cnt, lane, 32, total);
+        for (int32_t k0 = 0; k0 < total; k0 += 32) {
+            const int32_t k = k0 + lane;
+            // the last lane whose first edge is <= k owns edge k
+            int own = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const int32_t e = __shfl_sync(all, excl, own + step);
+                if (e <= k) own += step;
+            }
+            const int32_t at = k - __shfl_sync(all, excl, own), of = __shfl_sync(all, f, own);
+            const double2 *P = pool + __shfl_sync(all, src, own) + at;
+            DEdge *out = edges + __shfl_sync(all, dst, own) + at;
+            double et = 0, eb = 0, el = 0, er = 0;
+            bool any = false;
+            if (k < total) {
+                const double2 a = P[0], b = P[1];
+                add_edge(fills[of], out, a.x, a.y, b.x, b.y, et, eb, el, er, any);
+            }
+            merge_extents(st, of, any, et, eb, el, er);
+        }
+        // curves without a polyline, one after the other
+        for (uint32_t m = __ballot_sync(all, i >= 0); m; m &= m - 1) {
+            const int own = __ffs(m) - 1;
+            const int32_t ci = __shfl_sync(all, i, own), cf = __shfl_sync(all, f, own);
+            const NodeInfo inf = info[ci];
+            const z2d_node nd = nodes[ci];
+            double et = 0, eb = 0, el = 0, er = 0;
+            bool any = false;
+            curve_emit_warp(fills[cf], edges + st[cf].edge_base + inf.edge_off, inf, nd.p, lane, et, eb, el, er, any);
+            __syncwarp();
+            merge_extents(st, cf, any, et, eb, el, er);
+        }
     }
 }
 
@@ -1253,18 +1159,19 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     DevJob *d_jobs = reinterpret_cast<DevJob *>(dv + o_jobs);
     int32_t *d_cnt = reinterpret_cast<int32_t *>(dv + o_cnt);
 
-    // node info, then the per-node leaf counts of the curves' frontier items
+    // node info, then the curve queues and the nodes' fills
     const size_t info_bytes = (sizeof(NodeInfo) * (size_t)n_nodes + 255) & ~(size_t)255;
-    const size_t items_bytes = (sizeof(uint16_t) * kFrontier * (size_t)n_nodes + 255) & ~(size_t)255;
     const size_t st_bytes = (sizeof(FillState) * (size_t)n_fills + 255) & ~(size_t)255;
-    if (c.node_info.ensure(info_bytes + items_bytes + 3 * sizeof(int32_t) * (size_t)n_nodes) ||
+    if (c.node_info.ensure(info_bytes + (kCurveClasses + 2) * sizeof(int32_t) * (size_t)n_nodes) ||
         c.fill_state.ensure(st_bytes + sizeof(RasterFill) * (size_t)n_fills))
         return Z2D_ERR_OUT_OF_MEMORY;
     RasterFill *d_rf = reinterpret_cast<RasterFill *>(c.fill_state.as<uint8_t>() + st_bytes);
     NodeInfo *d_info = c.node_info.as<NodeInfo>();
-    uint16_t *d_items = reinterpret_cast<uint16_t *>(c.node_info.as<uint8_t>() + info_bytes);
-    int32_t *d_curves = reinterpret_cast<int32_t *>(c.node_info.as<uint8_t>() + info_bytes + items_bytes);  // 2 queues
-    int32_t *d_nfill = d_curves + 2 * (size_t)n_nodes;
+    // the curves to count, one queue per class, those to emit, then each
+    // node's fill
+    int32_t *d_curves = reinterpret_cast<int32_t *>(c.node_info.as<uint8_t>() + info_bytes);
+    int32_t *d_curves_emit = d_curves + kCurveClasses * (size_t)n_nodes;
+    int32_t *d_nfill = d_curves_emit + (size_t)n_nodes;
     FillState *d_st = c.fill_state.as<FillState>();
     Z2D_CUDA(cudaMemsetAsync(d_st, 0, sizeof(FillState) * (size_t)n_fills, c.stream));
     // each node's fill; nodes no fill owns (stroke commands' nodes, gaps) keep -1
@@ -1294,17 +1201,17 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         (unsigned)std::min<long long>(grid_for(n_nodes, kFlattenWarps), (long long)c.sm_count * curve_res);
     // per curve warp: kScratch leaf points per lane; then the curve pool
     const size_t scratch_pts = (size_t)curve_blocks * kFlattenWarps * 32 * kScratch;
-    // pool capacity: 16 points per node, or what the previous call asked for
+    // pool capacity: 32 points per node, or what the previous call asked for
     const int32_t pool_cap = (int32_t)std::min<long long>(
-        64ll << 20, std::max<long long>({1ll << 20, 16ll * n_nodes, c.pool_demand + c.pool_demand / 4}));
+        64ll << 20, std::max<long long>({1ll << 20, 32ll * n_nodes, c.pool_demand + c.pool_demand / 4}));
     if (c.curve_pool.ensure(sizeof(double2) * (scratch_pts + (size_t)pool_cap))) return Z2D_ERR_OUT_OF_MEMORY;
     double2 *d_scratch = c.curve_pool.as<double2>();
     double2 *d_pool = d_scratch + scratch_pts;
     cudaEvent_t tf = c.timer_begin(c.t_flatten);
     k_node_count_w<<<flat_blocks, 32 * kFlattenWarps, 0, c.stream>>>(d_nodes, d_nfill, d_fills, d_info, n_nodes,
                                                                     d_curves, d_cnt);
-    k_curve_count_w<<<curve_blocks, 32 * kFlattenWarps, 0, c.stream>>>(d_nodes, d_nfill, d_fills, d_info, d_curves,
-                                                                      d_cnt, d_items, d_cnt + CNT_STATUS, d_scratch,
+    k_curve_count_w<<<curve_blocks, 32 * kFlattenWarps, 0, c.stream>>>(d_nodes, d_nfill, d_fills, d_info, n_nodes,
+                                                                      d_curves, d_cnt, d_cnt + CNT_STATUS, d_scratch,
                                                                       d_pool, pool_cap);
     StrokeRun srun;
     if (n_sk > 0) {
@@ -1355,10 +1262,9 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     // extents start at +inf/-inf keys: min slots 0xFF.., max slots 0
     tf = c.timer_begin(c.t_flatten);
     k_node_emit_w<<<flat_blocks, 32 * kFlattenWarps, 0, c.stream>>>(d_nodes, d_nfill, d_fills, d_info, d_st, d_edges,
-                                                                   n_nodes, d_curves + n_nodes, d_cnt);
+                                                                   n_nodes, d_curves_emit, d_cnt);
     k_curve_emit_w<<<curve_blocks, 32 * kFlattenWarps, 0, c.stream>>>(d_nodes, d_nfill, d_fills, d_info, d_st,
-                                                                     d_edges, d_curves + n_nodes, d_cnt, d_items,
-                                                                     d_pool);
+                                                                     d_edges, d_curves_emit, d_cnt, d_pool);
     if (n_sk > 0) {
         const int rc = stroke_emit(c, srun, d_fills, d_st, d_edges);
         if (rc) return rc;

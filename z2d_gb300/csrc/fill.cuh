@@ -43,9 +43,7 @@ struct NodeInfo {
     int32_t n_emit; // edges emitted (one per lineTo the reference issues)
     int32_t n_added;
     int32_t edge_off;
-    int32_t chords; // curve whose edges are its subdivision leaves' chords (see k_node_emit_w)
-    int32_t pool;   // first of its leaves' points in the curve pool, or -1 (see k_curve_count_w)
-    int32_t _pad;
+    int32_t pool;   // first of its polyline's points in the curve pool, or -1 (see k_curve_count_w)
 };
 
 // Polygon.Edge plus its rounded active range: the edge is active on sample
@@ -209,11 +207,11 @@ enum : int32_t {
     CNT_MASK_LO = 2,  // + CNT_MASK_HI = 3
     CNT_EXACT = 4,
     CNT_STATUS = 5,
-    CNT_CURVES = 6,       // curves queued by k_node_count_w
-    CNT_CURVES_EMIT = 7,  // curves queued by k_node_emit_w
-    CNT_POOL = 8,         // points asked of the curve pool (64-bit pair, + 9)
-    CNT_QUEUE = 10,       // k_raster's work-queue counter (64-bit pair, + 11)
-    CNT_COUNT = 12
+    CNT_CURVES = 6,       // curves queued by k_node_count_w, per class (6 slots)
+    CNT_CURVES_EMIT = 12, // curves queued by k_node_emit_w
+    CNT_POOL = 14,        // points asked of the curve pool (64-bit pair, + 15)
+    CNT_QUEUE = 16,       // k_raster's work-queue counter (64-bit pair, + 17)
+    CNT_COUNT = 18
 };
 
 // action-mask byte of the exact path: bit 7 = clear first, bits 0-4 = coverage

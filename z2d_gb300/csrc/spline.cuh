@@ -230,10 +230,79 @@ static __device__ __noinline__ Knots de_casteljau(Knots &k) {
     return r;
 }
 
-// Depth-first subdivision (Spline.decomposeInto, Spline.zig:56-71) with an
-// explicit stack.  Calls emit(x, y) for every lineTo the reference issues,
-// including the final lineTo(d).  Returns false if the stack would overflow
-// (coordinates are bounded, so this does not happen for valid input).
+// Depth-first walk of a subtree (Spline.decomposeInto, Spline.zig:56-71)
+// with an explicit stack: leaf(k) for every subcurve that decomposeInto stops
+// at, in order.  `open` counts the pending second halves above the subtree,
+// so the stack bound is the whole curve's.  False if the stack would overflow
+// (coordinates are bounded, so this does not happen for valid input) or the
+// subtree does not end within kSplineMaxSplits tests.
+template <class L>
+__device__ __forceinline__ bool walk_leaves(const Knots &k0, bool is_leaf, int open, const Tol &tol, L &&leaf) {
+    if (is_leaf) {
+        leaf(k0);
+        return true;
+    }
+    Knots stack[kSplineStack];
+    int sp = 0;
+    int32_t budget = kSplineMaxSplits;  // bounds the walk even for pathological input
+    Knots k = k0;
+    while (true) {
+        if (--budget < 0) return false;
+        if (below_tol(k, tol)) {
+            leaf(k);
+            if (sp == 0) return true;
+            k = stack[--sp];
+            continue;
+        }
+        if (sp + open >= kSplineStack) return false;  // cannot recurse deeper
+        stack[sp++] = de_casteljau(k);                 // processed after the first half
+    }
+}
+
+// A curve's subdivision tree shared by 2^g neighbouring lanes: lane j
+// walks the subtree that the bits of j lead to (first level in the highest
+// bit, 0 for the first half), so the lanes' leaves, lane after lane, are the
+// curve's in order.  A leaf above level g belongs to the lane whose
+// remaining bits are 0.  Each lane goes down from the root by itself (g tests
+// and splits, without shared memory or exchange), which costs less than
+// one leaf per level.
+__device__ __forceinline__ bool lane_subtree(Knots &k, int g, int j, const Tol &tol, bool &is_leaf, int &open) {
+    is_leaf = false;
+    open = 0;
+    for (int l = g - 1; l >= 0; l--) {
+        if (below_tol(k, tol)) {
+            is_leaf = true;
+            return (j & ((2 << l) - 1)) == 0;
+        }
+        const Knots second = de_casteljau(k);
+        if ((j >> l) & 1) k = second;
+        else open++;
+    }
+    return true;
+}
+
+// A curve's length class, from a rough count of its leaves: halving divides
+// the second differences a - 2b + c and b - 2c + d by 4, so about
+// 2^k = (|second difference| / tolerance)^(1/2) leaves are left.  Class 0 is
+// k <= 3, then one class per k, class 5 k >= 8.
+constexpr int kCurveClasses = 6;
+__device__ __forceinline__ int curve_class(double ax, double ay, const double *p, double tol) {
+    float x[4], y[4], t;
+    bool ok = f32_trunc(ax, x[0]) && f32_trunc(ay, y[0]) && f32_trunc(tol, t);
+#pragma unroll
+    for (int i = 0; i < 3; i++) ok = ok && f32_trunc(p[2 * i], x[i + 1]) && f32_trunc(p[2 * i + 1], y[i + 1]);
+    if (!ok) return kCurveClasses - 1;
+    const float x1 = x[0] - 2.0f * x[1] + x[2], y1 = y[0] - 2.0f * y[1] + y[2];
+    const float x2 = x[1] - 2.0f * x[2] + x[3], y2 = y[1] - 2.0f * y[2] + y[3];
+    const float d = fmaxf(x1 * x1 + y1 * y1, x2 * x2 + y2 * y2);
+    float bound = 4096.0f * (t * t);  // 16^3 t^2
+    int c = 0;
+    for (; c < kCurveClasses - 1 && !(d <= bound); c++) bound *= 16.0f;
+    return c;
+}
+
+// Depth-first subdivision of one curve by one thread.  Calls emit(x, y) for
+// every lineTo the reference issues, including the final lineTo(d).
 template <class F>
 __device__ __forceinline__ bool spline_walk(double ax, double ay, const double *p, double tol, F &&emit) {
     const double bx = p[0], by = p[1], cx = p[2], cy = p[3], dx = p[4], dy = p[5];
@@ -241,31 +310,9 @@ __device__ __forceinline__ bool spline_walk(double ax, double ay, const double *
         emit(dx, dy);
         return true;
     }
-    const Tol t = make_tol(tol);
-    Knots stack[kSplineStack];
-    int sp = 0;
-    stack[sp++] = Knots{ax, ay, bx, by, cx, cy, dx, dy};
-    bool ok = true;
-    int32_t budget = kSplineMaxSplits;  // bounds the walk even for pathological input
-    while (sp > 0 && ok) {
-        Knots k = stack[--sp];
-        while (true) {
-            if (--budget < 0) {
-                ok = false;
-                break;
-            }
-            if (below_tol(k, t)) {
-                if (!pt_eq(k.ax, k.ay, ax, ay)) emit(k.ax, k.ay);
-                break;
-            }
-            const Knots second = de_casteljau(k);
-            if (sp >= kSplineStack) {  // cannot recurse deeper: give up on this branch
-                ok = false;
-                break;
-            }
-            stack[sp++] = second;  // processed after the first half
-        }
-    }
+    const bool ok = walk_leaves(Knots{ax, ay, bx, by, cx, cy, dx, dy}, false, 0, make_tol(tol), [&](const Knots &k) {
+        if (!pt_eq(k.ax, k.ay, ax, ay)) emit(k.ax, k.ay);
+    });
     emit(dx, dy);
     return ok;
 }

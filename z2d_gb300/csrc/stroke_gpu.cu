@@ -12,6 +12,8 @@
 // host builder; the curve subdivision is spline.cuh, shared with fills.
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "edges.cuh"
 #include "spline.cuh"
@@ -44,7 +46,8 @@ struct StrokeTot {
 
 // device pointers of one run
 struct State {
-    long long *raw_cnt, *raw_off;   // n_local + 1
+    long long *raw_cnt, *raw_off;   // (n_local << g) + 1
+    int g;                          // log2 of the lanes that share a node
     PenVertex *pen;                 // n_pen
     SubState *sub;                  // n_subs
     StrokeTot *tot;                 // n_strokes
@@ -53,7 +56,7 @@ struct State {
     double2 *raw_pt;
     int32_t *raw_sub;
     uint8_t *raw_mode;
-    int32_t *keep, *kept_off;       // R + 1
+    int32_t *kept_off;              // R + 1
     double2 *q_pt;
     int32_t *q_sub;
     uint8_t *q_mode;
@@ -106,90 +109,114 @@ __global__ void ks_local_sub(const SubpathDev *__restrict__ subs, int32_t n_subs
 
 // The points one node hands to the plotter: move_to its point, line_to its
 // end, curve_to Spline.decompose's lineTo calls (stroke_plotter.zig:126-150).
+// 2^g neighbouring lanes share a node: a curve's subdivision tree as in
+// lane_subtree (one thread walking a curve of 500 leaves took 0.68 ms, most
+// of a single stroke's call; 32 lanes take 0.03), the other nodes' point is
+// lane 0's.  emit(x, y) is called for the lane's points in order; false if
+// the subdivision gave up.
 template <class Emit>
-__device__ __forceinline__ bool node_points(const z2d_node *__restrict__ nodes, const SubpathDev &S, int32_t j,
-                                           double tol, Emit &&emit) {
-    const z2d_node nd = nodes[S.node0 + j];
-    if (j == 0 || nd.tag == Z2D_LINE_TO) {
-        emit(nd.p[0], nd.p[1]);
+__device__ __forceinline__ bool node_points(const z2d_node *__restrict__ nodes, const SubpathDev &S, int32_t n, int g,
+                                           int j, double tol, Emit &&emit) {
+    const z2d_node nd = nodes[S.node0 + n];
+    if (n == 0 || nd.tag == Z2D_LINE_TO) {
+        if (j == 0) emit(nd.p[0], nd.p[1]);
         return true;
     }
-    const Pt a = node_end(nodes[S.node0 + j - 1]);
-    return spline_walk(a.x, a.y, nd.p, tol, emit);
+    const Pt a = node_end(nodes[S.node0 + n - 1]);
+    const double *p = nd.p;
+    const int last = (1 << g) - 1;
+    bool ok = true;
+    if (!(pt_eq(a.x, a.y, p[0], p[1]) && pt_eq(p[2], p[3], p[4], p[5]))) {  // Spline.zig:39-42
+        const Tol t = make_tol(tol);
+        Knots k{a.x, a.y, p[0], p[1], p[2], p[3], p[4], p[5]};
+        bool is_leaf;
+        int open;
+        if (lane_subtree(k, g, j, t, is_leaf, open))
+            ok = walk_leaves(k, is_leaf, open, t, [&](const Knots &q) {
+                if (!pt_eq(q.ax, q.ay, a.x, a.y)) emit(q.ax, q.ay);
+            });
+    }
+    if (j == last) emit(p[4], p[5]);
+    return ok;
 }
 
+// Points per (node, lane), node after node.
 __global__ void ks_raw_count(const z2d_node *__restrict__ nodes, const SubpathDev *__restrict__ subs,
                              const int32_t *__restrict__ local_sub, const StrokeDev *__restrict__ strokes,
-                             long long n_local, long long *__restrict__ raw_cnt, int32_t *__restrict__ status) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n_local) return;
-    if (i == n_local) {
-        raw_cnt[i] = 0;
+                             long long n_local, int g, long long *__restrict__ raw_cnt, int32_t *__restrict__ status) {
+    const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = at >> g;
+    if (i >= n_local) {
+        if (at == n_local << g) raw_cnt[at] = 0;
         return;
     }
-    const int32_t sp = local_sub[i];
-    const SubpathDev S = subs[sp];
+    const SubpathDev S = subs[local_sub[i]];
     int32_t cnt = 0;
-    if (!node_points(nodes, S, (int32_t)(i - S.local0), strokes[S.stroke].tolerance, [&](double, double) { cnt++; }))
+    if (!node_points(nodes, S, (int32_t)(i - S.local0), g, (int)(at & ((1 << g) - 1)), strokes[S.stroke].tolerance,
+                     [&](double, double) { cnt++; }))
         atomicExch(status, Z2D_ERR_INVALID_STATE);
-    raw_cnt[i] = cnt;
+    raw_cnt[at] = cnt;
 }
 
 __global__ void ks_raw_emit(const z2d_node *__restrict__ nodes, const SubpathDev *__restrict__ subs,
                             const int32_t *__restrict__ local_sub, const StrokeDev *__restrict__ strokes,
-                            long long n_local, const long long *__restrict__ raw_off, long long n_raw,
+                            long long n_local, int g, const long long *__restrict__ raw_off,
                             double2 *__restrict__ raw_pt, int32_t *__restrict__ raw_sub,
-                            uint8_t *__restrict__ raw_mode, int32_t *__restrict__ keep) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_local) {
-        if (i == n_local) keep[n_raw] = 0;
-        return;
-    }
+                            uint8_t *__restrict__ raw_mode) {
+    const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = at >> g;
+    if (i >= n_local) return;
+    long long r = raw_off[at];
+    const long long r_end = raw_off[at + 1];
+    if (r == r_end) return;
     const int32_t sp = local_sub[i];
     const SubpathDev S = subs[sp];
-    const int32_t j = (int32_t)(i - S.local0);
+    const int32_t n = (int32_t)(i - S.local0);
     const StrokeDev &T = strokes[S.stroke];
-    const z2d_node nd = nodes[S.node0 + j];
-    // the previous point the plotter saw, for the degenerate-node check
-    Pt prev = j == 0 ? Pt{nd.p[0], nd.p[1]} : node_end(nodes[S.node0 + j - 1]);
-    const uint8_t mode = (j > 0 && nd.tag == Z2D_CURVE_TO) ? (uint8_t)Z2D_JOIN_ROUND : (uint8_t)T.join;
-    long long r = raw_off[i];
-    const long long r_end = raw_off[i + 1];
-    bool first = true;
-    node_points(nodes, S, j, T.tolerance, [&](double x, double y) {
+    const uint8_t mode =
+        (n > 0 && nodes[S.node0 + n].tag == Z2D_CURVE_TO) ? (uint8_t)Z2D_JOIN_ROUND : (uint8_t)T.join;
+    node_points(nodes, S, n, g, (int)(at & ((1 << g) - 1)), T.tolerance, [&](double x, double y) {
         if (r < r_end) {
             raw_pt[r] = make_double2(x, y);
             raw_sub[r] = sp;
             raw_mode[r] = mode;
-            keep[r] = (j == 0 && first) ? 1 : !sg::eq(Pt{x, y}, prev);
         }
-        first = false;
-        prev = Pt{x, y};
         r++;
     });
 }
 
-__global__ void ks_compact(const double2 *__restrict__ raw_pt, const int32_t *__restrict__ raw_sub,
-                           const uint8_t *__restrict__ raw_mode, const int32_t *__restrict__ keep,
-                           const int32_t *__restrict__ kept_off, long long n_raw, double2 *__restrict__ q_pt,
+// Whether the plotter keeps raw point r: the degenerate-node check against
+// the point before it of the same subpath.
+struct Keep {
+    const double2 *pt;
+    const int32_t *sub;
+    long long n;
+    __host__ __device__ __forceinline__ int32_t operator()(long long r) const {
+        if (r >= n) return 0;
+        if (r == 0 || sub[r] != sub[r - 1]) return 1;
+        const double2 a = pt[r - 1], b = pt[r];
+        return pt_eq(a.x, a.y, b.x, b.y) ? 0 : 1;
+    }
+};
+
+__global__ void ks_compact(const Keep keep, const uint8_t *__restrict__ raw_mode,
+                           const int32_t *__restrict__ kept_off, double2 *__restrict__ q_pt,
                            int32_t *__restrict__ q_sub, uint8_t *__restrict__ q_mode) {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_raw || !keep[r]) return;
+    if (r >= keep.n || !keep(r)) return;
     const int32_t q = kept_off[r];
-    q_pt[q] = raw_pt[r];
-    q_sub[q] = raw_sub[r];
+    q_pt[q] = keep.pt[r];
+    q_sub[q] = keep.sub[r];
     q_mode[q] = raw_mode[r];
 }
 
 // close_path / finish of the plotter (stroke_plotter.zig:152-230): what a
 // subpath of n kept points draws.
 __global__ void ks_sub_setup(const SubpathDev *__restrict__ subs, int32_t n_subs, const StrokeDev *__restrict__ strokes,
-                             const long long *__restrict__ raw_off, const int32_t *__restrict__ kept_off,
+                             int g, const long long *__restrict__ raw_off, const int32_t *__restrict__ kept_off,
                              const double2 *__restrict__ q_pt, SubState *__restrict__ sub) {
     const int32_t sp = blockIdx.x * blockDim.x + threadIdx.x;
     if (sp >= n_subs) return;
     const SubpathDev S = subs[sp];
-    const long long r0 = raw_off[S.local0], r1 = raw_off[S.local0 + S.n_nodes];
+    const long long r0 = raw_off[S.local0 << g], r1 = raw_off[(S.local0 + S.n_nodes) << g];
     SubState st;
     st.q0 = kept_off[r0];
     st.n = kept_off[r1] - st.q0;
@@ -619,7 +646,10 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     constexpr int T = 128;
     // ---- buffers known before counting
     Carve ca;
-    const size_t o_cnt = ca.take<long long>(run.n_local + 1), o_off = ca.take<long long>(run.n_local + 1);
+    // a warp per node while the device has room for all of them, else 8 lanes
+    st.g = run.n_local * 32 <= (long long)c.sm_count * 2048 ? 5 : 3;
+    const long long n_lanes = run.n_local << st.g;
+    const size_t o_cnt = ca.take<long long>(n_lanes + 1), o_off = ca.take<long long>(n_lanes + 1);
     const size_t o_lsub = ca.take<int32_t>(run.n_local + 1), o_pen = ca.take<PenVertex>(run.n_pen + 1);
     const size_t o_sub = ca.take<SubState>(run.n_subs + 1), o_tot = ca.take<StrokeTot>(run.n_strokes + 1);
     const size_t o_edges = ca.take<int32_t>(run.n_strokes + 1), o_totals = ca.take<long long>(2);
@@ -637,17 +667,17 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     cudaEvent_t ts = c.timer_begin(c.t_stroke);
     ks_pen<<<blocks_for(run.n_strokes, T), T, 0, c.stream>>>(run.strokes, run.n_strokes, run.trig, st.pen);
     ks_local_sub<<<blocks_for(run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, local_sub);
-    ks_raw_count<<<blocks_for(run.n_local + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes,
-                                                                      run.n_local, st.raw_cnt, d_status);
+    ks_raw_count<<<blocks_for(n_lanes + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes,
+                                                                  run.n_local, st.g, st.raw_cnt, d_status);
     size_t tmp = 0;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, st.raw_cnt, st.raw_off, run.n_local + 1, c.stream));
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, st.raw_cnt, st.raw_off, n_lanes + 1, c.stream));
     if (c.scan_tmp.ensure(tmp + 16)) return Z2D_ERR_OUT_OF_MEMORY;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, tmp, st.raw_cnt, st.raw_off, run.n_local + 1, c.stream));
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, tmp, st.raw_cnt, st.raw_off, n_lanes + 1, c.stream));
     c.launches += 4;
     long long *rb = nullptr;
     if (c.readback.ensure(64)) return Z2D_ERR_OUT_OF_MEMORY;
     rb = c.readback.as<long long>();
-    Z2D_CUDA(cudaMemcpyAsync(rb, st.raw_off + run.n_local, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
+    Z2D_CUDA(cudaMemcpyAsync(rb, st.raw_off + n_lanes, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
     Z2D_CUDA(cudaStreamSynchronize(c.stream));
     const long long R = rb[0];
     if (R < 0 || R >= 0x7FFFFFFFll) {
@@ -658,7 +688,7 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     // ---- buffers sized by the point count
     Carve cb;
     const size_t o_rpt = cb.take<double2>(R + 1), o_rsub = cb.take<int32_t>(R + 1), o_rmode = cb.take<uint8_t>(R + 1);
-    const size_t o_keep = cb.take<int32_t>(R + 1), o_kept = cb.take<int32_t>(R + 1);
+    const size_t o_kept = cb.take<int32_t>(R + 1);
     const size_t o_qpt = cb.take<double2>(R + 1), o_qsub = cb.take<int32_t>(R + 1), o_qmode = cb.take<uint8_t>(R + 1);
     const size_t o_ca = cb.take<long long>(R + 1), o_cb = cb.take<long long>(R + 1);
     const size_t o_oa = cb.take<long long>(R + 1), o_ob = cb.take<long long>(R + 1);
@@ -667,7 +697,6 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     st.raw_pt = reinterpret_cast<double2 *>(B + o_rpt);
     st.raw_sub = reinterpret_cast<int32_t *>(B + o_rsub);
     st.raw_mode = B + o_rmode;
-    st.keep = reinterpret_cast<int32_t *>(B + o_keep);
     st.kept_off = reinterpret_cast<int32_t *>(B + o_kept);
     st.q_pt = reinterpret_cast<double2 *>(B + o_qpt);
     st.q_sub = reinterpret_cast<int32_t *>(B + o_qsub);
@@ -677,17 +706,17 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     st.off_a = reinterpret_cast<long long *>(B + o_oa);
     st.off_b = reinterpret_cast<long long *>(B + o_ob);
 
-    ks_raw_emit<<<blocks_for(run.n_local + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes,
-                                                                     run.n_local, st.raw_off, R, st.raw_pt, st.raw_sub,
-                                                                     st.raw_mode, st.keep);
+    ks_raw_emit<<<blocks_for(n_lanes + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes, run.n_local,
+                                                            st.g, st.raw_off, st.raw_pt, st.raw_sub, st.raw_mode);
+    const Keep keep{st.raw_pt, st.raw_sub, R};
+    const auto kept = thrust::make_transform_iterator(thrust::make_counting_iterator(0ll), keep);
     size_t t1 = 0, t2 = 0;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, st.keep, st.kept_off, R + 1, c.stream));
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, kept, st.kept_off, R + 1, c.stream));
     Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, st.cnt_a, st.off_a, R + 1, c.stream));
     if (c.scan_tmp.ensure(std::max(t1, t2) + 16)) return Z2D_ERR_OUT_OF_MEMORY;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t1, st.keep, st.kept_off, R + 1, c.stream));
-    ks_compact<<<blocks_for(R, T), T, 0, c.stream>>>(st.raw_pt, st.raw_sub, st.raw_mode, st.keep, st.kept_off, R,
-                                                      st.q_pt, st.q_sub, st.q_mode);
-    ks_sub_setup<<<blocks_for(run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, run.strokes, st.raw_off,
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t1, kept, st.kept_off, R + 1, c.stream));
+    ks_compact<<<blocks_for(R, T), T, 0, c.stream>>>(keep, st.raw_mode, st.kept_off, st.q_pt, st.q_sub, st.q_mode);
+    ks_sub_setup<<<blocks_for(run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, run.strokes, st.g, st.raw_off,
                                                                  st.kept_off, st.q_pt, st.sub);
     ks_elem_count<<<blocks_for(R + 1, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.q_pt, st.q_sub,
                                                              st.q_mode, st.kept_off, R, st.cnt_a, st.cnt_b);
