@@ -568,6 +568,8 @@ static int prepare_fill(const z2d_surface &s, int32_t job, const z2d_node *nodes
         F.px_paint = convert_px(px, s.format);
         F.px_rgba = to_i16(convert_px(px, Z2D_FORMAT_RGBA));
         if (F.op == Z2D_OP_SRC_OVER && F.precision == Z2D_PRECISION_INTEGER) F.fast_kind = FAST_PIXEL_SRC_OVER;
+    } else if (F.op == Z2D_OP_SRC_OVER && F.precision == Z2D_PRECISION_INTEGER) {
+        F.fast_kind = FAST_SOURCE_SRC_OVER;
     }
     return Z2D_OK;
 }

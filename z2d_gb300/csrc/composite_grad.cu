@@ -7,11 +7,10 @@
 // calls and run-time dispatch on every level (source kind, gradient kind,
 // interpolation method, operator); here the gradient kind, the
 // interpolation space and the presence of a dither are template parameters
-// and everything is inlined, so a pixel is the offset (grad_fast.cuh, f64
-// only where its rounding is undecided), the stop search, the
-// interpolation and the two operators.  Each thread owns 16-byte chunks of
-// destination (4 pixels) and the matching 4 mask bytes; pixel coordinates
-// advance with the grid stride instead of being divided out per chunk.
+// and everything is inlined, so a pixel is its lanes in f32 (grad_f32.cuh;
+// where they are undecided, the double-word or f64 offset and the exact
+// colour) and the two operators.  Pixel coordinates advance with
+// the grid stride instead of being divided out per pixel.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -25,14 +24,6 @@ namespace {
 constexpr int kGradThreads = 256;
 
 enum : int { kLinRGB = 0, kSRGB = 1, kHSL = 2 };
-
-// Out of line: the f64 offsets (taken for a pixel in thousands) and
-// std.math.pow (three per sRGB pixel), so that each instantiation's loop
-// stays small enough for the instruction cache.
-__device__ __noinline__ float offset_f64_call(const DevGradient &g, int32_t x, int32_t y) {
-    return grad_offset_f64(g, x, y);
-}
-__device__ __noinline__ float gamma_call(float x) { return zpow(x, kGamma); }
 
 template <int KIND>
 __device__ __forceinline__ float offset_inline(const DevGradient &g, int32_t x, int32_t y) {
@@ -65,15 +56,10 @@ __device__ __forceinline__ float offset_of(const DevGradient &g, int32_t x, int3
     if constexpr (KIND == Z2D_GRADIENT_LINEAR) return offset_inline<KIND>(g, x, y);
     else return offset_call<KIND>(g, x, y);
 }
-// HSL.interpolate + toLinearRGB, out of line (fmod and the hue cases)
-__device__ __noinline__ RGBf hsl_call(RGBf a, RGBf b, float t, int method) {
-    return hsl_to_rgb(hsl_lerp_demul(a, b, t, method));
-}
-
 // The source's colour lanes at (x, y): interpolateEncode, or the dithered
 // linear colour encoded (Dither.getPixel)
 template <int KIND, int METHOD, bool DITH>
-__device__ __forceinline__ I16 grad_lanes(const DevSrc &s, const DevGradient &g, int32_t x, int32_t y) {
+__device__ __noinline__ I16 grad_lanes_exact(const DevSrc &s, const DevGradient &g, int32_t x, int32_t y) {
     const Search r = grad_search(g, offset_of<KIND>(g, x, y));
     const RGBf a = stop_prep(g, r.i0), b = stop_prep(g, r.i1);
     // (SRGB.interpolate then toLinearRGB, as interp_encode_prep /
@@ -104,42 +90,77 @@ __device__ __forceinline__ I16 grad_lanes(const DevSrc &s, const DevGradient &g,
     }
 }
 
+// The batch's second half for one pixel: dst_in(source lanes, mask), then the
+// operator on the destination word.
+__device__ __forceinline__ uint32_t grad_composite(int op, uint32_t w, I16 sl, uint32_t m8, int fmt) {
+    if (op == Z2D_OP_SRC_OVER) {  // two channels per 32-bit operation
+        const uint32_t L = i16_to_word(sl, word_order(fmt));
+        const uint32_t e = div255x2((L & 0x00FF00FFu) * m8), o = div255x2(((L >> 8) & 0x00FF00FFu) * m8);
+        return word_src_over(w, e | (o << 8), fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB);
+    }
+    // IntegerOps.dstIn(d = source, s = mask), then the operator
+    const I16 rl = int_op(Z2D_OP_DST_IN, sl, I16{0u, 0u, 0u, m8});
+    return i16_to_word(int_op_any(op, word_to_i16(w, fmt), rl), fmt);
+}
+
+// A lane takes a pixel at a time (32 neighbours per warp: coalesced, and the
+// body, a few hundred instructions, is compiled once); the pixels whose lanes
+// f32 does not decide (grad_f32.cuh) go to the warp's list, 32 of which are
+// evaluated exactly at a time: the exact evaluation, several times as long,
+// then never runs for one lane with 31 waiting.
 template <int KIND, int METHOD, bool DITH>
 __global__ void __launch_bounds__(kGradThreads) k_mask_grad(uint8_t *__restrict__ dst, const uint8_t *__restrict__ mask,
-                                                           int32_t W, size_t n_chunks, int32_t fmt, int32_t op,
+                                                           int32_t W, size_t n_px, int32_t fmt, int32_t op,
                                                            const DevSrc src) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    __shared__ unsigned long long lists[kGradThreads / 32][64];
+    const int lane = threadIdx.x & 31;
+    unsigned long long *list = lists[threadIdx.x >> 5];
     const DevGradient &g = *src.grad;
+    uint32_t *dw = reinterpret_cast<uint32_t *>(dst);
+    const int method = METHOD == kLinRGB ? Z2D_INTERP_LINEAR_RGB : METHOD == kSRGB ? Z2D_INTERP_SRGB : src.grad_method;
+    const int dither = DITH ? src.dither_type : Z2D_DITHER_NONE;
+    const float step = DITH ? dither_step_of(src.dither_scale) : 0.0f;
     const size_t first = (size_t)blockIdx.x * kGradThreads + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * kGradThreads;
-    // (x, y) of the first pixel of this thread's first chunk, then advanced
-    // by the stride (4 * stride pixels: q rows and r columns)
-    const size_t p0 = first * 4, sp = stride * 4;
-    int32_t y = (int32_t)(p0 / (size_t)W), x = (int32_t)(p0 - (size_t)y * W);
-    const int32_t q = (int32_t)(sp / (size_t)W), rr = (int32_t)(sp - (size_t)q * W);
-    for (size_t c = first; c < n_chunks; c += stride) {
-        uint4 v = reinterpret_cast<const uint4 *>(dst)[c];
-        const uint32_t mw = __ldcs(reinterpret_cast<const uint32_t *>(mask) + c);
-        uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        int32_t px = x, py = y;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const I16 sl = grad_lanes<KIND, METHOD, DITH>(src, g, px, py);
-            // IntegerOps.dstIn(d = source, s = mask), then the operator
-            const I16 rl = int_op(Z2D_OP_DST_IN, sl, I16{0u, 0u, 0u, (mw >> (8 * j)) & 0xFFu});
-            w[j] = i16_to_word(int_op_any(op, word_to_i16(w[j], fmt), rl), fmt);
-            if (++px == W) {
-                px = 0;
-                py++;
-            }
+    // (x, y) of this thread's first pixel, then advanced by the stride
+    // (q rows and r columns)
+    int32_t y = (int32_t)(first / (size_t)W), x = (int32_t)(first - (size_t)y * W);
+    const int32_t q = (int32_t)(stride / (size_t)W), r = (int32_t)(stride - (size_t)q * W);
+    int n = 0;  // pixels in the list
+    auto exact = [&](int at) {
+        const size_t p = (size_t)list[at];
+        const int32_t py = (int32_t)(p / (size_t)W), px = (int32_t)(p - (size_t)py * W);
+        dw[p] = grad_composite(op, dw[p], grad_lanes_exact<KIND, METHOD, DITH>(src, g, px, py), mask[p], fmt);
+    };
+#pragma unroll 1
+    for (size_t p0 = first - lane; p0 < n_px; p0 += stride) {
+        const size_t p = p0 + lane;
+        bool late = false;
+        if (p < n_px) {
+            const uint32_t w = dw[p], m8 = __ldcs(mask + p);
+            I16 sl;
+            if (grad_lanes_f32(KIND, method, dither, step, g, x, y, sl)) dw[p] = grad_composite(op, w, sl, m8, fmt);
+            else late = true;
         }
-        reinterpret_cast<uint4 *>(dst)[c] = make_uint4(w[0], w[1], w[2], w[3]);
-        x += rr;
+        const uint32_t m = __ballot_sync(kAll, late);
+        if (late) list[n + __popc(m & ((1u << lane) - 1u))] = p;
+        n += __popc(m);
+        if (n >= 32) {
+            __syncwarp();
+            n -= 32;
+            exact(n + lane);
+            __syncwarp();
+        }
+        x += r;
         y += q;
         if (x >= W) {
             x -= W;
             y++;
         }
     }
+    __syncwarp();
+    if (lane < n) exact(lane);
 }
 
 using GradKernel = void (*)(uint8_t *, const uint8_t *, int32_t, size_t, int32_t, int32_t, const DevSrc);
@@ -177,10 +198,8 @@ bool try_mask_grad(Ctx &c, const CompJob &J, bool flat) {
     }
     if (!s.grad || J.dst.fmt > Z2D_FORMAT_RGBA || o1.op < 0 || o1.op >= Z2D_OP_COUNT) return false;
     if (o0.src.sfc.fmt != Z2D_FORMAT_ALPHA8 || o0.src.sfc.w != J.dst.w || o0.src.sfc.h < J.dst.h) return false;
-    if ((reinterpret_cast<uintptr_t>(o0.src.sfc.data) & 3) != 0 || (reinterpret_cast<uintptr_t>(J.dst.data) & 15) != 0)
-        return false;
+    if ((reinterpret_cast<uintptr_t>(J.dst.data) & 3) != 0) return false;
     const size_t px = (size_t)J.dst.w * J.dst.h;
-    if (px % 4 != 0) return false;
     const int kind = s.grad_type, method = s.grad_method;
     if (kind < Z2D_GRADIENT_LINEAR || kind > Z2D_GRADIENT_CONIC) return false;
     GradKernel k = kind == Z2D_GRADIENT_LINEAR   ? pick_method<Z2D_GRADIENT_LINEAR>(method, dith)
@@ -193,12 +212,11 @@ bool try_mask_grad(Ctx &c, const CompJob &J, bool flat) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kGradThreads, 0) != cudaSuccess || occ <= 0) occ = 1;
         slot.store(occ, std::memory_order_relaxed);
     }
-    const size_t n_chunks = px / 4;
-    size_t blocks = (n_chunks + kGradThreads - 1) / kGradThreads;
+    size_t blocks = (px + kGradThreads - 1) / kGradThreads;
     const size_t cap = (size_t)c.sm_count * (size_t)occ;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) return true;
-    k<<<(unsigned)blocks, kGradThreads, 0, c.stream>>>(J.dst.data, o0.src.sfc.data, J.dst.w, n_chunks, J.dst.fmt, o1.op,
+    k<<<(unsigned)blocks, kGradThreads, 0, c.stream>>>(J.dst.data, o0.src.sfc.data, J.dst.w, px, J.dst.fmt, o1.op,
                                                       s);
     c.launches++;
     return true;

@@ -158,7 +158,8 @@ Z2D_HD bool crossing_f32(float fx, float fxi, float t, float limit, int32_t &n) 
 
 enum : int32_t {
     FAST_NONE = 0,
-    FAST_PIXEL_SRC_OVER = 1,  // pixel pattern, integer precision, src_over
+    FAST_PIXEL_SRC_OVER = 1,   // pixel pattern, integer precision, src_over
+    FAST_SOURCE_SRC_OVER = 2,  // gradient or dither pattern, integer precision, src_over
 };
 
 enum : int32_t {

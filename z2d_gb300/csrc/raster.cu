@@ -34,6 +34,14 @@ static __device__ __noinline__ I16 apply_ssaa(const FillCmd &F, int32_t x, int32
     return encode_raw(float_op_any(F.op, decode_raw(d), r));
 }
 
+// The source word (word_order) of a pixel of a FAST_SOURCE_SRC_OVER fill with
+// `opacity`: dst_in(pattern, opacity), the pattern itself at 255 (where
+// dst_in changes nothing).
+__device__ __forceinline__ uint32_t source_word(I16 s, uint32_t opacity, int fmt) {
+    const uint32_t L = i16_to_word(s, word_order(fmt));
+    return div255x2((L & 0x00FF00FFu) * opacity) | (div255x2(((L >> 8) & 0x00FF00FFu) * opacity) << 8);
+}
+
 // multisample.run's clears for unbounded operators (multisample.zig:96-110),
 // including its quirks: the rows below the draw box are cleared up to the
 // surface WIDTH, and the right-hand clear starts at x = 0.
@@ -108,6 +116,13 @@ __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const
     return R;
 }
 
+// The reference's evaluation, out of line: needed for one crossing in
+// thousands, and four copies of it in the crossing loop would be most of the
+// loop's code.
+static __device__ __noinline__ int32_t crossing_f64(const DEdge *__restrict__ e, int32_t sr) {
+    return (int32_t)round(e->x_start + (e->x_inc * (((double)sr + 0.5) - e->top)));
+}
+
 // Sample column, relative to the tile's first, where edge R crosses sample
 // row sub0 + r (r one of R.rows).
 __device__ __forceinline__ int32_t edge_crossing(const DEdge *__restrict__ edges, const RowEdge &R, int32_t r,
@@ -115,8 +130,7 @@ __device__ __forceinline__ int32_t edge_crossing(const DEdge *__restrict__ edges
     const float t = (R.t0 + (float)r) + R.rt_rest;
     int32_t n;
     if (crossing_f32(R.fx, R.fxi, t, R.lim, n)) return n + R.c0;
-    const DEdge &e = edges[R.id];
-    return (int32_t)round(e.x_start + (e.x_inc * (((double)(sub0 + r) + 0.5) - e.top))) - col0;
+    return crossing_f64(edges + R.id, sub0 + r) - col0;
 }
 
 // Inside bits of the lane's columns on the row's sample rows by the non-zero
@@ -212,6 +226,19 @@ static __device__ __noinline__ uint4 winding_bits(const void *bins, const DEdge 
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
+// The alpha formats' pixel access and src_over, out of line: the 4-byte
+// formats' loops stay small.
+static __device__ __noinline__ uint32_t load_alpha(uint8_t *data, int fmt, size_t i) {
+    return load_raw(DevSurface{data, fmt, 0, 0}, i);
+}
+static __device__ __noinline__ void store_alpha(uint8_t *data, int fmt, size_t i, uint32_t v) {
+    store_raw(DevSurface{data, fmt, 0, 0}, i, v);
+}
+static __device__ __noinline__ uint32_t alpha_src_over(uint32_t raw, uint32_t sa, int fmt) {
+    const uint32_t da = raw_to_i16(raw, fmt).a;
+    return i16_to_raw(I16{0, 0, 0, sa + da - (sa * da) / 255u}, fmt);
+}
+
 // One work item is one pixel row of a tile of 4 rows x 256 pixels.  The warp
 // walks the band's fills in call order: the fill's crossings with the row's
 // 4 (or 1) sample rows go to the planes, where lane l owns the 32 (or 8)
@@ -249,6 +276,13 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     const int4 *list = A.band_fills + JB.list_base + (long long)lb * (JB.fill1 - JB.fill0);
     const int32_t px0 = x0 + lane;  // this lane's first pixel; the others follow 32 apart
     constexpr uint32_t kAll = 0xffffffffu;
+    // The loops over sample rows are unrolled in the plain variant, where they
+    // are the kernel's work (2,000 paths 2.41 ms, not unrolled 2.70), not in
+    // the general one, where every warp is at another place of a large
+    // program and waits for instructions (240 gradient fills 0.78 ms, unrolled
+    // 1.05).  What a loop needs rarely is out of line for the same
+    // reason: with it inline the plain kernel had 86 KB of code instead of 61
+    // and 320 surfaces with strokes took 5.1 ms instead of 3.9.
     const uint32_t below = (1u << lane) - 1u;  // the lanes before this one
 
     for (int i = lane; i < kCovOff; i += 32) words[i] = 0u;
@@ -257,7 +291,12 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     {
         const DevSurface dst = JB.sfc;
 #pragma unroll
-        for (int q = 0; q < 8; q++) raw[q] = (px0 + 32 * q < W) ? load_raw(dst, (size_t)W * y + px0 + 32 * q) : 0u;
+        for (int q = 0; q < 8; q++) {
+            raw[q] = 0u;
+            if (px0 + 32 * q >= W) continue;
+            const size_t at = (size_t)W * y + px0 + 32 * q;
+            raw[q] = fmt <= Z2D_FORMAT_RGBA ? reinterpret_cast<const uint32_t *>(dst.data)[at] : load_alpha(dst.data, fmt, at);
+        }
     }
     __syncwarp();
 
@@ -322,10 +361,8 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 if (dense) flags = 4u;
                 for (int32_t base = dense ? ne : 0; base < ne; base += 32) {
                     const RowEdge R = row_edge<GATHER>(A.bins, A.edges, e0 + base + lane, base + lane < ne, sub0, sc, col0);
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        if (r >= sc) break;
-                        if (!((R.rows >> r) & 1u)) continue;
+                    auto cross = [&](int r) {
+                        if (!((R.rows >> r) & 1u)) return;
                         const int32_t c = edge_crossing(A.edges, R, r, sub0, col0);
                         if (c <= 0) {
                             const int32_t d = R.down ? -1 : 1;
@@ -345,6 +382,16 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                                 }
                             }
                         }
+                    };
+                    if constexpr (PLAIN) {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            if (r >= sc) break;
+                            cross(r);
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int r = 0; r < sc; r++) cross(r);
                     }
                 }
                 __syncwarp();
@@ -361,25 +408,13 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 // coverage of pixel q (0..16) of the lane's [8l, 8l+8) is byte
                 // q / 2 of cov_ev (q even) or cov_od (q odd)
                 uint32_t cov_ev = 0, cov_od = 0;
+                if constexpr (PLAIN) {
                 int32_t wl[4];  // winding left of the lane's columns (even-odd: its parity)
                 wl[0] = (int32_t)(int16_t)(l01 & 0xFFFF);
                 wl[1] = (l01 - wl[0]) >> 16;
                 wl[2] = (int32_t)(int16_t)(l23 & 0xFFFF);
                 wl[3] = (l23 - wl[2]) >> 16;
-                auto cover = [&](uint32_t bits) {
-                    if (direct) {  // one sample row: bit q is pixel q's sample
-#pragma unroll
-                        for (int q = 0; q < 8; q += 2) {
-                            cov_ev |= ((bits >> q) & 1u) << (4 * q);
-                            cov_od |= ((bits >> (q + 1)) & 1u) << (4 * q);
-                        }
-                    } else {  // nibble q holds pixel q's 4 samples of this row
-                        uint32_t n = bits - ((bits >> 1) & 0x55555555u);
-                        n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
-                        cov_ev += n & 0x0F0F0F0Fu;
-                        cov_od += (n >> 4) & 0x0F0F0F0Fu;
-                    }
-                };
+                uint32_t in[4] = {0u, 0u, 0u, 0u};  // inside bits of the lane's columns per sample row
                 if (eo) {
 #pragma unroll
                     for (int s = 0; s < 4; s++) {
@@ -390,25 +425,23 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                         // the crossings of the lanes before this one, and of
                         // the columns left of the tile
                         const uint32_t odd = __ballot_sync(kAll, __popc(t) & 1);
-                        const uint32_t in = (uint32_t)(__popc(odd & below) + wl[s]) & 1u;
+                        const uint32_t first = (uint32_t)(__popc(odd & below) + wl[s]) & 1u;
                         t ^= t << 1;
                         t ^= t << 2;
                         t ^= t << 4;
                         t ^= t << 8;
                         t ^= t << 16;
-                        cover(t ^ (0u - in));
+                        in[s] = t ^ (0u - first);
                     }
                 } else if (flags & 4u) {
                     if (!dense) {  // clear the planes
                         for (int i = lane; i < 4 * kSubWords; i += 32) words[i] = 0u;
                     }
-                    const uint4 in = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, sc, col0, words, lane);
-                    cover(in.x);
-                    if (sc > 1) {
-                        cover(in.y);
-                        cover(in.z);
-                        cover(in.w);
-                    }
+                    const uint4 v = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, sc, col0, words, lane);
+                    in[0] = v.x;
+                    in[1] = v.y;
+                    in[2] = v.z;
+                    in[3] = v.w;
                 } else {
                     uint32_t up[4], dn[4];
                     int32_t tot[4] = {0, 0, 0, 0};  // the lane's winding change
@@ -466,8 +499,131 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                                 if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
                             }
                         }
+                        in[s] = bits;
+                    }
+                }
+                if (direct) {  // one sample row: bit q is pixel q's sample
+#pragma unroll
+                    for (int q = 0; q < 8; q += 2) {
+                        cov_ev |= ((in[0] >> q) & 1u) << (4 * q);
+                        cov_od |= ((in[0] >> (q + 1)) & 1u) << (4 * q);
+                    }
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {  // nibble q holds pixel q's 4 samples of a row
+                        uint32_t n = in[s] - ((in[s] >> 1) & 0x55555555u);
+                        n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+                        cov_ev += n & 0x0F0F0F0Fu;
+                        cov_od += (n >> 4) & 0x0F0F0F0Fu;
+                    }
+                }
+                } else {
+                auto cover = [&](uint32_t bits) {
+                    if (direct) {  // one sample row: bit q is pixel q's sample
+                        cov_ev = (bits & 1u) | ((bits & 4u) << 6) | ((bits & 16u) << 12) | ((bits & 64u) << 18);
+                        bits >>= 1;
+                        cov_od = (bits & 1u) | ((bits & 4u) << 6) | ((bits & 16u) << 12) | ((bits & 64u) << 18);
+                    } else {  // nibble q holds pixel q's 4 samples of this row
+                        uint32_t n = bits - ((bits >> 1) & 0x55555555u);
+                        n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+                        cov_ev += n & 0x0F0F0F0Fu;
+                        cov_od += (n >> 4) & 0x0F0F0F0Fu;
+                    }
+                };
+                // winding (even-odd: its parity) left of the lane's columns,
+                // rows 0, 1 and 2, 3 packed
+                int32_t i01 = l01, i23 = l23;
+                uint4 counted = make_uint4(0u, 0u, 0u, 0u);
+                if (flags & 4u) {
+                    if (!dense) {  // clear the planes
+                        for (int i = lane; i < 4 * kSubWords; i += 32) words[i] = 0u;
+                    }
+                    counted = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, sc, col0, words, lane);
+                } else if (!eo) {
+                    int32_t tot[4] = {0, 0, 0, 0};  // the lane's winding change
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        const uint32_t *w = words + s * kSubWords + lane;
+                        tot[s] = __popc(w[0]) - __popc(w[32]);
+                        if (flags & 2u) tot[s] += __popc(w[64]) + __popc(w[128]) - __popc(w[96]) - __popc(w[160]);
+                    }
+                    const int32_t t01 = tot[0] + tot[1] * 65536, t23 = tot[2] + tot[3] * 65536;
+                    i01 = t01;
+                    i23 = t23;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int32_t u01 = __shfl_up_sync(kAll, i01, o);
+                        const int32_t u23 = __shfl_up_sync(kAll, i23, o);
+                        if (lane >= o) {
+                            i01 += u01;
+                            i23 += u23;
+                        }
+                    }
+                    i01 += l01 - t01;
+                    i23 += l23 - t23;
+                }
+                auto left_of = [&](int s) -> int32_t {
+                    const int32_t pair = s < 2 ? i01 : i23, low = (int32_t)(int16_t)(pair & 0xFFFF);
+                    return (s & 1) ? (pair - low) >> 16 : low;
+                };
+                if (eo) {
+#pragma unroll 1
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        uint32_t *w = words + s * kSubWords + lane;
+                        uint32_t t = *w;
+                        *w = 0u;
+                        // the crossings of the lanes before this one, and of
+                        // the columns left of the tile
+                        const uint32_t odd = __ballot_sync(kAll, __popc(t) & 1);
+                        const uint32_t first = (uint32_t)(__popc(odd & below) + left_of(s)) & 1u;
+                        t ^= t << 1;
+                        t ^= t << 2;
+                        t ^= t << 4;
+                        t ^= t << 8;
+                        t ^= t << 16;
+                        cover(t ^ (0u - first));
+                    }
+                } else if (flags & 4u) {
+                    cover(counted.x);
+                    if (!direct) {
+                        cover(counted.y);
+                        cover(counted.z);
+                        cover(counted.w);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int s = 0; s < 4; s++) {
+                        if (s >= sc) break;
+                        // the inside state changes where the winding leaves
+                        // or reaches zero
+                        uint32_t *w = words + s * kSubWords + lane;
+                        const uint32_t up = w[0], dn = w[32];
+                        w[0] = w[32] = 0u;
+                        int32_t wnd = left_of(s);
+                        uint32_t bits = wnd != 0 ? 0xFFFFFFFFu : 0u;
+                        if (flags & 2u) {
+                            const uint32_t u1 = w[64], d1 = w[96], u2 = w[128], d2 = w[160];
+                            w[64] = w[96] = w[128] = w[160] = 0u;
+                            for (uint32_t m = up | dn; m; m &= m - 1) {
+                                const int k = __ffs(m) - 1;
+                                const bool was = wnd != 0;
+                                wnd += (int32_t)(((up >> k) & 1u) + ((u1 >> k) & 1u) + ((u2 >> k) & 1u)) -
+                                       (int32_t)(((dn >> k) & 1u) + ((d1 >> k) & 1u) + ((d2 >> k) & 1u));
+                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                            }
+                        } else {
+                            for (uint32_t m = up | dn; m; m &= m - 1) {
+                                const int k = __ffs(m) - 1;
+                                const bool was = wnd != 0;
+                                wnd += (int32_t)((up >> k) & 1u) - (int32_t)((dn >> k) & 1u);
+                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                            }
+                        }
                         cover(bits);
                     }
+                }
                 }
                 // only the box's columns are drawn
                 const uint32_t box = __shfl_sync(kAll, my_box, src);
@@ -534,9 +690,8 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     for (int q = 0; q < 8; q++) {
                         if (!((blocks >> q) & 1u)) continue;
                         const int c = cov[32 * q];
-                        const uint32_t sa = __shfl_sync(kAll, s.a, c), da = raw_to_i16(raw[q], fmt).a;
-                        const uint32_t nv = i16_to_raw(I16{0, 0, 0, sa + da - (sa * da) / 255u}, fmt);
-                        raw[q] = c != 0 ? nv : raw[q];
+                        const uint32_t sa = __shfl_sync(kAll, s.a, c);
+                        if (c != 0) raw[q] = alpha_src_over(raw[q], sa, fmt);
                     }
                 }
                 continue;
@@ -545,6 +700,64 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
             const int32_t f = __shfl_sync(kAll, my_f, src);
             const FillState &S = A.st[f];
             const FillCmd &F = A.fills[f];
+            const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
+            if (((meta >> RF_FAST_SHIFT) & 3u) == FAST_SOURCE_SRC_OVER && !exact && fmt <= Z2D_FORMAT_RGBA &&
+                (!ssaa || has_alpha)) {
+                // A gradient or dither drawn by integer src_over.  A source
+                // pixel costs hundreds of instructions, so the covered
+                // pixels of the whole row are listed first and evaluated 32 at
+                // a time, whatever block they lie in.  (Supersampled, a
+                // pixel without coverage composites a clear source: without
+                // an alpha channel that would still rewrite its padding byte.)
+                if (!blocks) continue;
+                touched |= blocks;
+                // the planes, clear at this point, hold the colours and the
+                // list
+                uint8_t *at = reinterpret_cast<uint8_t *>(words + kTileCols);
+                int n = 0;
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    if (!((blocks >> q) & 1u)) continue;
+                    const bool on = cov[32 * q] != 0;
+                    const uint32_t m = __ballot_sync(kAll, on);
+                    if (on) at[n + __popc(m & below)] = (uint8_t)(32 * q + lane);
+                    n += __popc(m);
+                }
+                __syncwarp();
+                auto word_at = [&](int p, I16 s) {
+                    const int c = reinterpret_cast<const uint8_t *>(words + kCovOff)[p];
+                    const uint32_t op8 = ssaa ? ss_mask8(c, fmt) : c >= (direct ? 1 : 16) ? 255u : (uint32_t)(c * 16 - 1);
+                    words[p] = source_word(s, op8, fmt);
+                };
+                // in f32 first; what that does not decide goes to the front
+                // of the list (behind the reads) and is evaluated exactly
+                int late = 0;
+                for (int i0 = 0; i0 < n; i0 += 32) {
+                    const bool live = i0 + lane < n;
+                    const int p = live ? at[i0 + lane] : 0;
+                    I16 s;
+                    const bool ok = live && src_i16_f32(F.src, x0 + p, y, s);
+                    if (ok) word_at(p, s);
+                    const uint32_t m = __ballot_sync(kAll, live && !ok);
+                    if (live && !ok) at[late + __popc(m & below)] = (uint8_t)p;
+                    late += __popc(m);
+                    __syncwarp();
+                }
+                for (int i = lane; i < late; i += 32) {
+                    const int p = at[i];
+                    word_at(p, src_i16_slow(F.src, x0 + p, y, 0));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    if (!((blocks >> q) & 1u)) continue;
+                    if (cov[32 * q] != 0) raw[q] = word_src_over_x4(raw[q], words[32 * q + lane], has_alpha);
+                }
+                __syncwarp();
+                for (int i = lane; i < kTileCols + kTileCols / 4; i += 32) words[i] = 0u;
+                __syncwarp();
+                continue;
+            }
             // with a bounded operator only covered pixels are drawn
             const bool sparse = bounded && !ssaa && !exact;
 #pragma unroll 1
@@ -596,14 +809,14 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     }
     // the surface pointer is read again here rather than kept in registers
     // through the fill loop
-    DevSurface dst;
-    dst.data = MULTI ? *reinterpret_cast<uint8_t *const volatile *>(&A.jobs[jb].sfc.data) : A.job0.sfc.data;
-    dst.fmt = fmt;
-    dst.w = W;
-    dst.h = 0;  // unused by the stores
+    uint8_t *data = MULTI ? *reinterpret_cast<uint8_t *const volatile *>(&A.jobs[jb].sfc.data) : A.job0.sfc.data;
 #pragma unroll
     for (int q = 0; q < 8; q++)
-        if (((touched >> q) & 1u) && px0 + 32 * q < W) store_raw(dst, (size_t)W * y + px0 + 32 * q, raw[q]);
+        if (((touched >> q) & 1u) && px0 + 32 * q < W) {
+            const size_t at = (size_t)W * y + px0 + 32 * q;
+            if (fmt <= Z2D_FORMAT_RGBA) reinterpret_cast<uint32_t *>(data)[at] = raw[q];
+            else store_alpha(data, fmt, at, raw[q]);
+        }
 }
 
 // Persistent rasteriser: a grid of resident CTAs that take items from a

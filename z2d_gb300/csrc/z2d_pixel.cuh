@@ -589,6 +589,20 @@ Z2D_D float grad_offset_f64(const DevGradient &gr, int32_t x, int32_t y) {
     return (float)(ang / twopi);
 }
 
+static __device__ __noinline__ float offset_f64_call(const DevGradient &gr, int32_t x, int32_t y) {
+    return grad_offset_f64(gr, x, y);
+}
+// One kind's double-word evaluation, out of line; 2 where it does not decide
+// (an offset is at most 1).
+template <int MODE>
+static __device__ __noinline__ float offset_fast_call(const GradFast &F, bool tf, float fx, float fy) {
+    float t = 0.0f;
+    int done;
+    if constexpr (MODE == kFastLinear) done = fast_linear(F, tf, fx, fy, t);
+    else if constexpr (MODE == kFastConic) done = fast_conic(F, tf, fx, fy, t);
+    else done = fast_radial(F, tf, F.mode == kFastRadialA0, fx, fy, t);
+    return done ? t : 2.0f;
+}
 // Gradient.getOffset (src/gradient.zig:239-243, 349-372, 605-648, 731-741):
 // the double-word evaluation when it decides the f32 result, else the f64
 // code above (`slow` is set then).
@@ -598,15 +612,13 @@ Z2D_D float grad_offset_ex(const DevGradient &gr, int32_t x, int32_t y, bool &sl
     if (mode != kFastNone && (uint32_t)(x + (1 << 22)) < (1u << 23) && (uint32_t)(y + (1 << 22)) < (1u << 23)) {
         const float fx = (float)x + 0.5f, fy = (float)y + 0.5f;
         const bool tf = gr.has_tf != 0;
-        float t = 0.0f;
-        int done;
-        if (mode == kFastLinear) done = fast_linear(gr.fz, tf, fx, fy, t);
-        else if (mode == kFastConic) done = fast_conic(gr.fz, tf, fx, fy, t);
-        else done = fast_radial(gr.fz, tf, mode == kFastRadialA0, fx, fy, t);
-        if (done) return t;
+        const float t = mode == kFastLinear  ? offset_fast_call<kFastLinear>(gr.fz, tf, fx, fy)
+                        : mode == kFastConic ? offset_fast_call<kFastConic>(gr.fz, tf, fx, fy)
+                                             : offset_fast_call<kFastRadial>(gr.fz, tf, fx, fy);
+        if (t < 2.0f) return t;
     }
     slow = true;
-    return grad_offset_f64(gr, x, y);
+    return offset_f64_call(gr, x, y);
 }
 // Out of line: the kernels that composite every kind of source (the
 // rasteriser among them) keep their registers for their own loops.
@@ -694,6 +706,14 @@ Z2D_D HSLf hsl_lerp_demul(RGBf am, RGBf bm, float t, int polar) {
     if (o.a == 0.0f) return HSLf{o.h, 0.0f, 0.0f, o.a};
     return HSLf{o.h, o.s / o.a, o.l / o.a, o.a};
 }
+// The heavy steps of a gradient pixel, out of line: one copy each per
+// translation unit.  With them inlined into every place that evaluates a
+// source, the rasteriser's warps (each on a fill of its own) waited for
+// instructions most of the time.
+static __device__ __noinline__ float gamma_call(float x) { return zpow(x, kGamma); }
+static __device__ __noinline__ RGBf hsl_call(RGBf a, RGBf b, float t, int polar) {
+    return hsl_to_rgb(hsl_lerp_demul(a, b, t, polar));
+}
 // interpolateEncode: the integer lanes of the interpolated colour.
 Z2D_D I16 interp_encode_prep(int method, RGBf am, RGBf bm, float t) {
     if (method == Z2D_INTERP_LINEAR_RGB)
@@ -701,18 +721,18 @@ Z2D_D I16 interp_encode_prep(int method, RGBf am, RGBf bm, float t) {
                    enc_ch(lerpf(am.a, bm.a, t))};
     if (method == Z2D_INTERP_SRGB) {
         const RGBf d = rgb_lerp_demul(am, bm, t);
-        return encode_linear(RGBf{zpow(d.r, kGamma), zpow(d.g, kGamma), zpow(d.b, kGamma), d.a});
+        return encode_linear(RGBf{gamma_call(d.r), gamma_call(d.g), gamma_call(d.b), d.a});
     }
-    return encode_linear(hsl_to_rgb(hsl_lerp_demul(am, bm, t, method)));
+    return encode_linear(hsl_call(am, bm, t, method));
 }
 // interpolate: the linear colour (float precision, dither sources).
 Z2D_D RGBf interp_linear_prep(int method, RGBf am, RGBf bm, float t) {
     if (method == Z2D_INTERP_LINEAR_RGB) return rgb_lerp_demul(am, bm, t);
     if (method == Z2D_INTERP_SRGB) {
         const RGBf d = rgb_lerp_demul(am, bm, t);
-        return RGBf{zpow(d.r, kGamma), zpow(d.g, kGamma), zpow(d.b, kGamma), d.a};
+        return RGBf{gamma_call(d.r), gamma_call(d.g), gamma_call(d.b), d.a};
     }
-    return hsl_to_rgb(hsl_lerp_demul(am, bm, t, method));
+    return hsl_call(am, bm, t, method);
 }
 
 // -------------------------------------------------------------- dither
@@ -770,6 +790,12 @@ Z2D_D RGBf dither_linear(const DevSrc &s, int32_t x, int32_t y) {
                 fmaxf(0.0f, fminf(c.b + m * scale, 1.0f)), fmaxf(0.0f, fminf(c.a + m * scale, 1.0f))};
 }
 
+}  // namespace z2dg
+#if defined(__CUDACC__)
+#include "grad_f32.cuh"
+#endif
+namespace z2dg {
+
 // Source lanes at device position (x, y); `idx` is the flat index used for
 // SURFACE params.
 Z2D_D I16 src_i16(const DevSrc &s, int32_t x, int32_t y, size_t idx) {
@@ -807,7 +833,20 @@ namespace z2dg {
 // Out-of-line entry points for the heavy per-pixel paths, so that kernels
 // instantiated per format and precision do not each inline every source
 // and operator (keeps code size and build time small).
-static __device__ __noinline__ I16 src_i16_any(const DevSrc &s, int32_t x, int32_t y, size_t idx) { return src_i16(s, x, y, idx); }
+static __device__ __noinline__ I16 src_i16_slow(const DevSrc &s, int32_t x, int32_t y, size_t idx) { return src_i16(s, x, y, idx); }
+// A gradient source's lanes in f32; false where that does not decide them,
+// and for other sources.
+static __device__ __noinline__ bool src_i16_f32(const DevSrc &s, int32_t x, int32_t y, I16 &v) {
+    const bool dith = s.kind == SRC_DITHER && s.dither_source == Z2D_DITHER_SRC_GRADIENT;
+    if (s.kind != SRC_GRADIENT && !dith) return false;
+    return grad_lanes_f32(s.grad_type, s.grad_method, dith ? s.dither_type : Z2D_DITHER_NONE,
+                          dith ? dither_step_of(s.dither_scale) : 0.0f, *s.grad, x, y, v);
+}
+static __device__ __noinline__ I16 src_i16_any(const DevSrc &s, int32_t x, int32_t y, size_t idx) {
+    I16 v;
+    if (src_i16_f32(s, x, y, v)) return v;
+    return src_i16_slow(s, x, y, idx);
+}
 static __device__ __noinline__ F4 src_f4_any(const DevSrc &s, int32_t x, int32_t y, size_t idx) { return src_f4(s, x, y, idx); }
 static __device__ __noinline__ I16 int_op_any(int op, I16 d, I16 s) { return int_op(op, d, s); }
 static __device__ __noinline__ F4 float_op_any(int op, F4 d, F4 s) { return float_op(op, d, s); }
