@@ -107,3 +107,20 @@ def test_several_surfaces(gpu, oracle):
     gpu.ctx.synchronize()
     for (s, _), ref, size in zip(jobs, refs, sizes):
         assert np.array_equal(s.numpy(), ref.numpy()), size
+
+
+@pytest.mark.parametrize("aas", [("none",), ("none", "default"), ("default", "supersample_4x"), ("none", "supersample_4x")])
+@pytest.mark.parametrize("fmt", ["rgba", "xrgb", "alpha8"])
+def test_modes(gpu, oracle, aas, fmt):
+    """Batches of one anti-aliasing mode and of several: the plain variants and the general one."""
+    fills = [(PIX, _copies(1 + k % 5, 270, 11, True), FillOptions(anti_aliasing=aas[k % len(aas)],
+                                                                 fill_rule=("non_zero", "even_odd")[k % 2]))
+             for k in range(8)] + [(PIX, _off_surface(), FillOptions(anti_aliasing=aas[0]))]
+    a, b = _surface(fmt, 270, 11, 2), _surface(fmt, 270, 11, 2)
+    painter.fill_batch(a, fills, ctx=gpu.ctx)
+    for pat, nodes, opts in fills:
+        assert oracle.fill(b, pat, nodes, opts) == abi.OK
+    x, y = a.numpy(), b.numpy()
+    if fmt == "xrgb":  # the padding byte of a pixel without coverage is undefined in z2d (left as it was here)
+        x, y = x.reshape(-1, 4)[:, :3], y.reshape(-1, 4)[:, :3]
+    assert np.array_equal(x, y)

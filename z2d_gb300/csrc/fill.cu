@@ -698,9 +698,7 @@ __global__ void k_fill_setup(const FillCmd *__restrict__ fills, FillState *__res
              (F.rule == Z2D_FILL_EVEN_ODD ? RF_EVEN_ODD : 0u) | ((uint32_t)F.fast_kind << RF_FAST_SHIFT) |
              ((S.flags & FILL_EXACT) ? RF_EXACT : 0u) | ((S.flags & FILL_SS_ZERO) ? RF_SS_ZERO : 0u) |
              (bounded ? RF_BOUNDED : 0u);
-    R.px = (F.src.pix.r & 0xFFu) | ((F.src.pix.g & 0xFFu) << 8) | ((F.src.pix.b & 0xFFu) << 16) |
-           ((F.src.pix.a & 0xFFu) << 24);
-    R._pad[0] = R._pad[1] = 0;
+    R._pad[0] = R._pad[1] = R._pad[2] = 0;
     rf[f] = R;
 }
 
@@ -786,11 +784,21 @@ __global__ void k_bin_fill(const FillCmd *__restrict__ fills, const FillState *_
     });
 }
 
-// Edge -> fill map (edges of one fill are contiguous).
-__global__ void k_edge_fill(const FillState *__restrict__ st, int32_t n_fills, int32_t *__restrict__ edge_fill) {
+// Edge -> fill map (edges of one fill are contiguous), and the fill's source
+// word for every coverage: 17 words that a fill's every row and tile would
+// otherwise compute again, with a division per channel.
+__global__ void k_edge_fill(const FillState *__restrict__ st, const FillCmd *__restrict__ fills,
+                            const DevJob *__restrict__ jobs, int32_t *__restrict__ edge_fill,
+                            uint32_t *__restrict__ luts) {
     const int32_t f = blockIdx.x;
-    const FillState S = st[f];
-    for (int32_t k = threadIdx.x; k < S.n_edges; k += blockDim.x) edge_fill[S.edge_base + k] = f;
+    const FillState &S = st[f];
+    const int32_t e0 = S.edge_base, n = S.n_edges;
+    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) edge_fill[e0 + k] = f;
+    if (threadIdx.x < 32) {
+        const FillCmd &F = fills[f];
+        luts[32 * (size_t)f + threadIdx.x] =
+            F.fast_kind == FAST_PIXEL_SRC_OVER ? coverage_word(F, jobs[F.job].sfc.fmt, (int)threadIdx.x) : 0u;
+    }
 }
 
 // Ordered list of the fills touching each band (call order preserved by a
@@ -1163,9 +1171,10 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     const size_t info_bytes = (sizeof(NodeInfo) * (size_t)n_nodes + 255) & ~(size_t)255;
     const size_t st_bytes = (sizeof(FillState) * (size_t)n_fills + 255) & ~(size_t)255;
     if (c.node_info.ensure(info_bytes + (kCurveClasses + 2) * sizeof(int32_t) * (size_t)n_nodes) ||
-        c.fill_state.ensure(st_bytes + sizeof(RasterFill) * (size_t)n_fills))
+        c.fill_state.ensure(st_bytes + (sizeof(RasterFill) + 32 * sizeof(uint32_t)) * (size_t)n_fills))
         return Z2D_ERR_OUT_OF_MEMORY;
     RasterFill *d_rf = reinterpret_cast<RasterFill *>(c.fill_state.as<uint8_t>() + st_bytes);
+    uint32_t *d_luts = reinterpret_cast<uint32_t *>(d_rf + n_fills);  // per fill, its source word per coverage
     NodeInfo *d_info = c.node_info.as<NodeInfo>();
     // the curves to count, one queue per class, those to emit, then each
     // node's fill
@@ -1281,7 +1290,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         const int rc = poly_emit(c, pr, d_fills, d_st, d_edges);
         if (rc) return rc;
     }
-    k_edge_fill<<<n_fills, 128, 0, c.stream>>>(d_st, n_fills, d_edge_fill);
+    k_edge_fill<<<n_fills, 128, 0, c.stream>>>(d_st, d_fills, d_jobs, d_edge_fill, d_luts);
     k_fill_setup<<<grid_for(n_fills, 64), 64, 0, c.stream>>>(d_fills, d_st, n_fills, d_jobs, d_cnt, d_rf);
     c.timer_end(c.t_flatten, tf);
     c.launches += 4;
@@ -1390,6 +1399,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     A.band_count = d_band_count;
     A.band_fills = d_band_fills;
     A.rfills = d_rf;
+    A.luts = d_luts;
     A.tiles = d_tiles;
     A.masks = c.masks.as<uint8_t>();
     A.n_jobs = n_jobs;
@@ -1400,8 +1410,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     }
     // persistent grid: every SM filled to the kernel's residency (or the
     // tuned CTAs per SM), never more CTAs than tiles
-    RasterVariant variant{n_jobs > 1, false, n_exact == 0, false};
-    for (const FillCmd &F : fills) variant.plain &= F.fast_kind == FAST_PIXEL_SRC_OVER;
+    RasterVariant variant{n_jobs > 1, false, false, raster_mode(fills.data(), fills.size(), n_exact > 0)};
     int occ = 1;
     {
         const int rc = raster_occupancy(c, variant, occ);
@@ -1778,8 +1787,6 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         R.meta = ((uint32_t)F.op & RF_OP_MASK) | ((uint32_t)F.aa << RF_AA_SHIFT) |
                  (F.rule == Z2D_FILL_EVEN_ODD ? RF_EVEN_ODD : 0u) | ((uint32_t)F.fast_kind << RF_FAST_SHIFT) |
                  (bounded ? RF_BOUNDED : 0u);
-        R.px = (F.src.pix.r & 0xFFu) | ((F.src.pix.g & 0xFFu) << 8) | ((F.src.pix.b & 0xFFu) << 16) |
-               ((F.src.pix.a & 0xFFu) << 24);
     }
     done = true;
     if (n_fb == 0) return Z2D_OK;  // nothing is drawn
@@ -1880,7 +1887,8 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     const size_t o_list = o_cnt + al(sizeof(int32_t) * bcount.size());
     const size_t o_grad = o_list + al(sizeof(int4) * blist.size());
     const size_t o_tile = o_grad + al(sizeof(DevGradient) * std::max<size_t>(grads.size(), 1));
-    const size_t total = o_tile + al(sizeof(TileRec) * tiles.size());
+    const size_t o_lut = o_tile + al(sizeof(TileRec) * tiles.size());
+    const size_t total = o_lut + al(32 * sizeof(uint32_t) * n_fills);
     const int slot = c.small_slot;
     c.small_slot ^= 1;
     HostBuf &hb = c.small_stage[slot];
@@ -1903,6 +1911,11 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     memcpy(h + o_cnt, bcount.data(), sizeof(int32_t) * bcount.size());
     memcpy(h + o_list, blist.data(), sizeof(int4) * blist.size());
     if (!grads.empty()) memcpy(h + o_grad, grads.data(), sizeof(DevGradient) * grads.size());
+    uint32_t *lut = reinterpret_cast<uint32_t *>(h + o_lut);
+    for (size_t f = 0; f < n_fills; f++) {
+        if (fills[f].fast_kind != FAST_PIXEL_SRC_OVER) continue;  // (not read)
+        for (int k = 0; k <= 16; k++) lut[32 * f + k] = coverage_word(fills[f], J[(size_t)fills[f].job].sfc.fmt, k);
+    }
     Z2D_CUDA(cudaMemcpyAsync(dv, h, total, cudaMemcpyHostToDevice, c.stream));
     Z2D_CUDA(cudaEventRecord(c.small_done[slot], c.stream));
     if (n_tiles == 0) return Z2D_OK;
@@ -1919,6 +1932,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     A.band_fills = reinterpret_cast<const int4 *>(dv + o_list);
     A.rfills = reinterpret_cast<const RasterFill *>(dv + o_rf);
     A.tiles = reinterpret_cast<const TileRec *>(dv + o_tile);
+    A.luts = reinterpret_cast<const uint32_t *>(dv + o_lut);
     A.masks = nullptr;
     A.n_jobs = (int32_t)n_jobs;
     A.queue = nullptr;
@@ -1929,8 +1943,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         const int rs = c.await_surface();
         if (rs) return rs;
     }
-    RasterVariant variant{n_jobs > 1, true, true, true};
-    for (const FillCmd &F : fills) variant.plain &= F.fast_kind == FAST_PIXEL_SRC_OVER;
+    const RasterVariant variant{n_jobs > 1, true, true, raster_mode(fills.data(), n_fills, false)};
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
     const int rc = raster_launch(c, variant, A, (unsigned)n_tiles);
     if (rc) return rc;

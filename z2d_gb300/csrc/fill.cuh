@@ -181,15 +181,14 @@ struct FillState {
     int32_t cull_x0, cull_x1;   // columns a tile must overlap to be affected
 };
 
-// What k_raster reads of a fill on its common path, in two 16-byte loads
+// What k_raster reads of a fill on its common path
 // (written by k_fill_setup from the FillCmd and FillState).
 struct RasterFill {
     int32_t start_x, end_x, start_y, end_y;  // FillState's draw box
     uint32_t meta;  // RF_* fields below
-    uint32_t px;    // pattern pixel's RGBA lanes (FillCmd.px_rgba), one byte each: r | g << 8 | b << 16 | a << 24
-    int32_t _pad[2];
+    int32_t _pad[3];
 };
-static_assert(sizeof(RasterFill) == 32, "RasterFill: two 16-byte loads");
+static_assert(sizeof(RasterFill) == 32, "RasterFill: the box is one 16-byte load");
 enum : uint32_t {
     RF_OP_MASK = 0x1F,        // operator
     RF_AA_SHIFT = 5,          // anti-aliasing mode, 2 bits

@@ -13,15 +13,6 @@
 namespace z2dg {
 
 // --------------------------------------------------------- compositing
-// The supersample mask value of a pixel whose 4x4 sample block has n covered
-// samples, as 8-bit alpha: the mask is alpha8, or the surface's own format
-// for alpha4/2/1 surfaces (supersample.zig:69-83), each covered sample is
-// opaque, and downsampleBuffer averages the 16 (surface.zig:447-469).
-__device__ __forceinline__ uint32_t ss_mask8(int n, int fmt) {
-    if (fmt >= Z2D_FORMAT_ALPHA4) return scale_alpha(((uint32_t)n * fmt_max(fmt)) / 16u, fmt_bits(fmt), 8);
-    return ((uint32_t)n * 255u) / 16u;
-}
-
 // One pixel of the supersample batch [dst_in(dst = pattern, src = mask), op]
 // (supersample.zig:171-184) as StrideCompositor.runPrecision evaluates it
 // (compositor.zig:540-621): the mask reads as alpha-only lanes.
@@ -62,10 +53,10 @@ __device__ __forceinline__ bool msaa_unbounded_clear(const FillState &S, int32_t
 //     column, row and direction sends the (fill, row) to winding_bits.
 // Against 16-bit counters per column this is one atomic per crossing instead
 // of three, and the even-odd rule needs no walk over the crossings at all:
-// the inside bits are the prefix XOR of the toggles.  Issue bound: a fill
-// costs a row and tile of the 2,000-path 4096x4096 batch (2.9 M of them, 28
-// edges each on average) about 600 warp instructions instead of 1,250, and
-// the kernel takes 2.45 ms instead of 4.30.
+// the inside bits are the prefix XOR of the toggles.  Issue bound, on the
+// ALU pipe: a fill costs a row and tile of the 2,000-path 4096x4096 batch
+// (2.9 M of them, 28 edges each on average) about 700 warp instructions
+// instead of 1,250, and the kernel takes 2.08 ms instead of 4.30.
 constexpr int kPlanes = 6;
 constexpr int kSubWords = kPlanes * 32;         // one sample row
 constexpr int kDenseWords = 2 * 16 * 32 + 2 * 32;  // or winding_bits' counters
@@ -251,7 +242,7 @@ static __device__ __noinline__ uint32_t alpha_src_over(uint32_t raw, uint32_t sa
 // MULTI = false draws a one-surface batch from A.job0, whose fields are
 // kernel parameters (warp-uniform values that need no registers);
 // MULTI = true finds the tile's job in the job table.
-template <bool MULTI, bool PLAIN, bool GATHER>
+template <bool MULTI, int MODE, bool GATHER>
 __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t tile, const int warp, const int lane,
                                            uint32_t *words) {
     // tile -> (job, band, tile column)
@@ -276,8 +267,9 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     const int4 *list = A.band_fills + JB.list_base + (long long)lb * (JB.fill1 - JB.fill0);
     const int32_t px0 = x0 + lane;  // this lane's first pixel; the others follow 32 apart
     constexpr uint32_t kAll = 0xffffffffu;
+    constexpr bool PLAIN = MODE != kGeneral;
     // The loops over sample rows are unrolled in the plain variant, where they
-    // are the kernel's work (2,000 paths 2.41 ms, not unrolled 2.70), not in
+    // are the kernel's work (2,000 paths then 2.41 ms, not unrolled 2.70), not in
     // the general one, where every warp is at another place of a large
     // program and waits for instructions (240 gradient fills 0.78 ms, unrolled
     // 1.05).  What a loop needs rarely is out of line for the same
@@ -306,18 +298,17 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     // records in registers, before the first of them is drawn.
     for (int32_t k0 = 0; k0 < cnt; k0 += 32) {
         int32_t my_f = 0, my_e0 = 0, my_ne = 0;
-        uint32_t my_meta = 0, my_px = 0, my_box = 0;
+        uint32_t my_meta = 0, my_box = 0;
         bool hit = false;
         if (k0 + lane < cnt) {
             const int4 ent = list[k0 + lane];
             if (ent.z > x0 && ent.y < x0 + kTileCols) {
                 const int4 ra = __ldg(reinterpret_cast<const int4 *>(A.rfills + ent.x));
-                const int2 rb = __ldg(reinterpret_cast<const int2 *>(A.rfills + ent.x) + 2);
+                const uint32_t rb = __ldg(&A.rfills[ent.x].meta);
                 my_e0 = __ldg(A.bin_off + ent.w);
                 my_ne = __ldg(A.bin_off + ent.w + 1) - my_e0;
                 my_f = ent.x;
-                my_meta = (uint32_t)rb.x;
-                my_px = (uint32_t)rb.y;
+                my_meta = rb;
                 const int32_t aa = (int32_t)((my_meta >> RF_AA_SHIFT) & 3u);
                 const bool bounded = (my_meta & RF_BOUNDED) != 0;
                 const bool boxed = bounded || aa == Z2D_AA_SUPERSAMPLE_4X;  // touches only its box
@@ -342,7 +333,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
             const int32_t aa = (int32_t)((meta >> RF_AA_SHIFT) & 3u);
             const bool bounded = PLAIN || (meta & RF_BOUNDED) != 0;
             const bool ssaa = aa == Z2D_AA_SUPERSAMPLE_4X;
-            const bool direct = aa == Z2D_AA_NONE;
+            const bool direct = MODE == kPlainDirect || (MODE == kGeneral && aa == Z2D_AA_NONE);
             const bool exact = !PLAIN && (meta & RF_EXACT) != 0;
             const bool in_rows = PLAIN || (meta & RF_IN_ROWS) != 0;
             const int32_t sc = direct ? 1 : 4, per = 8 * sc, lg_per = direct ? 3 : 5;
@@ -485,18 +476,18 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                             const uint32_t u1 = w[64], d1 = w[96], u2 = w[128], d2 = w[160];
                             w[64] = w[96] = w[128] = w[160] = 0u;
                             for (uint32_t m = up[s] | dn[s]; m; m &= m - 1) {
-                                const int k = __ffs(m) - 1;
-                                const bool was = wnd != 0;
-                                wnd += (int32_t)(((up[s] >> k) & 1u) + ((u1 >> k) & 1u) + ((u2 >> k) & 1u)) -
-                                       (int32_t)(((dn[s] >> k) & 1u) + ((d1 >> k) & 1u) + ((d2 >> k) & 1u));
-                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                                const uint32_t k = m & (0u - m);  // the next column's bit
+                                const uint32_t was = wnd != 0 ? 0xFFFFFFFFu : 0u;
+                                wnd += (up[s] & k ? 1 : 0) + (u1 & k ? 1 : 0) + (u2 & k ? 1 : 0) - (dn[s] & k ? 1 : 0) -
+                                       (d1 & k ? 1 : 0) - (d2 & k ? 1 : 0);
+                                bits ^= (was ^ (wnd != 0 ? 0xFFFFFFFFu : 0u)) & (0u - k);
                             }
                         } else {
                             for (uint32_t m = up[s] | dn[s]; m; m &= m - 1) {
-                                const int k = __ffs(m) - 1;
-                                const bool was = wnd != 0;
-                                wnd += (int32_t)((up[s] >> k) & 1u) - (int32_t)((dn[s] >> k) & 1u);
-                                if ((wnd != 0) != was) bits ^= 0xFFFFFFFFu << k;
+                                const uint32_t k = m & (0u - m);
+                                const uint32_t was = wnd != 0 ? 0xFFFFFFFFu : 0u;
+                                wnd += (up[s] & k ? 1 : 0) - (dn[s] & k ? 1 : 0);
+                                bits ^= (was ^ (wnd != 0 ? 0xFFFFFFFFu : 0u)) & (0u - k);
                             }
                         }
                         in[s] = bits;
@@ -664,25 +655,17 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 // coverage both leave the pixel as it is.
                 // (A bounded fill outside its rows was skipped above.)
                 if (!blocks) continue;
-                const uint32_t pw = __shfl_sync(kAll, my_px, src);
-                const int full = direct ? 1 : 16;
-                // Lane k holds the source word for coverage k: the pixel at
-                // k = full, dst_in(pixel, opacity(k)) below it.
-                I16 s{pw & 0xFFu, (pw >> 8) & 0xFFu, (pw >> 16) & 0xFFu, pw >> 24};
-                if (lane < full) {
-                    const uint32_t op8 = ssaa ? ss_mask8(lane, fmt) : (uint32_t)max(lane * 16 - 1, 0);
-                    s = I16{(s.r * op8) / 255u, (s.g * op8) / 255u, (s.b * op8) / 255u, (s.a * op8) / 255u};
-                }
+                // Lane k holds the source word for coverage k (k_edge_fill).
+                const uint32_t lut_w = __ldg(A.luts + 32 * (size_t)__shfl_sync(kAll, my_f, src) + lane);
                 touched |= blocks;
                 if (fmt <= Z2D_FORMAT_RGBA) {
-                    const uint32_t lut_w = i16_to_word(s, word_order(fmt));
                     const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
                         if (!((blocks >> q) & 1u)) continue;
                         const int c = cov[32 * q];
                         const uint32_t L = __shfl_sync(kAll, lut_w, c);
-                        const uint32_t nv = word_src_over_x4(raw[q], L, has_alpha);
+                        const uint32_t nv = word_src_over_fma(raw[q], L, has_alpha);
                         raw[q] = c != 0 ? nv : raw[q];
                     }
                 } else {  // alpha formats: the alpha lane of src_over alone
@@ -690,7 +673,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     for (int q = 0; q < 8; q++) {
                         if (!((blocks >> q) & 1u)) continue;
                         const int c = cov[32 * q];
-                        const uint32_t sa = __shfl_sync(kAll, s.a, c);
+                        const uint32_t sa = __shfl_sync(kAll, lut_w, c);
                         if (c != 0) raw[q] = alpha_src_over(raw[q], sa, fmt);
                     }
                 }
@@ -751,7 +734,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     if (!((blocks >> q) & 1u)) continue;
-                    if (cov[32 * q] != 0) raw[q] = word_src_over_x4(raw[q], words[32 * q + lane], has_alpha);
+                    if (cov[32 * q] != 0) raw[q] = word_src_over_fma(raw[q], words[32 * q + lane], has_alpha);
                 }
                 __syncwarp();
                 for (int i = lane; i < kTileCols + kTileCols / 4; i += 32) words[i] = 0u;
@@ -829,8 +812,8 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 //    taken by a single warp: a warp that finishes a cheap row takes the
 //    next item at once instead of holding its CTA until the slowest warp of
 //    the tile is done.
-template <bool MULTI, bool CTA_ITEMS, bool PLAIN, bool GATHER = false>
-__global__ void __launch_bounds__(kRasterThreads, PLAIN ? 8 : 6) k_raster(const RasterArgs A) {
+template <bool MULTI, bool CTA_ITEMS, int MODE, bool GATHER = false>
+__global__ void __launch_bounds__(kRasterThreads, MODE != kGeneral ? 8 : 6) k_raster(const RasterArgs A) {
     extern __shared__ uint32_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *words = smem + warp * kWarpWords;
@@ -846,7 +829,7 @@ __global__ void __launch_bounds__(kRasterThreads, PLAIN ? 8 : 6) k_raster(const 
                 if (t >= A.n_items) break;
             }
             const int32_t tile = A.order ? A.order[t] : (int32_t)t;
-            raster_row<MULTI, PLAIN, GATHER>(A, tile, warp, lane, words);
+            raster_row<MULTI, MODE, GATHER>(A, tile, warp, lane, words);
             if (A.one_per_tile) break;
         }
     } else {
@@ -858,36 +841,33 @@ __global__ void __launch_bounds__(kRasterThreads, PLAIN ? 8 : 6) k_raster(const 
             const long long t = (long long)(item / kTileRows);
             const int32_t tile = A.order ? A.order[t] : (int32_t)t;
             __syncwarp();  // the previous item's reads of `words` are done before it is reset
-            raster_row<MULTI, PLAIN, GATHER>(A, tile, (int)(item % kTileRows), lane, words);
+            raster_row<MULTI, MODE, GATHER>(A, tile, (int)(item % kTileRows), lane, words);
         }
     }
 }
 
 static size_t raster_smem() { return sizeof(uint32_t) * kWarpWords * kTileRows; }
 
+template <int MODE, class F>
+static int of_mode(RasterVariant v, int k, F &&f) {
+    if (v.gather)  // (gathered edges come a tile per CTA)
+        return v.multi ? f(k_raster<true, true, MODE, true>, k) : f(k_raster<false, true, MODE, true>, k);
+    if (v.multi) return v.cta_items ? f(k_raster<true, true, MODE>, k) : f(k_raster<true, false, MODE>, k);
+    return v.cta_items ? f(k_raster<false, true, MODE>, k) : f(k_raster<false, false, MODE>, k);
+}
 template <class F>
 static int with_variant(RasterVariant v, F &&f) {
-    const int k = (v.gather ? 8 : 0) | (v.multi ? 4 : 0) | (v.cta_items ? 2 : 0) | (v.plain ? 1 : 0);
-    switch (k) {
-        case 0: return f(k_raster<false, false, false>, k);
-        case 1: return f(k_raster<false, false, true>, k);
-        case 2: return f(k_raster<false, true, false>, k);
-        case 3: return f(k_raster<false, true, true>, k);
-        case 4: return f(k_raster<true, false, false>, k);
-        case 5: return f(k_raster<true, false, true>, k);
-        case 6: return f(k_raster<true, true, false>, k);
-        case 7: return f(k_raster<true, true, true>, k);
-        case 10: return f(k_raster<false, true, false, true>, k);
-        case 11: return f(k_raster<false, true, true, true>, k);
-        case 14: return f(k_raster<true, true, false, true>, k);
-        case 15: return f(k_raster<true, true, true, true>, k);
-        default: return Z2D_ERR_INVALID_ARGUMENT;  // (gathered edges come a tile per CTA)
+    const int k = v.mode * 8 + ((v.gather ? 4 : 0) | (v.multi ? 2 : 0) | (v.cta_items ? 1 : 0));
+    switch (v.mode) {
+        case kPlain4x: return of_mode<kPlain4x>(v, k, f);
+        case kPlainDirect: return of_mode<kPlainDirect>(v, k, f);
+        default: return of_mode<kGeneral>(v, k, f);
     }
 }
 
 // A variant's resident CTAs per SM, asked once per variant.
 int raster_occupancy(Ctx &, RasterVariant v, int &ctas_per_sm) {
-    static std::atomic<int> cache[16];
+    static std::atomic<int> cache[24];
     return with_variant(v, [&](auto kernel, int k) -> int {
         int occ = cache[k].load(std::memory_order_relaxed);
         if (occ <= 0) {

@@ -8,6 +8,15 @@
 
 namespace z2dg {
 
+// The supersample mask value of a pixel whose 4x4 sample block has n covered
+// samples, as 8-bit alpha: the mask is alpha8, or the surface's own format
+// for alpha4/2/1 surfaces (supersample.zig:69-83), each covered sample is
+// opaque, and downsampleBuffer averages the 16 (surface.zig:447-469).
+Z2D_HD uint32_t ss_mask8(int n, int fmt) {
+    if (fmt >= Z2D_FORMAT_ALPHA4) return scale_alpha(((uint32_t)n * fmt_max(fmt)) / 16u, fmt_bits(fmt), 8);
+    return ((uint32_t)n * 255u) / 16u;
+}
+
 // An edge in the bin of one (fill, band): the f32 half of its DEdge and its
 // index, for the crossings that are evaluated in f64.
 struct BinEdge {
@@ -35,6 +44,7 @@ struct RasterArgs {
     const int32_t *band_count;  // per global band
     const int4 *band_fills;     // {fill, cull_x0, cull_x1, (fill, band) slot} per band, in call order
     const RasterFill *rfills;
+    const uint32_t *luts;       // 32 source words per fill (coverage_word)
     const TileRec *tiles;       // per tile (several surfaces only)
     const uint8_t *masks;
     int32_t n_jobs;
@@ -44,14 +54,42 @@ struct RasterArgs {
     int32_t one_per_tile;       // not persistent: CTA i draws the i-th tile of the queue
 };
 
+// What the fills of a batch have in common: pixel src_over fills
+// (FAST_PIXEL_SRC_OVER) none of which takes the exact path, all with 4x4
+// samples or all without anti-aliasing, or anything.
+enum : int { kGeneral = 0, kPlain4x = 1, kPlainDirect = 2 };
+inline int raster_mode(const FillCmd *fills, size_t n, bool any_exact) {
+    bool plain = !any_exact, direct = true, sampled = true;
+    for (size_t i = 0; i < n; i++) {
+        plain &= fills[i].fast_kind == FAST_PIXEL_SRC_OVER;
+        direct &= fills[i].aa == Z2D_AA_NONE;
+        sampled &= fills[i].aa != Z2D_AA_NONE;
+    }
+    return !plain ? kGeneral : sampled ? kPlain4x : direct ? kPlainDirect : kGeneral;
+}
+
+// The source word of a FAST_PIXEL_SRC_OVER fill for coverage k of a pixel:
+// the pixel at full coverage, dst_in(pixel, opacity(k)) below it; on the
+// alpha formats its alpha alone.  0 beyond full coverage.
+Z2D_HD uint32_t coverage_word(const FillCmd &F, int fmt, int k) {
+    const int full = F.aa == Z2D_AA_NONE ? 1 : 16;
+    if (k > full) return 0u;
+    I16 s = I16{F.src.pix.r & 0xFFu, F.src.pix.g & 0xFFu, F.src.pix.b & 0xFFu, F.src.pix.a & 0xFFu};
+    if (k < full) {
+        const uint32_t o = F.aa == Z2D_AA_SUPERSAMPLE_4X ? ss_mask8(k, fmt) : k == 0 ? 0u : (uint32_t)(k * 16 - 1);
+        s = I16{(s.r * o) / 255u, (s.g * o) / 255u, (s.b * o) / 255u, (s.a * o) / 255u};
+    }
+    return fmt <= Z2D_FORMAT_RGBA ? i16_to_word(s, word_order(fmt)) : s.a;
+}
+
 // How k_raster runs: `multi` for several surfaces, `cta_items` for a whole
-// tile per work item, `plain` when every fill of the batch is a pixel src_over
-// fill (FAST_PIXEL_SRC_OVER) and none takes the exact path; `gather` for bins
-// of edge indices and edges without their f32 fields, as the one-upload path's
-// host writes them (with records and fields from the host a call of 1,500
-// edges took 67 us instead of 56).
+// tile per work item, the mode, and `gather` for bins of edge indices and
+// edges without their f32 fields, as the one-upload path's host writes them
+// (with records and fields from the host a call of 1,500 edges took 67 us
+// instead of 56).
 struct RasterVariant {
-    bool multi, cta_items, plain, gather;
+    bool multi, cta_items, gather;
+    int mode;
 };
 int raster_occupancy(Ctx &c, RasterVariant v, int &ctas_per_sm);
 int raster_launch(Ctx &c, RasterVariant v, const RasterArgs &A, unsigned grid);
