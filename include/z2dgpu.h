@@ -428,6 +428,11 @@ Z2D_API int z2dgpu_png_encode(z2dgpu_ctx *ctx, const z2d_surface *surface, int32
  * Allocated like z2dgpu_png_encode's output. */
 Z2D_API int z2dgpu_png_scanlines(z2dgpu_ctx *ctx, const z2d_surface *surface, int32_t color_profile, uint8_t **out,
                                  size_t *out_len);
+/* The same into the caller's buffer of `cap` bytes; *out_len receives the
+ * size.  With out = NULL only the size is returned; a buffer that is too
+ * small is Z2D_ERR_OUT_OF_MEMORY (and *out_len the size it needs). */
+Z2D_API int z2dgpu_png_scanlines_into(z2dgpu_ctx *ctx, const z2d_surface *surface, int32_t color_profile, uint8_t *out,
+                                      size_t cap, size_t *out_len);
 /* Releases memory the library returned. */
 Z2D_API void z2dgpu_free(void *p);
 

@@ -75,3 +75,10 @@ def test_scene_export(oracle, name):
 def test_gamma_scene_export(oracle, name):
     scene, profile = EXPORT_SCENES[name]
     assert png.scanlines(scene(GpuBackend()), profile) == oracle.png_scanlines(scene(StrokeOracle(oracle)), profile)
+
+
+@pytest.mark.parametrize("w,h", [(1024, 1023), (1023, 1024), (1024, 1025), (2049, 1025), (3001, 1500)])
+def test_scanlines_in_pieces(oracle, w, h):
+    """Image data around and beyond the 4 MiB pieces it is read back in."""
+    s = _random_surface("rgba", w, h, w + h)
+    assert png.scanlines(s.to_device("cuda"), "srgb") == oracle.png_scanlines(s, "srgb")

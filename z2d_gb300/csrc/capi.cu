@@ -1469,9 +1469,11 @@ Z2D_API int z2dgpu_ctx_destroy(z2dgpu_ctx *c) {
     c->tune_collect(true);
     c->staging.release();
     c->readback.release();
+    c->export_stage.release();
     for (int i = 0; i < 2; i++) {
         c->small_stage[i].release();
         if (c->small_done[i]) cudaEventDestroy(c->small_done[i]);
+        if (c->export_done[i]) cudaEventDestroy(c->export_done[i]);
     }
     for (Ctx::Timer *t : {&c->t_raster, &c->t_composite, &c->t_flatten, &c->t_bins, &c->t_stroke, &c->t_export}) c->timer_collect(*t);
     if (c->copy_stream) {
@@ -1592,23 +1594,28 @@ Z2D_API int z2dgpu_stroke_contours(const z2d_node *nodes, size_t n_nodes, const 
     return Z2D_OK;
 }
 
-static int png_common(z2dgpu_ctx *c, const z2d_surface *surface, int32_t profile, bool file, uint8_t **out,
-                      size_t *out_len) {
-    if (!c || !out || !out_len) return Z2D_ERR_INVALID_ARGUMENT;
-    *out = nullptr;
-    *out_len = 0;
-    int rc = check_surface(surface);
+// Checks a PNG call's arguments and stages its surface.
+static int png_begin(z2dgpu_ctx *c, const z2d_surface *surface, int32_t profile, DevSurface &ds) {
+    const int rc = check_surface(surface);
     if (rc) return rc;
     if (profile != Z2D_PROFILE_NONE && profile != Z2D_PROFILE_LINEAR && profile != Z2D_PROFILE_SRGB) {
         set_error("png: bad color profile");
         return Z2D_ERR_INVALID_ARGUMENT;
     }
     Z2D_CUDA(cudaSetDevice(c->device));
+    return stage_in(*c, *surface, c->surface, ds);
+}
+
+Z2D_API int z2dgpu_png_encode(z2dgpu_ctx *c, const z2d_surface *surface, int32_t color_profile, uint8_t **out,
+                              size_t *out_len) {
+    if (!c || !out || !out_len) return Z2D_ERR_INVALID_ARGUMENT;
+    *out = nullptr;
+    *out_len = 0;
     DevSurface ds;
-    rc = stage_in(*c, *surface, c->surface, ds);
+    int rc = png_begin(c, surface, color_profile, ds);
     if (rc) return rc;
     std::vector<uint8_t> bytes;
-    rc = file ? png_file(*c, ds, profile, bytes) : png_scanlines(*c, ds, profile, bytes);
+    rc = png_file(*c, ds, color_profile, bytes);
     if (rc) return rc;
     uint8_t *p = static_cast<uint8_t *>(malloc(std::max<size_t>(1, bytes.size())));
     if (!p) return Z2D_ERR_OUT_OF_MEMORY;
@@ -1618,14 +1625,44 @@ static int png_common(z2dgpu_ctx *c, const z2d_surface *surface, int32_t profile
     return Z2D_OK;
 }
 
-Z2D_API int z2dgpu_png_encode(z2dgpu_ctx *c, const z2d_surface *surface, int32_t color_profile, uint8_t **out,
-                              size_t *out_len) {
-    return png_common(c, surface, color_profile, true, out, out_len);
-}
-
 Z2D_API int z2dgpu_png_scanlines(z2dgpu_ctx *c, const z2d_surface *surface, int32_t color_profile, uint8_t **out,
                                  size_t *out_len) {
-    return png_common(c, surface, color_profile, false, out, out_len);
+    if (!c || !out || !out_len) return Z2D_ERR_INVALID_ARGUMENT;
+    *out = nullptr;
+    *out_len = 0;
+    DevSurface ds;
+    int rc = png_begin(c, surface, color_profile, ds);
+    if (rc) return rc;
+    const size_t n = png_scanlines_size(ds.fmt, ds.w, ds.h);
+    uint8_t *p = static_cast<uint8_t *>(malloc(std::max<size_t>(1, n)));
+    if (!p) return Z2D_ERR_OUT_OF_MEMORY;
+    rc = png_scanlines(*c, ds, color_profile, p);
+    if (rc) {
+        free(p);
+        return rc;
+    }
+    *out = p;
+    *out_len = n;
+    return Z2D_OK;
+}
+
+Z2D_API int z2dgpu_png_scanlines_into(z2dgpu_ctx *c, const z2d_surface *surface, int32_t color_profile, uint8_t *out,
+                                      size_t cap, size_t *out_len) {
+    if (!c || !out_len) return Z2D_ERR_INVALID_ARGUMENT;
+    *out_len = 0;
+    int rc = check_surface(surface);
+    if (rc) return rc;
+    const size_t n = png_scanlines_size(surface->format, surface->width, surface->height);
+    if (!out || cap < n) {
+        *out_len = n;
+        return out ? Z2D_ERR_OUT_OF_MEMORY : Z2D_OK;
+    }
+    DevSurface ds;
+    rc = png_begin(c, surface, color_profile, ds);
+    if (rc) return rc;
+    rc = png_scanlines(*c, ds, color_profile, out);
+    if (!rc) *out_len = n;
+    return rc;
 }
 
 Z2D_API void z2dgpu_free(void *p) { free(p); }

@@ -121,6 +121,9 @@ struct Ctx {
     int small_slot = 0;
     DevBuf small_params;
     cudaEvent_t done = nullptr;
+    // PNG rows on their way back: two pinned slots and their copies' events
+    HostBuf export_stage;
+    cudaEvent_t export_done[2] = {nullptr, nullptr};
     // upload of a host surface overlapping the flatten kernels: the copy runs
     // on copy_stream after call_start (the call's first point on `stream`);
     // `stream` waits for surface_ready before the first kernel that reads the
@@ -147,7 +150,8 @@ struct Ctx {
 namespace z2dg {
 // The PNG exporter (png.cu): the unfiltered scanline stream of a device
 // surface as export_png.zig encodes it, and the whole PNG file.
-int png_scanlines(Ctx &c, const DevSurface &s, int profile, std::vector<uint8_t> &raw);
+size_t png_scanlines_size(int32_t fmt, int32_t w, int32_t h);
+int png_scanlines(Ctx &c, const DevSurface &s, int profile, uint8_t *out);
 int png_file(Ctx &c, const DevSurface &s, int profile, std::vector<uint8_t> &png);
 }  // namespace z2dg
 

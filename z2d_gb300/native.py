@@ -103,6 +103,9 @@ def load(build_if_missing: bool = True):
             getattr(lib, name).argtypes = [C.c_void_p, P(abi.z2d_surface), C.c_int32, P(P(C.c_uint8)),
                                            P(C.c_size_t)]
             getattr(lib, name).restype = C.c_int
+        lib.z2dgpu_png_scanlines_into.argtypes = [C.c_void_p, P(abi.z2d_surface), C.c_int32, C.c_void_p, C.c_size_t,
+                                                  P(C.c_size_t)]
+        lib.z2dgpu_png_scanlines_into.restype = C.c_int
         lib.z2dgpu_free.argtypes = [C.c_void_p]
         lib.z2dgpu_free.restype = None
         lib.z2dgpu_gradient_offsets.argtypes = [C.c_void_p, P(abi.z2d_gradient), C.c_int32, C.c_int32, C.c_int32,
