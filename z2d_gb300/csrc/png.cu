@@ -46,6 +46,66 @@ __device__ __forceinline__ uint32_t srgb_encode(uint32_t c, bool gamma) {
     return (uint32_t)roundf(255.0f * v);
 }
 
+// Rows of the formats with four output bytes (RGBA, ARGB).  A warp takes 128
+// neighbouring pixels of a row, a lane 32 apart; the pixels' bytes start at
+// any byte (1 + 4 W bytes a row), so each lane shifts its left neighbour's
+// last bytes in front of its own and stores aligned words; only the ends of
+// a warp's run are stored byte by byte.  The gamma of a channel byte comes
+// from a table (std.math.pow was most of the kernel).  2561x1441 with the
+// sRGB profile: 34 us, a thread per pixel with byte stores and pow 57.
+constexpr int kRowGroups = 4;
+__global__ void __launch_bounds__(256) k_png_rgba(DevSurface s, int srgb, uint8_t *__restrict__ out,
+                                                  long long row_bytes, int32_t per_row, long long n_chunks) {
+    __shared__ uint8_t enc[256];
+    enc[threadIdx.x] = (uint8_t)(srgb ? srgb_encode(threadIdx.x, true) : threadIdx.x);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint32_t *px = reinterpret_cast<const uint32_t *>(s.data);
+    for (long long c = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); c < n_chunks; c += (long long)gridDim.x * 8) {
+        const int32_t y = (int32_t)(c / per_row), x0 = (int32_t)(c - (long long)y * per_row) * (32 * kRowGroups);
+        uint32_t w[kRowGroups];
+#pragma unroll
+        for (int q = 0; q < kRowGroups; q++) {
+            const int32_t x = x0 + 32 * q + lane;
+            w[q] = x < s.w ? px[(size_t)y * s.w + x] : 0u;
+        }
+        uint8_t *row = out + y * row_bytes;
+        if (x0 == 0 && lane == 0) row[0] = 0;  // filter type: none
+        const int sh = (int)((reinterpret_cast<uintptr_t>(row) + 1) & 3);
+        uint32_t carry = 0;  // the pixel before this group's first
+#pragma unroll
+        for (int q = 0; q < kRowGroups; q++) {
+            const int32_t x = x0 + 32 * q + lane;
+            const I16 p = word_to_i16(w[q], s.fmt);
+            // RGBA16.demultiply (pixel_vector.zig:27-60): x / a as
+            // umulhi(x, ceil(2^32 / a)), exact for x <= 255 * 255 (the error
+            // x / 2^32 stays below 1 / a); alpha encodes to itself
+            const uint32_t m = p.a > 1u ? 0xFFFFFFFFu / p.a + 1u : 0u;
+            auto channel = [&](uint32_t v) -> uint32_t {
+                v = p.a == 0 ? 0u : p.a == 1 ? v * 255u : __umulhi(v * 255u, m);
+                return v < 256u ? enc[v] : (srgb ? srgb_encode(v, true) : v) & 0xFFu;
+            };
+            const uint32_t v = channel(p.r) | (channel(p.g) << 8) | (channel(p.b) << 16) | (p.a << 24);
+            const uint32_t up = __shfl_up_sync(0xffffffffu, v, 1), last = __shfl_sync(0xffffffffu, v, 31);
+            const uint32_t prev = lane == 0 ? carry : up;
+            carry = last;
+            if (x >= s.w) continue;
+            uint8_t *o = row + 1 + 4ll * x;
+            if (sh == 0) {
+                *reinterpret_cast<uint32_t *>(o) = v;
+                continue;
+            }
+            if (x == x0) {  // the run's first pixel: its bytes up to the next word
+                for (int b = 0; b < 4 - sh; b++) o[b] = (uint8_t)(v >> (8 * b));
+            } else {
+                *reinterpret_cast<uint32_t *>(o - sh) = (prev >> (8 * (4 - sh))) | (v << (8 * sh));
+            }
+            if (x == s.w - 1 || x == x0 + 32 * kRowGroups - 1)  // and the last one's beyond its word
+                for (int b = 4 - sh; b < 4; b++) o[b] = (uint8_t)(v >> (8 * b));
+        }
+    }
+}
+
 __global__ void k_png_rows(DevSurface s, int srgb, uint8_t *__restrict__ out, long long row_bytes,
                            long long units_per_row, long long n_units) {
     const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -65,29 +125,16 @@ __global__ void k_png_rows(DevSurface s, int srgb, uint8_t *__restrict__ out, lo
     if (fmt <= Z2D_FORMAT_RGBA) {
         const uint32_t w = reinterpret_cast<const uint32_t *>(s.data)[(size_t)y * s.w + k];
         const I16 p = word_to_i16(w, fmt);
-        uint32_t r = p.r, g = p.g, b = p.b, a = p.a;
-        const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
-        if (has_alpha) {  // RGBA16.demultiply (pixel_vector.zig:27-60)
-            // x / a as umulhi(x, ceil(2^32 / a)): exact for x <= 255 * 255
-            // (the error x / 2^32 stays below 1 / a)
-            const uint32_t m = a > 1u ? 0xFFFFFFFFu / a + 1u : 0u;
-            r = a == 0 ? 0 : (a == 1 ? r * 255u : __umulhi(r * 255u, m));
-            g = a == 0 ? 0 : (a == 1 ? g * 255u : __umulhi(g * 255u, m));
-            b = a == 0 ? 0 : (a == 1 ? b * 255u : __umulhi(b * 255u, m));
-        } else {
-            a = 255;
-        }
-        if (srgb) {
+        uint32_t r = p.r, g = p.g, b = p.b;
+        if (srgb) {  // RGB, XRGB (k_png_rgba takes the formats with alpha)
             r = srgb_encode(r, true);
             g = srgb_encode(g, true);
             b = srgb_encode(b, true);
-            a = srgb_encode(a, false);
         }
-        uint8_t *o = row + 1 + k * (has_alpha ? 4 : 3);
+        uint8_t *o = row + 1 + k * 3;
         o[0] = (uint8_t)r;
         o[1] = (uint8_t)g;
         o[2] = (uint8_t)b;
-        if (has_alpha) o[3] = (uint8_t)a;
     } else if (fmt == Z2D_FORMAT_ALPHA8) {
         row[1 + k] = s.data[(size_t)y * s.w + k];
     } else {  // one output byte: 8 / bits pixels, the first in the high bits
@@ -238,7 +285,15 @@ int png_scanlines(Ctx &c, const DevSurface &s, int profile, uint8_t *out) {
         if (!e) Z2D_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     uint8_t *d = c.surface2.as<uint8_t>(), *stage = c.export_stage.as<uint8_t>();
     const long long n_units = units * s.h;
-    if (n_units > 0) {
+    if (fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB) {
+        const int32_t per_row = (s.w + 32 * kRowGroups - 1) / (32 * kRowGroups);
+        const long long chunks = (long long)per_row * s.h;
+        cudaEvent_t te = c.timer_begin(c.t_export);
+        k_png_rgba<<<(unsigned)std::min<long long>((chunks + 7) / 8, (long long)c.sm_count * 8), 256, 0, c.stream>>>(
+            s, profile == Z2D_PROFILE_SRGB ? 1 : 0, d, row_bytes, per_row, chunks);
+        c.timer_end(c.t_export, te);
+        c.launches++;
+    } else if (n_units > 0) {
         cudaEvent_t te = c.timer_begin(c.t_export);
         k_png_rows<<<(unsigned)((n_units + 255) / 256), 256, 0, c.stream>>>(s, profile == Z2D_PROFILE_SRGB ? 1 : 0, d,
                                                                           row_bytes, units, n_units);
