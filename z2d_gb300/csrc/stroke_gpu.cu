@@ -12,8 +12,6 @@
 // host builder; the curve subdivision is spline.cuh, shared with fills.
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
-#include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
 
 #include "edges.cuh"
 #include "spline.cuh"
@@ -39,9 +37,31 @@ struct SubState {
     int32_t kind;    // SK_*
     int32_t pcw;     // direction of the first join (the plotter's `clockwise`)
 };
-// per stroke: its outer points [a0, a0 + na) and inner points [b0, b0 + nb)
-struct StrokeTot {
-    long long a0, na, b0, nb;
+// counts or offsets of outer (a) and inner (b) contour points
+struct Count2 {
+    long long a, b;
+};
+struct Sum2 {
+    __host__ __device__ __forceinline__ Count2 operator()(const Count2 &x, const Count2 &y) const {
+        return Count2{x.a + y.a, x.b + y.b};
+    }
+};
+// per subpath: its outer points [ra, ra + sa) and inner points
+// [rb, rb + sb), the fill that draws it and what turns a point's position
+// into its edge's index within that fill
+struct Region {
+    int32_t ra, sa, rb, sb;
+    int32_t fill, edge_a, edge_b, closed;
+};
+// The points of an element that is a join, found when it is counted: the
+// outer side's first and last point with a run of pen vertices around the
+// join's point between them, the inner side's first and last point with the
+// join's point between them.
+enum : int32_t { EL_JOIN = 1, EL_SWITCHED = 2, EL_CW = 4, EL_TWO_OUTER = 8, EL_THREE_INNER = 16 };
+struct Elem {
+    Pt o1, o2, i1, i2;
+    int32_t start, cnt;  // pen vertices
+    int32_t flags, _pad;
 };
 
 // device pointers of one run
@@ -50,19 +70,21 @@ struct State {
     int g;                          // log2 of the lanes that share a node
     PenVertex *pen;                 // n_pen
     SubState *sub;                  // n_subs
-    StrokeTot *tot;                 // n_strokes
+    Region *region;                 // n_subs
     long long *totals;              // outer, inner totals (read back)
     // sized by the raw point count R
     double2 *raw_pt;
     int32_t *raw_sub;
     uint8_t *raw_mode;
-    int32_t *kept_off;              // R + 1
+    int32_t *keep, *kept_off;       // R + 1
     double2 *q_pt;
     int32_t *q_sub;
     uint8_t *q_mode;
-    long long *cnt_a, *cnt_b, *off_a, *off_b;  // R + 1
-    // contour points
+    Elem *elem;                     // R
+    Count2 *cnt, *off;              // R + 1
+    // contour points, and each one's subpath
     double2 *pa, *pb;
+    int32_t *a_sub, *b_sub;
 };
 
 __device__ __forceinline__ Tf tf_of(const StrokeDev &s) {
@@ -75,36 +97,39 @@ __device__ __forceinline__ Pt node_end(const z2d_node &nd) {
 // ----------------------------------------------------------------- pens
 // Pen.init (Pen.zig:25-88) from the host's cos/sin table: vertex points
 // through the CTM, then the slopes to either neighbour.
-__global__ void ks_pen(const StrokeDev *__restrict__ strokes, int32_t n_strokes, const double *__restrict__ trig,
+// A block per stroke, a thread per vertex (each evaluates its neighbours'
+// points again, which gives the same bits).
+__global__ void ks_pen(const StrokeDev *__restrict__ strokes, const double *__restrict__ trig,
                        PenVertex *__restrict__ pen) {
-    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_strokes) return;
-    const StrokeDev S = strokes[s];
+    const StrokeDev &S = strokes[blockIdx.x];
     const int32_t n = S.pen_n;
-    if (n <= 0) return;
     const Tf ctm = tf_of(S);
     const double radius = S.thickness / 2;
     PenVertex *v = pen + S.pen_off;
     const double *t = trig + 2 * (size_t)S.pen_tab;
-    for (int32_t i = 0; i < n; i++) {
+    auto point = [&](int32_t i) {
         double dx = radius * t[2 * i], dy = radius * t[2 * i + 1];
         sg::user_to_device_distance(ctm, dx, dy);
-        v[i].point = Pt{dx, dy};
-    }
-    for (int32_t i = 0; i < n; i++) {
+        return Pt{dx, dy};
+    };
+    for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const int32_t next = (i >= n - 1) ? 0 : i + 1;
         const int32_t prev = max(0, i == 0 ? n - 1 : i - 1);
-        v[i].slope_cw = sg::slope(v[prev].point, v[i].point);
-        v[i].slope_ccw = sg::slope(v[i].point, v[next].point);
+        PenVertex p;
+        p.point = point(i);
+        p.slope_cw = sg::slope(point(prev), p.point);
+        p.slope_ccw = sg::slope(p.point, point(next));
+        v[i] = p;
     }
 }
 
 // ------------------------------------------------------------ raw points
+// A warp per subpath.
 __global__ void ks_local_sub(const SubpathDev *__restrict__ subs, int32_t n_subs, int32_t *__restrict__ local_sub) {
-    const int32_t sp = blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t sp = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (sp >= n_subs) return;
-    const SubpathDev S = subs[sp];
-    for (int32_t j = 0; j < S.n_nodes; j++) local_sub[S.local0 + j] = sp;
+    const int32_t l0 = subs[sp].local0, n = subs[sp].n_nodes;
+    for (int32_t j = threadIdx.x & 31; j < n; j += 32) local_sub[l0 + j] = sp;
 }
 
 // The points one node hands to the plotter: move_to its point, line_to its
@@ -185,26 +210,30 @@ __global__ void ks_raw_emit(const z2d_node *__restrict__ nodes, const SubpathDev
 
 // Whether the plotter keeps raw point r: the degenerate-node check against
 // the point before it of the same subpath.
-struct Keep {
-    const double2 *pt;
-    const int32_t *sub;
-    long long n;
-    __host__ __device__ __forceinline__ int32_t operator()(long long r) const {
-        if (r >= n) return 0;
-        if (r == 0 || sub[r] != sub[r - 1]) return 1;
-        const double2 a = pt[r - 1], b = pt[r];
-        return pt_eq(a.x, a.y, b.x, b.y) ? 0 : 1;
+__global__ void ks_keep(const double2 *__restrict__ raw_pt, const int32_t *__restrict__ raw_sub, long long n_raw,
+                        int32_t *__restrict__ keep) {
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > n_raw) return;
+    int32_t k = 0;
+    if (r < n_raw) {
+        k = 1;
+        if (r > 0 && raw_sub[r] == raw_sub[r - 1]) {
+            const double2 a = raw_pt[r - 1], b = raw_pt[r];
+            k = pt_eq(a.x, a.y, b.x, b.y) ? 0 : 1;
+        }
     }
-};
+    keep[r] = k;
+}
 
-__global__ void ks_compact(const Keep keep, const uint8_t *__restrict__ raw_mode,
-                           const int32_t *__restrict__ kept_off, double2 *__restrict__ q_pt,
+__global__ void ks_compact(const double2 *__restrict__ raw_pt, const int32_t *__restrict__ raw_sub,
+                           const uint8_t *__restrict__ raw_mode, const int32_t *__restrict__ keep,
+                           const int32_t *__restrict__ kept_off, long long n_raw, double2 *__restrict__ q_pt,
                            int32_t *__restrict__ q_sub, uint8_t *__restrict__ q_mode) {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= keep.n || !keep(r)) return;
+    if (r >= n_raw || !keep[r]) return;
     const int32_t q = kept_off[r];
-    q_pt[q] = keep.pt[r];
-    q_sub[q] = keep.sub[r];
+    q_pt[q] = raw_pt[r];
+    q_sub[q] = raw_sub[r];
     q_mode[q] = raw_mode[r];
 }
 
@@ -268,46 +297,38 @@ struct Out {
 };
 
 // join (stroke_plotter.zig:405-545) at p1 between p0->p1 and p1->p2, with
-// the subpath's first-join direction pcw.
-template <class O>
-__device__ __forceinline__ void join(O &o, const StrokeDev &T, const Tf &ctm, const PenVertex *pen, int mode, Pt p0,
-                                     Pt p1, Pt p2, bool pcw) {
-    if (sg::eq(p0, p1) || sg::eq(p1, p2)) return;
+// the subpath's first-join direction pcw: where outer and inner trade places
+// (EL_SWITCHED) the outer points go to the inner contour.
+__device__ __forceinline__ Elem join(const StrokeDev &T, const Tf &ctm, const PenVertex *pen, int mode, Pt p0, Pt p1,
+                                     Pt p2, bool pcw) {
+    Elem e;
+    e.start = e.cnt = 0;
+    e.flags = 0;
+    if (sg::eq(p0, p1) || sg::eq(p1, p2)) return e;
     const Face in = sg::face_init(p0, p1, T.thickness, ctm);
     const Face out = sg::face_init(p1, p2, T.thickness, ctm);
     const int cmp = sg::compare(in.dev_slope, out.dev_slope);
     const bool jcw = cmp < 0;
-    const bool sw = jcw != pcw;  // outer and inner trade places
-    auto outer = [&](Pt p) {
-        if (sw) o.B(p);
-        else o.A(p);
-    };
-    auto inner = [&](Pt p) {
-        if (sw) o.A(p);
-        else o.B(p);
-    };
-    if (cmp == 0) {
-        outer(jcw ? in.p1_ccw : in.p1_cw);
-        inner(jcw ? in.p1_cw : in.p1_ccw);
-        return;
+    e.flags = EL_JOIN | (jcw != pcw ? EL_SWITCHED : 0) | (jcw ? EL_CW : 0);
+    e.o1 = jcw ? in.p1_ccw : in.p1_cw;
+    e.i1 = jcw ? in.p1_cw : in.p1_ccw;
+    if (cmp == 0) return e;
+    e.flags |= EL_THREE_INNER;
+    e.i2 = jcw ? out.p0_cw : out.p0_ccw;
+    if (mode == Z2D_JOIN_MITER && sg::compare_for_miter_limit(in.dev_slope, out.dev_slope, T.miter_limit)) {
+        e.o1 = sg::intersect(in, out, jcw);
+        return e;
     }
-    if (mode == Z2D_JOIN_MITER || mode == Z2D_JOIN_BEVEL) {
-        if (mode == Z2D_JOIN_MITER && sg::compare_for_miter_limit(in.dev_slope, out.dev_slope, T.miter_limit)) {
-            outer(sg::intersect(in, out, jcw));
-        } else {
-            outer(jcw ? in.p1_ccw : in.p1_cw);
-            outer(jcw ? out.p0_ccw : out.p0_cw);
-        }
-    } else {
-        outer(jcw ? in.p1_ccw : in.p1_cw);
-        int32_t start;
-        const int32_t cnt = sg::pen_range(pen, T.pen_n, in.dev_slope, out.dev_slope, jcw, start);
-        o.pen(!sw, p1, pen, T.pen_n, start, cnt, jcw);
-        outer(jcw ? out.p0_ccw : out.p0_cw);
-    }
-    inner(jcw ? in.p1_cw : in.p1_ccw);
-    inner(p1);
-    inner(jcw ? out.p0_cw : out.p0_ccw);
+    e.flags |= EL_TWO_OUTER;
+    e.o2 = jcw ? out.p0_ccw : out.p0_cw;
+    if (mode != Z2D_JOIN_MITER && mode != Z2D_JOIN_BEVEL)
+        e.cnt = sg::pen_range(pen, T.pen_n, in.dev_slope, out.dev_slope, jcw, e.start);
+    return e;
+}
+__device__ __forceinline__ Count2 join_count(const Elem &e) {
+    if (!(e.flags & EL_JOIN)) return Count2{0, 0};
+    const long long o = 1 + e.cnt + ((e.flags & EL_TWO_OUTER) ? 1 : 0), i = (e.flags & EL_THREE_INNER) ? 3 : 1;
+    return (e.flags & EL_SWITCHED) ? Count2{i, o} : Count2{o, i};
 }
 
 // Face.cap (Face.zig:156-246), to A
@@ -335,9 +356,10 @@ __device__ __forceinline__ void cap(O &o, const StrokeDev &T, const Tf &ctm, con
     }
 }
 
-// Everything element k of a subpath contributes (see stroke_gpu.cuh).
+// What element k of a subpath contributes (see stroke_gpu.cuh): caps and dots
+// go to `o`, a join is returned (flags 0: none).
 template <class O>
-__device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVertex *pen, const SubState &st,
+__device__ __forceinline__ Elem element(O &o, const StrokeDev &T, const PenVertex *pen, const SubState &st,
                                         const double2 *__restrict__ q_pt, const uint8_t *__restrict__ q_mode,
                                         int32_t k) {
     const int32_t n = st.n;
@@ -350,6 +372,8 @@ __device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVerte
     // Every case below draws at most two caps or one join; they are
     // gathered into one cap call and one join call, so that the kernel
     // holds a single copy of each.
+    Elem none;
+    none.flags = none.cnt = 0;
     int n_caps = 0, jmode = -1;
     Pt c0{}, c1{}, j0{}, j1{}, j2{};
     bool ccw = pcw;
@@ -359,9 +383,9 @@ __device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVerte
                 const Pt c = P(0);
                 for (int32_t i = 0; i < T.pen_n; i++) o.A(Pt{c.x + pen[i].point.x, c.y + pen[i].point.y});
             }
-            return;
+            return none;
         case SK_SINGLE:  // plotSingle (stroke_plotter.zig:232-279): caps of b->a, then a->b
-            if (k != 0) return;
+            if (k != 0) return none;
             n_caps = 2;
             c0 = P(1);
             c1 = P(0);
@@ -391,7 +415,7 @@ __device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVerte
                 j1 = P(k);
                 j2 = P(k + 1);
             } else if (k == n - 1) {
-                if (back_to_start) return;
+                if (back_to_start) return none;
                 jmode = T.join;
                 j0 = P(n - 2);
                 j1 = P(n - 1);
@@ -404,7 +428,7 @@ __device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVerte
             }
             break;
         }
-        default: return;
+        default: return none;
     }
 #pragma unroll 1
     for (int i = 0; i < n_caps; i++) {
@@ -413,152 +437,162 @@ __device__ __forceinline__ void element(O &o, const StrokeDev &T, const PenVerte
         c0 = c1;
         c1 = t;
     }
-    if (jmode >= 0) join(o, T, ctm, pen, jmode, j0, j1, j2, pcw);
+    if (jmode >= 0) return join(T, ctm, pen, jmode, j0, j1, j2, pcw);
+    return none;
 }
 
 __global__ void ks_elem_count(const SubpathDev *__restrict__ subs, const StrokeDev *__restrict__ strokes,
                               const PenVertex *__restrict__ pen, const SubState *__restrict__ sub,
                               const double2 *__restrict__ q_pt, const int32_t *__restrict__ q_sub,
                               const uint8_t *__restrict__ q_mode, const int32_t *__restrict__ kept_off,
-                              long long n_raw, long long *__restrict__ cnt_a, long long *__restrict__ cnt_b) {
+                              long long n_raw, Elem *__restrict__ elem, Count2 *__restrict__ cnt) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q > n_raw) return;
     const long long n_kept = kept_off[n_raw];
     if (q >= n_kept) {
-        cnt_a[q] = 0;
-        cnt_b[q] = 0;
+        cnt[q] = Count2{0, 0};
         return;
     }
     const int32_t sp = q_sub[q];
     const SubState st = sub[sp];
     const StrokeDev T = strokes[subs[sp].stroke];
     Out<false> o;
-    element(o, T, pen + T.pen_off, st, q_pt, q_mode, (int32_t)(q - st.q0));
-    cnt_a[q] = o.na;
-    cnt_b[q] = o.nb;
+    const Elem e = element(o, T, pen + T.pen_off, st, q_pt, q_mode, (int32_t)(q - st.q0));
+    elem[q] = e;
+    cnt[q] = (e.flags & EL_JOIN) ? join_count(e) : Count2{o.na, o.nb};
 }
 
+// Per stroke its edge count, per subpath its regions of the contour arrays.
 __global__ void ks_stroke_tot(const StrokeDev *__restrict__ strokes, int32_t n_strokes,
-                              const SubState *__restrict__ sub, const long long *__restrict__ off_a,
-                              const long long *__restrict__ off_b, long long n_raw, StrokeTot *__restrict__ tot,
+                              const SubpathDev *__restrict__ subs, int32_t n_subs, const SubState *__restrict__ sub,
+                              const Count2 *__restrict__ off, long long n_raw, Region *__restrict__ region,
                               int32_t *__restrict__ stroke_edges, long long *__restrict__ totals) {
-    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) {
-        totals[0] = off_a[n_raw];
-        totals[1] = off_b[n_raw];
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        totals[0] = off[n_raw].a;
+        totals[1] = off[n_raw].b;
     }
-    if (s >= n_strokes) return;
-    const StrokeDev S = strokes[s];
-    StrokeTot t{0, 0, 0, 0};
-    if (S.n_sub > 0) {
-        const int32_t e0 = sub[S.sub0].q0;
+    // the stroke's points: [first, last) of the kept points
+    auto ends = [&](const StrokeDev &S, Count2 &c0, Count2 &c1) {
         const SubState last = sub[S.sub0 + S.n_sub - 1];
-        const int32_t e1 = last.q0 + last.n;
-        t.a0 = off_a[e0];
-        t.na = off_a[e1] - t.a0;
-        t.b0 = off_b[e0];
-        t.nb = off_b[e1] - t.b0;
+        c0 = off[sub[S.sub0].q0];
+        c1 = off[last.q0 + last.n];
+    };
+    if (i < n_strokes) {
+        const StrokeDev &S = strokes[i];
+        Count2 c0{0, 0}, c1{0, 0};
+        if (S.n_sub > 0) ends(S, c0, c1);
+        const long long e = (c1.a - c0.a) + (c1.b - c0.b);
+        stroke_edges[i] = e > 0x7FFFFFFFll ? -1 : (int32_t)e;
     }
-    tot[s] = t;
-    const long long e = t.na + t.nb;
-    stroke_edges[s] = e > 0x7FFFFFFFll ? -1 : (int32_t)e;
+    if (i < n_subs) {
+        const StrokeDev &S = strokes[subs[i].stroke];
+        const SubState st = sub[i];
+        Count2 c0, c1;
+        ends(S, c0, c1);
+        const Count2 r0 = off[st.q0], r1 = off[st.q0 + st.n];
+        Region R;
+        R.ra = (int32_t)r0.a;
+        R.sa = (int32_t)(r1.a - r0.a);
+        R.rb = (int32_t)r0.b;
+        R.sb = (int32_t)(r1.b - r0.b);
+        R.fill = S.fill;
+        R.edge_a = (int32_t)-c0.a;
+        R.edge_b = (int32_t)(c1.a - c0.a - c0.b);
+        R.closed = st.kind == SK_CLOSED ? 1 : 0;
+        region[i] = R;
+    }
 }
 
-// Region layout of one element: where its A points start and where its B
-// points end (B points are stored in contour order, i.e. reversed).
-struct Place {
-    long long ra, sa, rb, sb;  // the subpath's outer and inner regions
-    long long pos_a, end_b;
-};
-__device__ __forceinline__ Place place(const SubState &st, int32_t k, long long q, const long long *__restrict__ off_a,
-                                       const long long *__restrict__ off_b) {
-    Place p;
-    p.ra = off_a[st.q0];
-    p.sa = off_a[st.q0 + st.n] - p.ra;
-    p.rb = off_b[st.q0];
-    p.sb = off_b[st.q0 + st.n] - p.rb;
-    long long t_b;
-    if (st.kind == SK_CLOSED) {
-        // the closing joins come last: elements 1..n-1, then 0
-        const long long a0 = off_a[st.q0 + 1] - p.ra, b0 = off_b[st.q0 + 1] - p.rb;
-        p.pos_a = k >= 1 ? off_a[q] - a0 : p.ra + p.sa - a0;
-        t_b = k >= 1 ? off_b[q] - p.rb - b0 : p.sb - b0;
-    } else {
-        p.pos_a = off_a[q];
-        t_b = off_b[q] - p.rb;
-    }
-    p.end_b = p.rb + p.sb - t_b;
-    return p;
-}
-
+// Writes every element's points to their contour positions: outer points in
+// element order, inner points in reverse (B points are prepended); a closed
+// subpath's closing joins come last: elements 1..n-1, then 0.
 __global__ void ks_elem_emit(const SubpathDev *__restrict__ subs, const StrokeDev *__restrict__ strokes,
                              const PenVertex *__restrict__ pen, const SubState *__restrict__ sub,
-                             const double2 *__restrict__ q_pt, const int32_t *__restrict__ q_sub,
-                             const uint8_t *__restrict__ q_mode, const int32_t *__restrict__ kept_off, long long n_raw,
-                             const long long *__restrict__ off_a, const long long *__restrict__ off_b,
-                             double2 *__restrict__ pa, double2 *__restrict__ pb) {
+                             const Region *__restrict__ region, const double2 *__restrict__ q_pt,
+                             const int32_t *__restrict__ q_sub, const uint8_t *__restrict__ q_mode,
+                             const int32_t *__restrict__ kept_off, long long n_raw, const Elem *__restrict__ elem,
+                             const Count2 *__restrict__ off, double2 *__restrict__ pa, double2 *__restrict__ pb,
+                             int32_t *__restrict__ a_sub, int32_t *__restrict__ b_sub) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= kept_off[n_raw]) return;
     const int32_t sp = q_sub[q];
     const SubState st = sub[sp];
+    const Region R = region[sp];
     const int32_t k = (int32_t)(q - st.q0);
-    const StrokeDev T = strokes[subs[sp].stroke];
-    const Place pl = place(st, k, q, off_a, off_b);
+    const StrokeDev &T = strokes[subs[sp].stroke];
+    const Count2 at = off[q], next = off[q + 1];
+    const long long na = next.a - at.a, nb = next.b - at.b;
+    long long pos_a = at.a, t_b = at.b - R.rb;
+    if (st.kind == SK_CLOSED) {
+        const Count2 o1 = off[st.q0 + 1];
+        const long long a0 = o1.a - R.ra, b0 = o1.b - R.rb;
+        pos_a = k >= 1 ? at.a - a0 : R.ra + R.sa - a0;
+        t_b = k >= 1 ? at.b - R.rb - b0 : R.sb - b0;
+    }
+    const long long end_b = (long long)R.rb + R.sb - t_b;
+    for (long long i = 0; i < na; i++) a_sub[pos_a + i] = sp;
+    for (long long i = 0; i < nb; i++) b_sub[end_b - 1 - i] = sp;
+    const Elem e = elem[q];
     Out<true> o;
-    o.pa = pa + pl.pos_a;
-    o.pb_end = pb + pl.end_b;
+    o.pa = pa + pos_a;
+    o.pb_end = pb + end_b;
     o.scale = T.scale;
-    element(o, T, pen + T.pen_off, st, q_pt, q_mode, k);
+    if (!(e.flags & EL_JOIN)) {  // caps and dots
+        if (na + nb > 0) {
+            const StrokeDev S = T;
+            element(o, S, pen + S.pen_off, st, q_pt, q_mode, k);
+        }
+        return;
+    }
+    const bool sw = (e.flags & EL_SWITCHED) != 0;
+    auto outer = [&](Pt p) {
+        if (sw) o.B(p);
+        else o.A(p);
+    };
+    auto inner = [&](Pt p) {
+        if (sw) o.A(p);
+        else o.B(p);
+    };
+    const double2 c = q_pt[q];
+    const Pt p1{c.x, c.y};
+    outer(e.o1);
+    if (e.cnt > 0) o.pen(!sw, p1, pen + T.pen_off, T.pen_n, e.start, e.cnt, (e.flags & EL_CW) != 0);
+    if (e.flags & EL_TWO_OUTER) outer(e.o2);
+    inner(e.i1);
+    if (e.flags & EL_THREE_INNER) {
+        inner(p1);
+        inner(e.i2);
+    }
 }
 
 // Polygon.addEdgesFromContour: every contour point to the next one (the
-// last back to the first).  An open subpath's contour is its outer region
-// followed by its inner region.
-__global__ void ks_edges(const SubpathDev *__restrict__ subs, const StrokeDev *__restrict__ strokes,
-                         const SubState *__restrict__ sub, const int32_t *__restrict__ q_sub,
-                         const int32_t *__restrict__ kept_off, long long n_raw, const long long *__restrict__ cnt_a,
-                         const long long *__restrict__ cnt_b, const long long *__restrict__ off_a,
-                         const long long *__restrict__ off_b, const StrokeTot *__restrict__ tot,
-                         const double2 *__restrict__ pa, const double2 *__restrict__ pb,
+// last back to the first), a thread per point.  An open subpath's contour is
+// its outer region followed by its inner region.
+__global__ void ks_edges(const Region *__restrict__ region, const double2 *__restrict__ pa,
+                         const double2 *__restrict__ pb, const int32_t *__restrict__ a_sub,
+                         const int32_t *__restrict__ b_sub, long long n_a, long long n_b,
                          const FillCmd *__restrict__ fills, FillState *__restrict__ st_fill,
                          DEdge *__restrict__ edges) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = q < kept_off[n_raw];
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t f = -1;
     double et = 0, eb = 0, el = 0, er = 0;
     bool any = false;
-    if (live) {
-        const int32_t sp = q_sub[q];
-        const SubState st = sub[sp];
-        const int32_t k = (int32_t)(q - st.q0);
-        const int32_t s = subs[sp].stroke;
-        f = strokes[s].fill;
-        const FillCmd F = fills[f];
-        const StrokeTot t = tot[s];
-        const Place pl = place(st, k, q, off_a, off_b);
-        DEdge *out = edges + st_fill[f].edge_base;
-        const bool closed = st.kind == SK_CLOSED;
-        const long long na = cnt_a[q], nb = cnt_b[q];
-        for (long long i = 0; i < na; i++) {
-            const long long pos = pl.pos_a + i;
-            const double2 a = pa[pos];
-            long long nx = pos + 1;
-            double2 b;
-            if (nx < pl.ra + pl.sa) b = pa[nx];
-            else if (!closed && pl.sb > 0) b = pb[pl.rb];
-            else b = pa[pl.ra];
-            add_edge(F, out + (pos - t.a0), a.x, a.y, b.x, b.y, et, eb, el, er, any);
+    if (t < n_a + n_b) {
+        const bool outer = t < n_a;
+        const int32_t pos = (int32_t)(outer ? t : t - n_a);
+        const Region R = region[outer ? a_sub[pos] : b_sub[pos]];
+        f = R.fill;
+        double2 a, b;
+        if (outer) {
+            a = pa[pos];
+            b = pos + 1 < R.ra + R.sa ? pa[pos + 1] : !R.closed && R.sb > 0 ? pb[R.rb] : pa[R.ra];
+        } else {
+            a = pb[pos];
+            b = pos + 1 < R.rb + R.sb ? pb[pos + 1] : !R.closed ? pa[R.ra] : pb[R.rb];
         }
-        for (long long i = 0; i < nb; i++) {
-            const long long pos = pl.end_b - nb + i;
-            const double2 a = pb[pos];
-            long long nx = pos + 1;
-            double2 b;
-            if (nx < pl.rb + pl.sb) b = pb[nx];
-            else if (!closed) b = pa[pl.ra];
-            else b = pb[pl.rb];
-            add_edge(F, out + (t.na + pos - t.b0), a.x, a.y, b.x, b.y, et, eb, el, er, any);
-        }
+        DEdge *out = edges + st_fill[f].edge_base + (pos + (outer ? R.edge_a : R.edge_b));
+        add_edge(fills[f], out, a.x, a.y, b.x, b.y, et, eb, el, er, any);
     }
     merge_extents(st_fill, f, any, et, eb, el, er);
 }
@@ -651,7 +685,7 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     const long long n_lanes = run.n_local << st.g;
     const size_t o_cnt = ca.take<long long>(n_lanes + 1), o_off = ca.take<long long>(n_lanes + 1);
     const size_t o_lsub = ca.take<int32_t>(run.n_local + 1), o_pen = ca.take<PenVertex>(run.n_pen + 1);
-    const size_t o_sub = ca.take<SubState>(run.n_subs + 1), o_tot = ca.take<StrokeTot>(run.n_strokes + 1);
+    const size_t o_sub = ca.take<SubState>(run.n_subs + 1), o_reg = ca.take<Region>(run.n_subs + 1);
     const size_t o_edges = ca.take<int32_t>(run.n_strokes + 1), o_totals = ca.take<long long>(2);
     if (c.stroke_a.ensure(ca.off)) return Z2D_ERR_OUT_OF_MEMORY;
     uint8_t *A = c.stroke_a.as<uint8_t>();
@@ -660,13 +694,13 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     int32_t *local_sub = reinterpret_cast<int32_t *>(A + o_lsub);
     st.pen = reinterpret_cast<PenVertex *>(A + o_pen);
     st.sub = reinterpret_cast<SubState *>(A + o_sub);
-    st.tot = reinterpret_cast<StrokeTot *>(A + o_tot);
+    st.region = reinterpret_cast<Region *>(A + o_reg);
     run.stroke_edges = reinterpret_cast<int32_t *>(A + o_edges);
     st.totals = reinterpret_cast<long long *>(A + o_totals);
 
     cudaEvent_t ts = c.timer_begin(c.t_stroke);
-    ks_pen<<<blocks_for(run.n_strokes, T), T, 0, c.stream>>>(run.strokes, run.n_strokes, run.trig, st.pen);
-    ks_local_sub<<<blocks_for(run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, local_sub);
+    ks_pen<<<(unsigned)run.n_strokes, 64, 0, c.stream>>>(run.strokes, run.trig, st.pen);
+    ks_local_sub<<<blocks_for(32ll * run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, local_sub);
     ks_raw_count<<<blocks_for(n_lanes + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes,
                                                                   run.n_local, st.g, st.raw_cnt, d_status);
     size_t tmp = 0;
@@ -688,42 +722,40 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     // ---- buffers sized by the point count
     Carve cb;
     const size_t o_rpt = cb.take<double2>(R + 1), o_rsub = cb.take<int32_t>(R + 1), o_rmode = cb.take<uint8_t>(R + 1);
-    const size_t o_kept = cb.take<int32_t>(R + 1);
+    const size_t o_keep = cb.take<int32_t>(R + 1), o_kept = cb.take<int32_t>(R + 1);
     const size_t o_qpt = cb.take<double2>(R + 1), o_qsub = cb.take<int32_t>(R + 1), o_qmode = cb.take<uint8_t>(R + 1);
-    const size_t o_ca = cb.take<long long>(R + 1), o_cb = cb.take<long long>(R + 1);
-    const size_t o_oa = cb.take<long long>(R + 1), o_ob = cb.take<long long>(R + 1);
+    const size_t o_el = cb.take<Elem>(R + 1), o_c = cb.take<Count2>(R + 1), o_o = cb.take<Count2>(R + 1);
     if (c.stroke_b.ensure(cb.off)) return Z2D_ERR_OUT_OF_MEMORY;
     uint8_t *B = c.stroke_b.as<uint8_t>();
     st.raw_pt = reinterpret_cast<double2 *>(B + o_rpt);
     st.raw_sub = reinterpret_cast<int32_t *>(B + o_rsub);
     st.raw_mode = B + o_rmode;
+    st.keep = reinterpret_cast<int32_t *>(B + o_keep);
     st.kept_off = reinterpret_cast<int32_t *>(B + o_kept);
     st.q_pt = reinterpret_cast<double2 *>(B + o_qpt);
     st.q_sub = reinterpret_cast<int32_t *>(B + o_qsub);
     st.q_mode = B + o_qmode;
-    st.cnt_a = reinterpret_cast<long long *>(B + o_ca);
-    st.cnt_b = reinterpret_cast<long long *>(B + o_cb);
-    st.off_a = reinterpret_cast<long long *>(B + o_oa);
-    st.off_b = reinterpret_cast<long long *>(B + o_ob);
+    st.elem = reinterpret_cast<Elem *>(B + o_el);
+    st.cnt = reinterpret_cast<Count2 *>(B + o_c);
+    st.off = reinterpret_cast<Count2 *>(B + o_o);
 
     ks_raw_emit<<<blocks_for(n_lanes + 1, T), T, 0, c.stream>>>(run.nodes, run.subs, local_sub, run.strokes, run.n_local,
                                                             st.g, st.raw_off, st.raw_pt, st.raw_sub, st.raw_mode);
-    const Keep keep{st.raw_pt, st.raw_sub, R};
-    const auto kept = thrust::make_transform_iterator(thrust::make_counting_iterator(0ll), keep);
+    ks_keep<<<blocks_for(R + 1, T), T, 0, c.stream>>>(st.raw_pt, st.raw_sub, R, st.keep);
     size_t t1 = 0, t2 = 0;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, kept, st.kept_off, R + 1, c.stream));
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, st.cnt_a, st.off_a, R + 1, c.stream));
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, st.keep, st.kept_off, R + 1, c.stream));
+    Z2D_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, t2, st.cnt, st.off, Sum2{}, Count2{0, 0}, R + 1, c.stream));
     if (c.scan_tmp.ensure(std::max(t1, t2) + 16)) return Z2D_ERR_OUT_OF_MEMORY;
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t1, kept, st.kept_off, R + 1, c.stream));
-    ks_compact<<<blocks_for(R, T), T, 0, c.stream>>>(keep, st.raw_mode, st.kept_off, st.q_pt, st.q_sub, st.q_mode);
+    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t1, st.keep, st.kept_off, R + 1, c.stream));
+    ks_compact<<<blocks_for(R, T), T, 0, c.stream>>>(st.raw_pt, st.raw_sub, st.raw_mode, st.keep, st.kept_off, R,
+                                                      st.q_pt, st.q_sub, st.q_mode);
     ks_sub_setup<<<blocks_for(run.n_subs, T), T, 0, c.stream>>>(run.subs, run.n_subs, run.strokes, st.g, st.raw_off,
                                                                  st.kept_off, st.q_pt, st.sub);
     ks_elem_count<<<blocks_for(R + 1, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.q_pt, st.q_sub,
-                                                             st.q_mode, st.kept_off, R, st.cnt_a, st.cnt_b);
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t2, st.cnt_a, st.off_a, R + 1, c.stream));
-    Z2D_CUDA(cub::DeviceScan::ExclusiveSum(c.scan_tmp.ptr, t2, st.cnt_b, st.off_b, R + 1, c.stream));
-    ks_stroke_tot<<<blocks_for(std::max(run.n_strokes, 1), T), T, 0, c.stream>>>(
-        run.strokes, run.n_strokes, st.sub, st.off_a, st.off_b, R, st.tot, run.stroke_edges, st.totals);
+                                                             st.q_mode, st.kept_off, R, st.elem, st.cnt);
+    Z2D_CUDA(cub::DeviceScan::ExclusiveScan(c.scan_tmp.ptr, t2, st.cnt, st.off, Sum2{}, Count2{0, 0}, R + 1, c.stream));
+    ks_stroke_tot<<<blocks_for(std::max(run.n_strokes, run.n_subs), T), T, 0, c.stream>>>(
+        run.strokes, run.n_strokes, run.subs, run.n_subs, st.sub, st.off, R, st.region, run.stroke_edges, st.totals);
     c.timer_end(c.t_stroke, ts);
     c.launches += 9;
     return Z2D_OK;
@@ -738,17 +770,21 @@ int stroke_emit(Ctx &c, StrokeRun &run, const FillCmd *d_fills, FillState *d_st,
     }
     Carve cc;
     const size_t o_pa = cc.take<double2>(run.n_a + 1), o_pb = cc.take<double2>(run.n_b + 1);
+    const size_t o_as = cc.take<int32_t>(run.n_a + 1), o_bs = cc.take<int32_t>(run.n_b + 1);
     if (c.stroke_c.ensure(cc.off)) return Z2D_ERR_OUT_OF_MEMORY;
     st.pa = reinterpret_cast<double2 *>(c.stroke_c.as<uint8_t>() + o_pa);
     st.pb = reinterpret_cast<double2 *>(c.stroke_c.as<uint8_t>() + o_pb);
+    st.a_sub = reinterpret_cast<int32_t *>(c.stroke_c.as<uint8_t>() + o_as);
+    st.b_sub = reinterpret_cast<int32_t *>(c.stroke_c.as<uint8_t>() + o_bs);
     constexpr int T = 128;
     const long long R = run.raw;
     cudaEvent_t ts = c.timer_begin(c.t_stroke);
-    ks_elem_emit<<<blocks_for(R, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.q_pt, st.q_sub,
-                                                        st.q_mode, st.kept_off, R, st.off_a, st.off_b, st.pa, st.pb);
-    ks_edges<<<blocks_for(R, T), T, 0, c.stream>>>(run.subs, run.strokes, st.sub, st.q_sub, st.kept_off, R, st.cnt_a,
-                                                    st.cnt_b, st.off_a, st.off_b, st.tot, st.pa, st.pb, d_fills, d_st,
-                                                    d_edges);
+    ks_elem_emit<<<blocks_for(R, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.region, st.q_pt, st.q_sub,
+                                                        st.q_mode, st.kept_off, R, st.elem, st.off, st.pa, st.pb,
+                                                        st.a_sub, st.b_sub);
+    if (run.n_a + run.n_b > 0)
+        ks_edges<<<blocks_for(run.n_a + run.n_b, T), T, 0, c.stream>>>(st.region, st.pa, st.pb, st.a_sub, st.b_sub,
+                                                                        run.n_a, run.n_b, d_fills, d_st, d_edges);
     c.timer_end(c.t_stroke, ts);
     c.launches += 2;
     return Z2D_OK;
