@@ -51,8 +51,10 @@ namespace z2dg {
 
 // ------------------------------------------------------------ kernels
 // The sequential walk of fill_plotter.plot over one fill's nodes, one warp
-// per fill: the warp stages 32 nodes at a time in shared memory, lane 0
-// walks them, and the warp writes their NodeInfo back.
+// per fill: the warp stages 32 nodes at a time in shared memory, takes runs of
+// segments together, lane 0 walks the rest, and the warp writes their
+// NodeInfo back.  Bound by the latency of the walk (1,024 glyphs of 113
+// nodes: node by node 45 us, now 13).
 constexpr int kScanWarps = 4;
 struct ScanStage {
     double x[32], y[32];    // node end point (curve: p[4], p[5])
@@ -106,9 +108,40 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_fill_scan(const z2d_node *_
             S.ey[lane] = inf.ey;
         }
         __syncwarp();
-        if (lane == 0) {
-            const int32_t m = min(32, n_nodes - base);
-            for (int32_t k = 0; k < m; k++) {
+        // Runs of line_to and curve_to nodes whose start is the node before
+        // (all but the first after a close_path) need no walk: their starts,
+        // counts and edge offsets are a scan over the lanes.  Lane 0 walks the
+        // others one at a time.
+        const int32_t m = min(32, n_nodes - base);
+        const uint32_t plain = __ballot_sync(0xffffffffu, valid && base + lane > 0 &&
+                                                              (S.tag[lane] == Z2D_LINE_TO || S.tag[lane] == Z2D_CURVE_TO) &&
+                                                              S.n_emit[lane] >= 0);
+        for (int32_t k = 0; k < m;) {
+            const uint32_t rest = plain >> k;
+            const int32_t run = (rest & 1u) ? min(m - k, __ffs(~rest) == 0 ? 32 : __ffs(~rest) - 1) : 0;
+            if (run >= 2) {
+                const bool in = lane >= k && lane < k + run;
+                int32_t incl = in ? S.n_emit[lane] : 0, add = in ? S.n_added[lane] : 0;
+                const int32_t mine = incl;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                add = __reduce_add_sync(0xffffffffu, min(add, 3));
+                if (in) {
+                    S.off[lane] = off + incl - mine;
+                    S.sx[lane] = lane == k ? lx : S.x[lane - 1];
+                    S.sy[lane] = lane == k ? ly : S.y[lane - 1];
+                }
+                off += __shfl_sync(0xffffffffu, incl, 31);
+                count = min(count + add, 3);
+                lx = S.x[k + run - 1];
+                ly = S.y[k + run - 1];
+                k += run;
+                continue;
+            }
+            if (lane == 0) {
                 S.off[k] = off;
                 int32_t ne;
                 const double px = S.x[k], py = S.y[k];
@@ -171,6 +204,12 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_fill_scan(const z2d_node *_
                 S.n_emit[k] = ne;
                 off += ne;
             }
+            // lane 0's state for the runs
+            off = __shfl_sync(0xffffffffu, off, 0);
+            count = __shfl_sync(0xffffffffu, count, 0);
+            lx = __shfl_sync(0xffffffffu, lx, 0);
+            ly = __shfl_sync(0xffffffffu, ly, 0);
+            k++;
         }
         __syncwarp();
         if (valid) {
@@ -816,6 +855,42 @@ __device__ __forceinline__ int32_t job_of(const DevJob *__restrict__ jobs, int32
     return lo;
 }
 
+// The same with a warp per band, for jobs of few fills: a CTA per band
+// spends its time starting and meeting at barriers (16,384 bands of one fill:
+// 43 us, a warp each 11).
+__global__ void __launch_bounds__(256) k_band_lists_w(const FillState *__restrict__ st, const DevJob *__restrict__ jobs,
+                                                      int32_t n_jobs, int32_t n_gbands,
+                                                      int32_t *__restrict__ band_count, int4 *__restrict__ band_fills,
+                                                      TileRec *__restrict__ tiles) {
+    const int32_t gb = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (gb >= n_gbands) return;
+    const int32_t j = job_of(jobs, n_jobs, gb, [](const DevJob &J) { return (long long)J.gband_base; });
+    const DevJob &J = jobs[j];
+    const int32_t lb = gb - J.gband_base, b = J.band_lo + lb, nf = J.fill1 - J.fill0;
+    if (tiles) {
+        const int32_t nc = J.tcol_hi - J.tcol_lo + 1;
+        for (int32_t t = lane; t < nc; t += 32) tiles[J.tile_base + (long long)lb * nc + t] = TileRec{j, lb, t, 0};
+    }
+    int4 *out = band_fills + J.list_base + (long long)lb * nf;
+    int32_t n = 0;
+    for (int32_t f0 = J.fill0; f0 < J.fill1; f0 += 32) {
+        const int32_t f = f0 + lane;
+        bool hit = false;
+        int4 ent = make_int4(f, 0, 0, 0);
+        if (f < J.fill1) {
+            const FillState &S = st[f];
+            hit = S.active && b >= S.band0 && b <= S.band1;
+            ent.y = S.cull_x0;
+            ent.z = S.cull_x1;
+            ent.w = S.fb_base + (b - S.band0);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) out[n + __popc(m & ((1u << lane) - 1u))] = ent;
+        n += __popc(m);
+    }
+    if (lane == 0) band_count[gb] = n;
+}
+
 // One CTA per global band: the job's fills touching the band, in call order
 // (ordered compaction), with the tile-column range each one can affect and
 // the fill's (fill, band) slot of the band, and (several surfaces) the
@@ -1374,7 +1449,12 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     int32_t *d_band_count = c.band_fills.as<int32_t>();
     TileRec *d_tiles = n_jobs > 1 ? reinterpret_cast<TileRec *>(c.band_fills.as<uint8_t>() + count_bytes) : nullptr;
     int4 *d_band_fills = reinterpret_cast<int4 *>(c.band_fills.as<uint8_t>() + count_bytes + tile_bytes);
-    k_band_lists<<<(unsigned)n_gbands, 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, d_band_count, d_band_fills, d_tiles);
+    if (n_slots <= 256 * n_gbands)  // few fills a job on average
+        k_band_lists_w<<<grid_for(32 * n_gbands, 256), 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, (int32_t)n_gbands,
+                                                                            d_band_count, d_band_fills, d_tiles);
+    else
+        k_band_lists<<<(unsigned)n_gbands, 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, d_band_count, d_band_fills,
+                                                               d_tiles);
     c.launches++;
 
     // ---- exact path
