@@ -1,0 +1,28 @@
+"""The curve flattener's error test in fixed point: wherever chord_test
+decides, it is the f64 comparison, on random and adversarial curves and their
+subcurves (tests/chord_check.cu, built with nvcc as host code and run on
+the CPU)."""
+import os
+import shutil
+import subprocess
+import tempfile
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+def test_chord_test_matches_f64():
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not found")
+    with tempfile.TemporaryDirectory() as d:
+        exe = os.path.join(d, "chord_check")
+        subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O2", "-std=c++17",
+                        "-Xcompiler", "-ffp-contract=off",
+                        "-I", os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "z2d_gb300", "csrc"),
+                        os.path.join(HERE, "chord_check.cu"), "-o", exe], check=True)
+        r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "wrong 0" in r.stdout, r.stdout

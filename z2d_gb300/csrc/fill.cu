@@ -290,10 +290,11 @@ struct LaneCurve {
     bool ok = true;
 };
 template <class P>
-__device__ __forceinline__ LaneCurve walk_lane(double sx, double sy, const double *p, const Tol &tol, int g, int j,
+__device__ __forceinline__ LaneCurve walk_lane(double sx, double sy, const double *p, double tolerance, int g, int j,
                                                P &&leaf_start) {
     LaneCurve r;
     Knots k{sx, sy, p[0], p[1], p[2], p[3], p[4], p[5]};
+    const Tol tol = make_tol(tolerance, k);
     bool is_leaf;
     int open;
     if (!lane_subtree(k, g, j, tol, is_leaf, open)) return r;
@@ -380,9 +381,9 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_count_w(const z2d_n
 // leaves), fewer while the grid has lanes to spare.  The lanes of a warp then
 // have walks of like length, and the splits that every lane of a curve
 // repeats stay few against the leaves.  (A warp per curve left most lanes
-// idle on short curves: 1,024 glyphs of 110 curves 655 us, now 157; 320
-// surfaces with 16 k fills 2.1 ms, now 0.76; 2,000 paths of long curves 396
-// us, now 285.  Three classes of 1, 8 and 32 lanes: 222, 925 and 309 us.)
+// idle on short curves: 1,024 glyphs of 110 curves 655 us, in classes 157; 320
+// surfaces with 16 k fills 2.1 ms, then 0.76; 2,000 paths of long curves 396
+// us, then 285.  Three classes of 1, 8 and 32 lanes: 222, 925 and 309 us.)
 // A curve's edges are its leaves' chords when every leaf start but the first
 // differs from the curve's start (consecutive leaves share their end points,
 // so the lineTo sequence start, a1, a2, ..., d is the chord sequence): such a
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_curve_count_w(const z2d_
             sy = pv.tag == Z2D_CURVE_TO ? pv.p[5] : pv.p[1];
             dx = nd.p[4];
             dy = nd.p[5];
-            r = walk_lane(sx, sy, nd.p, make_tol(fills[node_fill[i]].tol), g, j, [&](int32_t m, const Knots &q) {
+            r = walk_lane(sx, sy, nd.p, fills[node_fill[i]].tol, g, j, [&](int32_t m, const Knots &q) {
                 if (m < kScratch) scr[m * 32 + lane] = make_double2(q.ax, q.ay);
             });
             if (!r.ok) atomicExch(status, Z2D_ERR_INVALID_STATE);
@@ -495,8 +496,7 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_curve_count_w(const z2d_
 // one walk, emitted by another.
 __device__ __forceinline__ void curve_emit_warp(const FillCmd &F, DEdge *out, const NodeInfo &inf, const double *p,
                                                 int lane, double &et, double &eb, double &el, double &er, bool &any) {
-    const Tol tol = make_tol(F.tol);
-    const LaneCurve r = walk_lane(inf.sx, inf.sy, p, tol, 5, lane, [](int32_t, const Knots &) {});
+    const LaneCurve r = walk_lane(inf.sx, inf.sy, p, F.tol, 5, lane, [](int32_t, const Knots &) {});
     __syncwarp();
     double px, py;
     prev_point_scan(r.cnt > 0, r.lx, r.ly, inf.sx, inf.sy, lane, 32, px, py);
@@ -505,7 +505,7 @@ __device__ __forceinline__ void curve_emit_warp(const FillCmd &F, DEdge *out, co
     const double ex = r.cnt > 0 ? r.lx : px, ey = r.cnt > 0 ? r.ly : py;
     if (r.cnt > 0) {
         int32_t k = off;
-        walk_lane(inf.sx, inf.sy, p, tol, 5, lane, [&](int32_t, const Knots &q) {
+        walk_lane(inf.sx, inf.sy, p, F.tol, 5, lane, [&](int32_t, const Knots &q) {
             if (pt_eq(q.ax, q.ay, inf.sx, inf.sy)) return;
             if (k < inf.n_emit) add_edge(F, out + k, px, py, q.ax, q.ay, et, eb, el, er, any);
             k++;

@@ -19,7 +19,7 @@ struct Knots {
 };
 
 // Spline.Knots.errorSq (Spline.zig:83-123)
-__device__ __forceinline__ double error_sq(const Knots &k) {
+__host__ __device__ __forceinline__ double error_sq(const Knots &k) {
     double bx = k.bx - k.ax, by = k.by - k.ay, cx = k.cx - k.ax, cy = k.cy - k.ay;
     if (k.ax != k.dx || k.ay != k.dy) {
         const double dx = k.dx - k.ax, dy = k.dy - k.ay;
@@ -47,17 +47,22 @@ __device__ __forceinline__ double error_sq(const Knots &k) {
 // f64 -> f32 by truncating the mantissa (relative error < 2^-23) with
 // integer operations only, so that no FP64 instruction is spent on it.
 // False outside f32's normal range (zero excepted).
-__device__ __forceinline__ bool f32_trunc(double v, float &out) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+__host__ __device__ __forceinline__ float f32_from(uint32_t b) {
+    float f;
+    memcpy(&f, &b, 4);
+    return f;
+}
+__host__ __device__ __forceinline__ bool f32_trunc(double v, float &out) {
+    const uint64_t b = f64_bits(v);
     const uint32_t hi = (uint32_t)(b >> 32);
     const uint32_t sign = hi & 0x80000000u;
     if ((b << 1) == 0ull) {
-        out = __uint_as_float(sign);
+        out = f32_from(sign);
         return true;
     }
     const int32_t fe = (int32_t)((hi >> 20) & 0x7FFu) - 1023 + 127;
     if (fe <= 0 || fe >= 255) return false;
-    out = __uint_as_float(sign | ((uint32_t)fe << 23) | ((uint32_t)(b >> 29) & 0x7FFFFFu));
+    out = f32_from(sign | ((uint32_t)fe << 23) | ((uint32_t)(b >> 29) & 0x7FFFFFu));
     return true;
 }
 
@@ -133,6 +138,7 @@ __device__ __forceinline__ int error_sq_lt_f32(double bx64, double by64, double 
 // From the knots' coordinates, truncated to f32 (error < 2u of each) and
 // subtracted in f32 (one more rounding): no f64 instruction at all, at the
 // price of wider bounds (the coordinates' size instead of the differences').
+// Serves the curves whose coordinates do not take chord_test's fixed point.
 __device__ __forceinline__ int error_sq_lt_f32_pts(double ax64, double ay64, double bx64, double by64, double cx64,
                                                    double cy64, double dx64, double dy64, bool proj, float tol2f,
                                                    float tol2e) {
@@ -151,30 +157,136 @@ __device__ __forceinline__ int error_sq_lt_f32_pts(double ax64, double ay64, dou
                                 tol2f, tol2e);
 }
 
-// The squared tolerance of a subdivision, in f64 and as a truncated f32
-// with its error bound.
+// The squared tolerance of a subdivision, in f64, as a truncated f32 with its
+// error bound, and as a bracket in the curve's fixed-point units (chord_test).
 struct Tol {
     double d;
     float f, e;
     bool f_ok;
+    float lo, hi;
+    uint32_t shift0;
 };
-__device__ __forceinline__ Tol make_tol(double tol) {
+
+__host__ __device__ __forceinline__ Tol make_tol(double tol) {
     Tol t;
     t.d = tol * tol;  // decomposeInto's tolerance argument (Spline.zig:52)
     t.f = 0.0f;
     t.f_ok = f32_trunc(t.d, t.f);
     t.e = 4.0f * 5.9604644775390625e-8f * t.f;
+    t.lo = -1.0f;  // the bracket that decides nothing
+    t.hi = f32_from(0x7F800000u);
+    t.shift0 = 0;
+    return t;
+}
+// One curve's tolerance.  The fixed-point unit is 2^-29 of the power of two
+// at or below the curve's largest coordinate, so that every coordinate of
+// the curve and of its subcurves (a split's points lie between their ends,
+// each coordinate) takes 31 bits with the sign.
+__host__ __device__ __forceinline__ Tol make_tol(double tol, const Knots &k) {
+    Tol t = make_tol(tol);
+    uint32_t m = 0;
+    const double c[8] = {k.ax, k.ay, k.bx, k.by, k.cx, k.cy, k.dx, k.dy};
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t h = (uint32_t)(f64_bits(c[i]) >> 32) & 0x7FFFFFFFu;
+        m = m > h ? m : h;
+    }
+    const uint32_t e = m >> 20;
+    t.shift0 = e + 2;
+    if (t.f_ok && e >= 1023 - 40 && e <= 1023 + 40) {
+        const float unit = f32_from((127u + 1052u - e) << 23);  // units per 1
+        const float u2 = (t.f * unit) * unit;
+        if (u2 > 1e-18f && u2 < 1e18f) {
+            t.lo = u2 * (1.0f - 3.814697265625e-6f);  // -+ 2^-18
+            t.hi = u2 * (1.0f + 3.814697265625e-6f);
+        }
+    }
     return t;
 }
 
+// floor-like fixed point of one coordinate: within one unit below x (the
+// magnitude truncated, its bits inverted where x is negative).
+__host__ __device__ __forceinline__ int32_t to_fixed(double x, uint32_t shift0) {
+    const uint64_t b = f64_bits(x);
+    const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+    const uint32_t sh = shift0 - ((hi >> 20) & 0x7FFu);
+#ifdef __CUDA_ARCH__
+    const uint32_t m = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+    const uint32_t q = __funnelshift_rc(m, 0u, sh);
+#else
+    const uint32_t m = (hi << 11) | (lo >> 21) | 0x80000000u;
+    const uint32_t q = sh >= 32u ? 0u : m >> sh;
+#endif
+    return (int32_t)q ^ ((int32_t)hi >> 31);
+}
+
+// errorSq(k) < tol2 from fixed-point coordinates: 1 / 0 where the error
+// bounds allow the decision, -1 otherwise.  The differences are exact integers
+// within one unit of the true ones; f32 takes over from there.  With d the
+// chord, a control point p (from a) that projects before d's end is at
+// squared distance cross(p, d)^2 / |d|^2, and the comparison with tol2 needs
+// no division; past the end it is |p - d|^2.
+//
+// Bounds: an input (a difference, at most L in size) is off by at most
+// 1 + uL, u = 2^-24; K = 1 + 4uL covers it and, by K times the other
+// factor, the roundings of a product.  A sum of two products of p and d is
+// then within K (P + 2 S) + 2 K^2 of its true value, with P = |px| + |py|
+// and S = |dx| + |dy|; the bounds below have 6 % on top of that for their own
+// roundings, and the tolerance's bracket (2^-18) covers the relative
+// roundings of the squares and products that are compared.
+//
+// f32 copies of the coordinates, subtracted, left 1.8 % of the tests on a
+// 4096-pixel canvas to the f64 differences, which one warp in two then
+// waited for; a unit is 64 times finer than their last place, and leaves
+// 0.03 %.
+__host__ __device__ __forceinline__ int chord_test(const Knots &k, const Tol &t) {
+    const uint32_t s0 = t.shift0;
+    const int32_t ax = to_fixed(k.ax, s0), ay = to_fixed(k.ay, s0);
+    const float dx = (float)(to_fixed(k.dx, s0) - ax), dy = (float)(to_fixed(k.dy, s0) - ay);
+    const float p[2][2] = {{(float)(to_fixed(k.bx, s0) - ax), (float)(to_fixed(k.by, s0) - ay)},
+                           {(float)(to_fixed(k.cx, s0) - ax), (float)(to_fixed(k.cy, s0) - ay)}};
+    const float L = fmaxf(fmaxf(fmaxf(fabsf(p[0][0]), fabsf(p[0][1])), fmaxf(fabsf(p[1][0]), fabsf(p[1][1]))),
+                          fmaxf(fabsf(dx), fabsf(dy)));
+    const float K = 1.0f + 2.384185791015625e-7f * L;  // 1 + 4 u L
+    const float S = fabsf(dx) + fabsf(dy);
+    const float dd = dx * dx + dy * dy, m_dd = 2.125f * K * (S + K);
+    const float dd_lo = dd - m_dd, dd_hi = dd + m_dd;
+    if (!(dd_lo > 0.0f)) return -1;
+    bool below = true, above = false;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const float px = p[i][0], py = p[i][1];
+        const float P = fabsf(px) + fabsf(py);
+        const float m = 1.0625f * K * (P + 2.0f * S + 2.0f * K);
+        const float diff = (px * dx + py * dy) - dd;
+        if (diff < -(m + m_dd)) {
+            const float c = fabsf(px * dy - py * dx);
+            const float lo = fmaxf(c - m, 0.0f), hi = c + m;
+            below = below && hi * hi < t.lo * dd_lo;
+            above = above || lo * lo > t.hi * dd_hi;
+        } else if (diff > m + m_dd) {
+            const float vx = px - dx, vy = py - dy;
+            const float n = vx * vx + vy * vy, mn = 4.25f * K * (fabsf(vx) + fabsf(vy) + 2.125f * K);
+            below = below && n + mn < t.lo;
+            above = above || n - mn > t.hi;
+        } else {
+            return -1;
+        }
+    }
+    return above ? 0 : below ? 1 : -1;
+}
+
 // errorSq(k) < t.d, exactly as the f64 comparison decides it.
-// The rarely needed tests of below_tol, out of line so that the
-// subdivision loops that inline below_tol stay small in the instruction
-// cache.
-static __device__ __noinline__ bool below_tol_slow(Knots k, Tol t, bool proj) {
+// The rarely needed tests, out of line so that the subdivision loops stay
+// small in the instruction cache.
+static __device__ __noinline__ bool below_tol_slow(Knots k, Tol t) {
     if (t.f_ok) {
-        const int r = error_sq_lt_f32(k.bx - k.ax, k.by - k.ay, k.cx - k.ax, k.cy - k.ay, proj, k.dx - k.ax,
-                                      k.dy - k.ay, t.f, t.e);
+        const bool proj = !pt_eq(k.ax, k.ay, k.dx, k.dy);
+        int r = -1;
+        if (t.lo < 0.0f) r = error_sq_lt_f32_pts(k.ax, k.ay, k.bx, k.by, k.cx, k.cy, k.dx, k.dy, proj, t.f, t.e);
+        if (r < 0)
+            r = error_sq_lt_f32(k.bx - k.ax, k.by - k.ay, k.cx - k.ax, k.cy - k.ay, proj, k.dx - k.ax, k.dy - k.ay, t.f,
+                                t.e);
         if (r >= 0) return r != 0;
     }
     return error_sq(k) < t.d;
@@ -182,16 +294,12 @@ static __device__ __noinline__ bool below_tol_slow(Knots k, Tol t, bool proj) {
 
 // Out of line, like the split: the subdivision loops stay small in the
 // instruction cache and the curve kernels need 96 registers instead of
-// 118-124 (flatten of the 2,000-path batch 0.68 -> 0.59 ms).
+// 118-124 (flatten of the 2,000-path batch 0.68 -> 0.59 ms).  The
+// fixed-point test took the count of that batch from 285 to 185 us.
 static __device__ __noinline__ bool below_tol(const Knots &k, const Tol &t) {
-    const bool proj = !pt_eq(k.ax, k.ay, k.dx, k.dy);
-    if (t.f_ok) {
-        // from the coordinates first (no f64), then from the exact f64
-        // differences, then errorSq itself
-        const int r = error_sq_lt_f32_pts(k.ax, k.ay, k.bx, k.by, k.cx, k.cy, k.dx, k.dy, proj, t.f, t.e);
-        if (r >= 0) return r != 0;
-    }
-    return below_tol_slow(k, t, proj);
+    const int r = chord_test(k, t);
+    if (r >= 0) return r != 0;
+    return below_tol_slow(k, t);
 }
 
 // x / 2.  For normal x whose half is normal this only lowers the exponent,
@@ -310,7 +418,8 @@ __device__ __forceinline__ bool spline_walk(double ax, double ay, const double *
         emit(dx, dy);
         return true;
     }
-    const bool ok = walk_leaves(Knots{ax, ay, bx, by, cx, cy, dx, dy}, false, 0, make_tol(tol), [&](const Knots &k) {
+    const Knots k0{ax, ay, bx, by, cx, cy, dx, dy};
+    const bool ok = walk_leaves(k0, false, 0, make_tol(tol, k0), [&](const Knots &k) {
         if (!pt_eq(k.ax, k.ay, ax, ay)) emit(k.ax, k.ay);
     });
     emit(dx, dy);

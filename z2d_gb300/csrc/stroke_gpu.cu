@@ -152,8 +152,8 @@ __device__ __forceinline__ bool node_points(const z2d_node *__restrict__ nodes, 
     const int last = (1 << g) - 1;
     bool ok = true;
     if (!(pt_eq(a.x, a.y, p[0], p[1]) && pt_eq(p[2], p[3], p[4], p[5]))) {  // Spline.zig:39-42
-        const Tol t = make_tol(tol);
         Knots k{a.x, a.y, p[0], p[1], p[2], p[3], p[4], p[5]};
+        const Tol t = make_tol(tol, k);
         bool is_leaf;
         int open;
         if (lane_subtree(k, g, j, t, is_leaf, open))
