@@ -764,7 +764,7 @@ __device__ __forceinline__ void for_edge_bands(const FillCmd *__restrict__ fills
     const int32_t stride = gridDim.x * blockDim.x;
     for (int32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n_edges; base += stride) {
         const int32_t i = base + lane;
-        int32_t nb = 0, fb0 = 0;
+        int32_t nb = 0, fb0 = 0, row0 = 0;  // row0: the first band's first sample row, | 1 with 4 a pixel
         if (i < n_edges) {
             const int32_t f = edge_fill[i];
             if (f >= 0) {
@@ -773,6 +773,8 @@ __device__ __forceinline__ void for_edge_bands(const FillCmd *__restrict__ fills
                 if (S.active && !(S.flags & FILL_EXACT) && edge_bands(edges[i], fills[f], S, b0, b1)) {
                     nb = b1 - b0 + 1;
                     fb0 = S.fb_base + (b0 - S.band0);
+                    const int32_t S_ = (int32_t)fills[f].scale;
+                    row0 = b0 * kTileRows * S_ | (S_ == 4 ? 1 : 0);
                 }
             }
         }
@@ -795,7 +797,9 @@ __device__ __forceinline__ void for_edge_bands(const FillCmd *__restrict__ fills
             }
             const int32_t o_excl = __shfl_sync(0xffffffffu, excl, owner);
             const int32_t o_fb0 = __shfl_sync(0xffffffffu, fb0, owner);
-            if (k < total) visit(base + owner, o_fb0 + (k - o_excl));
+            const int32_t o_row0 = __shfl_sync(0xffffffffu, row0, owner);
+            const int32_t rows = (o_row0 & 1) ? 4 * kTileRows : kTileRows;
+            if (k < total) visit(base + owner, o_fb0 + (k - o_excl), (o_row0 & ~1) + (k - o_excl) * rows, rows);
         }
     }
 }
@@ -803,7 +807,7 @@ __device__ __forceinline__ void for_edge_bands(const FillCmd *__restrict__ fills
 __global__ void k_bin_count(const FillCmd *__restrict__ fills, const FillState *__restrict__ st,
                             const DEdge *__restrict__ edges, const int32_t *__restrict__ edge_fill, int32_t n_edges,
                             int32_t *__restrict__ fb_count, int32_t *__restrict__ status) {
-    for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t, int32_t fb) {
+    for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t, int32_t fb, int32_t, int32_t) {
         if (atomicAdd(&fb_count[fb], 1) >= kMaxBandEdges) atomicExch(status, Z2D_ERR_INVALID_ARGUMENT);
     });
 }
@@ -814,12 +818,14 @@ __global__ void k_bin_count(const FillCmd *__restrict__ fills, const FillState *
 __global__ void k_bin_fill(const FillCmd *__restrict__ fills, const FillState *__restrict__ st,
                            const DEdge *__restrict__ edges, const int32_t *__restrict__ edge_fill, int32_t n_edges,
                            int32_t *__restrict__ fb_cursor, BinEdge *__restrict__ bins) {
-    for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t edge, int32_t fb) {
+    for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t edge, int32_t fb, int32_t row, int32_t rows) {
         const int4 a = __ldg(reinterpret_cast<const int4 *>(edges + edge));
         const int2 r = __ldg(reinterpret_cast<const int2 *>(&edges[edge].rt));
+        const BinEdge B = bin_edge(a.x, __int_as_float(a.y), __int_as_float(a.z), __int_as_float(a.w), r.x, r.y, edge,
+                                   row, rows);
         int4 *out = reinterpret_cast<int4 *>(bins + atomicAdd(&fb_cursor[fb], 1));
-        out[0] = a;
-        out[1] = make_int4(r.x, r.y, edge, 0);
+        out[0] = make_int4(B.c, __float_as_int(B.fx), __float_as_int(B.fxi), __float_as_int(B.t));
+        out[1] = make_int4((int32_t)B.rows, __float_as_int(B.limit), B.id, 0);
     });
 }
 

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "fill.cuh"
 
@@ -17,14 +18,42 @@ Z2D_HD uint32_t ss_mask8(int n, int fmt) {
     return ((uint32_t)n * 255u) / 16u;
 }
 
-// An edge in the bin of one (fill, band): the f32 half of its DEdge and its
-// index, for the crossings that are evaluated in f64.
+// An edge in the bin of one (fill, band), as a pixel row of the band needs
+// it: the crossing with the band's sample row s is
+//   xi + round(fx + fxi (t + s)),  c = xi - kRoundMagicBits,
+// if bit s of `rows` is set and f32 decides it (limit); bit 31 is set for a
+// downward edge.  `id` is the edge's index, for f64.
 struct BinEdge {
-    int32_t xi;
-    float fx, fxi, fdt;
-    int32_t rt, rb;
+    int32_t c;
+    float fx, fxi, t;
+    uint32_t rows;
+    float limit;
     int32_t id, _pad;
 };
+// The record of an edge (its DEdge fields) for the n sample rows from `row`.
+// A pixel row evaluates fma(fxi, r, fma(fxi, t + w, fx)) with s = w + r.
+// With T >= |t|, |t + w| and the largest t + s, p = |fxi| T and u = 2^-24, the
+// error is at most u (2 p (slope) + 3 p (t: the conversion and two sums)
+// + 3 |fxi| (fdt) + 2 (fx) + 2 (1 + p) (the multiply-adds)), within the bound
+// of crossing_limit.
+Z2D_HD BinEdge bin_edge(int32_t xi, float fx, float fxi, float fdt, int32_t rt, int32_t rb, int32_t id, int32_t row,
+                        int32_t n) {
+    BinEdge B;
+    const int32_t rel = row - rt;
+    const int32_t lo = rel < 0 ? -rel : 0, hi = rb - row < n ? rb - row : n;
+    B.c = (int32_t)((uint32_t)xi - (uint32_t)kRoundMagicBits);
+    B.fx = fx;
+    B.fxi = fxi;
+    B.t = (float)rel + fabsf(fdt);
+    B.rows = lo < hi ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+    uint32_t dir;
+    memcpy(&dir, &fdt, 4);
+    B.rows |= dir & 0x80000000u;
+    B.limit = crossing_limit(fxi, (float)(rel + hi > 1 - rel ? rel + hi : 1 - rel));
+    B.id = id;
+    B._pad = 0;
+    return B;
+}
 static_assert(sizeof(BinEdge) == 32, "BinEdge: two 16-byte accesses");
 
 // A tile of a batch of several surfaces: its surface, its band counted
