@@ -541,9 +541,12 @@ __global__ void __launch_bounds__(32 * kFlattenWarps) k_node_emit_w(const z2d_no
                 DEdge *out = edges + st[f].edge_base + inf.edge_off;
                 const bool straight = nd.tag == Z2D_CURVE_TO && pt_eq(inf.sx, inf.sy, nd.p[0], nd.p[1]) &&
                                       pt_eq(nd.p[2], nd.p[3], nd.p[4], nd.p[5]);
-                if (nd.tag == Z2D_LINE_TO) add_edge(F, out, inf.sx, inf.sy, nd.p[0], nd.p[1], et, eb, el, er, any);
-                else if (nd.tag == Z2D_CLOSE_PATH) add_edge(F, out, inf.sx, inf.sy, inf.ex, inf.ey, et, eb, el, er, any);
-                else if (straight) add_edge(F, out, inf.sx, inf.sy, nd.p[4], nd.p[5], et, eb, el, er, any);
+                // one add_edge for lanes of every kind
+                const int last = nd.tag == Z2D_CURVE_TO ? 4 : 0;
+                const bool close = nd.tag == Z2D_CLOSE_PATH;
+                if (nd.tag == Z2D_LINE_TO || close || straight)
+                    add_edge(F, out, inf.sx, inf.sy, close ? inf.ex : nd.p[last], close ? inf.ey : nd.p[last + 1], et,
+                             eb, el, er, any);
                 else curve = true;  // k_curve_emit_w emits it
             }
         }
