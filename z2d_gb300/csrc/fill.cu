@@ -1594,7 +1594,7 @@ constexpr int kSmallMaxDepth = 40;  // below the device subdivision bound
 
 struct HostFlatten {
     const FillCmd &F;
-    std::vector<DEdge> &edges;
+    std::vector<SmallEdge> &edges;
     size_t max_edges;
     double et = 0, eb = 0, el = 0, er = 0;
     bool any = false, overflow = false;
@@ -1609,25 +1609,23 @@ struct HostFlatten {
             return;
         }
         const double ax = x0 * F.edge_scale, ay = y0 * F.edge_scale, bx = x1 * F.edge_scale, by = y1 * F.edge_scale;
-        DEdge e{};
+        SmallEdge e{};
         if (ay < by) {
             e.top = ay;
             e.x_start = ax;
             e.x_inc = (bx - ax) / (by - ay);
-            e.rb = (int32_t)std::round(by);
+            e.rb2 = 2 * (int32_t)std::round(by) + 1;
         } else if (ay > by) {
             e.top = by;
             e.x_start = bx;
             e.x_inc = (ax - bx) / (ay - by);
-            e.rb = (int32_t)std::round(ay);
+            e.rb2 = 2 * (int32_t)std::round(ay);
         } else {
-            e.rt = 1;
-            e.rb = 0;
+            e.rt = 1;  // rb = 0: never active
             edges.push_back(e);
             return;
         }
         e.rt = (int32_t)std::round(e.top);
-        e.fdt = ay < by ? -0.0f : 0.0f;  // (k_raster's gathering variants fill the f32 fields in)
         const double bot = ay < by ? by : ay;
         const double l = ax < bx ? ax : bx, r = ax < bx ? bx : ax;
         if (!any) {
@@ -1827,7 +1825,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     for (const DevGradient &g : grads)
         if (g.n_stops > kMaxStops) return Z2D_OK;
     // ---- flatten every fill (fill_plotter.plot)
-    static thread_local std::vector<DEdge> edges;
+    static thread_local std::vector<SmallEdge> edges;
     static thread_local std::vector<FillState> st;
     static thread_local std::vector<RasterFill> rf;
     static thread_local std::vector<double> ext;  // et, eb, el, er per fill
@@ -1933,8 +1931,8 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
             if (!S.active) continue;
             const int32_t S_ = (int32_t)fills[f].scale;
             for (int32_t k = 0; k < S.n_edges; k++) {
-                const DEdge &e = edges[(size_t)(S.edge_base + k)];
-                const int32_t lo = std::max(e.rt, S.start_y * S_), hi = std::min(e.rb, (S.end_y + 1) * S_);
+                const SmallEdge &e = edges[(size_t)(S.edge_base + k)];
+                const int32_t lo = std::max(e.rt, S.start_y * S_), hi = std::min(e.rb2 >> 1, (S.end_y + 1) * S_);
                 if (lo >= hi) continue;
                 const int32_t b0 = lo / (kTileRows * S_), b1 = (hi - 1) / (kTileRows * S_);
                 for (int32_t b = b0; b <= b1; b++) visit(S.fb_base + (b - S.band0), S.edge_base + k);
@@ -1987,7 +1985,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     const size_t o_jobs = 0, o_fill = al(sizeof(DevJob) * n_jobs);
     const size_t o_st = o_fill + al(sizeof(FillCmd) * n_fills), o_rf = o_st + al(sizeof(FillState) * n_fills);
     const size_t o_edges = o_rf + al(sizeof(RasterFill) * n_fills);
-    const size_t o_bins = o_edges + al(sizeof(DEdge) * std::max<size_t>(edges.size(), 1));
+    const size_t o_bins = o_edges + al(sizeof(SmallEdge) * std::max<size_t>(edges.size(), 1));
     const size_t o_off = o_bins + al(sizeof(int32_t) * bins.size());
     const size_t o_cnt = o_off + al(sizeof(int32_t) * ((size_t)n_fb + 1));
     const size_t o_list = o_cnt + al(sizeof(int32_t) * bcount.size());
@@ -2019,7 +2017,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         if (grad_of_fill[f] >= 0) hf[f].src.grad = dgrads + grad_of_fill[f];
     memcpy(h + o_st, st.data(), sizeof(FillState) * n_fills);
     memcpy(h + o_rf, rf.data(), sizeof(RasterFill) * n_fills);
-    if (!edges.empty()) memcpy(h + o_edges, edges.data(), sizeof(DEdge) * edges.size());
+    if (!edges.empty()) memcpy(h + o_edges, edges.data(), sizeof(SmallEdge) * edges.size());
     memcpy(h + o_bins, bins.data(), sizeof(int32_t) * bins.size());
     if (!tiles.empty()) memcpy(h + o_tile, tiles.data(), sizeof(TileRec) * tiles.size());
     memcpy(h + o_off, off.data(), sizeof(int32_t) * ((size_t)n_fb + 1));
@@ -2047,7 +2045,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     A.jobs = reinterpret_cast<const DevJob *>(dv + o_jobs);
     A.fills = reinterpret_cast<const FillCmd *>(dv + o_fill);
     A.st = reinterpret_cast<const FillState *>(dv + o_st);
-    A.edges = reinterpret_cast<const DEdge *>(dv + o_edges);
+    A.edges = dv + o_edges;
     A.bins = dv + o_bins;
     A.bin_off = reinterpret_cast<const int32_t *>(dv + o_off);
     A.band_count = reinterpret_cast<const int32_t *>(dv + o_cnt);

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "raster.cuh"
 #include "raster_px.cuh"
@@ -77,7 +78,7 @@ struct RowEdge {
 // record is read by every row and tile column of its band (2,000 paths: with
 // rows, t and limit worked out here 2.07 ms, now 1.97).
 template <bool GATHER>
-__device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const DEdge *__restrict__ edges,
+__device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const void *__restrict__ edges,
                                             int32_t bin, bool valid, int32_t sub0, int32_t off, int32_t sc,
                                             int32_t col0) {
     RowEdge R{};
@@ -85,15 +86,14 @@ __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const
     BinEdge B;
     if constexpr (GATHER) {
         const int32_t id = __ldg(reinterpret_cast<const int32_t *>(bins) + bin);
-        const int4 a = __ldg(reinterpret_cast<const int4 *>(edges + id));
-        const int4 b = __ldg(reinterpret_cast<const int4 *>(edges + id) + 1);
-        const int4 c = __ldg(reinterpret_cast<const int4 *>(edges + id) + 2);
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id);
+        const int4 b = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id + 1);
         DEdge e;
-        e.x_start = __hiloint2double(b.w, b.z);
-        e.x_inc = __hiloint2double(c.y, c.x);
-        e.top = __hiloint2double(c.w, c.z);
-        edge_fields(e, a.w < 0);
-        B = bin_edge(e.xi, e.fx, e.fxi, e.fdt, b.x, b.y, id, sub0 - off, kTileRows * sc);
+        e.x_start = __hiloint2double(a.y, a.x);
+        e.x_inc = __hiloint2double(a.w, a.z);
+        e.top = __hiloint2double(b.y, b.x);
+        edge_fields(e, (b.w & 1) != 0);
+        B = bin_edge(e.xi, e.fx, e.fxi, e.fdt, b.z, b.w >> 1, id, sub0 - off, kTileRows * sc);
     } else {
         const int4 a = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin);
         const int4 b = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin + 1);
@@ -113,17 +113,20 @@ __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const
 // The reference's evaluation, out of line: needed for one crossing in
 // thousands, and four copies of it in the crossing loop would be most of the
 // loop's code.
-static __device__ __noinline__ int32_t crossing_f64(const DEdge *__restrict__ e, int32_t sr) {
-    return (int32_t)round(e->x_start + (e->x_inc * (((double)sr + 0.5) - e->top)));
+static __device__ __noinline__ int32_t crossing_f64(double x_start, double x_inc, double top, int32_t sr) {
+    return (int32_t)round(x_start + (x_inc * (((double)sr + 0.5) - top)));
 }
 
 // Sample column, relative to the tile's first, where edge R crosses sample
 // row sub0 + r (r one of R.rows).
-__device__ __forceinline__ int32_t edge_crossing(const DEdge *__restrict__ edges, const RowEdge &R, int32_t r,
+template <bool GATHER>
+__device__ __forceinline__ int32_t edge_crossing(const void *__restrict__ edges, const RowEdge &R, int32_t r,
                                                  int32_t sub0, int32_t col0) {
     int32_t n;
     if (crossing_f32(R.v0, R.fxi, (float)r, R.lim, n)) return n + R.c0;
-    return crossing_f64(edges + R.id, sub0 + r) - col0;
+    using E = std::conditional_t<GATHER, SmallEdge, DEdge>;
+    const E *e = reinterpret_cast<const E *>(edges) + R.id;
+    return crossing_f64(e->x_start, e->x_inc, e->top, sub0 + r) - col0;
 }
 
 // Inside bits of the lane's columns on the row's sample rows by the non-zero
@@ -139,7 +142,7 @@ __device__ __forceinline__ int32_t edge_crossing(const DEdge *__restrict__ edges
 // registers of the common path.
 constexpr int32_t kDenseEdges = 256;
 template <bool GATHER>
-static __device__ __noinline__ uint4 winding_bits(const void *bins, const DEdge *edges, int32_t e0, int32_t ne,
+static __device__ __noinline__ uint4 winding_bits(const void *bins, const void *edges, int32_t e0, int32_t ne,
                                                   int32_t sub0, int32_t off, int32_t sc, int32_t col0, uint32_t *words,
                                                   int lane) {
     constexpr uint32_t kBias2 = 0x80008000u;
@@ -159,7 +162,7 @@ static __device__ __noinline__ uint4 winding_bits(const void *bins, const DEdge 
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 if (!((R.rows >> (s0 + h)) & 1u)) continue;
-                const int32_t c = edge_crossing(edges, R, s0 + h, sub0, col0);
+                const int32_t c = edge_crossing<GATHER>(edges, R, s0 + h, sub0, col0);
                 if (c <= 0) {
                     left += R.down ? (h ? -65536 : -1) : (h ? 65536 : 1);
                 } else if (c < 32 * per) {
@@ -357,7 +360,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     const RowEdge R = row_edge<GATHER>(A.bins, A.edges, e0 + base + lane, base + lane < ne, sub0, off, sc, col0);
                     auto cross = [&](int r) {
                         if (!((R.rows >> r) & 1u)) return;
-                        const int32_t c = edge_crossing(A.edges, R, r, sub0, col0);
+                        const int32_t c = edge_crossing<GATHER>(A.edges, R, r, sub0, col0);
                         if (c <= 0) {
                             const int32_t d = R.down ? -1 : 1;
                             if (r < 2) l01 += r == 0 ? d : d * 65536;

@@ -56,6 +56,15 @@ Z2D_HD BinEdge bin_edge(int32_t xi, float fx, float fxi, float fdt, int32_t rt, 
 }
 static_assert(sizeof(BinEdge) == 32, "BinEdge: two 16-byte accesses");
 
+// An edge as the one-upload path's host writes it: what its f32 fields are
+// made from, in 32 bytes (the upload of a call of 1,500 edges is most of what
+// its tables weigh).
+struct SmallEdge {
+    double x_start, x_inc, top;
+    int32_t rt, rb2;  // rb2: 2 rb, + 1 for a downward edge
+};
+static_assert(sizeof(SmallEdge) == 32, "SmallEdge: two 16-byte accesses");
+
 // A tile of a batch of several surfaces: its surface, its band counted
 // from the surface's first touched one, and its tile column.
 struct TileRec {
@@ -67,7 +76,7 @@ struct RasterArgs {
     const DevJob *jobs;
     const FillCmd *fills;
     const FillState *st;
-    const DEdge *edges;
+    const void *edges;          // DEdge, or (gather) SmallEdge
     const void *bins;           // BinEdge records, or (gather) int32 indices of `edges`
     const int32_t *bin_off;
     const int32_t *band_count;  // per global band
