@@ -13,6 +13,7 @@
 // Both evaluate the batch per pixel exactly like runPrecision's lanes.
 #include <cuda_runtime.h>
 
+#define Z2D_HEAVY_CALL __device__ __forceinline__  // (z2d_pixel.cuh)
 #include "z2d_internal.h"
 
 namespace z2dg {
@@ -214,19 +215,27 @@ static void launch_fmt(Ctx &c, const CompJob &J, bool flat) {
 
 int launch_composite(Ctx &c, const CompJob &J) {
     if (J.y1 <= J.y0 || J.line_w <= 0) return Z2D_OK;
-    // The flat kernel applies when the region is the whole surface, the
-    // surface is a whole number of 16-byte chunks and every surface param
-    // has the destination's geometry.
-    bool flat = J.dst_x == 0 && J.dst_y == 0 && J.dsx == 0 && J.y0 == 0 && J.y1 == J.dst.h && J.line_w == J.dst.w;
-    const size_t bytes = ((size_t)J.dst.w * J.dst.h * fmt_bits(J.dst.fmt) + 7) / 8;
-    if (bytes % 16 != 0 || (reinterpret_cast<uintptr_t>(J.dst.data) & 15) != 0) flat = false;
-    for (int k = 0; k < J.n_ops && flat; k++) {
+    // whole: the region is the whole surface and every surface param has the
+    // destination's geometry.  The flat kernel also wants a whole number of
+    // 16-byte chunks.
+    bool whole = J.dst_x == 0 && J.dst_y == 0 && J.dsx == 0 && J.y0 == 0 && J.y1 == J.dst.h && J.line_w == J.dst.w;
+    bool computed = false;  // a gradient source, dithered or not
+    for (int k = 0; k < J.n_ops; k++) {
         const CompOp &o = J.ops[k];
-        if (o.dst.kind == SRC_SURFACE && (o.dst.sfc.w != J.dst.w || o.dst.sfc.h < J.dst.h)) flat = false;
-        if (o.src.kind == SRC_SURFACE && (o.src.sfc.w != J.dst.w || o.src.sfc.h < J.dst.h)) flat = false;
+        if (o.dst.kind == SRC_SURFACE && (o.dst.sfc.w != J.dst.w || o.dst.sfc.h < J.dst.h)) whole = false;
+        if (o.src.kind == SRC_SURFACE && (o.src.sfc.w != J.dst.w || o.src.sfc.h < J.dst.h)) whole = false;
+        for (const DevSrc *d : {&o.dst, &o.src}) computed |= d->kind == SRC_GRADIENT || d->kind == SRC_DITHER;
     }
+    const size_t bytes = ((size_t)J.dst.w * J.dst.h * fmt_bits(J.dst.fmt) + 7) / 8;
+    // A flat thread draws 16 bytes, which are 16 to 128 pixels of an alpha
+    // format, one after the other: with a gradient's few hundred instructions
+    // for each, the region kernel's thread per byte keeps the chip busier
+    // (1704 x 860 linear on alpha4 97 us, now 54; conic sRGB on alpha1 130, now
+    // 107).
+    const bool flat = whole && bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(J.dst.data) & 15) == 0 &&
+                      !(computed && J.dst.fmt > Z2D_FORMAT_RGBA);
     cudaEvent_t t0 = c.timer_begin(c.t_composite);
-    if (try_mask_batch(c, J, flat) || try_mask_grad(c, J, flat) || try_layer(c, J)) {
+    if (try_mask_batch(c, J, whole) || try_mask_grad(c, J, whole) || try_layer(c, J)) {
     } else if (J.precision == Z2D_PRECISION_FLOAT) {
         launch_fmt<Z2D_PRECISION_FLOAT>(c, J, flat);
     } else {

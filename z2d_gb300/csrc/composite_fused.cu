@@ -25,6 +25,7 @@
 // once, with several 16-byte loads in flight per thread before any compute.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 #include <utility>
@@ -76,7 +77,7 @@ struct PackedTable {
 
 template <int FMT, int OP>
 __global__ void __launch_bounds__(kFusedThreads) k_mask_packed(uint8_t *__restrict__ dst, const uint8_t *__restrict__ mask,
-                                                               size_t n_items, uint32_t spa) {
+                                                               size_t n_items, uint32_t n_tail, uint32_t spa) {
     constexpr int BITS = FMT == Z2D_FORMAT_ALPHA4 ? 4 : FMT == Z2D_FORMAT_ALPHA2 ? 2 : 1;
     constexpr uint32_t MAXV = (1u << BITS) - 1u;
     using TB = PackedTable<BITS>;
@@ -131,6 +132,19 @@ __global__ void __launch_bounds__(kFusedThreads) k_mask_packed(uint8_t *__restri
             }
             d[it] = U::put(out);
         }
+    }
+    // the pixels after the last whole item, a byte per thread
+    constexpr uint32_t PER = 8 / BITS;
+    const uint32_t first = threadIdx.x * PER;
+    if (blockIdx.x + 1 == gridDim.x && first < n_tail) {
+        uint8_t *const b = dst + n_items * (2 * BITS) + threadIdx.x;
+        uint32_t v = *b;
+        for (uint32_t k = 0; k < PER && first + k < n_tail; k++) {
+            const uint32_t raw = (v >> (k * BITS)) & MAXV;
+            const uint32_t pos = ((uint32_t)mask[n_items * 16 + first + k] << TB::POS_M) | (raw << TB::LOGB);
+            v = (v & ~(MAXV << (k * BITS))) | (((words[pos >> 5] >> (pos & 31u)) & MAXV) << (k * BITS));
+        }
+        *b = (uint8_t)v;
     }
 }
 
@@ -191,7 +205,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_mask_float(uint8_t *__restric
     }
 }
 
-using PackedKernel = void (*)(uint8_t *, const uint8_t *, size_t, uint32_t);
+using PackedKernel = void (*)(uint8_t *, const uint8_t *, size_t, uint32_t, uint32_t);
 using FloatKernel = void (*)(uint8_t *, const uint8_t *, size_t, F4);
 
 template <int FMT, int... OPS>
@@ -224,10 +238,8 @@ static size_t grid_for(std::atomic<int> &slot, K k, const Ctx &c, size_t units, 
 }
 
 // Integer mask batch on alpha4 / alpha2 / alpha1 (the shape is checked by
-// try_mask_batch).  Needs a whole number of 16-pixel items and a
-// destination aligned to its per-item vector.
+// try_mask_batch).  Needs a destination aligned to its per-item vector.
 bool launch_mask_packed(Ctx &c, uint8_t *dst, int fmt, const uint8_t *mask, size_t px, int op, const I16 &spx) {
-    if (px % 16 != 0) return false;
     const int bits = fmt_bits(fmt);
     if ((reinterpret_cast<uintptr_t>(dst) & (uintptr_t)(2 * bits - 1)) != 0) return false;
     const std::make_integer_sequence<int, Z2D_OP_COUNT> ops{};
@@ -241,9 +253,8 @@ bool launch_mask_packed(Ctx &c, uint8_t *dst, int fmt, const uint8_t *mask, size
     }
     const size_t smem = bits == 4 ? PackedTable<4>::SMEM : bits == 2 ? PackedTable<2>::SMEM : PackedTable<1>::SMEM;
     const size_t n_items = px / 16;
-    const size_t blocks = grid_for(g_packed_occ[slot][op], k, c, n_items, smem);
-    if (blocks == 0) return true;
-    k<<<(unsigned)blocks, kFusedThreads, smem, c.stream>>>(dst, mask, n_items, spx.a);
+    const size_t blocks = std::max<size_t>(grid_for(g_packed_occ[slot][op], k, c, n_items, smem), 1);  // (1: a tail alone)
+    k<<<(unsigned)blocks, kFusedThreads, smem, c.stream>>>(dst, mask, n_items, (uint32_t)(px % 16), spx.a);
     c.launches++;
     return true;
 }

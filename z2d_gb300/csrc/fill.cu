@@ -3,8 +3,8 @@
 //
 // Pipeline (one launch each, all on the context stream):
 //   k_node_count_w  32 nodes per warp: how many edges each line/curve
-//                 emits (Bezier subdivision of Spline.zig:37-165; curves
-//                 subdivided by the whole warp)
+//                 emits; k_curve_count_w subdivides the curves among them
+//                 (Spline.zig:37-165), 1 to 32 lanes a curve
 //   stroke_count  device-stroked commands (stroke_gpu.cu): their polygons'
 //                 edge counts
 //   k_fill_scan   warp per fill: the sequential part of fill_plotter.plot
@@ -16,13 +16,14 @@
 //   k_fill_setup  thread per fill: Polygon.inBox and the draw box of
 //                 multisample.run / direct.run
 //   k_bin_count / k_bin_fill   (edge, 4-row band) lists per fill
-//   k_band_lists  CTA per band: the fills touching the band, in call order
+//   k_band_lists  CTA or warp per band: the fills touching the band, in call
+//                 order
 //   k_exact       thread per degenerate fill: literal restatement of the
 //                 sorted-span rasteriser, writing a per-pixel action mask
-//   k_raster      CTA per 4x256 tile: for each fill in order, winding deltas
-//                 per sub-scanline in shared memory, a warp prefix scan per
-//                 sub-scanline, coverage, then z2d's span compositing rules
-//                 (raster/shared.zig) applied to the tile held in registers.
+//   k_raster      (raster.cu) per pixel row of a 4x256 tile: for each fill in
+//                 order, crossings as bit planes in shared memory, inside
+//                 bits, coverage, then z2d's span compositing rules
+//                 (raster/shared.zig) on pixels held in registers.
 //
 // Why the winding scan equals z2d's sorted spans: on every sub-scanline
 // z2d sorts the active edges' rounded crossings, keeps the 0<->non-zero

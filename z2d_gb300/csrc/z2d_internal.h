@@ -255,7 +255,7 @@ int fill_jobs(Ctx &c, const z2d_job *jobs, size_t n_jobs, const z2d_node *nodes,
 const char *last_error();
 // Launches the whole-surface mask batch [dst_in(pixel, alpha8 mask), op]
 // when J has that shape (composite_mask.cu); returns false otherwise.
-bool try_mask_batch(Ctx &c, const CompJob &J, bool flat);
+bool try_mask_batch(Ctx &c, const CompJob &J, bool whole);
 // The same batch in float precision (4-byte formats, alpha8) and on the
 // packed alpha formats in integer precision (composite_fused.cu); false
 // when the surface does not fit the kernel's layout.
@@ -263,7 +263,7 @@ bool launch_mask_float(Ctx &c, uint8_t *dst, int fmt, const uint8_t *mask, size_
 bool launch_mask_packed(Ctx &c, uint8_t *dst, int fmt, const uint8_t *mask, size_t px, int op, const I16 &spx);
 // The same batch with a gradient or dithered-gradient source on the 4-byte
 // formats in integer precision (composite_grad.cu).
-bool try_mask_grad(Ctx &c, const CompJob &J, bool flat);
+bool try_mask_grad(Ctx &c, const CompJob &J, bool whole);
 // One surface composited onto another, 4-byte formats in integer precision
 // (composite_layer.cu).
 bool try_layer(Ctx &c, const CompJob &J);

@@ -594,13 +594,22 @@ Z2D_D float grad_offset_f64(const DevGradient &gr, int32_t x, int32_t y) {
     return (float)(ang / twopi);
 }
 
-static __device__ __noinline__ float offset_f64_call(const DevGradient &gr, int32_t x, int32_t y) {
+// The heavy steps of a gradient pixel are out of line, one copy each per
+// translation unit (with them inlined into every place that evaluates a
+// source, the rasteriser's warps, each on a fill of its own, waited for
+// instructions most of the time), unless the unit defines otherwise: the
+// general compositor's float kernels, where all warps run the same
+// source, lose 4-13 % to the calls.
+#ifndef Z2D_HEAVY_CALL
+#define Z2D_HEAVY_CALL static __device__ __noinline__
+#endif
+Z2D_HEAVY_CALL float offset_f64_call(const DevGradient &gr, int32_t x, int32_t y) {
     return grad_offset_f64(gr, x, y);
 }
 // One kind's double-word evaluation, out of line; 2 where it does not decide
 // (an offset is at most 1).
 template <int MODE>
-static __device__ __noinline__ float offset_fast_call(const GradFast &F, bool tf, float fx, float fy) {
+Z2D_HEAVY_CALL float offset_fast_call(const GradFast &F, bool tf, float fx, float fy) {
     float t = 0.0f;
     int done;
     if constexpr (MODE == kFastLinear) done = fast_linear(F, tf, fx, fy, t);
@@ -711,12 +720,8 @@ Z2D_D HSLf hsl_lerp_demul(RGBf am, RGBf bm, float t, int polar) {
     if (o.a == 0.0f) return HSLf{o.h, 0.0f, 0.0f, o.a};
     return HSLf{o.h, o.s / o.a, o.l / o.a, o.a};
 }
-// The heavy steps of a gradient pixel, out of line: one copy each per
-// translation unit.  With them inlined into every place that evaluates a
-// source, the rasteriser's warps (each on a fill of its own) waited for
-// instructions most of the time.
-static __device__ __noinline__ float gamma_call(float x) { return zpow(x, kGamma); }
-static __device__ __noinline__ RGBf hsl_call(RGBf a, RGBf b, float t, int polar) {
+Z2D_HEAVY_CALL float gamma_call(float x) { return zpow(x, kGamma); }
+Z2D_HEAVY_CALL RGBf hsl_call(RGBf a, RGBf b, float t, int polar) {
     return hsl_to_rgb(hsl_lerp_demul(a, b, t, polar));
 }
 // interpolateEncode: the integer lanes of the interpolated colour.
@@ -859,6 +864,7 @@ static __device__ __noinline__ F4 float_op_any(int op, F4 d, F4 s) { return floa
 // Source lanes with the pixel case inline.
 __device__ __forceinline__ I16 src_i16_fast(const DevSrc &s, int32_t x, int32_t y, size_t idx) {
     if (s.kind == SRC_PIXEL) return s.pix;
+    if (s.kind == SRC_SURFACE) return src_i16_slow(s, x, y, idx);
     return src_i16_any(s, x, y, idx);
 }
 __device__ __forceinline__ F4 src_f4_fast(const DevSrc &s, int32_t x, int32_t y, size_t idx) {
