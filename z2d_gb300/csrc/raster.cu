@@ -57,7 +57,7 @@ __device__ __forceinline__ bool msaa_unbounded_clear(const FillState &S, int32_t
 // the inside bits are the prefix XOR of the toggles.  Issue bound, on the
 // ALU pipe: a fill costs a row and tile of the 2,000-path 4096x4096 batch
 // (2.9 M of them, 28 edges each on average) about 690 warp instructions
-// instead of 1,250, and the kernel takes 1.97 ms instead of 4.30.
+// instead of 1,250, and the kernel takes 1.93 ms instead of 4.30.
 constexpr int kPlanes = 6;
 constexpr int kSubWords = kPlanes * 32;         // one sample row
 constexpr int kDenseWords = 2 * 16 * 32 + 2 * 32;  // or winding_bits' counters
@@ -76,7 +76,7 @@ struct RowEdge {
 // Bin entry `bin` for the pixel row whose sc sample rows begin at row `off` of
 // the band's.  What does not depend on the pixel row is in the record: a
 // record is read by every row and tile column of its band (2,000 paths: with
-// rows, t and limit worked out here 2.07 ms, now 1.97).
+// rows, t and limit worked out here 2.07 ms, with the record 1.97).
 template <bool GATHER>
 __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const void *__restrict__ edges,
                                             int32_t bin, bool valid, int32_t sub0, int32_t off, int32_t sc,
@@ -818,8 +818,16 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 //    taken by a single warp: a warp that finishes a cheap row takes the
 //    next item at once instead of holding its CTA until the slowest warp of
 //    the tile is done.
+// CTAs per SM: nine of the plain variants for one surface (56 registers;
+// 2,000 paths with 7, 8, 9, 10 and 11: 2.08, 1.97, 1.93, 1.95 and 2.09 ms),
+// eight for several surfaces (320 surfaces with 7, 8 and 9: 3.14, 3.06 and
+// 3.15 ms: the job's fields take registers), six of the general ones (240
+// gradient fills with 4, 6 and 8: 0.82, 0.75 and 0.77 ms).
+constexpr int raster_ctas(bool multi, int mode, bool gather) {
+    return mode == kGeneral ? 6 : multi || gather ? 8 : 9;
+}
 template <bool MULTI, bool CTA_ITEMS, int MODE, bool GATHER = false>
-__global__ void __launch_bounds__(kRasterThreads, MODE != kGeneral ? 8 : 6) k_raster(const RasterArgs A) {
+__global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, GATHER)) k_raster(const RasterArgs A) {
     extern __shared__ uint32_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *words = smem + warp * kWarpWords;
