@@ -1789,7 +1789,7 @@ size_t estimate_edges(const z2d_node *nodes, int32_t n, double tol) {
 
 // A small call's tables as a kernel's parameters: the launch carries them, so
 // no copy engine, event or staging slot is between the call and its raster
-// kernel.  Such calls are bound by their driver calls and by the wait of the
+// kernel.  Such calls are bound by their CUDA calls and by the wait of the
 // raster kernel for its tables (the 300x300 star from Python: copied 16.4 us,
 // now 14.3).  Larger tables stay with the copy: a launch's parameters are
 // written by the host a second time, and end at 32 KB.

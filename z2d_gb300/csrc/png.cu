@@ -272,7 +272,7 @@ size_t png_scanlines_size(int32_t fmt, int32_t w, int32_t h) {
 // rows come back through two pinned slots: while one piece is on its way the
 // host pool copies the last one to where the caller wants it (touching its
 // fresh pages from several threads).  A copy into pageable memory instead
-// runs at the driver's staging rate: the call took 1.9 ms for 14.8 MB, now 0.46.
+// runs at the rate of CUDA's own staging: the call took 1.9 ms for 14.8 MB, now 0.46.
 int png_scanlines(Ctx &c, const DevSurface &s, int profile, uint8_t *out) {
     constexpr size_t kPiece = (size_t)4 << 20;
     const int fmt = s.fmt;
