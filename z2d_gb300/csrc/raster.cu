@@ -285,7 +285,10 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 
     for (int i = lane; i < kCovOff; i += 32) words[i] = 0u;
     uint32_t raw[8];
-    uint32_t touched = 0;  // blocks of 32 pixels to store (the same in every lane)
+    // This lane's pixels that some fill has drawn, a bit per block: only those
+    // are stored.  (Their neighbours may be another stream's to draw: a block
+    // stored whole would put back what it held when this row began.)
+    uint32_t touched = 0;
     {
         const DevSurface dst = JB.sfc;
 #pragma unroll
@@ -663,7 +666,6 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 if (!blocks) continue;
                 // Lane k holds the source word for coverage k (k_edge_fill).
                 const uint32_t lut_w = __ldg(A.luts + 32 * (size_t)__shfl_sync(kAll, my_f, src) + lane);
-                touched |= blocks;
                 if (fmt <= Z2D_FORMAT_RGBA) {
                     const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
 #pragma unroll
@@ -673,6 +675,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                         const uint32_t L = __shfl_sync(kAll, lut_w, c);
                         const uint32_t nv = word_src_over_fma(raw[q], L, has_alpha);
                         raw[q] = c != 0 ? nv : raw[q];
+                        touched |= c != 0 ? 1u << q : 0u;
                     }
                 } else {  // alpha formats: the alpha lane of src_over alone
 #pragma unroll
@@ -680,7 +683,9 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                         if (!((blocks >> q) & 1u)) continue;
                         const int c = cov[32 * q];
                         const uint32_t sa = __shfl_sync(kAll, lut_w, c);
-                        if (c != 0) raw[q] = alpha_src_over(raw[q], sa, fmt);
+                        if (c == 0) continue;
+                        raw[q] = alpha_src_over(raw[q], sa, fmt);
+                        touched |= 1u << q;
                     }
                 }
                 continue;
@@ -699,7 +704,6 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 // pixel without coverage composites a clear source: without
                 // an alpha channel that would still rewrite its padding byte.)
                 if (!blocks) continue;
-                touched |= blocks;
                 // the planes, clear at this point, hold the colours and the
                 // list
                 uint8_t *at = reinterpret_cast<uint8_t *>(words + kTileCols);
@@ -740,7 +744,9 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     if (!((blocks >> q) & 1u)) continue;
-                    if (cov[32 * q] != 0) raw[q] = word_src_over_fma(raw[q], words[32 * q + lane], has_alpha);
+                    if (cov[32 * q] == 0) continue;
+                    raw[q] = word_src_over_fma(raw[q], words[32 * q + lane], has_alpha);
+                    touched |= 1u << q;
                 }
                 __syncwarp();
                 for (int i = lane; i < kTileCols + kTileCols / 4; i += 32) words[i] = 0u;
@@ -787,7 +793,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                         rq = i16_to_raw(d, fmt);
                     }
                 }
-                if (!__any_sync(kAll, on)) continue;
+                if (!on) continue;
                 touched |= 1u << q;
 #pragma unroll
                 for (int j = 0; j < 8; j++)
