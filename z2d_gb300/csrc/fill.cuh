@@ -94,7 +94,7 @@ Z2D_HD bool edge_fields(DEdge &e, bool down) {
     bool neg;
     bool ok = fixed_coord(e.x_start, w, f, neg);
     const float fx = frac_f32(f);
-    e.xi = neg ? -(int32_t)w : (int32_t)w;
+    e.xi = (int32_t)(neg ? 0u - w : w);
     e.fx = neg ? -fx : fx;
     uint64_t b;
     memcpy(&b, &e.x_inc, 8);
@@ -109,7 +109,7 @@ Z2D_HD bool edge_fields(DEdge &e, bool down) {
     const uint32_t up = f >> 31;
     const float r = frac_f32(f), m = (float)up;
     const float d = neg ? (0.5f - m) + r : (0.5f + m) - r;
-    e.rt = neg ? -(int32_t)(w + up) : (int32_t)(w + up);
+    e.rt = (int32_t)(neg ? 0u - (w + up) : w + up);
     e.fdt = down ? -d : d;
     if (!(ok && top_ok)) e.fx = f32_of_bits(0x7FC00000u);
     return top_ok;

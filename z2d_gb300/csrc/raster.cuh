@@ -30,7 +30,8 @@ struct BinEdge {
     float limit;
     int32_t id, _pad;
 };
-// The record of an edge (its DEdge fields) for the n sample rows from `row`.
+// The record of an edge (its DEdge fields) for the n sample rows from `row`
+// (>= 0).
 // A pixel row evaluates fma(fxi, r, fma(fxi, t + w, fx)) with s = w + r.
 // With T >= |t|, |t + w| and the largest t + s, p = |fxi| T and u = 2^-24, the
 // error is at most u (2 p (slope) + 3 p (t: the conversion and two sums)
@@ -39,17 +40,22 @@ struct BinEdge {
 Z2D_HD BinEdge bin_edge(int32_t xi, float fx, float fxi, float fdt, int32_t rt, int32_t rb, int32_t id, int32_t row,
                         int32_t n) {
     BinEdge B;
-    const int32_t rel = row - rt;
-    const int32_t lo = rel < 0 ? -rel : 0, hi = rb - row < n ? rb - row : n;
+    // rt and rb are the ends of an edge of any length, saturated at the ends of
+    // the int32 range: they are compared with the band before they are
+    // subtracted from it
+    const int32_t lo = rt <= row ? 0 : rt - row < n ? rt - row : n;
+    const int32_t hi = rb <= row ? 0 : rb - row < n ? rb - row : n;
+    const uint32_t away = rt <= row ? (uint32_t)row - (uint32_t)rt : (uint32_t)rt - (uint32_t)row;
+    const float rel = rt <= row ? (float)away : -(float)away;
     B.c = (int32_t)((uint32_t)xi - (uint32_t)kRoundMagicBits);
     B.fx = fx;
     B.fxi = fxi;
-    B.t = (float)rel + fabsf(fdt);
+    B.t = rel + fabsf(fdt);
     B.rows = lo < hi ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
     uint32_t dir;
     memcpy(&dir, &fdt, 4);
     B.rows |= dir & 0x80000000u;
-    B.limit = crossing_limit(fxi, (float)(rel + hi > 1 - rel ? rel + hi : 1 - rel));
+    B.limit = crossing_limit(fxi, fmaxf(rel + (float)hi, 1.0f - rel));
     B.id = id;
     B._pad = 0;
     return B;
