@@ -1,0 +1,20 @@
+// Host check of the index arithmetic of grids with a warp per item: the item
+// numbers at and beyond 2^27, where the thread's own number passes 32 bits.
+#include <cstdint>
+#include <cstdio>
+
+#include "fill.cuh"
+
+using namespace z2dg;
+
+int main() {
+    long long wrong = 0;
+    for (uint32_t threads : {256u})
+        for (long long item : {0ll, 1ll, (1ll << 27) - 1, 1ll << 27, (1ll << 27) + 5, 1ll << 30, (1ll << 31) - 1}) {
+            const uint32_t per = threads / 32;
+            const uint32_t block = (uint32_t)(item / per), first = (uint32_t)(item % per) * 32;
+            for (uint32_t lane : {0u, 31u}) wrong += warp_number(block, threads, first + lane) != item;
+        }
+    printf("wrong %lld\n", wrong);
+    return wrong ? 1 : 0;
+}

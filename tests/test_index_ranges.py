@@ -1,0 +1,50 @@
+"""Index arithmetic at the sizes where 32 bits end: on the host
+(tests/index_check.cu, built with nvcc as host code), and batches of more
+than 2^27 four-row bands on the GPU."""
+import os
+import shutil
+import subprocess
+import tempfile
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+def test_item_numbers():
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not found")
+    with tempfile.TemporaryDirectory() as d:
+        exe = os.path.join(d, "index_check")
+        subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O2", "-std=c++17",
+                        "-I", os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "z2d_gb300", "csrc"),
+                        os.path.join(HERE, "index_check.cu"), "-o", exe], check=True)
+        r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+def test_more_than_2_27_bands():
+    """66 surfaces of one column and 2^23 - 1 rows, each filled from top to
+    bottom: 66 * 2^21 bands of one fill."""
+    torch = pytest.importorskip("torch")
+    from z2d_gb300 import painter
+    from z2d_gb300.native import Context
+    from z2d_gb300.path import Path
+    from z2d_gb300.surface import Surface
+    from z2d_gb300.types import FillOptions, Pattern, Pixel
+    if torch.cuda.mem_get_info()[0] < 32 << 30:
+        pytest.skip("needs 32 GB of device memory")
+    h = (1 << 23) - 1
+    nodes = Path().move_to(0, 0).line_to(1, 0).line_to(1, h).line_to(0, h).close().to_array()
+    pat = Pattern.from_pixel(Pixel.rgba(0, 0, 0, 200))
+    dev = [Surface.init("alpha8", 1, h).to_device("cuda") for _ in range(66)]
+    torch.cuda.synchronize()
+    ctx = Context(0)
+    painter.fill_jobs([(d, [(pat, nodes, FillOptions())]) for d in dev], ctx=ctx)
+    ctx.synchronize()
+    ctx.close()
+    for k, d in enumerate(dev):
+        assert bool((d.data == 200).all()), f"surface {k}"

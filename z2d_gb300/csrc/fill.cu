@@ -872,8 +872,9 @@ __global__ void __launch_bounds__(256) k_band_lists_w(const FillState *__restric
                                                       int32_t n_jobs, int32_t n_gbands,
                                                       int32_t *__restrict__ band_count, int4 *__restrict__ band_fills,
                                                       TileRec *__restrict__ tiles) {
-    const int32_t gb = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (gb >= n_gbands) return;
+    const long long at = warp_number(blockIdx.x, blockDim.x, threadIdx.x);
+    if (at >= n_gbands) return;
+    const int32_t gb = (int32_t)at, lane = threadIdx.x & 31;
     const int32_t j = job_of(jobs, n_jobs, gb, [](const DevJob &J) { return (long long)J.gband_base; });
     const DevJob &J = jobs[j];
     const int32_t lb = gb - J.gband_base, b = J.band_lo + lb, nf = J.fill1 - J.fill0;

@@ -61,6 +61,12 @@ struct DEdge {
 
 static_assert(sizeof(DEdge) == 48, "DEdge layout: 16-byte f32 block, ranges, f64 fields");
 
+// A thread's warp among all of its grid's, for grids of one warp per item: with
+// 2^27 items and more the thread's own number does not fit 32 bits.
+Z2D_HD long long warp_number(uint32_t block, uint32_t threads, uint32_t thread) {
+    return ((long long)block * threads + thread) >> 5;
+}
+
 Z2D_HD float f32_of_bits(uint32_t b) {
     float f;
     memcpy(&f, &b, 4);
