@@ -9,7 +9,7 @@ using namespace z2dg;
 
 int main() {
     long long wrong = 0;
-    for (uint32_t threads : {256u})
+    for (uint32_t threads : {128u, 256u})
         for (long long item : {0ll, 1ll, (1ll << 27) - 1, 1ll << 27, (1ll << 27) + 5, 1ll << 30, (1ll << 31) - 1}) {
             const uint32_t per = threads / 32;
             const uint32_t block = (uint32_t)(item / per), first = (uint32_t)(item % per) * 32;

@@ -126,10 +126,10 @@ __global__ void ks_pen(const StrokeDev *__restrict__ strokes, const double *__re
 // ------------------------------------------------------------ raw points
 // A warp per subpath.
 __global__ void ks_local_sub(const SubpathDev *__restrict__ subs, int32_t n_subs, int32_t *__restrict__ local_sub) {
-    const int32_t sp = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const long long sp = warp_number(blockIdx.x, blockDim.x, threadIdx.x);
     if (sp >= n_subs) return;
     const int32_t l0 = subs[sp].local0, n = subs[sp].n_nodes;
-    for (int32_t j = threadIdx.x & 31; j < n; j += 32) local_sub[l0 + j] = sp;
+    for (int32_t j = threadIdx.x & 31; j < n; j += 32) local_sub[l0 + j] = (int32_t)sp;
 }
 
 // The points one node hands to the plotter: move_to its point, line_to its
