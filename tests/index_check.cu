@@ -1,9 +1,11 @@
 // Host check of the index arithmetic of grids with a warp per item: the item
-// numbers at and beyond 2^27, where the thread's own number passes 32 bits.
+// numbers at and beyond 2^27, where the thread's own number passes 32 bits;
+// and of the stroker's slots per node and lane, from 2^28 nodes on.
 #include <cstdint>
 #include <cstdio>
 
 #include "fill.cuh"
+#include "stroke_gpu.cuh"
 
 using namespace z2dg;
 
@@ -15,6 +17,9 @@ int main() {
             const uint32_t block = (uint32_t)(item / per), first = (uint32_t)(item % per) * 32;
             for (uint32_t lane : {0u, 31u}) wrong += warp_number(block, threads, first + lane) != item;
         }
+    for (int g : {0, 3, 5})
+        for (int32_t node : {0, 1, (1 << 26) - 1, 1 << 28, (1 << 28) + 3, 0x7FFFFFFF})
+            wrong += lane_slot(node, g) != (long long)node * (1 << g);
     printf("wrong %lld\n", wrong);
     return wrong ? 1 : 0;
 }

@@ -171,7 +171,7 @@ __global__ void ks_raw_count(const z2d_node *__restrict__ nodes, const SubpathDe
                              long long n_local, int g, long long *__restrict__ raw_cnt, int32_t *__restrict__ status) {
     const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = at >> g;
     if (i >= n_local) {
-        if (at == n_local << g) raw_cnt[at] = 0;
+        if (at == lane_slot(n_local, g)) raw_cnt[at] = 0;
         return;
     }
     const SubpathDev S = subs[local_sub[i]];
@@ -245,7 +245,7 @@ __global__ void ks_sub_setup(const SubpathDev *__restrict__ subs, int32_t n_subs
     const int32_t sp = blockIdx.x * blockDim.x + threadIdx.x;
     if (sp >= n_subs) return;
     const SubpathDev S = subs[sp];
-    const long long r0 = raw_off[S.local0 << g], r1 = raw_off[(S.local0 + S.n_nodes) << g];
+    const long long r0 = raw_off[lane_slot(S.local0, g)], r1 = raw_off[lane_slot((long long)S.local0 + S.n_nodes, g)];
     SubState st;
     st.q0 = kept_off[r0];
     st.n = kept_off[r1] - st.q0;
@@ -682,7 +682,7 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     Carve ca;
     // a warp per node while the device has room for all of them, else 8 lanes
     st.g = run.n_local * 32 <= (long long)c.sm_count * 2048 ? 5 : 3;
-    const long long n_lanes = run.n_local << st.g;
+    const long long n_lanes = lane_slot(run.n_local, st.g);
     const size_t o_cnt = ca.take<long long>(n_lanes + 1), o_off = ca.take<long long>(n_lanes + 1);
     const size_t o_lsub = ca.take<int32_t>(run.n_local + 1), o_pen = ca.take<PenVertex>(run.n_pen + 1);
     const size_t o_sub = ca.take<SubState>(run.n_subs + 1), o_reg = ca.take<Region>(run.n_subs + 1);

@@ -59,6 +59,10 @@ struct StrokeSet {
     bool empty() const { return strokes.empty() && polys.empty(); }
 };
 
+// The first of a node's 2^g slots in the per-lane counts (stroke_gpu.cu): up
+// to 2^31 nodes of 8 lanes, more than 32 bits hold.
+Z2D_HD long long lane_slot(long long node, int g) { return node << g; }
+
 // The contours of the host-built polygons on the device (structure of
 // arrays over all contours, in order): contour k is points
 // [start[k], start[k] + n[k]) of the point array, drawn by fill[k], its
