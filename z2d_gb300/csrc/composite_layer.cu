@@ -109,7 +109,7 @@ bool try_layer(Ctx &c, const CompJob &J) {
     A.rows = J.y1 - J.y0;
     A.dst_fmt = J.dst.fmt;
     A.src_fmt = s.fmt;
-    A.per_row = (J.line_w + kLayerChunk - 1) / kLayerChunk;
+    A.per_row = row_chunks(J.line_w, kLayerChunk);
     const long long blocks = ((long long)A.per_row * A.rows + kLayerWarps - 1) / kLayerWarps;
     if (blocks > 0x7FFFFFFFll) return false;
     const std::make_integer_sequence<int, Z2D_OP_COUNT> ops{};

@@ -286,7 +286,7 @@ int png_scanlines(Ctx &c, const DevSurface &s, int profile, uint8_t *out) {
     uint8_t *d = c.surface2.as<uint8_t>(), *stage = c.export_stage.as<uint8_t>();
     const long long n_units = units * s.h;
     if (fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB) {
-        const int32_t per_row = (s.w + 32 * kRowGroups - 1) / (32 * kRowGroups);
+        const int32_t per_row = row_chunks(s.w, 32 * kRowGroups);
         const long long chunks = (long long)per_row * s.h;
         cudaEvent_t te = c.timer_begin(c.t_export);
         k_png_rgba<<<(unsigned)std::min<long long>((chunks + 7) / 8, (long long)c.sm_count * 8), 256, 0, c.stream>>>(

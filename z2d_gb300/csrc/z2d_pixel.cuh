@@ -23,6 +23,8 @@ constexpr int kMaxStops = 32;
 Z2D_HD int fmt_bits(int f) {
     return f == Z2D_FORMAT_ALPHA8 ? 8 : f == Z2D_FORMAT_ALPHA4 ? 4 : f == Z2D_FORMAT_ALPHA2 ? 2 : f == Z2D_FORMAT_ALPHA1 ? 1 : 32;
 }
+// Runs of `per` pixels in a row of n >= 1, for any n of 31 bits.
+Z2D_HD int32_t row_chunks(int32_t n, int32_t per) { return (n - 1) / per + 1; }
 Z2D_HD bool fmt_packed(int f) { return f >= Z2D_FORMAT_ALPHA4; }
 Z2D_HD bool fmt_has_color(int f) { return f <= Z2D_FORMAT_RGBA; }
 Z2D_HD bool fmt_has_alpha(int f) { return f == Z2D_FORMAT_ARGB || f == Z2D_FORMAT_RGBA || f >= Z2D_FORMAT_ALPHA8; }
