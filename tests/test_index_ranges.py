@@ -68,3 +68,29 @@ def test_layer_of_the_widest_row():
     torch.cuda.synchronize()
     same = torch.equal(dst, src)  # 255 * s / 255
     assert same
+
+
+@pytest.mark.gpu
+def test_gradient_on_the_widest_rows():
+    """A gradient through a mask onto two rows of 2^31 - 1 alpha8 pixels: beyond
+    its end every pixel of both rows has the last stop's alpha."""
+    torch = pytest.importorskip("torch")
+    from z2d_gb300 import compositor
+    from z2d_gb300.surface import Surface
+    from z2d_gb300.types import Color, Gradient, Operation, Pattern
+    w, end = (1 << 31) - 1, 1 << 20
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 24 GB of device memory")
+    mask = torch.full((2 * w,), 255, dtype=torch.uint8, device="cuda")
+    dst = torch.zeros(2 * w, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    g = Gradient.linear(0, 0, end, 0)
+    g.add_stop(0.0, Color.rgb(0, 0, 0, 0)).add_stop(1.0, Color.rgb(0, 0, 0, 1))
+    compositor.SurfaceCompositor.run(Surface("alpha8", w, 2, dst), 0, 0,
+                                     [Operation("dst_in", dst=Pattern.from_gradient(g), src=Surface("alpha8", w, 2, mask)),
+                                      Operation("src")])
+    torch.cuda.synchronize()
+    for y in (0, 1):
+        row = dst[y * w:(y + 1) * w]
+        first, other = int(row[0]), int((row[end:] != 255).sum())
+        assert first == 0 and other == 0, f"row {y}"

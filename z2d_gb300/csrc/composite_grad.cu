@@ -162,11 +162,12 @@ __global__ void __launch_bounds__(kGradThreads) k_mask_grad(uint8_t *__restrict_
             exact(n + lane);
             __syncwarp();
         }
-        x += r;
         y += q;
-        if (x >= W) {
-            x -= W;
+        if (x >= W - r) {  // (x + r may not fit)
+            x -= W - r;
             y++;
+        } else {
+            x += r;
         }
     }
     __syncwarp();
