@@ -47,6 +47,7 @@ int DevBuf::ensure(size_t bytes) {
     ptr = nullptr;
     cap = 0;
     if (cudaMalloc(&ptr, n) != cudaSuccess) {
+        cudaGetLastError();  // not the next launch's error: the caller may do with less
         ptr = nullptr;
         set_errorf("device allocation of %zu bytes failed", n);
         return 1;

@@ -818,16 +818,22 @@ __global__ void k_bin_count(const FillCmd *__restrict__ fills, const FillState *
 
 // The rasteriser reads an edge once per tile column and row of a band: the
 // bin holds what it reads, one coalesced 32-byte record per entry, instead of
-// an index to gather it by.
+// an index to gather it by (RECORDS; without, the index: BinKind).
+template <bool RECORDS>
 __global__ void k_bin_fill(const FillCmd *__restrict__ fills, const FillState *__restrict__ st,
                            const DEdge *__restrict__ edges, const int32_t *__restrict__ edge_fill, int32_t n_edges,
-                           int32_t *__restrict__ fb_cursor, BinEdge *__restrict__ bins) {
+                           int32_t *__restrict__ fb_cursor, void *__restrict__ bins) {
     for_edge_bands(fills, st, edges, edge_fill, n_edges, [&](int32_t edge, int32_t fb, int32_t row, int32_t rows) {
+        const int32_t at = atomicAdd(&fb_cursor[fb], 1);
+        if constexpr (!RECORDS) {
+            reinterpret_cast<int32_t *>(bins)[at] = edge;
+            return;
+        }
         const int4 a = __ldg(reinterpret_cast<const int4 *>(edges + edge));
         const int2 r = __ldg(reinterpret_cast<const int2 *>(&edges[edge].rt));
         const BinEdge B = bin_edge(a.x, __int_as_float(a.y), __int_as_float(a.z), __int_as_float(a.w), r.x, r.y, edge,
                                    row, rows);
-        int4 *out = reinterpret_cast<int4 *>(bins + atomicAdd(&fb_cursor[fb], 1));
+        int4 *out = reinterpret_cast<int4 *>(reinterpret_cast<BinEdge *>(bins) + at);
         out[0] = make_int4(B.c, __float_as_int(B.fx), __float_as_int(B.fxi), __float_as_int(B.t));
         out[1] = make_int4((int32_t)B.rows, __float_as_int(B.limit), B.id, 0);
     });
@@ -1442,21 +1448,30 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         set_error("a fill has more than 32000 edges inside one 4-row band");
         return rb[1];
     }
-    if (c.bins.ensure(sizeof(BinEdge) * (size_t)std::max(n_bin_entries, 1))) return Z2D_ERR_OUT_OF_MEMORY;
-    // scatter with the counts array reused as cursors
-    Z2D_CUDA(cudaMemcpyAsync(d_fb_cnt, d_fb_off, sizeof(int32_t) * (size_t)(n_fb + 1), cudaMemcpyDeviceToDevice, c.stream));
-    tb = c.timer_begin(c.t_bins);
-    if (n_edges > 0 && n_bin_entries > 0) {
-        k_bin_fill<<<grid_for(n_edges, 256), 256, 0, c.stream>>>(d_fills, d_st, d_edges, d_edge_fill, n_edges, d_fb_cnt,
-                                                                  c.bins.as<BinEdge>());
-        c.launches++;
-    }
-
-    // ---- ordered fill lists per global band
+    // the band lists and the exact path's masks, then the bins: what is left
+    // decides whether they hold records or, an eighth of them, indices
     const size_t count_bytes = ((sizeof(int32_t) * (size_t)n_gbands) + 15) & ~(size_t)15;
     const size_t tile_bytes = n_jobs > 1 ? sizeof(TileRec) * (size_t)n_tiles : 0;
     if (c.band_fills.ensure(count_bytes + tile_bytes + sizeof(int4) * (size_t)std::max(n_slots, 1ll)))
         return Z2D_ERR_OUT_OF_MEMORY;
+    // masks plus per-fill work arrays
+    if (n_exact > 0 && c.masks.ensure((size_t)mask_bytes + 64)) return Z2D_ERR_OUT_OF_MEMORY;
+    BinKind bin_kind = kBinRecords;
+    if (c.bins.ensure(sizeof(BinEdge) * (size_t)std::max(n_bin_entries, 1))) {
+        bin_kind = kBinIndex;
+        if (c.bins.ensure(sizeof(int32_t) * (size_t)std::max(n_bin_entries, 1))) return Z2D_ERR_OUT_OF_MEMORY;
+    }
+    // scatter with the counts array reused as cursors
+    Z2D_CUDA(cudaMemcpyAsync(d_fb_cnt, d_fb_off, sizeof(int32_t) * (size_t)(n_fb + 1), cudaMemcpyDeviceToDevice, c.stream));
+    tb = c.timer_begin(c.t_bins);
+    if (n_edges > 0 && n_bin_entries > 0) {
+        const auto bin_fill = bin_kind == kBinRecords ? k_bin_fill<true> : k_bin_fill<false>;
+        bin_fill<<<grid_for(n_edges, 256), 256, 0, c.stream>>>(d_fills, d_st, d_edges, d_edge_fill, n_edges, d_fb_cnt,
+                                                                c.bins.ptr);
+        c.launches++;
+    }
+
+    // ---- ordered fill lists per global band
     int32_t *d_band_count = c.band_fills.as<int32_t>();
     TileRec *d_tiles = n_jobs > 1 ? reinterpret_cast<TileRec *>(c.band_fills.as<uint8_t>() + count_bytes) : nullptr;
     int4 *d_band_fills = reinterpret_cast<int4 *>(c.band_fills.as<uint8_t>() + count_bytes + tile_bytes);
@@ -1470,9 +1485,6 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
 
     // ---- exact path
     if (n_exact > 0) {
-        // mask plus per-fill work arrays (3 ints per edge, 8-byte aligned)
-        const size_t need = (size_t)mask_bytes + 64;
-        if (c.masks.ensure(need)) return Z2D_ERR_OUT_OF_MEMORY;
         Z2D_CUDA(cudaMemsetAsync(c.masks.ptr, 0, (size_t)mask_bytes, c.stream));
         k_exact<<<grid_for(n_fills, 32), 32, 0, c.stream>>>(d_fills, d_st, d_edges, n_fills, d_jobs, c.masks.as<uint8_t>());
         c.launches++;
@@ -1485,7 +1497,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     A.fills = d_fills;
     A.st = d_st;
     A.edges = d_edges;
-    A.bins = c.bins.as<BinEdge>();
+    A.bins = c.bins.ptr;
     A.bin_off = d_fb_off;
     A.band_count = d_band_count;
     A.band_fills = d_band_fills;
@@ -1501,7 +1513,8 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     }
     // persistent grid: every SM filled to the kernel's residency (or the
     // tuned CTAs per SM), never more CTAs than tiles
-    RasterVariant variant{n_jobs > 1, false, false, raster_mode(fills.data(), fills.size(), n_exact > 0)};
+    RasterVariant variant{n_jobs > 1, false, bin_kind, raster_mode(fills.data(), fills.size(), n_exact > 0)};
+    if (bin_kind == kBinIndex) variant.mode = kGeneral;
     int occ = 1;
     {
         const int rc = raster_occupancy(c, variant, occ);
@@ -1511,7 +1524,9 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     const TuneKey key = tune_key(n_jobs, n_tiles, n_slots, n_gbands);
     c.last_key = key;
     RasterPlan plan{c.raster_ctas_per_sm, c.raster_order, c.raster_cta_items, -1};
-    if (!c.raster_forced) {
+    if (bin_kind == kBinIndex) {  // (one schedule: its variants draw rows)
+        plan = RasterPlan{0, 0, 0, -1};
+    } else if (!c.raster_forced) {
         c.tune_collect(false);
         plan = tune_pick(key);
     }
@@ -2065,7 +2080,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         const int rs = c.await_surface();
         if (rs) return rs;
     }
-    const RasterVariant variant{n_jobs > 1, true, true, raster_mode(fills.data(), n_fills, false)};
+    const RasterVariant variant{n_jobs > 1, true, kBinSmall, raster_mode(fills.data(), n_fills, false)};
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
     const int rc = raster_launch(c, variant, A, (unsigned)n_tiles);
     if (rc) return rc;

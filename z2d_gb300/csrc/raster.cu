@@ -77,14 +77,14 @@ struct RowEdge {
 // the band's.  What does not depend on the pixel row is in the record: a
 // record is read by every row and tile column of its band (2,000 paths: with
 // rows, t and limit worked out here 2.07 ms, with the record 1.97).
-template <bool GATHER>
+template <int BINS>
 __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const void *__restrict__ edges,
                                             int32_t bin, bool valid, int32_t sub0, int32_t off, int32_t sc,
                                             int32_t col0) {
     RowEdge R{};
     if (!valid) return R;
     BinEdge B;
-    if constexpr (GATHER) {
+    if constexpr (BINS == kBinSmall) {
         const int32_t id = __ldg(reinterpret_cast<const int32_t *>(bins) + bin);
         const int4 a = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id);
         const int4 b = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id + 1);
@@ -94,6 +94,13 @@ __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const
         e.top = __hiloint2double(b.y, b.x);
         edge_fields(e, (b.w & 1) != 0);
         B = bin_edge(e.xi, e.fx, e.fxi, e.fdt, b.z, b.w >> 1, id, sub0 - off, kTileRows * sc);
+    } else if constexpr (BINS == kBinIndex) {
+        const int32_t id = __ldg(reinterpret_cast<const int32_t *>(bins) + bin);
+        const DEdge *e = reinterpret_cast<const DEdge *>(edges) + id;
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(e));
+        const int2 b = __ldg(reinterpret_cast<const int2 *>(&e->rt));
+        B = bin_edge(a.x, __int_as_float(a.y), __int_as_float(a.z), __int_as_float(a.w), b.x, b.y, id, sub0 - off,
+                     kTileRows * sc);
     } else {
         const int4 a = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin);
         const int4 b = __ldg(reinterpret_cast<const int4 *>(bins) + 2 * (size_t)bin + 1);
@@ -119,12 +126,12 @@ static __device__ __noinline__ int32_t crossing_f64(double x_start, double x_inc
 
 // Sample column, relative to the tile's first, where edge R crosses sample
 // row sub0 + r (r one of R.rows).
-template <bool GATHER>
+template <int BINS>
 __device__ __forceinline__ int32_t edge_crossing(const void *__restrict__ edges, const RowEdge &R, int32_t r,
                                                  int32_t sub0, int32_t col0) {
     int32_t n;
     if (crossing_f32(R.v0, R.fxi, (float)r, R.lim, n)) return n + R.c0;
-    using E = std::conditional_t<GATHER, SmallEdge, DEdge>;
+    using E = std::conditional_t<BINS == kBinSmall, SmallEdge, DEdge>;
     const E *e = reinterpret_cast<const E *>(edges) + R.id;
     return crossing_f64(e->x_start, e->x_inc, e->top, sub0 + r) - col0;
 }
@@ -141,7 +148,7 @@ __device__ __forceinline__ int32_t edge_crossing(const void *__restrict__ edges,
 // themselves, paths much smaller than their detail).  Out of line, for the
 // registers of the common path.
 constexpr int32_t kDenseEdges = 256;
-template <bool GATHER>
+template <int BINS>
 static __device__ __noinline__ uint4 winding_bits(const void *bins, const void *edges, int32_t e0, int32_t ne,
                                                   int32_t sub0, int32_t off, int32_t sc, int32_t col0, uint32_t *words,
                                                   int lane) {
@@ -158,11 +165,11 @@ static __device__ __noinline__ uint4 winding_bits(const void *bins, const void *
         if (s0 >= sc) break;
         int32_t left = 0;  // rows s0 and s0 + 1 as lo + 65536 hi
         for (int32_t base = 0; base < ne; base += 32) {
-            const RowEdge R = row_edge<GATHER>(bins, edges, e0 + base + lane, base + lane < ne, sub0, off, sc, col0);
+            const RowEdge R = row_edge<BINS>(bins, edges, e0 + base + lane, base + lane < ne, sub0, off, sc, col0);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 if (!((R.rows >> (s0 + h)) & 1u)) continue;
-                const int32_t c = edge_crossing<GATHER>(edges, R, s0 + h, sub0, col0);
+                const int32_t c = edge_crossing<BINS>(edges, R, s0 + h, sub0, col0);
                 if (c <= 0) {
                     left += R.down ? (h ? -65536 : -1) : (h ? 65536 : 1);
                 } else if (c < 32 * per) {
@@ -248,7 +255,7 @@ static __device__ __noinline__ uint32_t alpha_src_over(uint32_t raw, uint32_t sa
 // MULTI = false draws a one-surface batch from A.job0, whose fields are
 // kernel parameters (warp-uniform values that need no registers);
 // MULTI = true finds the tile's job in the job table.
-template <bool MULTI, int MODE, bool GATHER>
+template <bool MULTI, int MODE, int BINS>
 __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t tile, const int warp, const int lane,
                                            uint32_t *words) {
     // tile -> (job, band, tile column)
@@ -360,10 +367,10 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 const bool dense = !eo && ne >= kDenseEdges;
                 if (dense) flags = 4u;
                 for (int32_t base = dense ? ne : 0; base < ne; base += 32) {
-                    const RowEdge R = row_edge<GATHER>(A.bins, A.edges, e0 + base + lane, base + lane < ne, sub0, off, sc, col0);
+                    const RowEdge R = row_edge<BINS>(A.bins, A.edges, e0 + base + lane, base + lane < ne, sub0, off, sc, col0);
                     auto cross = [&](int r) {
                         if (!((R.rows >> r) & 1u)) return;
-                        const int32_t c = edge_crossing<GATHER>(A.edges, R, r, sub0, col0);
+                        const int32_t c = edge_crossing<BINS>(A.edges, R, r, sub0, col0);
                         if (c <= 0) {
                             const int32_t d = R.down ? -1 : 1;
                             if (r < 2) l01 += r == 0 ? d : d * 65536;
@@ -437,7 +444,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     if (!dense) {  // clear the planes
                         for (int i = lane; i < 4 * kSubWords; i += 32) words[i] = 0u;
                     }
-                    const uint4 v = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, off, sc, col0, words, lane);
+                    const uint4 v = winding_bits<BINS>(A.bins, A.edges, e0, ne, sub0, off, sc, col0, words, lane);
                     in[0] = v.x;
                     in[1] = v.y;
                     in[2] = v.z;
@@ -538,7 +545,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     if (!dense) {  // clear the planes
                         for (int i = lane; i < 4 * kSubWords; i += 32) words[i] = 0u;
                     }
-                    counted = winding_bits<GATHER>(A.bins, A.edges, e0, ne, sub0, off, sc, col0, words, lane);
+                    counted = winding_bits<BINS>(A.bins, A.edges, e0, ne, sub0, off, sc, col0, words, lane);
                 } else if (!eo) {
                     int32_t tot[4] = {0, 0, 0, 0};  // the lane's winding change
 #pragma unroll
@@ -829,11 +836,11 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 // eight for several surfaces (320 surfaces with 7, 8 and 9: 3.14, 3.06 and
 // 3.15 ms: the job's fields take registers), six of the general ones (240
 // gradient fills with 4, 6 and 8: 0.82, 0.75 and 0.77 ms).
-constexpr int raster_ctas(bool multi, int mode, bool gather) {
-    return mode == kGeneral ? 6 : multi || gather ? 8 : 9;
+constexpr int raster_ctas(bool multi, int mode, int bins) {
+    return mode == kGeneral ? 6 : multi || bins != kBinRecords ? 8 : 9;
 }
-template <bool MULTI, bool CTA_ITEMS, int MODE, bool GATHER = false>
-__global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, GATHER)) k_raster(const RasterArgs A) {
+template <bool MULTI, bool CTA_ITEMS, int MODE, int BINS = kBinRecords>
+__global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, BINS)) k_raster(const RasterArgs A) {
     extern __shared__ uint32_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *words = smem + warp * kWarpWords;
@@ -849,7 +856,7 @@ __global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, GATHE
                 if (t >= A.n_items) break;
             }
             const int32_t tile = A.order ? A.order[t] : (int32_t)t;
-            raster_row<MULTI, MODE, GATHER>(A, tile, warp, lane, words);
+            raster_row<MULTI, MODE, BINS>(A, tile, warp, lane, words);
             if (A.one_per_tile) break;
         }
     } else {
@@ -861,7 +868,7 @@ __global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, GATHE
             const long long t = (long long)(item / kTileRows);
             const int32_t tile = A.order ? A.order[t] : (int32_t)t;
             __syncwarp();  // the previous item's reads of `words` are done before it is reset
-            raster_row<MULTI, MODE, GATHER>(A, tile, (int)(item % kTileRows), lane, words);
+            raster_row<MULTI, MODE, BINS>(A, tile, (int)(item % kTileRows), lane, words);
         }
     }
 }
@@ -870,14 +877,17 @@ static size_t raster_smem() { return sizeof(uint32_t) * kWarpWords * kTileRows; 
 
 template <int MODE, class F>
 static int of_mode(RasterVariant v, int k, F &&f) {
-    if (v.gather)  // (gathered edges come a tile per CTA)
-        return v.multi ? f(k_raster<true, true, MODE, true>, k) : f(k_raster<false, true, MODE, true>, k);
+    if (v.bins == kBinSmall)
+        return v.multi ? f(k_raster<true, true, MODE, kBinSmall>, k) : f(k_raster<false, true, MODE, kBinSmall>, k);
     if (v.multi) return v.cta_items ? f(k_raster<true, true, MODE>, k) : f(k_raster<true, false, MODE>, k);
     return v.cta_items ? f(k_raster<false, true, MODE>, k) : f(k_raster<false, false, MODE>, k);
 }
 template <class F>
 static int with_variant(RasterVariant v, F &&f) {
-    const int k = v.mode * 8 + ((v.gather ? 4 : 0) | (v.multi ? 2 : 0) | (v.cta_items ? 1 : 0));
+    const int k = (v.mode * 3 + v.bins) * 4 + ((v.multi ? 2 : 0) | (v.cta_items ? 1 : 0));
+    if (v.bins == kBinIndex)
+        return v.multi ? f(k_raster<true, false, kGeneral, kBinIndex>, k)
+                       : f(k_raster<false, false, kGeneral, kBinIndex>, k);
     switch (v.mode) {
         case kPlain4x: return of_mode<kPlain4x>(v, k, f);
         case kPlainDirect: return of_mode<kPlainDirect>(v, k, f);
@@ -887,7 +897,7 @@ static int with_variant(RasterVariant v, F &&f) {
 
 // A variant's resident CTAs per SM, asked once per variant.
 int raster_occupancy(Ctx &, RasterVariant v, int &ctas_per_sm) {
-    static std::atomic<int> cache[24];
+    static std::atomic<int> cache[36];
     return with_variant(v, [&](auto kernel, int k) -> int {
         int occ = cache[k].load(std::memory_order_relaxed);
         if (occ <= 0) {

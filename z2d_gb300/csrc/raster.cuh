@@ -82,8 +82,8 @@ struct RasterArgs {
     const DevJob *jobs;
     const FillCmd *fills;
     const FillState *st;
-    const void *edges;          // DEdge, or (gather) SmallEdge
-    const void *bins;           // BinEdge records, or (gather) int32 indices of `edges`
+    const void *edges;          // DEdge, or (kBinSmall) SmallEdge
+    const void *bins;           // BinEdge records, or int32 indices of `edges` (BinKind)
     const int32_t *bin_off;
     const int32_t *band_count;  // per global band
     const int4 *band_fills;     // {fill, cull_x0, cull_x1, (fill, band) slot} per band, in call order
@@ -126,13 +126,18 @@ Z2D_HD uint32_t coverage_word(const FillCmd &F, int fmt, int k) {
     return fmt <= Z2D_FORMAT_RGBA ? i16_to_word(s, word_order(fmt)) : s.a;
 }
 
+// What the bins of (fill, band) hold: the edges' records, or indices of edges
+// whose records every pixel row works out, either of the one-upload path's
+// SmallEdge (with records from the host a call of 1,500 edges took 67 us
+// instead of 56) or of DEdge, where the device has no room for the records.
+enum BinKind : int { kBinRecords = 0, kBinSmall = 1, kBinIndex = 2 };
+
 // How k_raster runs: `multi` for several surfaces, `cta_items` for a whole
-// tile per work item, the mode, and `gather` for bins of edge indices and
-// edges without their f32 fields, as the one-upload path's host writes them
-// (with records and fields from the host a call of 1,500 edges took 67 us
-// instead of 56).
+// tile per work item, the mode, and what the bins hold.  kBinSmall comes with
+// a tile per item, kBinIndex with a row per item and in the general mode only.
 struct RasterVariant {
-    bool multi, cta_items, gather;
+    bool multi, cta_items;
+    BinKind bins;
     int mode;
 };
 int raster_occupancy(Ctx &c, RasterVariant v, int &ctas_per_sm);
