@@ -7,11 +7,12 @@ import gc
 import numpy as np
 import pytest
 
+from backends import StrokeOracle
 from z2d_gb300 import abi, painter
 from z2d_gb300.native import Context
 from z2d_gb300.path import Path
 from z2d_gb300.surface import Surface
-from z2d_gb300.types import FillOptions, Pattern, Pixel
+from z2d_gb300.types import FillOptions, Pattern, Pixel, StrokeOptions
 
 pytestmark = pytest.mark.gpu
 GB = 1 << 30
@@ -67,3 +68,54 @@ def test_bins_of_indices(oracle, fmt, op, many):
         one = Surface.init(fmt, 40, 8)
         assert oracle.fill(one, *fills[0]) == abi.OK
         assert np.array_equal(small.to_host().numpy(), one.numpy())
+
+
+def _scratch_of(call):
+    """What a call leaves allocated on the device."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.synchronize()
+    ctx = Context(0)
+    before = torch.cuda.mem_get_info()[0]
+    call(ctx)
+    ctx.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    return used
+
+
+def _wave():
+    return Path().move_to(4, 30).curve_to(10, -20, 30, 70, 36, 8).line_to(20, 20).line_to(5, 5).to_array()
+
+
+def _stroke_beside(oracle, big, less):
+    """A stroke `big` off the surface and a small one on it, with `less` bytes
+    fewer than the first call of its kind took."""
+    pytest.importorskip("torch")
+    pat = Pattern.from_pixel(Pixel.rgba(10, 200, 70, 255))
+    opts = [StrokeOptions(line_width=2), StrokeOptions(line_width=5, line_join="round", line_cap="round")]
+    ref = Surface.init("rgba", 40, 40)
+    assert StrokeOracle(oracle).stroke(ref, pat, _wave(), opts[1]) == abi.OK
+    dev = [Surface.init("rgba", 40, 40).to_device("cuda") for _ in range(2)]
+
+    def draw(k):
+        return lambda ctx: painter.draw_jobs([(dev[k], [("stroke", pat, big, opts[0]), ("stroke", pat, _wave(), opts[1])])],
+                                             ctx=ctx)
+    used = _scratch_of(draw(0))
+    ctx = Context(0)
+    with only_free(used - less):
+        draw(1)(ctx)
+        ctx.synchronize()
+        ctx.close()
+    for d in dev:
+        assert np.array_equal(d.to_host().numpy(), ref.numpy())
+
+
+def test_stroke_without_kept_joins(oracle):
+    """Strokes of some 20 M points: their joins are 80 bytes each."""
+    one = Path().move_to(0, -2e5).curve_to(1e6, -4e6, 2e6, -1e5, 3e6, -4e6)
+    points = sum(len(c) for c in painter.stroke_contours(one.to_array(), StrokeOptions(line_width=2))[0]) // 5
+    p = Path()
+    n = (20 << 20) // points + 1
+    for k in range(n):
+        p.move_to(0, -2e5).curve_to(1e6, -4e6, 2e6, -1e5, 3e6, -4e6)
+    _stroke_beside(oracle, p.to_array(), 40 * points * n)

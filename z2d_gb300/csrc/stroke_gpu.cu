@@ -80,7 +80,7 @@ struct State {
     double2 *q_pt;
     int32_t *q_sub;
     uint8_t *q_mode;
-    Elem *elem;                     // R
+    Elem *elem;                     // R, or null: not kept
     Count2 *cnt, *off;              // R + 1
     // contour points, and each one's subpath
     double2 *pa, *pb;
@@ -458,7 +458,7 @@ __global__ void ks_elem_count(const SubpathDev *__restrict__ subs, const StrokeD
     const StrokeDev T = strokes[subs[sp].stroke];
     Out<false> o;
     const Elem e = element(o, T, pen + T.pen_off, st, q_pt, q_mode, (int32_t)(q - st.q0));
-    elem[q] = e;
+    if (elem) elem[q] = e;
     cnt[q] = (e.flags & EL_JOIN) ? join_count(e) : Count2{o.na, o.nb};
 }
 
@@ -506,7 +506,9 @@ __global__ void ks_stroke_tot(const StrokeDev *__restrict__ strokes, int32_t n_s
 
 // Writes every element's points to their contour positions: outer points in
 // element order, inner points in reverse (B points are prepended); a closed
-// subpath's closing joins come last: elements 1..n-1, then 0.
+// subpath's closing joins come last: elements 1..n-1, then 0.  KEPT: the joins
+// are in `elem`; without (scarce), they are found a second time.
+template <bool KEPT>
 __global__ void ks_elem_emit(const SubpathDev *__restrict__ subs, const StrokeDev *__restrict__ strokes,
                              const PenVertex *__restrict__ pen, const SubState *__restrict__ sub,
                              const Region *__restrict__ region, const double2 *__restrict__ q_pt,
@@ -533,17 +535,17 @@ __global__ void ks_elem_emit(const SubpathDev *__restrict__ subs, const StrokeDe
     const long long end_b = (long long)R.rb + R.sb - t_b;
     for (long long i = 0; i < na; i++) a_sub[pos_a + i] = sp;
     for (long long i = 0; i < nb; i++) b_sub[end_b - 1 - i] = sp;
-    const Elem e = elem[q];
+    Elem e;
+    if constexpr (KEPT) e = elem[q];
     Out<true> o;
     o.pa = pa + pos_a;
     o.pb_end = pb + end_b;
     o.scale = T.scale;
-    if (!(e.flags & EL_JOIN)) {  // caps and dots
-        if (na + nb > 0) {
-            const StrokeDev S = T;
-            element(o, S, pen + S.pen_off, st, q_pt, q_mode, k);
-        }
-        return;
+    if (!KEPT || !(e.flags & EL_JOIN)) {  // caps and dots
+        if (na + nb == 0) return;
+        const StrokeDev S = T;
+        e = element(o, S, pen + S.pen_off, st, q_pt, q_mode, k);
+        if (!(e.flags & EL_JOIN)) return;
     }
     const bool sw = (e.flags & EL_SWITCHED) != 0;
     auto outer = [&](Pt p) {
@@ -654,6 +656,15 @@ struct Carve {
     }
 };
 
+// Whether scratch that a call can do without would leave the device too little
+// for the rest of it: the rest of a stroke takes three to six times as much.
+bool scarce(size_t bytes) {
+    if (bytes < ((size_t)1 << 30)) return false;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+    return bytes > free_bytes / 8;
+}
+
 }  // namespace
 
 int poly_emit(Ctx &c, const PolyRun &run, const FillCmd *d_fills, FillState *d_st, DEdge *d_edges) {
@@ -724,8 +735,13 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     const size_t o_rpt = cb.take<double2>(R + 1), o_rsub = cb.take<int32_t>(R + 1), o_rmode = cb.take<uint8_t>(R + 1);
     const size_t o_keep = cb.take<int32_t>(R + 1), o_kept = cb.take<int32_t>(R + 1);
     const size_t o_qpt = cb.take<double2>(R + 1), o_qsub = cb.take<int32_t>(R + 1), o_qmode = cb.take<uint8_t>(R + 1);
-    const size_t o_el = cb.take<Elem>(R + 1), o_c = cb.take<Count2>(R + 1), o_o = cb.take<Count2>(R + 1);
-    if (c.stroke_b.ensure(cb.off)) return Z2D_ERR_OUT_OF_MEMORY;
+    const size_t o_c = cb.take<Count2>(R + 1), o_o = cb.take<Count2>(R + 1);
+    // the joins are kept where the device has room for them (a stroke of 500
+    // leaves 449 us without, with them and an edge per contour point 335)
+    const size_t without = cb.off, o_el = cb.take<Elem>(R + 1);
+    bool kept = c.stroke_b.cap >= cb.off || !scarce(cb.off - without);
+    if (kept && c.stroke_b.ensure(cb.off)) kept = false;
+    if (!kept && c.stroke_b.ensure(without)) return Z2D_ERR_OUT_OF_MEMORY;
     uint8_t *B = c.stroke_b.as<uint8_t>();
     st.raw_pt = reinterpret_cast<double2 *>(B + o_rpt);
     st.raw_sub = reinterpret_cast<int32_t *>(B + o_rsub);
@@ -735,7 +751,7 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     st.q_pt = reinterpret_cast<double2 *>(B + o_qpt);
     st.q_sub = reinterpret_cast<int32_t *>(B + o_qsub);
     st.q_mode = B + o_qmode;
-    st.elem = reinterpret_cast<Elem *>(B + o_el);
+    st.elem = kept ? reinterpret_cast<Elem *>(B + o_el) : nullptr;
     st.cnt = reinterpret_cast<Count2 *>(B + o_c);
     st.off = reinterpret_cast<Count2 *>(B + o_o);
 
@@ -779,9 +795,10 @@ int stroke_emit(Ctx &c, StrokeRun &run, const FillCmd *d_fills, FillState *d_st,
     constexpr int T = 128;
     const long long R = run.raw;
     cudaEvent_t ts = c.timer_begin(c.t_stroke);
-    ks_elem_emit<<<blocks_for(R, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.region, st.q_pt, st.q_sub,
-                                                        st.q_mode, st.kept_off, R, st.elem, st.off, st.pa, st.pb,
-                                                        st.a_sub, st.b_sub);
+    const auto elem_emit = st.elem ? ks_elem_emit<true> : ks_elem_emit<false>;
+    elem_emit<<<blocks_for(R, T), T, 0, c.stream>>>(run.subs, run.strokes, st.pen, st.sub, st.region, st.q_pt, st.q_sub,
+                                                     st.q_mode, st.kept_off, R, st.elem, st.off, st.pa, st.pb, st.a_sub,
+                                                     st.b_sub);
     if (run.n_a + run.n_b > 0)
         ks_edges<<<blocks_for(run.n_a + run.n_b, T), T, 0, c.stream>>>(st.region, st.pa, st.pb, st.a_sub, st.b_sub,
                                                                         run.n_a, run.n_b, d_fills, d_st, d_edges);
