@@ -12,7 +12,7 @@ from z2d_gb300 import abi, painter
 from z2d_gb300.native import Context
 from z2d_gb300.path import Path
 from z2d_gb300.surface import Surface
-from z2d_gb300.types import FillOptions, Pattern, Pixel, StrokeOptions
+from z2d_gb300.types import NODE_DTYPE, FillOptions, Pattern, Pixel, StrokeOptions
 
 pytestmark = pytest.mark.gpu
 GB = 1 << 30
@@ -119,3 +119,14 @@ def test_stroke_without_kept_joins(oracle):
     for k in range(n):
         p.move_to(0, -2e5).curve_to(1e6, -4e6, 2e6, -1e5, 3e6, -4e6)
     _stroke_beside(oracle, p.to_array(), 40 * points * n)
+
+
+def test_stroke_with_a_lane_a_node(oracle):
+    """9 M stroked nodes: their counts are 128 bytes each with 8 lanes a node,
+    16 with one."""
+    n = 9_000_000
+    k = np.arange(n)
+    big = np.zeros(n, NODE_DTYPE)
+    big["tag"] = np.where(k == 0, abi.MOVE_TO, abi.LINE_TO)
+    big["p"][:, 0], big["p"][:, 1] = 10.0 * (k % 2), -100.0 - k % 1000
+    _stroke_beside(oracle, big, 64 * n)

@@ -690,14 +690,23 @@ int stroke_count(Ctx &c, StrokeRun &run, int32_t *d_status) {
     run.state = &st;
     constexpr int T = 128;
     // ---- buffers known before counting
+    // A warp per node while the device has room for all of them, else 8 lanes;
+    // one where the lanes' counts are scarce memory.
     Carve ca;
-    // a warp per node while the device has room for all of them, else 8 lanes
-    st.g = run.n_local * 32 <= (long long)c.sm_count * 2048 ? 5 : 3;
-    const long long n_lanes = lane_slot(run.n_local, st.g);
-    const size_t o_cnt = ca.take<long long>(n_lanes + 1), o_off = ca.take<long long>(n_lanes + 1);
-    const size_t o_lsub = ca.take<int32_t>(run.n_local + 1), o_pen = ca.take<PenVertex>(run.n_pen + 1);
-    const size_t o_sub = ca.take<SubState>(run.n_subs + 1), o_reg = ca.take<Region>(run.n_subs + 1);
-    const size_t o_edges = ca.take<int32_t>(run.n_strokes + 1), o_totals = ca.take<long long>(2);
+    long long n_lanes = 0;
+    size_t o_cnt, o_off, o_lsub, o_pen, o_sub, o_reg, o_edges, o_totals;
+    auto carve = [&](int g) {
+        ca = Carve{};
+        st.g = g;
+        n_lanes = lane_slot(run.n_local, g);
+        o_cnt = ca.take<long long>(n_lanes + 1), o_off = ca.take<long long>(n_lanes + 1);
+        o_lsub = ca.take<int32_t>(run.n_local + 1), o_pen = ca.take<PenVertex>(run.n_pen + 1);
+        o_sub = ca.take<SubState>(run.n_subs + 1), o_reg = ca.take<Region>(run.n_subs + 1);
+        o_edges = ca.take<int32_t>(run.n_strokes + 1), o_totals = ca.take<long long>(2);
+    };
+    carve(run.n_local * 32 <= (long long)c.sm_count * 2048 ? 5 : 3);
+    if (c.stroke_a.cap < ca.off && (scarce(2 * sizeof(long long) * (size_t)n_lanes) || c.stroke_a.ensure(ca.off)))
+        carve(0);
     if (c.stroke_a.ensure(ca.off)) return Z2D_ERR_OUT_OF_MEMORY;
     uint8_t *A = c.stroke_a.as<uint8_t>();
     st.raw_cnt = reinterpret_cast<long long *>(A + o_cnt);
