@@ -70,6 +70,37 @@ def test_bins_of_indices(oracle, fmt, op, many):
         assert np.array_equal(small.to_host().numpy(), one.numpy())
 
 
+def test_tiles_not_sorted():
+    """16 surfaces of one column and 2^21 bands each: 2.1 GB of records fit, the
+    0.8 GB that sorting the tiles takes do not beside them."""
+    torch = pytest.importorskip("torch")
+    h = (1 << 23) - 1
+    nodes = Path().move_to(0, 0).line_to(1, 0).line_to(1, h).line_to(0, h).close().to_array()
+    pat = Pattern.from_pixel(Pixel.rgba(0, 0, 0, 200))
+    dev = [Surface.init("alpha8", 1, h).to_device("cuda") for _ in range(16)]
+    torch.cuda.synchronize()
+
+    def draw(ctx):
+        painter.fill_jobs([(d, [(pat, nodes, FillOptions())]) for d in dev], ctx=ctx)
+    ctx = Context(0)
+    ctx.set_raster(0, 0, 0)
+    before = torch.cuda.mem_get_info()[0]
+    draw(ctx)
+    ctx.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    ctx = Context(0)
+    ctx.set_raster(0, 1, 0)
+    with only_free(used + GB // 4):
+        draw(ctx)
+        ctx.synchronize()
+        ctx.close()
+    twice = 200 + 200 - 200 * 200 // 255
+    for k, d in enumerate(dev):
+        other = int((d.data != twice).sum())
+        assert other == 0, f"surface {k}"
+
+
 def _scratch_of(call):
     """What a call leaves allocated on the device."""
     torch = pytest.importorskip("torch")

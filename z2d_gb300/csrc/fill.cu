@@ -1551,23 +1551,25 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     A.n_items = (unsigned long long)n_tiles * (plan.cta_items ? 1 : kTileRows);
     A.order = nullptr;
     if (plan.order == 1 && n_tiles > 1) {
-        // longest bands first: tiles sorted by their band's fill count
+        // longest bands first: tiles sorted by their band's fill count (in tile
+        // order where there is no room to sort them)
         const size_t nt = (size_t)n_tiles;
         size_t sort_bytes = 0;
         cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, (const int32_t *)nullptr, (int32_t *)nullptr,
                                                   (const int32_t *)nullptr, (int32_t *)nullptr, (int)nt, 0, 32,
                                                   c.stream);
         const size_t arr = (sizeof(int32_t) * nt + 255) & ~(size_t)255;
-        if (c.tile_order.ensure(4 * arr + sort_bytes)) return Z2D_ERR_OUT_OF_MEMORY;
-        uint8_t *b = c.tile_order.as<uint8_t>();
-        int32_t *cost = reinterpret_cast<int32_t *>(b), *idx = reinterpret_cast<int32_t *>(b + arr);
-        int32_t *cost_s = reinterpret_cast<int32_t *>(b + 2 * arr), *order = reinterpret_cast<int32_t *>(b + 3 * arr);
-        k_tile_cost<<<grid_for((long long)nt, 256), 256, 0, c.stream>>>(d_jobs, n_jobs, d_band_count, (int32_t)nt, cost,
-                                                                         idx);
-        Z2D_CUDA(cub::DeviceRadixSort::SortPairsDescending(b + 4 * arr, sort_bytes, cost, cost_s, idx, order, (int)nt,
-                                                           0, 32, c.stream));
-        c.launches += 2;
-        A.order = order;
+        if (c.tile_order.ensure(4 * arr + sort_bytes) == 0) {
+            uint8_t *b = c.tile_order.as<uint8_t>();
+            int32_t *cost = reinterpret_cast<int32_t *>(b), *idx = reinterpret_cast<int32_t *>(b + arr);
+            int32_t *cost_s = reinterpret_cast<int32_t *>(b + 2 * arr), *order = reinterpret_cast<int32_t *>(b + 3 * arr);
+            k_tile_cost<<<grid_for((long long)nt, 256), 256, 0, c.stream>>>(d_jobs, n_jobs, d_band_count, (int32_t)nt,
+                                                                             cost, idx);
+            Z2D_CUDA(cub::DeviceRadixSort::SortPairsDescending(b + 4 * arr, sort_bytes, cost, cost_s, idx, order,
+                                                               (int)nt, 0, 32, c.stream));
+            c.launches += 2;
+            A.order = order;
+        }
     }
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
     variant.cta_items = plan.cta_items != 0;
