@@ -871,11 +871,12 @@ __device__ __forceinline__ int32_t job_of(const DevJob *__restrict__ jobs, int32
     return lo;
 }
 
-// The same with a warp per band, for jobs of few fills: a CTA per band
+constexpr int32_t kWarpFills = 512;
+// With a warp per band, for the jobs of at most max_fills fills: a CTA per band
 // spends its time starting and meeting at barriers (16,384 bands of one fill:
 // 43 us, a warp each 11).
 __global__ void __launch_bounds__(256) k_band_lists_w(const FillState *__restrict__ st, const DevJob *__restrict__ jobs,
-                                                      int32_t n_jobs, int32_t n_gbands,
+                                                      int32_t n_jobs, int32_t n_gbands, int32_t max_fills,
                                                       int32_t *__restrict__ band_count, int4 *__restrict__ band_fills,
                                                       TileRec *__restrict__ tiles) {
     const long long at = warp_number(blockIdx.x, blockDim.x, threadIdx.x);
@@ -884,6 +885,7 @@ __global__ void __launch_bounds__(256) k_band_lists_w(const FillState *__restric
     const int32_t j = job_of(jobs, n_jobs, gb, [](const DevJob &J) { return (long long)J.gband_base; });
     const DevJob &J = jobs[j];
     const int32_t lb = gb - J.gband_base, b = J.band_lo + lb, nf = J.fill1 - J.fill0;
+    if (nf > max_fills) return;
     if (tiles) {
         const int32_t nc = J.tcol_hi - J.tcol_lo + 1;
         for (int32_t t = lane; t < nc; t += 32) tiles[J.tile_base + (long long)lb * nc + t] = TileRec{j, lb, t, 0};
@@ -908,19 +910,22 @@ __global__ void __launch_bounds__(256) k_band_lists_w(const FillState *__restric
     if (lane == 0) band_count[gb] = n;
 }
 
-// One CTA per global band: the job's fills touching the band, in call order
+// One CTA per global band from gb0 on, of the jobs of more than max_fills
+// fills: the job's fills touching the band, in call order
 // (ordered compaction), with the tile-column range each one can affect and
 // the fill's (fill, band) slot of the band, and (several surfaces) the
 // records of the band's tiles.
 __global__ void __launch_bounds__(256) k_band_lists(const FillState *__restrict__ st, const DevJob *__restrict__ jobs,
-                                                    int32_t n_jobs, int32_t *__restrict__ band_count,
+                                                    int32_t n_jobs, int32_t gb0, int32_t max_fills,
+                                                    int32_t *__restrict__ band_count,
                                                     int4 *__restrict__ band_fills, TileRec *__restrict__ tiles) {
-    const int32_t gb = blockIdx.x;
+    const int32_t gb = gb0 + (int32_t)blockIdx.x;
     const int32_t j = job_of(jobs, n_jobs, gb, [](const DevJob &J) { return (long long)J.gband_base; });
     const DevJob J = jobs[j];
     const int32_t lb = gb - J.gband_base;
     const int32_t b = J.band_lo + lb;
     const int32_t nf = J.fill1 - J.fill0;
+    if (nf <= max_fills) return;
     if (tiles) {
         const int32_t nc = J.tcol_hi - J.tcol_lo + 1;
         for (int32_t t = threadIdx.x; t < nc; t += blockDim.x)
@@ -1475,13 +1480,28 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     int32_t *d_band_count = c.band_fills.as<int32_t>();
     TileRec *d_tiles = n_jobs > 1 ? reinterpret_cast<TileRec *>(c.band_fills.as<uint8_t>() + count_bytes) : nullptr;
     int4 *d_band_fills = reinterpret_cast<int4 *>(c.band_fills.as<uint8_t>() + count_bytes + tile_bytes);
-    if (n_slots <= 256 * n_gbands)  // few fills a job on average
+    // A warp per band where the jobs have few fills on average, and then a CTA
+    // for the bands of the jobs of more than kWarpFills: 2,000 surfaces of one
+    // fill beside one of n, all bins and lists: n = 256 by warps 50.5 us, by
+    // CTAs 54.7; 512 58.1 and 54.4; 1,024 68.9 and 57.8; 4,096 142 and 75.
+    const int32_t max_fills = n_slots <= 256 * n_gbands ? kWarpFills : 0;
+    if (max_fills > 0) {
         k_band_lists_w<<<grid_for(32 * n_gbands, 256), 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, (int32_t)n_gbands,
-                                                                            d_band_count, d_band_fills, d_tiles);
-    else
-        k_band_lists<<<(unsigned)n_gbands, 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, d_band_count, d_band_fills,
-                                                               d_tiles);
-    c.launches++;
+                                                                            max_fills, d_band_count, d_band_fills,
+                                                                            d_tiles);
+        c.launches++;
+    }
+    long long gb0 = n_gbands, gb1 = 0;  // from the first of the other jobs' bands to the last
+    for (const DevJob &J : jobs)
+        if (J.fill1 - J.fill0 > max_fills && J.band_hi >= J.band_lo) {
+            gb0 = std::min<long long>(gb0, J.gband_base);
+            gb1 = (long long)J.gband_base + (J.band_hi - J.band_lo + 1);
+        }
+    if (gb0 < gb1) {
+        k_band_lists<<<(unsigned)(gb1 - gb0), 256, 0, c.stream>>>(d_st, d_jobs, n_jobs, (int32_t)gb0, max_fills,
+                                                                 d_band_count, d_band_fills, d_tiles);
+        c.launches++;
+    }
 
     // ---- exact path
     if (n_exact > 0) {
