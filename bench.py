@@ -1115,7 +1115,7 @@ def run_ours(args):
                   "calls": PLAIN_FILLS, "note": f"z2dgpu_fill per path, first {PLAIN_FILLS} fills",
                   "latency_us": {"p50": call_us[len(call_us) // 2], "p99": call_us[int(len(call_us) * 0.99) - 1],
                                  "note": "host wall time per painter.fill call, Python marshalling included (a "
-                                         "short path returns once its one upload and raster launch are queued; "
+                                         "short path returns once its raster launch, with its tables, is queued; "
                                          "a longer one after the pipeline's size readbacks)"}},
         "star_300": star,
         "jobs": jobs,

@@ -266,8 +266,7 @@ Z2D_API int z2dgpu_ctx_create(z2dgpu_ctx **out, int device, void *stream);
 Z2D_API int z2dgpu_ctx_destroy(z2dgpu_ctx *ctx);
 /* Blocks until all work queued on the context's stream has finished. */
 Z2D_API int z2dgpu_ctx_synchronize(z2dgpu_ctx *ctx);
-/* Number of kernels this context has launched since creation (the kernel that
- * carries a small call's tables in place of a copy is not counted). */
+/* Number of kernels this context has launched since creation. */
 Z2D_API uint64_t z2dgpu_ctx_launch_count(const z2dgpu_ctx *ctx);
 
 /* Kernel timing: when enabled, the context brackets its dominant kernels

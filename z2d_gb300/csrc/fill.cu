@@ -1135,7 +1135,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     const int32_t n_fills = (int32_t)fills.size();
     const int32_t n_jobs = (int32_t)jobs.size();
     if (n_fills == 0 || n_nodes == 0 || n_jobs == 0) return Z2D_OK;
-    if (!strokes) {  // few short fills: one upload, one launch
+    if (!strokes) {  // few short fills: one launch
         bool done = false;
         const int rc = run_small_jobs(c, jobs, nodes, fills, grads, grad_of_fill, done);
         if (rc || done) return rc;
@@ -1608,8 +1608,9 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
 // ------------------------------------------------------- small fills
 // One fill of a short path: everything up to the rasteriser runs on the
 // host (a few microseconds for a few hundred edges) and reaches the device
-// in one upload, so the call costs one copy and one launch instead of the
-// pipeline's launches and size readbacks.  The host steps restate the same
+// with the rasteriser's one launch (tables of up to 8 KB, its parameters) or
+// in one copy in front of it, instead of the pipeline's launches and size
+// readbacks.  The host steps restate the same
 // z2d code as the device kernels, with the same f64 operations in the same
 // order (the host is compiled without FP contraction), so the edges, the
 // fill's box and the tiles are the device pipeline's; bins list a band's
@@ -1825,23 +1826,6 @@ size_t estimate_edges(const z2d_node *nodes, int32_t n, double tol) {
 
 }  // namespace
 
-// A small call's tables as a kernel's parameters: the launch carries them, so
-// no copy engine, event or staging slot is between the call and its raster
-// kernel.  Such calls are bound by their CUDA calls and by the wait of the
-// raster kernel for its tables (the 300x300 star from Python: copied 16.4 us,
-// now 14.3).  Larger tables stay with the copy: a launch's parameters are
-// written by the host a second time, and end at 32 KB.
-constexpr size_t kParamBytes = 8192;
-struct ParamBlob {
-    uint4 v[kParamBytes / sizeof(uint4)];
-};
-constexpr int kPutThreads = 64;
-__global__ void __launch_bounds__(kPutThreads) k_put_params(const __grid_constant__ ParamBlob P, uint4 *__restrict__ out,
-                                                            int32_t n) {
-    const int32_t i = (int32_t)(blockIdx.x * kPutThreads + threadIdx.x);
-    if (i < n) out[i] = P.v[i];
-}
-
 int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, const std::vector<FillCmd> &fills,
                    const std::vector<DevGradient> &grads, const std::vector<int32_t> &grad_of_fill, bool &done) {
     done = false;
@@ -2019,7 +2003,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
             bcount[(size_t)(jb.gband_base + lb)] = k;
         }
     }
-    // ---- one upload
+    // ---- the tables, laid out as the device reads them
     auto al = [](size_t v) { return (v + 15) & ~(size_t)15; };
     const size_t o_jobs = 0, o_fill = al(sizeof(DevJob) * n_jobs);
     const size_t o_st = o_fill + al(sizeof(FillCmd) * n_fills), o_rf = o_st + al(sizeof(FillState) * n_fills);
@@ -2032,14 +2016,17 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     const size_t o_tile = o_grad + al(sizeof(DevGradient) * grads.size());
     const size_t o_lut = o_tile + al(sizeof(TileRec) * tiles.size());
     const size_t total = o_lut + al(32 * sizeof(uint32_t) * n_fills);
-    if (c.small_params.ensure(total)) return Z2D_ERR_OUT_OF_MEMORY;
-    uint8_t *dv = c.small_params.as<uint8_t>(), *h;
+    // (as the launch's parameters, or by a copy: k_raster_small)
     const bool by_param = total <= kParamBytes;
     ParamBlob blob;
+    uint8_t *h;
+    uintptr_t dv = 0;  // the device's tables (parameters: offsets)
     int slot = 0;
     if (by_param) {
         h = reinterpret_cast<uint8_t *>(blob.v);
     } else {
+        if (c.small_params.ensure(total)) return Z2D_ERR_OUT_OF_MEMORY;
+        dv = reinterpret_cast<uintptr_t>(c.small_params.ptr);
         slot = c.small_slot;
         c.small_slot ^= 1;
         HostBuf &hb = c.small_stage[slot];
@@ -2053,7 +2040,7 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     memcpy(hf, fills.data(), sizeof(FillCmd) * n_fills);
     const DevGradient *dgrads = reinterpret_cast<const DevGradient *>(dv + o_grad);
     for (size_t f = 0; f < n_fills; f++)
-        if (grad_of_fill[f] >= 0) hf[f].src.grad = dgrads + grad_of_fill[f];
+        hf[f].src.grad = grad_of_fill[f] >= 0 ? dgrads + grad_of_fill[f] : nullptr;
     memcpy(h + o_st, st.data(), sizeof(FillState) * n_fills);
     memcpy(h + o_rf, rf.data(), sizeof(RasterFill) * n_fills);
     if (!edges.empty()) memcpy(h + o_edges, edges.data(), sizeof(SmallEdge) * edges.size());
@@ -2068,13 +2055,8 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         if (fills[f].fast_kind != FAST_PIXEL_SRC_OVER) continue;  // (not read)
         for (int k = 0; k <= 16; k++) lut[32 * f + k] = coverage_word(fills[f], J[(size_t)fills[f].job].sfc.fmt, k);
     }
-    if (by_param) {
-        const int32_t n = (int32_t)(total / sizeof(uint4));
-        k_put_params<<<(unsigned)((n + kPutThreads - 1) / kPutThreads), kPutThreads, 0, c.stream>>>(
-            blob, reinterpret_cast<uint4 *>(dv), n);  // (stands for the upload: not counted as a launch)
-        Z2D_CUDA(cudaGetLastError());
-    } else {
-        Z2D_CUDA(cudaMemcpyAsync(dv, h, total, cudaMemcpyHostToDevice, c.stream));
+    if (!by_param) {
+        Z2D_CUDA(cudaMemcpyAsync(c.small_params.ptr, h, total, cudaMemcpyHostToDevice, c.stream));
         Z2D_CUDA(cudaEventRecord(c.small_done[slot], c.stream));
     }
     if (n_tiles == 0) return Z2D_OK;
@@ -2084,8 +2066,8 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     A.jobs = reinterpret_cast<const DevJob *>(dv + o_jobs);
     A.fills = reinterpret_cast<const FillCmd *>(dv + o_fill);
     A.st = reinterpret_cast<const FillState *>(dv + o_st);
-    A.edges = dv + o_edges;
-    A.bins = dv + o_bins;
+    A.edges = reinterpret_cast<const SmallEdge *>(dv + o_edges);
+    A.bins = reinterpret_cast<const int32_t *>(dv + o_bins);
     A.bin_off = reinterpret_cast<const int32_t *>(dv + o_off);
     A.band_count = reinterpret_cast<const int32_t *>(dv + o_cnt);
     A.band_fills = reinterpret_cast<const int4 *>(dv + o_list);
@@ -2102,9 +2084,11 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
         const int rs = c.await_surface();
         if (rs) return rs;
     }
-    const RasterVariant variant{n_jobs > 1, true, kBinSmall, raster_mode(fills.data(), n_fills, false)};
+    const int mode = raster_mode(fills.data(), n_fills, false);
     cudaEvent_t t0 = c.timer_begin(c.t_raster);
-    const int rc = raster_launch(c, variant, A, (unsigned)n_tiles);
+    const int rc = by_param ? raster_launch_small(c, n_jobs > 1, mode, A, blob, (int32_t)(total / sizeof(uint4)),
+                                                  (int32_t)n_fills, (unsigned)n_tiles)
+                            : raster_launch(c, RasterVariant{n_jobs > 1, true, kBinSmall, mode}, A, (unsigned)n_tiles);
     if (rc) return rc;
     c.timer_end(c.t_raster, t0);
     return Z2D_OK;

@@ -244,8 +244,8 @@ struct DevJob {
 // Nodes that no fill owns are skipped; device-stroked
 // commands (`strokes`, fills with stroke >= 0) read their nodes from the
 // same array; fills with poly >= 0 draw a host-built polygon of `strokes`.
-// A call with few short fills, on one surface or many, in a single upload
-// and a single launch: the host flattens the paths (fill_plotter.plot,
+// A call with few short fills, on one surface or many, in a single launch,
+// with its tables as parameters or in one copy before it: the host flattens the paths (fill_plotter.plot,
 // Spline.decompose, Polygon.addEdge), sets the fills up (inBox,
 // multisample.run's draw box), bins their edges and lays out the band
 // lists; the rasteriser draws the tiles.  Sets `done` = false without

@@ -77,6 +77,14 @@ struct RowEdge {
 // the band's.  What does not depend on the pixel row is in the record: a
 // record is read by every row and tile column of its band (2,000 paths: with
 // rows, t and limit worked out here 2.07 ms, with the record 1.97).
+// (Tables in global memory are read through the read-only path.)
+template <int BINS, class T>
+__device__ __forceinline__ T table(const T *p) {
+    if constexpr (BINS == kBinShared) return *p;
+    else return __ldg(p);
+}
+template <int BINS>
+constexpr bool kSmallEdges = BINS == kBinSmall || BINS == kBinShared;
 template <int BINS>
 __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const void *__restrict__ edges,
                                             int32_t bin, bool valid, int32_t sub0, int32_t off, int32_t sc,
@@ -84,10 +92,10 @@ __device__ __forceinline__ RowEdge row_edge(const void *__restrict__ bins, const
     RowEdge R{};
     if (!valid) return R;
     BinEdge B;
-    if constexpr (BINS == kBinSmall) {
-        const int32_t id = __ldg(reinterpret_cast<const int32_t *>(bins) + bin);
-        const int4 a = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id);
-        const int4 b = __ldg(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id + 1);
+    if constexpr (kSmallEdges<BINS>) {
+        const int32_t id = table<BINS>(reinterpret_cast<const int32_t *>(bins) + bin);
+        const int4 a = table<BINS>(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id);
+        const int4 b = table<BINS>(reinterpret_cast<const int4 *>(edges) + 2 * (size_t)id + 1);
         DEdge e;
         e.x_start = __hiloint2double(a.y, a.x);
         e.x_inc = __hiloint2double(a.w, a.z);
@@ -131,7 +139,7 @@ __device__ __forceinline__ int32_t edge_crossing(const void *__restrict__ edges,
                                                  int32_t sub0, int32_t col0) {
     int32_t n;
     if (crossing_f32(R.v0, R.fxi, (float)r, R.lim, n)) return n + R.c0;
-    using E = std::conditional_t<BINS == kBinSmall, SmallEdge, DEdge>;
+    using E = std::conditional_t<kSmallEdges<BINS>, SmallEdge, DEdge>;
     const E *e = reinterpret_cast<const E *>(edges) + R.id;
     return crossing_f64(e->x_start, e->x_inc, e->top, sub0 + r) - col0;
 }
@@ -261,7 +269,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
     // tile -> (job, band, tile column)
     int32_t jb = 0, lb, col;
     if constexpr (MULTI) {
-        const int4 t = __ldg(reinterpret_cast<const int4 *>(A.tiles + tile));
+        const int4 t = table<BINS>(reinterpret_cast<const int4 *>(A.tiles + tile));
         jb = t.x;
         lb = t.y;
         col = t.z;
@@ -319,10 +327,10 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
         if (k0 + lane < cnt) {
             const int4 ent = list[k0 + lane];
             if (ent.z > x0 && ent.y < x0 + kTileCols) {
-                const int4 ra = __ldg(reinterpret_cast<const int4 *>(A.rfills + ent.x));
-                const uint32_t rb = __ldg(&A.rfills[ent.x].meta);
-                my_e0 = __ldg(A.bin_off + ent.w);
-                my_ne = __ldg(A.bin_off + ent.w + 1) - my_e0;
+                const int4 ra = table<BINS>(reinterpret_cast<const int4 *>(A.rfills + ent.x));
+                const uint32_t rb = table<BINS>(&A.rfills[ent.x].meta);
+                my_e0 = table<BINS>(A.bin_off + ent.w);
+                my_ne = table<BINS>(A.bin_off + ent.w + 1) - my_e0;
                 my_f = ent.x;
                 my_meta = rb;
                 const int32_t aa = (int32_t)((my_meta >> RF_AA_SHIFT) & 3u);
@@ -672,7 +680,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                 // (A bounded fill outside its rows was skipped above.)
                 if (!blocks) continue;
                 // Lane k holds the source word for coverage k (k_edge_fill).
-                const uint32_t lut_w = __ldg(A.luts + 32 * (size_t)__shfl_sync(kAll, my_f, src) + lane);
+                const uint32_t lut_w = table<BINS>(A.luts + 32 * (size_t)__shfl_sync(kAll, my_f, src) + lane);
                 if (fmt <= Z2D_FORMAT_RGBA) {
                     const bool has_alpha = fmt == Z2D_FORMAT_RGBA || fmt == Z2D_FORMAT_ARGB;
 #pragma unroll
@@ -873,12 +881,54 @@ __global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, BINS)
     }
 }
 
+// A CTA per tile of a small call, whose tables are the launch's parameters: no
+// copy, event or staging slot is between the call and its one launch.  Each CTA
+// takes them to shared memory first.  Such calls are bound by their CUDA calls
+// and by the wait for the tables (the 300x300 star from Python: copied 16.4 us,
+// written by a launch of their own in front 13.8, now 11.6).
+// Larger tables stay with the copy: a launch's parameters are written by the
+// host a second time, and end at 32 KB.
+template <bool MULTI, int MODE>
+__global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, kBinShared))
+    k_raster_small(const __grid_constant__ RasterArgs A, const __grid_constant__ ParamBlob P, int32_t n, int32_t n_fills) {
+    extern __shared__ uint32_t smem[];
+    __shared__ uint4 tables[kParamBytes / sizeof(uint4)];
+    for (int32_t i = threadIdx.x; i < n; i += kRasterThreads) tables[i] = P.v[i];
+    __syncthreads();
+    RasterArgs B = A;
+    auto place = [&](auto *&p) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(reinterpret_cast<uintptr_t>(tables) +
+                                                                  reinterpret_cast<uintptr_t>(p));
+    };
+    place(B.jobs);
+    place(B.fills);
+    place(B.st);
+    place(B.edges);
+    place(B.bins);
+    place(B.bin_off);
+    place(B.band_count);
+    place(B.band_fills);
+    place(B.rfills);
+    place(B.luts);
+    place(B.tiles);
+    if constexpr (MODE == kGeneral) {
+        for (int32_t f = threadIdx.x; f < n_fills; f += kRasterThreads) {
+            FillCmd &F = const_cast<FillCmd &>(B.fills[f]);
+            if (F.src.grad) place(F.src.grad);
+        }
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    raster_row<MULTI, MODE, kBinShared>(B, (int32_t)blockIdx.x, warp, lane, smem + warp * kWarpWords);
+}
+
 static size_t raster_smem() { return sizeof(uint32_t) * kWarpWords * kTileRows; }
 
 template <int MODE, class F>
 static int of_mode(RasterVariant v, int k, F &&f) {
-    if (v.bins == kBinSmall)
-        return v.multi ? f(k_raster<true, true, MODE, kBinSmall>, k) : f(k_raster<false, true, MODE, kBinSmall>, k);
+    if constexpr (MODE != kPlainDirect)
+        if (v.bins == kBinSmall)
+            return v.multi ? f(k_raster<true, true, MODE, kBinSmall>, k) : f(k_raster<false, true, MODE, kBinSmall>, k);
     if (v.multi) return v.cta_items ? f(k_raster<true, true, MODE>, k) : f(k_raster<true, false, MODE>, k);
     return v.cta_items ? f(k_raster<false, true, MODE>, k) : f(k_raster<false, false, MODE>, k);
 }
@@ -917,6 +967,16 @@ int raster_launch(Ctx &c, RasterVariant v, const RasterArgs &A, unsigned grid) {
         Z2D_CUDA(cudaGetLastError());
         return Z2D_OK;
     });
+}
+
+int raster_launch_small(Ctx &c, bool multi, int mode, const RasterArgs &A, const ParamBlob &P, int32_t n, int32_t n_fills,
+                        unsigned grid) {
+    const auto kernel = mode == kPlain4x ? (multi ? k_raster_small<true, kPlain4x> : k_raster_small<false, kPlain4x>)
+                                         : (multi ? k_raster_small<true, kGeneral> : k_raster_small<false, kGeneral>);
+    kernel<<<grid, kRasterThreads, raster_smem(), c.stream>>>(A, P, n, n_fills);
+    c.launches++;
+    Z2D_CUDA(cudaGetLastError());
+    return Z2D_OK;
 }
 
 }  // namespace z2dg

@@ -130,17 +130,29 @@ Z2D_HD uint32_t coverage_word(const FillCmd &F, int fmt, int k) {
 // whose records every pixel row works out, either of the one-upload path's
 // SmallEdge (with records from the host a call of 1,500 edges took 67 us
 // instead of 56) or of DEdge, where the device has no room for the records.
-enum BinKind : int { kBinRecords = 0, kBinSmall = 1, kBinIndex = 2 };
+// kBinShared is kBinSmall with all of a call's tables in shared memory.
+enum BinKind : int { kBinRecords = 0, kBinSmall = 1, kBinIndex = 2, kBinShared = 3 };
 
 // How k_raster runs: `multi` for several surfaces, `cta_items` for a whole
-// tile per work item, the mode, and what the bins hold.  kBinSmall comes with
-// a tile per item, kBinIndex with a row per item and in the general mode only.
+// tile per work item, the mode, and what the bins hold.  kBinSmall and
+// kBinShared come with a tile per item and 4x4 samples, kBinIndex with a row
+// per item and in the general mode only.
 struct RasterVariant {
     bool multi, cta_items;
     BinKind bins;
     int mode;
 };
+
+// A small call's tables, as a parameter of its one launch.
+constexpr size_t kParamBytes = 8192;
+struct ParamBlob {
+    uint4 v[kParamBytes / sizeof(uint4)];
+};
 int raster_occupancy(Ctx &c, RasterVariant v, int &ctas_per_sm);
 int raster_launch(Ctx &c, RasterVariant v, const RasterArgs &A, unsigned grid);
+// A CTA per tile of a call whose tables are the first n words of P: A's
+// pointers, and those of its fills' gradients, are offsets into them.
+int raster_launch_small(Ctx &c, bool multi, int mode, const RasterArgs &A, const ParamBlob &P, int32_t n, int32_t n_fills,
+                        unsigned grid);
 
 }  // namespace z2dg

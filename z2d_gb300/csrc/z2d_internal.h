@@ -113,8 +113,8 @@ struct Ctx {
     std::vector<stroke::Polygon> poly_cache;
     HostBuf staging;    // pinned upload staging
     HostBuf readback;   // pinned readback
-    // the one-upload path of few short fills (fill.cu, run_small_jobs):
-    // two pinned staging slots, each free again once its upload event has
+    // the one-upload path of few short fills (fill.cu, run_small_jobs), for
+    // tables that are not the launch's parameters: two pinned staging slots, each free again once its upload event has
     // passed, and the device copy of the latest upload (stream ordered)
     HostBuf small_stage[2];
     cudaEvent_t small_done[2] = {nullptr, nullptr};
