@@ -1541,7 +1541,7 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
         if (rc) return rc;
     }
     // the schedule: forced on the context, or the tuner's for this kind of pass
-    const TuneKey key = tune_key(n_jobs, n_tiles, n_slots, n_gbands);
+    const TuneKey key = tune_key(n_jobs, variant.mode, n_tiles, n_slots, n_gbands);
     c.last_key = key;
     RasterPlan plan{c.raster_ctas_per_sm, c.raster_order, c.raster_cta_items, -1};
     if (bin_kind == kBinIndex) {  // (one schedule: its variants draw rows)

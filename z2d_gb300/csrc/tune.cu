@@ -13,15 +13,17 @@
 // The fourth candidate shape is no persistence at all: one CTA per tile, as
 // many CTAs as tiles, in queue order, scheduled by the hardware.
 //
-// The tuner keys a pass by (one surface or many, log2 of its tiles, log2 of
-// the mean fills per band list).  The first passes of a new key each run a
-// different candidate schedule with CUDA events around the raster launch;
-// once every candidate has run, the fastest is kept for the key.  Decisions
-// are cached in a JSON file (raster_tune.json beside libz2dgpu.so, or the
-// path in Z2D_TUNE_FILE) and loaded on first use, so a later process starts
-// from them.  Z2D_TUNE=off keeps the default schedule (one CTA per tile, in
-// tile order).  Every schedule draws the same pixels: tiles are disjoint and
-// each row's fills run in call order whatever the queue order.
+// The tuner keys a pass by (one surface or many, the kernel's mode, log2 of its
+// tiles, log2 of the mean fills per band list).  The first passes of a new key
+// each run a different candidate schedule with CUDA events around the raster
+// launch; once every candidate has run, the fastest is kept for the key.
+// Decisions are cached in a JSON file (raster_tune.json beside libz2dgpu.so, or
+// the path in Z2D_TUNE_FILE) and loaded on first use, so a later process
+// starts from them.  Lines without a mode, of a table measured before the
+// kernel had modes, are not taken.  Z2D_TUNE=off keeps the default schedule
+// (one CTA per tile, in tile order).  Every schedule draws the same pixels:
+// tiles are disjoint and each row's fills run in call order whatever the queue
+// order.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
@@ -44,7 +46,7 @@ struct Candidate {
     int ctas, order, cta_items;
 };
 // CTAs per SM: -1 = not persistent (one CTA per tile, dispatched in queue
-// order), 0 = as many as fit (6 for k_raster), else that many
+// order), 0 = as many as fit (6 to 9 of k_raster), else that many
 constexpr Candidate kCandidates[] = {{-1, 0, 1}, {-1, 1, 1}, {0, 0, 0}, {0, 1, 0},
                                      {0, 0, 1}, {0, 1, 1}, {4, 0, 0}, {2, 1, 0}};
 constexpr int kNumCandidates = sizeof(kCandidates) / sizeof(kCandidates[0]);
@@ -71,7 +73,7 @@ std::string tune_path() {
     return "raster_tune.json";
 }
 
-// {"multi": m, "tiles": t, "load": l, "ctas": c, "order": o, "cta_items": i, "ms": x} per line
+// {"multi": m, "mode": d, "tiles": t, "load": l, "ctas": c, "order": o, "cta_items": i, "ms": x} per line
 void load_locked() {
     g_loaded = true;
     FILE *f = std::fopen(tune_path().c_str(), "r");
@@ -82,9 +84,9 @@ void load_locked() {
         int ctas = 0, order = 0, items = 0;
         double ms = 0;
         if (std::sscanf(line,
-                        " {\"multi\": %d, \"tiles\": %d, \"load\": %d, \"ctas\": %d, \"order\": %d, \"cta_items\": %d, "
-                        "\"ms\": %lf",
-                        &k.multi, &k.tiles, &k.load, &ctas, &order, &items, &ms) != 7)
+                        " {\"multi\": %d, \"mode\": %d, \"tiles\": %d, \"load\": %d, \"ctas\": %d, \"order\": %d, "
+                        "\"cta_items\": %d, \"ms\": %lf",
+                        &k.multi, &k.mode, &k.tiles, &k.load, &ctas, &order, &items, &ms) != 8)
             continue;
         for (int i = 0; i < kNumCandidates; i++)
             if (kCandidates[i].ctas == ctas && kCandidates[i].order == order && kCandidates[i].cta_items == items)
@@ -104,9 +106,9 @@ void save_locked() {
         const Candidate &c = kCandidates[e.best];
         const double ms = e.n[e.best] ? e.ms[e.best] / e.n[e.best] : 0.0;
         std::fprintf(f,
-                     "{\"multi\": %d, \"tiles\": %d, \"load\": %d, \"ctas\": %d, \"order\": %d, \"cta_items\": %d, "
-                     "\"ms\": %.4f, \"candidates_ms\": [",
-                     kv.first.multi, kv.first.tiles, kv.first.load, c.ctas, c.order, c.cta_items, ms);
+                     "{\"multi\": %d, \"mode\": %d, \"tiles\": %d, \"load\": %d, \"ctas\": %d, \"order\": %d, "
+                     "\"cta_items\": %d, \"ms\": %.4f, \"candidates_ms\": [",
+                     kv.first.multi, kv.first.mode, kv.first.tiles, kv.first.load, c.ctas, c.order, c.cta_items, ms);
         for (int i = 0; i < kNumCandidates; i++)  // every candidate's time, for the record (0: not measured here)
             std::fprintf(f, "%s%.4f", i ? ", " : "", e.n[i] ? e.ms[i] / e.n[i] : 0.0);
         std::fprintf(f, "]}\n");
@@ -125,9 +127,10 @@ int mode_locked() {
 
 }  // namespace
 
-TuneKey tune_key(int32_t n_jobs, long long n_tiles, long long n_slots, long long n_gbands) {
+TuneKey tune_key(int32_t n_jobs, int mode, long long n_tiles, long long n_slots, long long n_gbands) {
     TuneKey k{};
     k.multi = n_jobs > 1 ? 1 : 0;
+    k.mode = mode;
     k.tiles = n_tiles > 0 ? (int)std::log2((double)n_tiles) : 0;
     const double load = n_gbands > 0 ? (double)n_slots / (double)n_gbands : 0.0;
     k.load = (int)std::log2(1.0 + load);

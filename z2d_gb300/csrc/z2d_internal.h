@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/z2dgpu.h"
@@ -45,12 +46,13 @@ struct HostBuf {
 };
 
 // The rasteriser's schedule tuner (tune.cu): a pass is keyed by whether it
-// draws one surface or many, log2 of its tiles and log2 of the mean fills
-// per band list.
+// draws one surface or many, the rasteriser's mode (what its fills have in
+// common: kernels of different residency), log2 of its tiles and log2 of the
+// mean fills per band list.
 struct TuneKey {
-    int multi, tiles, load;
+    int multi, mode, tiles, load;
     bool operator<(const TuneKey &o) const {
-        return multi != o.multi ? multi < o.multi : tiles != o.tiles ? tiles < o.tiles : load < o.load;
+        return std::tie(multi, mode, tiles, load) < std::tie(o.multi, o.mode, o.tiles, o.load);
     }
 };
 struct RasterPlan {
@@ -64,7 +66,7 @@ struct TunePending {
     int candidate;
     cudaEvent_t start, stop;
 };
-TuneKey tune_key(int32_t n_jobs, long long n_tiles, long long n_slots, long long n_gbands);
+TuneKey tune_key(int32_t n_jobs, int mode, long long n_tiles, long long n_slots, long long n_gbands);
 RasterPlan tune_pick(const TuneKey &k);
 void tune_report(const TuneKey &k, int candidate, float ms);
 // 1: decided (ctas, order set), 0: still exploring, -1: tuning off
@@ -104,7 +106,7 @@ struct Ctx {
     int raster_order = 0;
     int raster_cta_items = 1;
     std::vector<TunePending> tune_pending;  // tuner measurements not yet read
-    TuneKey last_key{-1, 0, 0};             // key of the last pass
+    TuneKey last_key{-1, 0, 0, 0};            // key of the last pass
     void tune_collect(bool wait);
     DevBuf tile_order;          // cost-ordered queue: keys, indices, sorted copies, sort scratch
     DevBuf pad_buf;             // padded copies of packed surfaces (PackedPads)
