@@ -40,13 +40,6 @@ __device__ __forceinline__ int32_t round_i32(double v) {
     if (ok) return r;
     return f64_round_i32_hw(v);
 }
-__device__ __forceinline__ float to_f32(double v) {
-    bool ok;
-    const float r = f64_to_f32(v, ok);
-    if (ok) return r;
-    return f64_to_f32_hw(v);
-}
-
 __device__ __forceinline__ void add_edge(const FillCmd &F, DEdge *out, double x0, double y0, double x1, double y1,
                                          double &et, double &eb, double &el, double &er, bool &any) {
     // Polygon.addEdge (Polygon.zig:61-109)

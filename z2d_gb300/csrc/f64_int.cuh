@@ -280,7 +280,6 @@ static __device__ __noinline__ double f64_add_hw(double a, double b) { return a 
 static __device__ __noinline__ double f64_mul_hw(double a, double b) { return a * b; }
 static __device__ __noinline__ double f64_div_hw(double a, double b) { return a / b; }
 static __device__ __noinline__ int32_t f64_round_i32_hw(double x) { return (int32_t)round(x); }
-static __device__ __noinline__ float f64_to_f32_hw(double x) { return (float)x; }
 
 // a / b through the integer long division (an f64 division is several f64
 // instructions), out of line: one copy serves every call site.

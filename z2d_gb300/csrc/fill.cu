@@ -1525,7 +1525,6 @@ int run_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, int32_t n
     A.luts = d_luts;
     A.tiles = d_tiles;
     A.masks = c.masks.as<uint8_t>();
-    A.n_jobs = n_jobs;
     A.job0 = jobs[0];
     {
         const int rc = c.await_surface();  // a host surface's upload
@@ -2075,7 +2074,6 @@ int run_small_jobs(Ctx &c, std::vector<DevJob> &jobs, const z2d_node *nodes, con
     A.tiles = reinterpret_cast<const TileRec *>(dv + o_tile);
     A.luts = reinterpret_cast<const uint32_t *>(dv + o_lut);
     A.masks = nullptr;
-    A.n_jobs = (int32_t)n_jobs;
     A.queue = nullptr;
     A.n_items = (unsigned long long)n_tiles;
     A.order = nullptr;

@@ -91,7 +91,6 @@ struct RasterArgs {
     const uint32_t *luts;       // 32 source words per fill (coverage_word)
     const TileRec *tiles;       // per tile (several surfaces only)
     const uint8_t *masks;
-    int32_t n_jobs;
     unsigned long long *queue;  // work-queue counter, zero at launch
     unsigned long long n_items; // tiles (CTA items) or tiles x rows (warp items)
     const int32_t *order;       // tile order of the queue, or null (tile index order)
