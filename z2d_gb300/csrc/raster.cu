@@ -729,6 +729,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                     const bool on = cov[32 * q] != 0;
                     const uint32_t m = __ballot_sync(kAll, on);
                     if (on) at[n + __popc(m & below)] = (uint8_t)(32 * q + lane);
+                    touched |= on ? 1u << q : 0u;
                     n += __popc(m);
                 }
                 __syncwarp();
@@ -759,9 +760,7 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     if (!((blocks >> q) & 1u)) continue;
-                    if (cov[32 * q] == 0) continue;
-                    raw[q] = word_src_over_fma(raw[q], words[32 * q + lane], has_alpha);
-                    touched |= 1u << q;
+                    if (cov[32 * q] != 0) raw[q] = word_src_over_fma(raw[q], words[32 * q + lane], has_alpha);
                 }
                 __syncwarp();
                 for (int i = lane; i < kTileCols + kTileCols / 4; i += 32) words[i] = 0u;
@@ -808,8 +807,8 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
                         rq = i16_to_raw(d, fmt);
                     }
                 }
-                if (!on) continue;
-                touched |= 1u << q;
+                if (!__any_sync(kAll, on)) continue;
+                touched |= on ? 1u << q : 0u;
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     if (q == j) raw[j] = rq;
