@@ -57,7 +57,7 @@ __device__ __forceinline__ bool msaa_unbounded_clear(const FillState &S, int32_t
 // the inside bits are the prefix XOR of the toggles.  Issue bound, on the
 // ALU pipe: a fill costs a row and tile of the 2,000-path 4096x4096 batch
 // (2.9 M of them, 28 edges each on average) about 690 warp instructions
-// instead of 1,250, and the kernel takes 1.93 ms instead of 4.30.
+// instead of 1,250, and the kernel takes 1.95 ms instead of 4.30.
 constexpr int kPlanes = 6;
 constexpr int kSubWords = kPlanes * 32;         // one sample row
 constexpr int kDenseWords = 2 * 16 * 32 + 2 * 32;  // or winding_bits' counters
@@ -839,7 +839,8 @@ __device__ __forceinline__ void raster_row(const RasterArgs &A, const int32_t ti
 //    next item at once instead of holding its CTA until the slowest warp of
 //    the tile is done.
 // CTAs per SM: nine of the plain variants for one surface (56 registers;
-// 2,000 paths with 7, 8, 9, 10 and 11: 2.08, 1.97, 1.93, 1.95 and 2.09 ms),
+// 2,000 paths with 7, 8, 9, 10 and 11: 2.08, 1.97, 1.93, 1.95 and 2.09 ms, when
+// whole blocks were stored),
 // eight for several surfaces (320 surfaces with 7, 8 and 9: 3.14, 3.06 and
 // 3.15 ms: the job's fields take registers), six of the general ones (240
 // gradient fills with 4, 6 and 8: 0.82, 0.75 and 0.77 ms).
@@ -886,7 +887,11 @@ __global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, BINS)
 // and by the wait for the tables (the 300x300 star from Python: copied 16.4 us,
 // written by a launch of their own in front 13.8, now 11.6).
 // Larger tables stay with the copy: a launch's parameters are written by the
-// host a second time, and end at 32 KB.
+// host a second time, read by every CTA, and end at 32 KB.  A call alone and
+// waited for: a polygon of 90 segments, just below 8 KB, 27.8 us and copied
+// 28.8; of 130, above it, 30.2 and 29.3; of 280 36.3 and 33.5 (among others
+// parameters are the faster way for all of them: 13, 14 and 17 us against 17,
+// 17.5 and 21).
 template <bool MULTI, int MODE>
 __global__ void __launch_bounds__(kRasterThreads, raster_ctas(MULTI, MODE, kBinShared))
     k_raster_small(const __grid_constant__ RasterArgs A, const __grid_constant__ ParamBlob P, int32_t n, int32_t n_fills) {

@@ -1,5 +1,5 @@
 // raster_px.cuh -- one pixel of a fill or hairline composited onto a
-// surface, and raw pixel access, shared by the rasteriser (fill.cu) and the
+// surface, and raw pixel access, shared by the rasteriser (raster.cu) and the
 // hairline rasteriser (hairline.cu).
 #pragma once
 #include <cuda_runtime.h>

@@ -321,8 +321,8 @@ __device__ __forceinline__ double lerp_half(double a, double b) {
 }
 
 // Knots.deCasteljau (Spline.zig:128-152): k becomes the first half, the
-// second half is returned.  Out of line: one copy serves the frontier
-// expansion and the depth-first walks (flatten of the 2,000-path batch
+// second half is returned.  Out of line: one copy serves the descent to a
+// lane's subtree and the depth-first walks (flatten of the 2,000-path batch
 // 0.72 -> 0.68 ms against the inlined copies).
 static __device__ __noinline__ Knots de_casteljau(Knots &k) {
     const double abx = lerp_half(k.ax, k.bx), aby = lerp_half(k.ay, k.by);
