@@ -275,9 +275,9 @@ Z2D_API uint64_t z2dgpu_ctx_launch_count(const z2dgpu_ctx *ctx);
  * synchronizes the context.  No reference counterpart (instrumentation). */
 Z2D_API int z2dgpu_ctx_set_timing(z2dgpu_ctx *ctx, int enable);
 /* The rasteriser's schedule on this context (no counterpart in z2d).  By
- * default an autotuner picks it per kind of pass (one surface or many, its
- * number of tiles, the mean fills per band) by timing the candidates on the
- * first passes of each kind, and caches its choices in raster_tune.json
+ * default an autotuner picks it per kind of pass (one surface or many, the
+ * kernel's mode, its number of tiles, the mean fills per band) by timing the
+ * candidates on the first passes of each kind, and caches its choices in raster_tune.json
  * beside the library (Z2D_TUNE_FILE overrides the path; Z2D_TUNE=off keeps
  * the default schedule).  ctas_per_sm >= -1 forces a schedule: the grid
  * (-1 = one CTA per tile, not persistent; 0 = a persistent grid of as many
